@@ -34,7 +34,7 @@ def build(ref_dir: str | None = REF_DIR) -> None:
     """Compile the C restatement, and the reference's own sources when they are
     present on this machine."""
     subprocess.check_call(["make", "-s", "-C", _HERE])
-    if ref_dir and os.path.isdir(ref_dir):
+    if ref_dir and os.path.isfile(os.path.join(ref_dir, "kernels", "ternary_gemv.cu")):
         subprocess.check_call(["make", "-s", "-C", _HERE, "ref", f"REF={ref_dir}"])
         pkg_lib = os.path.join(os.path.dirname(_HERE), "ternary_llm_b200", "libtllm_b200.so")
         if os.path.exists(pkg_lib):      # drop-in checks link against the built library

@@ -1,5 +1,6 @@
-// Grouped-query attention over prompts on the 5th-generation tensor cores (BF16, head sizes 64 and
-// 128; the other sizes run on mma.sync, grouped_attention.cu).
+// Grouped-query attention over prompts on the 5th-generation tensor cores (head sizes 64 and 128):
+// BF16 for the models of mixer layers (their other sizes run on mma.sync, grouped_attention.cu), FP16
+// for the LLaMA design (its other sizes run on attention.cu).
 //
 // A CTA takes 128 queries of one head and walks over tiles of 128 positions that some of its queries
 // sees; two CTAs share an SM, so that one's softmax runs beside the other's products.  Roles: a TMA
@@ -8,10 +9,23 @@
 //   softmax        a thread reads its row; the weights go back over S as two BF16 numbers each
 //   O += P V       weights from tensor memory, values as they lie in the cache (feature-major
 //                  operand); the high and the low parts are two products
-// The running maximum moves only when it grows by more than 2^8: the sums stay far inside FP32, and
-// the output in tensor memory is rescaled a few times per row at most.  All mbarrier waits are
-// bounded (see dense_gemm.cu).
+// The running maximum moves only when it grows by more than 2^8 (FP16: 2^4): the sums stay far inside
+// FP32, and the output in tensor memory is rescaled a few times per row at most.  FP16 weights carry a
+// factor of 2^10, which the division by their sum takes out again: the largest is then between 2^10 and
+// 2^14, and a weight keeps 22 bits in its two parts down to 2^-13 of the largest (below that the parts
+// hold it to 2^-35 of the largest).  A position that a query does not see enters its product with the
+// weight 0, so a NaN or an infinity among the values of such a position in the query's last tile
+// reaches the query.
+//
+// FP16, 32 heads over 8 key/value heads, one launch among others, against the form with a CTA per query
+// and key/value head on the CUDA cores (attention.cu), which read every position once per query: 2000
+// queries 2210 -> 116 us (head size 64), 6733 -> 127 us (128); 300 queries 82 -> 15 and 256 -> 17 us;
+// 2 queries 6.8 -> 6.9 and 9.9 -> 8.2 us; 2 queries behind 1000 positions 35.7 -> 33.3 and 60 -> 36 us.
+// It is taken from two queries on.  All mbarrier waits are bounded (see dense_gemm.cu).
+#include <type_traits>
+
 #include "launch.cuh"
+#include "layer.cuh"
 #include "mixers.cuh"
 #include "tcgen05.cuh"
 
@@ -23,21 +37,45 @@ using namespace gemm;
 
 constexpr int kTile = 128, kThreads = 192;
 constexpr int kBlock = kTile * 128;                 // bytes of 64 columns of a tile: 128-byte rows
+constexpr int kMinQueries = 2;                      // FP16; one query splits the positions (attention.cu)
 constexpr uint32_t kTmemCols = 256;                 // S and the weights: 128, O: 128
-constexpr float kLog2e = 1.4426950408889634f, kSlack = 8.f;
+constexpr float kLog2e = 1.4426950408889634f;
 
+template <typename T> struct Operand;
+template <> struct Operand<bf16> {
+    using Pair = __nv_bfloat162;
+    static constexpr uint32_t kFormats = (1u << 7) | (1u << 10);
+    static constexpr float kSlack = 8.f, kLift = 0.f;
+    static constexpr CUtensorMapDataType kMap = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    static __device__ __forceinline__ Pair pair(float x, float y) { return __floats2bfloat162_rn(x, y); }
+    static __device__ __forceinline__ float2 floats(Pair p) { return __bfloat1622float2(p); }
+};
+template <> struct Operand<half> {
+    using Pair = half2;
+    static constexpr uint32_t kFormats = 0;
+    static constexpr float kSlack = 4.f, kLift = 10.f;
+    static constexpr CUtensorMapDataType kMap = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    static __device__ __forceinline__ Pair pair(float x, float y) { return __floats2half2_rn(x, y); }
+    static __device__ __forceinline__ float2 floats(Pair p) { return __half22float2(p); }
+};
+
+// Keys of sequence b and key/value head g lie in rows (b * kv_heads + g) * head_rows + position and
+// columns g * k_cols .. of their map, values alike.
+template <typename T>
 struct PromptArgs {
-    bf16* out;
-    int ld_out, heads, per_kv, dim, vdim, n, pos0, chunk, cache_rows;
+    T* out;
+    int ld_out, per_kv, kv_heads, dim, vdim, n, pos0, chunk, cache_rows;
+    int head_rows, k_cols, v_cols;
     float scale2, out_scale;
     int* err;
 };
 
 __device__ __forceinline__ int chunk_start(int pos, int chunk) { return chunk > 0 ? pos / chunk * chunk : 0; }
 
+template <typename T>
 __device__ __forceinline__ uint32_t idesc(int n, bool feature_major)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((feature_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+    return (1u << 4) | Operand<T>::kFormats | ((feature_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
 }
 // operand whose rows are the contracted index: blocks of 64 features kBlock apart, groups of 8 rows 1024 bytes apart
 __device__ __forceinline__ uint64_t feature_major_desc(uint32_t addr)
@@ -74,10 +112,12 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 
 enum Bar { kQFull, kKFull, kKEmpty, kVFull, kVEmpty, kSFull, kPReady, kPvDone, kBars };
 
+template <typename T>
 __global__ void __launch_bounds__(kThreads, 2)
 grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                         const __grid_constant__ CUtensorMap map_v, const PromptArgs a)
+                         const __grid_constant__ CUtensorMap map_v, const PromptArgs<T> a)
 {
+    using Op = Operand<T>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[kBars];
@@ -85,7 +125,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __shared__ int abort_flag;
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.y, g = h / a.per_kv, q0 = (gridDim.x - 1 - blockIdx.x) * kTile;       // longest first
+    const int h = blockIdx.y, g = h / a.per_kv, seq = blockIdx.z, q0 = (gridDim.x - 1 - blockIdx.x) * kTile;       // longest first
     const int nq = min(kTile, a.n - q0), first = a.pos0 + q0, hi = first + nq;                    // positions of the queries
     const int lo = chunk_start(first, a.chunk) & ~(kTile - 1), lo_last = chunk_start(hi - 1, a.chunk);
     const int tiles = (hi - lo + kTile - 1) / kTile, nd = a.dim / 64, ne = a.vdim / 64;
@@ -114,10 +154,11 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             int issued = 0;                                     // tiles whose copies were issued: keys, then values
+            const int head_row = (seq * a.kv_heads + g) * a.head_rows;
             mbar_expect_tx(bar(kQFull), nd * kBlock);
-            for (int j = 0; j < nd; j++) tma_load_2d(qs + j * kBlock, &map_q, h * a.dim + j * 64, q0, bar(kQFull));
+            for (int j = 0; j < nd; j++) tma_load_2d(qs + j * kBlock, &map_q, h * a.dim + j * 64, seq * a.n + q0, bar(kQFull));
             for (int i = 0; i < 2 * tiles; i++, issued++) {
-                const int t = i >> 1, row = (lo + t * kTile) % a.cache_rows;
+                const int t = i >> 1, row = head_row + (lo + t * kTile) % a.cache_rows;
                 const bool v = i & 1;
                 if (!mbar_wait(bar(v ? kVEmpty : kKEmpty), (t & 1) ^ 1, abortp)) {
                     abort_flag = 1;
@@ -126,8 +167,8 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 const int blocks = v ? ne : nd;
                 mbar_expect_tx(bar(v ? kVFull : kKFull), blocks * kBlock);
                 for (int j = 0; j < blocks; j++) {
-                    if (v) tma_load_2d(vs + j * kBlock, &map_v, g * a.vdim + j * 64, row, bar(kVFull));
-                    else tma_load_2d(ks + j * kBlock, &map_k, g * a.dim + j * 64, row, bar(kKFull));
+                    if (v) tma_load_2d(vs + j * kBlock, &map_v, g * a.v_cols + j * 64, row, bar(kVFull));
+                    else tma_load_2d(ks + j * kBlock, &map_k, g * a.k_cols + j * 64, row, bar(kKFull));
                 }
             }
             // after an abort the copies still in flight must land before the shared memory goes away
@@ -140,7 +181,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     } else if (warp == 5) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            const uint32_t id_s = idesc(kTile, false), id_o = idesc(a.vdim, true);
+            const uint32_t id_s = idesc<T>(kTile, false), id_o = idesc<T>(a.vdim, true);
             bool ok = mbar_wait(bar(kQFull), 0, abortp);
             int done = 0;                                       // tiles whose last product was issued
             for (int t = 0; ok && t < tiles; t++) {
@@ -199,7 +240,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     s[i][j] = __float_as_uint(v);
                     mx = fmaxf(mx, v);
                 }
-            const bool grows = mx > m + kSlack || (m == -INFINITY && mx > m);
+            const bool grows = mx > m + Op::kSlack || (m == -INFINITY && mx > m);
             if (__any_sync(0xffffffffu, grows)) {
                 const float f = grows ? exp2_neg(m - mx) : 1.f;               // 0 where nothing was seen before
                 if (grows) {
@@ -218,7 +259,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     }
                 }
             }
-            const float ref = m == -INFINITY ? 0.f : m;
+            const float ref = (m == -INFINITY ? 0.f : m) - Op::kLift;
 #pragma unroll
             for (int half = 0; half < 2; half++) {                            // 64 positions: 32 words of high, 32 of low parts
                 uint32_t ph[32], pl[32];
@@ -227,9 +268,9 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     const float p0 = exp2_neg(__uint_as_float(s[2 * half + (j >> 4)][2 * (j & 15)]) - ref);
                     const float p1 = exp2_neg(__uint_as_float(s[2 * half + (j >> 4)][2 * (j & 15) + 1]) - ref);
                     l += p0 + p1;
-                    const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
-                    const float2 r = __bfloat1622float2(b);
-                    const __nv_bfloat162 c = __floats2bfloat162_rn(p0 - r.x, p1 - r.y);
+                    const typename Op::Pair b = Op::pair(p0, p1);
+                    const float2 r = Op::floats(b);
+                    const typename Op::Pair c = Op::pair(p0 - r.x, p1 - r.y);
                     ph[j] = *reinterpret_cast<const uint32_t*>(&b);
                     pl[j] = *reinterpret_cast<const uint32_t*>(&c);
                 }
@@ -252,20 +293,26 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(kPvDone), (tiles - 1) & 1, abortp));
         if (ok) {
             fence_after();
-            const float f = a.out_scale / l;
-            bf16* op = a.out + (size_t)(q0 + tid) * a.ld_out + (size_t)h * a.vdim;
+            // a row without a positive sum: zeros from the FP16 operator, as from its decode form
+            const bool zeros = std::is_same<T, half>::value && !(l > 0.f);
+            const float f = zeros ? 1.f : a.out_scale / l;
+            T* op = a.out + ((size_t)seq * a.n + q0 + tid) * a.ld_out + (size_t)h * a.vdim;
 #pragma unroll 1
             for (int c = 0; c < a.vdim; c += 32) {
                 uint32_t o[32];
                 tmem_ld32(row_o + c, o);
                 wait_ld();
+                if (zeros) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) o[j] = 0;
+                }
                 if (tid < nq) {
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        __nv_bfloat162 w[4];
+                        typename Op::Pair w[4];
 #pragma unroll
                         for (int i = 0; i < 4; i++)
-                            w[i] = __floats2bfloat162_rn(__uint_as_float(o[8 * j + 2 * i]) * f, __uint_as_float(o[8 * j + 2 * i + 1]) * f);
+                            w[i] = Op::pair(__uint_as_float(o[8 * j + 2 * i]) * f, __uint_as_float(o[8 * j + 2 * i + 1]) * f);
                         *reinterpret_cast<uint4*>(op + c + 8 * j) = *reinterpret_cast<const uint4*>(w);
                     }
                 }
@@ -285,16 +332,34 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
 size_t smem_bytes(int dim, int vdim) { return (size_t)(2 * (dim / 64) + vdim / 64) * kBlock + 1024; }
 
-int encode(EncodeTiledFn enc, CUtensorMap* map, const bf16* p, int cols, int rows, size_t ld)
+template <typename T>
+int encode(EncodeTiledFn enc, CUtensorMap* map, const T* p, int cols, size_t rows, size_t ld)
 {
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(bf16)};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(T)};
     const cuuint32_t box[2] = {64, (cuuint32_t)kTile};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = enc(map, Operand<T>::kMap, 2, const_cast<T*>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(TLLM_ERR_LAUNCH, "grouped_prompt: cuTensorMapEncodeTiled failed with %d", (int)r);
     return TLLM_OK;
+}
+
+template <typename T>
+int launch(PromptArgs<T>& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, int heads, int batch, cudaStream_t stream)
+{
+    p.err = device_error_flag();
+    if (!p.err) return fail(TLLM_ERR_LAUNCH, "device scratch unavailable");
+    static bool attr[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "grouped_prompt: no current device");
+    if (!attr[dev]) {
+        cudaFuncSetAttribute(grouped_prompt_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(128, 128));
+        attr[dev] = true;
+    }
+    return launch_pdl("grouped_prompt", grouped_prompt_tc_kernel<T>, dim3((p.n + kTile - 1) / kTile, heads, batch), dim3(kThreads),
+                      smem_bytes(p.dim, p.vdim), stream, mq, mk, mv, p);
 }
 
 }  // namespace
@@ -318,31 +383,58 @@ int launch_grouped_prompt_tcgen05(const GroupedArgs<bf16>& a, cudaStream_t strea
     if ((st = encode(enc, &mq, a.proj + a.q_off, a.heads * a.dim, a.g.seq_len, a.ld))) return st;
     if ((st = encode(enc, &mk, kc, a.kv_heads * a.dim, a.cache_rows, (size_t)a.kv_heads * a.dim))) return st;
     if ((st = encode(enc, &mv, vc, a.kv_heads * a.vdim, a.cache_rows, (size_t)a.kv_heads * a.vdim))) return st;
-    PromptArgs p;
+    PromptArgs<bf16> p = {};
     p.out = a.out;
     p.ld_out = a.ld_out;
-    p.heads = a.heads;
     p.per_kv = a.heads / a.kv_heads;
+    p.kv_heads = a.kv_heads;
     p.dim = a.dim;
     p.vdim = a.vdim;
     p.n = a.g.seq_len;
     p.pos0 = a.g.start_pos;
     p.chunk = a.chunk;
     p.cache_rows = a.cache_rows;
+    p.head_rows = 0;
+    p.k_cols = a.dim;
+    p.v_cols = a.vdim;
     p.scale2 = a.scale * kLog2e;
     p.out_scale = a.out_scale;
-    p.err = device_error_flag();
-    if (!p.err) return fail(TLLM_ERR_LAUNCH, "device scratch unavailable");
-    static bool attr[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "grouped_prompt: no current device");
-    if (!attr[dev]) {
-        cudaFuncSetAttribute(grouped_prompt_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(128, 128));
-        attr[dev] = true;
-    }
-    return launch_pdl("grouped_prompt", grouped_prompt_tc_kernel, dim3((a.g.seq_len + kTile - 1) / kTile, a.heads), dim3(kThreads),
-                      smem_bytes(a.dim, a.vdim), stream, mq, mk, mv, p);
+    return launch(p, mq, mk, mv, a.heads, 1, stream);
+}
+
+bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_kv_heads, int head_dim,
+                                int seq_len, int kv_len_max)
+{
+    // rows of a map are addressed with 32-bit coordinates
+    return (head_dim == 64 || head_dim == 128) && seq_len >= kMinQueries && (long long)batch * n_kv_heads * kv_len_max < (1ll << 30) &&
+           (long long)batch * seq_len < (1ll << 30) && batch <= 65535 &&
+           ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) |
+             reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+}
+
+int launch_attention_prompt(const half* q, const half* k_cache, const half* v_cache, half* out, int batch, int n_heads, int n_kv_heads,
+                            int head_dim, int seq_len, int kv_len, int kv_len_max, cudaStream_t stream)
+{
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return fail(TLLM_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from this driver");
+    const size_t rows = (size_t)batch * n_kv_heads * kv_len_max;
+    CUtensorMap mq, mk, mv;
+    int st;
+    if ((st = encode(enc, &mq, q, n_heads * head_dim, (size_t)batch * seq_len, (size_t)n_heads * head_dim))) return st;
+    if ((st = encode(enc, &mk, k_cache, head_dim, rows, head_dim))) return st;
+    if ((st = encode(enc, &mv, v_cache, head_dim, rows, head_dim))) return st;
+    PromptArgs<half> p = {};
+    p.out = out;
+    p.ld_out = n_heads * head_dim;
+    p.per_kv = n_heads / n_kv_heads;
+    p.kv_heads = n_kv_heads;
+    p.dim = p.vdim = head_dim;
+    p.n = seq_len;
+    p.pos0 = kv_len - seq_len;
+    p.cache_rows = p.head_rows = kv_len_max;
+    p.scale2 = kLog2e / sqrtf((float)head_dim);
+    p.out_scale = 1.f;
+    return launch(p, mq, mk, mv, n_heads, batch, stream);
 }
 
 }  // namespace tllm

@@ -1,0 +1,61 @@
+"""Attention of several FP16 queries on tcgen05 (csrc/grouped_prompt.cu) behind attention_forward,
+against the numpy restatement in 64 bits: edges of the 128-query and 128-position tiles, queries
+behind a context, both head sizes, groups of heads, several sequences, full caches."""
+import numpy as np
+import pytest
+import torch
+
+import ternary_llm_b200 as tl
+from ternary_llm_b200 import layer_ops as ops
+
+pytestmark = pytest.mark.gpu
+f16 = np.float16
+
+
+def exact(q, kc, vc, kv_len):
+    b, s, h, d = q.shape
+    group = h // kc.shape[1]
+    out = np.empty(q.shape)
+    seen = np.arange(kv_len)[None, :] <= kv_len - s + np.arange(s)[:, None]
+    for i in range(b):
+        for j in range(h):
+            k, v = kc[i, j // group, :kv_len].astype(np.float64), vc[i, j // group, :kv_len].astype(np.float64)
+            z = np.where(seen, q[i, :, j].astype(np.float64) @ k.T / np.sqrt(d), -np.inf)
+            p = np.exp(z - z.max(axis=1, keepdims=True))
+            out[i, :, j] = (p / p.sum(axis=1, keepdims=True)) @ v
+    return out
+
+
+@pytest.mark.parametrize("b,hq,hk,hd", [(1, 8, 2, 64), (2, 4, 4, 128), (1, 32, 8, 128)])
+@pytest.mark.parametrize("seq,kv_len,mx", [(2, 2, 8), (8, 8, 8), (8, 400, 512), (127, 127, 130), (128, 128, 128), (129, 129, 256), (130, 387, 387),
+                                           (300, 300, 512), (257, 640, 640)])
+def test_prompt_attention(b, hq, hk, hd, seq, kv_len, mx):
+    rng = np.random.default_rng(seq * 1000 + kv_len + hd)
+    q = (3.0 * rng.standard_normal((b, seq, hq, hd))).astype(f16)
+    kc = rng.standard_normal((b, hk, mx, hd)).astype(f16)
+    vc = rng.standard_normal((b, hk, mx, hd)).astype(f16)
+    kc[:, :, kv_len:], vc[:, :, kv_len:] = np.nan, np.nan       # nothing behind the last position is used
+    out = torch.zeros(q.shape, dtype=torch.float16, device="cuda")
+    args = [torch.from_numpy(t).cuda() for t in (q, kc, vc)]
+    ops.attention_forward(*args, out, b, hq, hk, hd, seq, kv_len, mx)
+    tl.check_device_errors()
+    want = exact(q, kc, vc, kv_len)
+    # FP16 rounding of the result; scores of up to 30 in FP32 sums of 64 or 128 terms move a weight by
+    # less than 30 * 128 * 2^-24 = 2.3e-4 of itself in the worst case, and the mean of values by a tenth of that
+    err = np.abs(out.cpu().numpy().astype(np.float64) - want)
+    assert (err <= 2.0 ** -11 * np.abs(want) + 2e-5 * np.abs(vc[:, :, :kv_len].astype(np.float64)).max()).all(), err.max()
+
+
+def test_scores_far_apart():
+    """One position's score far above the others', first, last or in between: the running maximum
+    moves, and the weights of the others are nothing."""
+    hd, n = 64, 300
+    for hot in (0, 127, 128, 200):
+        rng = np.random.default_rng(hot)
+        q, kc, vc = (rng.standard_normal(s).astype(f16) for s in ((1, n, 1, hd), (1, 1, n, hd), (1, 1, n, hd)))
+        q[..., 0], kc[..., 0], kc[0, 0, hot, 0] = 30.0, 0.0, 30.0
+        out = torch.zeros(q.shape, dtype=torch.float16, device="cuda")
+        ops.attention_forward(*[torch.from_numpy(t).cuda() for t in (q, kc, vc)], out, 1, 1, 1, hd, n, n, n)
+        want = exact(q, kc, vc, n)
+        err = np.abs(out.cpu().numpy().astype(np.float64) - want)
+        assert (err <= 2.0 ** -11 * np.abs(want) + 1e-4).all(), (hot, err.max())

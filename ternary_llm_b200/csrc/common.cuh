@@ -76,6 +76,19 @@ int noalloc_error_check(cudaStream_t stream);
 bool gemm_tcgen05_supported(int M, int N, int K);
 int launch_gemm_tcgen05(const half* A, const uint8_t* packed, half* C, int M, int N, int K, cudaStream_t stream);
 
+// A few rows on prepared weights (gemm_rows.cu).  out[i]: rows row0 .. row0 + rows of the matrix go to y[m, rows].
+struct RowsOut {
+    half* y;
+    int row0, rows;
+};
+int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream);
+
+// y[m, rows] = x[m, cols] . W^T, FP16 activations, on the kernel for these sizes: passes of the
+// streaming GEMV (four vectors share one over the weights), gemm_rows.cu, or the tcgen05 GEMM.
+constexpr int kRowsMax = 32;
+bool linear_takes_rows(int m, int rows, int cols);
+int launch_linear_f16(const uint8_t* packed, const half* x, half* y, int m, int rows, int cols, cudaStream_t stream);
+
 // ---- small device helpers --------------------------------------------------
 __device__ __forceinline__ float warp_sum(float v)
 {

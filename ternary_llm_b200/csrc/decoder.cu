@@ -120,18 +120,21 @@ int pack_group(LlamaDecoder* D, int count, const tllm_b200_ternary_weight* const
     return TLLM_OK;
 }
 
-// y[n_tokens, rows] = x[n_tokens, cols] . W^T with FP16 activations: the tcgen05 GEMM for
-// token batches, passes of the streaming GEMV for a few tokens.
+// y[n_tokens, rows] = x[n_tokens, cols] . W^T with FP16 activations
 int linear_f16(const PackedW& w, const half* x, half* y, int n_tokens, cudaStream_t stream)
 {
-    if (n_tokens > 8 && gemm_tcgen05_supported(n_tokens, w.rows, w.cols))
-        return launch_gemm_tcgen05(x, w.p, y, n_tokens, w.rows, w.cols, stream);
-    return launch_gemv_packed(w.p, x, y, n_tokens, w.rows, w.cols, stream);
+    return launch_linear_f16(w.p, x, y, n_tokens, w.rows, w.cols, stream);
 }
 
+// all: the matrices as one where they are packed back to back
 int linear_multi(LlamaDecoder* D, int count, const PackedW* const* w, half* const* y, const half* x, bool int8,
-                 int n_tokens, cudaStream_t stream)
+                 int n_tokens, cudaStream_t stream, const PackedW* all = nullptr)
 {
+    if (n_tokens > 1 && all && all->p && linear_takes_rows(n_tokens, all->rows, all->cols)) {
+        RowsOut out[TLLM_MAX_FUSED];
+        for (int i = 0, row = 0; i < count; row += w[i++]->rows) out[i] = {y[i], row, w[i]->rows};
+        return launch_gemm_rows(all->p, x, out, count, n_tokens, all->cols, stream);
+    }
     const uint8_t* p[TLLM_MAX_FUSED];
     int rows[TLLM_MAX_FUSED];
     for (int i = 0; i < count; i++) {
@@ -218,7 +221,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
         } else {
             const PackedW* w[3] = {&L.q, &L.k, &L.v};
             half* y[3] = {qb, kb, vb};
-            TRY(linear_multi(D, 3, w, y, D->hidden, i8, n, s));
+            TRY(linear_multi(D, 3, w, y, D->hidden, i8, n, s, &L.qkv));
         }
         TRY(launch_rope(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, bsz, seq_n, c.n_heads, c.n_kv_heads,
                         c.head_dim, start_pos, pos_dev, c.rope_theta, c.max_seq_len, 1, s));
@@ -245,7 +248,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
         } else {
             const PackedW* w[2] = {&L.gate, &L.up};
             half* y[2] = {gb, ub};
-            TRY(linear_multi(D, 2, w, y, D->hidden, i8, n, s));
+            TRY(linear_multi(D, 2, w, y, D->hidden, i8, n, s, &L.gate_up));
         }
         TRY(launch_silu_mul(gb, ub, gb, (long long)n * inter, xq, xs, s));
         {

@@ -36,31 +36,47 @@ inline void prefer_max_shared(const void* kernel)
 }
 
 
-// cluster_x: CTAs along x that form a cluster
+// The launch itself.  cluster_x: CTAs along x that form a cluster; carveout: wanted shared-memory part of the
+// SM's L1 and shared memory in per cent, negative for the kernel's own setting
 template <typename... KArgs, typename... Args>
-int launch_pdl_cluster(const char* what, void (*kernel)(KArgs...), int cluster_x, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                       Args... args)
+int launch_pdl_split(const char* what, void (*kernel)(KArgs...), int cluster_x, int carveout, dim3 grid, dim3 block, size_t smem,
+                     cudaStream_t stream, Args... args)
 {
-    prefer_max_shared(reinterpret_cast<const void*>(kernel));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = cluster_x;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[3];
+    int n = 0;
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+    if (cluster_x > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster_x;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (carveout >= 0) {
+        at[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at[n++].val.sharedMemCarveout = carveout;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = cluster_x > 1 ? 2 : 1;
+    cfg.numAttrs = n;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(TLLM_ERR_LAUNCH, "%s launch: %s", what, cudaGetErrorString(e));
     }
     return TLLM_OK;
+}
+
+template <typename... KArgs, typename... Args>
+int launch_pdl_cluster(const char* what, void (*kernel)(KArgs...), int cluster_x, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                       Args... args)
+{
+    prefer_max_shared(reinterpret_cast<const void*>(kernel));
+    return launch_pdl_split(what, kernel, cluster_x, -1, grid, block, smem, stream, args...);
 }
 
 template <typename... KArgs, typename... Args>

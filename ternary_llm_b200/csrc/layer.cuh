@@ -23,6 +23,9 @@ int launch_embedding(const half* table, const int* indices, half* out, int n_tok
 int launch_fp16_gemv(const half* w, const half* x, half* y, int rows, int cols, cudaStream_t stream);
 // y[b, r] = W[r, :] . x[b, :] for `batch` vectors (x [batch, cols], y [batch, rows]).
 int launch_fp16_gemv_batched(const half* w, const half* x, half* y, int batch, int rows, int cols, cudaStream_t stream);
+// The two above on the tensor cores (fp16_rows.cu), which they take where it is supported.
+bool fp16_rows_supported(const half* w, const half* x, int cols);
+int launch_fp16_rows(const half* w, const half* x, half* y, int m, int rows, int cols, cudaStream_t stream);
 int launch_fp16_gemm(const half* A, const half* B, half* C, int M, int N, int K, cudaStream_t stream);
 // part_val / part_idx: 64 entries each; counter: one zero-initialised unsigned; pos: when not
 // null, *pos is advanced by one together with the token (the decode loop's cache position).

@@ -384,9 +384,9 @@ int launch_embedding(const half* table, const int* indices, half* out, int n_tok
 // FP16 GEMV   y[r] = half(sum_c float(W[r, c]) * float(x[c]))    reference: kernels/elementwise.cu:158-201
 // ---------------------------------------------------------------------------
 // The lm_head of the 1B configuration is 525 MB of FP16, twice the ternary bytes of the
-// whole layer stack, so this kernel is HBM-bound like the ternary GEMV: x is staged in
-// shared memory once per CTA, each warp streams whole rows with 128-bit loads, four
-// loads in flight per lane, FP32 accumulation.
+// whole layer stack; columns in whole windows go to the tensor cores (fp16_rows.cu).  For the
+// other shapes: x is staged in shared memory once per CTA, each warp streams whole rows with
+// 128-bit loads where the alignment allows, four loads in flight per lane, FP32 accumulation.
 constexpr int kFp16GemvWarps = 8;
 
 __global__ void __launch_bounds__(kFp16GemvWarps * 32)
@@ -448,6 +448,7 @@ int launch_fp16_gemv(const half* w, const half* x, half* y, int rows, int cols, 
     if (rows == 0) return TLLM_OK;
     const size_t smem = (size_t)cols * sizeof(half);
     if (smem > 200 * 1024) return fail(TLLM_ERR_SHAPE, "fp16_gemv: cols=%d exceeds %d", cols, 100 * 1024);
+    if (fp16_rows_supported(w, x, cols)) return launch_fp16_rows(w, x, y, 1, rows, cols, stream);
     static bool attr[64] = {};
     static int sms[64] = {};
     int dev = 0;
@@ -532,6 +533,7 @@ int launch_fp16_gemv_batched(const half* w, const half* x, half* y, int batch, i
     if (batch == 1) return launch_fp16_gemv(w, x, y, rows, cols, stream);
     const size_t smem = (size_t)kFp16GemvVecs * cols * sizeof(half);
     if (smem > 200 * 1024) return fail(TLLM_ERR_SHAPE, "fp16_gemv (batched): cols=%d exceeds %d", cols, 200 * 1024 / 16);
+    if (fp16_rows_supported(w, x, cols)) return launch_fp16_rows(w, x, y, batch, rows, cols, stream);
     static bool attr[64] = {};
     static int sms[64] = {};
     int dev = 0;

@@ -1,0 +1,48 @@
+"""The dense FP16 head on the tensor cores (csrc/fp16_rows.cu): edges of the 16-row blocks, odd and even
+numbers of 128-column windows, one vector and batches that fill one, two and more column blocks of the MMA
+or need a second pass, against 64 bits."""
+import numpy as np
+import pytest
+import torch
+
+import ternary_llm_b200 as tl
+from ternary_llm_b200 import layer_ops as ops
+from ternary_llm_b200 import tllm_format as tf
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [1, 15, 17, 2400, 40001])
+@pytest.mark.parametrize("cols", [128, 384, 2048, 14336])
+def test_one_vector(rows, cols):
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    w = (0.02 * torch.randn(rows, cols, generator=gen, device="cuda")).half()
+    x = torch.randn(cols, generator=gen, device="cuda").half()
+    y = torch.full((rows + 16,), 7.0, dtype=torch.float16, device="cuda")
+    ops.fp16_gemv(w, x, y[:rows], rows, cols)
+    torch.cuda.synchronize()
+    assert (y[rows:] == 7.0).all()
+    want = w.double() @ x.double()
+    # cols FP32 roundings of at most the sum of magnitudes, then one to FP16
+    bound = cols * 2.0 ** -24 * (w.double().abs() @ x.double().abs()) + 2.0 ** -11 * want.abs() + 2.0 ** -25
+    assert ((y[:rows].double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("batch", [2, 8, 9, 17, 25, 40])
+def test_batch_equals_single_sequences(batch):
+    """No layer's sums depend on the vectors beside them: with the layers' products on the same kernel (up to 32
+    rows), a sequence's logits in a batch are those of the same sequence in another place of it."""
+    cfg = tf.TllmConfig(vocab_size=1003, hidden_dim=256, intermediate_dim=512, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64,
+                        max_seq_len=16, rope_theta=10000.0, rms_norm_eps=1e-5)
+    model = tf.random_model(cfg, seed=5)
+    dec = tl.Decoder(model, int8_decode=False, max_batch=batch)
+    tokens = torch.from_numpy(np.random.default_rng(batch).integers(0, cfg.vocab_size, batch).astype(np.int32)).cuda()
+    got = dec.forward_batch(tokens, 0).clone()
+    turned = dec.forward_batch(tokens.flip(0).contiguous(), 0).clone()
+    assert torch.equal(got, turned.flip(0))
+    for b in {0, batch // 2, batch - 1}:
+        one = dec.forward_seq(0, tokens[b:b + 1], 0).double()
+        # two FP16 roundings per operator of one layer, on different kernels
+        assert (got[b].double() - one).norm() <= 1e-2 * one.norm()
+    tl.check_device_errors()
+    dec.close()

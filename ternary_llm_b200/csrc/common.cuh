@@ -72,21 +72,22 @@ int launch_gemv_packed_noalloc(const uint8_t* packed, const half* x, half* y, in
                                cudaStream_t stream);
 int noalloc_error_check(cudaStream_t stream);
 
-// tcgen05 prefill GEMM on prepared weights (gemm_tcgen05.cu).
-bool gemm_tcgen05_supported(int M, int N, int K);
-int launch_gemm_tcgen05(const half* A, const uint8_t* packed, half* C, int M, int N, int K, cudaStream_t stream);
-
-// A few rows on prepared weights (gemm_rows.cu).  out[i]: rows row0 .. row0 + rows of the matrix go to y[m, rows].
+// out[i]: rows row0 .. row0 + rows of matrices packed back to back go to y[m, rows].
 struct RowsOut {
     half* y;
     int row0, rows;
 };
+// tcgen05 prompt GEMM on prepared weights (gemm_tcgen05.cu); glu: y = silu(gate) * up of [gate|up].
+int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out, int nout, bool glu, int M, int K, cudaStream_t stream);
+
+// A few rows on prepared weights (gemm_rows.cu).
 int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream);
 
 // y[m, rows] = x[m, cols] . W^T, FP16 activations, on the kernel for these sizes: passes of the
 // streaming GEMV (four vectors share one over the weights), gemm_rows.cu, or the tcgen05 GEMM.
 constexpr int kRowsMax = 32;
 bool linear_takes_rows(int m, int rows, int cols);
+int launch_linear_out(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream);
 int launch_linear_f16(const uint8_t* packed, const half* x, half* y, int m, int rows, int cols, cudaStream_t stream);
 
 // ---- small device helpers --------------------------------------------------

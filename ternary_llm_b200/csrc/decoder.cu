@@ -130,10 +130,10 @@ int linear_f16(const PackedW& w, const half* x, half* y, int n_tokens, cudaStrea
 int linear_multi(LlamaDecoder* D, int count, const PackedW* const* w, half* const* y, const half* x, bool int8,
                  int n_tokens, cudaStream_t stream, const PackedW* all = nullptr)
 {
-    if (n_tokens > 1 && all && all->p && linear_takes_rows(n_tokens, all->rows, all->cols)) {
+    if (n_tokens > 1 && all && all->p && (n_tokens > 8 || linear_takes_rows(n_tokens, all->rows, all->cols))) {
         RowsOut out[TLLM_MAX_FUSED];
         for (int i = 0, row = 0; i < count; row += w[i++]->rows) out[i] = {y[i], row, w[i]->rows};
-        return launch_gemm_rows(all->p, x, out, count, n_tokens, all->cols, stream);
+        return launch_linear_out(all->p, x, out, count, n_tokens, all->cols, stream);
     }
     const uint8_t* p[TLLM_MAX_FUSED];
     int rows[TLLM_MAX_FUSED];

@@ -292,26 +292,30 @@ int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, i
 //     and its block fixed point answers a non-finite activation with NaN in every output
 //   m = 4: one GEMV pass reads 24 tiles per warp before its staging is paid back, and long rows lengthen
 //     that staging: 4096 x 4096 6.9, here 5.3; 4096 x 14336 13.4, here 12.5; 16384 x 2048 6.5, here 7.1
-//   m = 5..24: two GEMV passes or a tcgen05 tile per 128 features: 4096 x 4096, m = 8: 13.5, here 5.6;
-//     m = 24: 13.6, here 8.0; 28672 x 4096, m = 8: 21.3, here 24.3 (two passes win there)
-//   m = 25..32: the tcgen05 kernel once its tiles fill the SMs: 4096 x 14336 29.7, here 21.1;
-//     28672 x 4096 34.6, here 42.9
+//   m = 5..8: two GEMV passes: 4096 x 4096, m = 8: 13.5, here 5.6; 28672 x 4096, m = 8: 21.3, here 24.3
+//   m = 9..32: the tcgen05 kernel (here / there): 2048 x 2048, m = 32 6.4 / 6.5; 4096 x 4096, m = 24 7.9 / 8.8;
+//     16384 x 2048, m = 16 9.7 / 8.8; 28672 x 4096, m = 9 29.8 / 25.0; 4096 x 14336, m = 16 15.4 / 16.2, m = 24
+//     18.1 / 16.5
 bool linear_takes_rows(int m, int rows, int cols)
 {
     const long long tiles = (long long)((rows + kTileRows - 1) / kTileRows) * (cols / kGroup);
     if (m < 4 || m > kRowsMax) return false;
     if (m == 4) return tiles <= 12288 || cols >= 12288;
     if (m <= 8) return tiles <= 40000;
-    return m <= 24 || rows < 14336;
+    return tiles <= 12288 || (m <= 16 && cols >= 8192 && rows <= 4096);
+}
+
+// Matrices packed back to back on this kernel or the tcgen05 GEMM (m > 8, or where this one is taken).
+int launch_linear_out(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream)
+{
+    if (linear_takes_rows(m, out[nout - 1].row0 + out[nout - 1].rows, cols)) return launch_gemm_rows(packed, x, out, nout, m, cols, stream);
+    return launch_gemm_tcgen05(x, packed, out, nout, false, m, cols, stream);
 }
 
 int launch_linear_f16(const uint8_t* packed, const half* x, half* y, int m, int rows, int cols, cudaStream_t stream)
 {
-    if (linear_takes_rows(m, rows, cols)) {
-        const RowsOut out = {y, 0, rows};
-        return launch_gemm_rows(packed, x, &out, 1, m, cols, stream);
-    }
-    if (m > 8) return launch_gemm_tcgen05(x, packed, y, m, rows, cols, stream);
+    const RowsOut out = {y, 0, rows};
+    if (m > 8 || linear_takes_rows(m, rows, cols)) return launch_linear_out(packed, x, &out, 1, m, cols, stream);
     return launch_gemv_packed(packed, x, y, m, rows, cols, stream);
 }
 

@@ -1,32 +1,45 @@
-// Prefill GEMM  C[M,N] = A[M,K] . W^T  on the 5th-generation tensor cores (sm_100a).
+// Prompt GEMM  C[M,N] = A[M,K] . W^T  on the 5th-generation tensor cores (sm_100a).
 //
-// W is ternary with one FP16 scale per 128 weights along K.  The product
-// scale * t is exactly representable in FP16, so the weight operand is expanded to
-// FP16 {-s, 0, +s} and a plain FP16 x FP16 -> FP32 contraction over the whole K
-// gives the reference result with nothing but FP32 accumulation rounding.
+// W is ternary with one FP16 scale per 128 weights along K.  The product scale * t is exactly
+// representable in FP16, so the weight operand is expanded to FP16 {-s, 0, +s} and a plain
+// FP16 x FP16 -> FP32 contraction over the whole K gives the reference result with nothing but
+// FP32 accumulation rounding.
 //
-// One CTA computes a tile of 128 output features x 256 tokens:
-//   * the weight tile is the MMA's A operand and lives in TENSOR MEMORY: four
-//     expander warps (one thread per feature row = one TMEM lane) read the row's
-//     packed 2-bit codes (packed_layout.cuh) straight from global/L2 and expand 128
-//     weights per stage: the codes c = t + 1 of two weights become the selector of one
-//     PRMT into the byte table {-s, 0, +s} of the group's scale (an integer multiply-add
-//     builds the selector), which yields the FP16 pair directly; tcgen05.st writes
-//     them.  The expanded weights never touch shared memory, which leaves its
-//     bandwidth to the activation operand;
-//   * the activation tile [256 tokens x 128 K] is the B operand in shared memory,
-//     brought by TMA (two 128-byte-swizzled boxes of 64 K per stage, 3 stages);
-//   * one thread issues tcgen05.mma (kind::f16, M=128, N=256, K=16; A from TMEM, B
-//     from a shared-memory descriptor) into a 128 x 256 FP32 accumulator in TMEM;
-//   * the expander warps then read the accumulator back with tcgen05.ld and store
-//     C (a TMEM lane is an output feature, so a warp writes 32 adjacent features
-//     of one token at a time).
-// TMEM: columns 0..255 accumulator, 256..383 two weight stages of 64 columns.
-// All mbarrier waits are bounded; a wait that gives up sets the device error flag
-// and every role falls through to the common exit, where TMEM is released.
+// Bound: the tensor pipe for long prompts (4 clocks a token of a tile and scale group); the chain of
+// expansion, MMA and hand-overs, about 700 clocks a scale group, for tiles of few tokens.  A tile is
+// 128 features x TM tokens, TM any multiple of 16 up to 192: the launch picks the TM (and a split of K)
+// with which the tiles come out even over the SMs.  One persistent CTA per SM, whose warps run ahead
+// of one another over the tiles' scale groups:
+//   * one warp loads the activations by TMA, a scale group (two boxes of 64 columns, 128-byte swizzled rows) a
+//     stage, four to eight stages; another one the packed codes, one box of 8 row blocks x 544 bytes per scale
+//     group, six ahead.  (Read by the expanders from global memory one group ahead, a group took a
+//     microsecond whatever the tile, the latency of a load from HBM.)
+//   * twelve warps expand: one thread per feature row = one lane of tensor memory, three warps per
+//     lane quarter on every third group (28672 x 4096, 37 tokens: two sets 30.4 us, three 26.5, four 26.1).
+//     The codes c = t + 1 of two weights are the selector of one PRMT into the byte table {-s, 0, +s}, which
+//     yields the FP16 pair; tcgen05.st writes it.  The expanded weights are the MMA's A operand in TENSOR
+//     MEMORY and never touch shared memory.
+//   * one warp issues tcgen05.mma (kind::f16, M=128, N=TM, K=16) into one of two accumulators.  A stage is one
+//     wait (activations and weights arrive on one barrier), eight MMAs and one commit, and the warp's loop is
+//     uniform with an elected lane for the MMAs: as the loop of one thread, with a barrier and a commit for
+//     either operand, the issue alone took 2000 clocks a stage;
+//   * four warps empty the other accumulator with tcgen05.ld and store C (a lane is an output feature, so a
+//     warp stores 32 adjacent features of one token at a time).
+// Tensor memory: two accumulators of TM columns (a multiple of 32 apart), then two to four weight
+// stages of 64 columns.
+// Too few tiles for the SMs: K is split over the CTAs of a cluster; each leaves its FP32 sums in its
+// shared memory, and each adds all of them, in rank order, for its share of the tokens.
+// All mbarrier waits are bounded; a wait that gives up sets the device error flag, every role waits for
+// its own copies and MMAs (bounded again) and falls through to the common exit.
+//
+// us, of tiles of 128 x 256 or fewer tokens without all this and now (weights from HBM): 4096 x 4096, 37 tokens
+// 13.3 -> 9.3, 300: 26.5 -> 16.3; 4096 x 14336, 37: 29.8 -> 17.0, 300: 60 -> 34.2; 28672 x 4096, 300: 104 -> 62, 2048:
+// 333 (1445 TFLOP/s); 2048 x 8192, 300: 29.2 -> 16.8.
+#include <climits>
 #include <mutex>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "packed_layout.cuh"
 #include "tcgen05.cuh"
 
@@ -34,50 +47,35 @@ namespace tllm {
 
 namespace gemm {
 
-constexpr int kTileN = 128;          // output features per CTA (MMA M, TMEM lanes)
-constexpr int kStageK = 128;         // K per pipeline stage = one scale group
-constexpr int kAStages = 2;          // weight stages in tensor memory
-constexpr int kBoxK = 64;            // TMA box inner extent (128 bytes of FP16)
-constexpr int kThreads = 256;
-constexpr int kAColsPerStage = kStageK / 2;            // 64 columns of FP16 pairs
-
-// Per token-tile size TM (tokens per CTA = MMA N): 256 for long prefills; 128/64/32 for
-// short ones and for decode batches, where two CTAs share an SM (half the shared memory
-// and half the tensor memory each) so that twice as many warps expand weights.
-template <int TM>
-struct Cfg {
-    static constexpr int kBoxBytes = TM * kBoxK * 2;
-    static constexpr int kStageBytes = 2 * kBoxBytes;                    // TM x 128 K x FP16
-    static constexpr int kBStages = (TM == 256) ? 3 : (TM == 128) ? 3 : (TM == 64) ? 6 : 8;
-    static constexpr int kAccCols = TM;                                  // FP32 accumulator columns
-    static constexpr int kTmemCols = (TM == 256) ? 512 : 256;            // power of two >= TM + 128
-    static constexpr int kCtasPerSm = (TM == 256) ? 1 : 2;
-    static constexpr size_t kSmem = (size_t)kBStages * kStageBytes + 1024;
-};
+constexpr int kTileN = 128;          // features per tile (MMA M, TMEM lanes)
+constexpr int kBoxK = 64;            // columns per activation box (128 bytes of FP16)
+constexpr int kACols = kGroup / 2;   // tensor-memory columns of a weight stage (FP16 pairs)
+constexpr int kMaxTm = 192;
+constexpr int kMaxB = 8;             // activation stages, upper bound
+constexpr int kMaxA = 4;             // weight stages, upper bound
+constexpr int kCodes = 6;            // scale groups of codes in shared memory
+constexpr int kCodeBytes = kTileN / kTileRows * kTileBytes;
+constexpr int kSets = 3;             // sets of four expander warps
+constexpr int kOutWarp = 4 + 4 * kSets;
+constexpr int kThreads = (kOutWarp + 4) * 32;        // warps 0-3: activations, MMA, codes, none; expanders; four for outputs
+constexpr int kTmemCols = 512;
+// All of it for every tile: a CTA that takes the whole tensor memory shares its SM with no other kernel's that needs some.
+constexpr size_t kSmem = 226 * 1024;
+constexpr int kMaxSplit = 8;
 
 struct Args {
-    const uint8_t* packed;     // packed weights [ceil(N/16)][K/128] tiles
-    half* C;                   // [M, N]
-    int M, N, K, groups;       // groups = K / 128
-    int nrb;                   // ceil(N / 16)
+    RowsOut out[TLLM_MAX_FUSED];     // row ranges of the matrix and where they go; unused ones start past every row
+    int M, N, groups;                // tokens; rows of W (of the gate where glu is set); K / 128
+    int mt, tiles, split;            // token tiles; tiles; CTAs per tile
+    int tm, acc_stride, na, nb;      // tokens per tile; columns between accumulators; weight and activation stages
+    int glu, up_rb;                  // rows n and 16 * up_rb + n are gate and up of output n
     int* err;
-    // split-K (gridDim.z > 1): CTA z contracts stages [z*groups/ks, (z+1)*groups/ks) and writes an
-    // FP32 partial tile; the CTA of a tile that arrives last adds the partials in z order.
-    float* ws;                 // [tile][z][tokens of the tile][128] FP32
-    unsigned* counters;        // [tiles], zero between launches
 };
 
-// kind::f16 instruction descriptor: FP16 x FP16 -> FP32, both operands K-major.
-template <int TM>
-__device__ __forceinline__ uint32_t make_idesc()
+// kind::f16 instruction descriptor: FP16 x FP16 -> FP32, both operands K-major, M = 128
+__device__ __forceinline__ uint32_t make_idesc(int tm)
 {
-    uint32_t d = 0;
-    d |= 1u << 4;                          // D format F32
-    d |= 0u << 7;                          // A format F16
-    d |= 0u << 10;                         // B format F16
-    d |= (uint32_t)(TM >> 3) << 17;        // N
-    d |= (uint32_t)(kTileN >> 4) << 24;    // M
-    return d;
+    return (1u << 4) | ((uint32_t)(tm >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
@@ -100,49 +98,88 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
-template <int TM>
-__global__ void __launch_bounds__(kThreads, Cfg<TM>::kCtasPerSm)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const Args a)
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr)
 {
-    constexpr int kBStages = Cfg<TM>::kBStages, kStageBytes = Cfg<TM>::kStageBytes, kBoxBytes = Cfg<TM>::kBoxBytes;
-    constexpr int kAccCols = Cfg<TM>::kAccCols, kTmemCols = Cfg<TM>::kTmemCols, kTileM = TM;
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ half glu_out(float g, float u) { return __float2half_rn(g / (1.0f + expf(-g)) * u); }
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
+    return p != 0;
+}
+
+// A place in a ring of n slots: the slot and the parity of its uses.
+struct Ring {
+    int slot = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void step(int n, int by = 1)
+    {
+        slot += by;
+        while (slot >= n) {
+            slot -= n;
+            phase ^= 1;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Args a)
+{
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment for the 128-byte swizzle atoms
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t bars[2 * kBStages + 2 * kAStages + 1];
+    __shared__ __align__(8) uint64_t bars[2 * kMaxB + 2 * kCodes + 5];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
-    __shared__ int last_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n0 = blockIdx.x * kTileN;          // first output feature of the tile
-    const int m0 = blockIdx.y * kTileM;          // first token of the tile
-    const int ks = gridDim.z;
-    const int it0 = (int)(((long long)blockIdx.z * a.groups) / ks);          // first scale group of this CTA
-    const int nstages = (int)(((long long)(blockIdx.z + 1) * a.groups) / ks) - it0;   // one scale group per stage
+    const int tm = a.tm, nb = a.nb, na = a.na;
+    const int split = a.split, rank = blockIdx.x % split, first = blockIdx.x / split, step = gridDim.x / split;
+    const int it0 = (int)((long long)rank * a.groups / split);                       // scale groups of this CTA
+    const int nst = (int)((long long)(rank + 1) * a.groups / split) - it0;
+    const int box_bytes = tm * kBoxK * 2, stage_bytes = 2 * box_bytes;
+    const int rb_tile = a.glu ? kTileN / kTileRows / 2 : kTileN / kTileRows;           // row blocks of a tile (of the gate)
+    uint8_t* codes = smem + nb * stage_bytes;
 
     const uint32_t bar0 = smem_u32(bars);
-    auto full_b = [&](int s) { return bar0 + 8u * s; };
-    auto empty_b = [&](int s) { return bar0 + 8u * (kBStages + s); };
-    auto full_a = [&](int s) { return bar0 + 8u * (2 * kBStages + s); };
-    auto empty_a = [&](int s) { return bar0 + 8u * (2 * kBStages + kAStages + s); };
-    const uint32_t acc_full = bar0 + 8u * (2 * kBStages + 2 * kAStages);
+    // full: a stage's activations (one arrival and their bytes) and expanded weights (four warps); done: its MMAs
+    auto full = [&](int s) { return bar0 + 8u * s; };
+    auto done = [&](int s) { return bar0 + 8u * (kMaxB + s); };
+    auto full_c = [&](int s) { return bar0 + 8u * (2 * kMaxB + s); };
+    auto empty_c = [&](int s) { return bar0 + 8u * (2 * kMaxB + kCodes + s); };
+    auto acc_full = [&](int s) { return bar0 + 8u * (2 * kMaxB + 2 * kCodes + s); };
+    auto acc_empty = [&](int s) { return bar0 + 8u * (2 * kMaxB + 2 * kCodes + 2 + s); };
+    const uint32_t drained = bar0 + 8u * (2 * kMaxB + 2 * kCodes + 4);
 
     if (tid == 0) {
-        for (int s = 0; s < kBStages; s++) {
-            mbar_init(full_b(s), 1);
-            mbar_init(empty_b(s), 1);
+        for (int s = 0; s < kMaxB; s++) {
+            mbar_init(full(s), 5);
+            mbar_init(done(s), 1);
         }
-        for (int s = 0; s < kAStages; s++) {
-            mbar_init(full_a(s), 128);
-            mbar_init(empty_a(s), 1);
+        for (int s = 0; s < kCodes; s++) {
+            mbar_init(full_c(s), 1);
+            mbar_init(empty_c(s), 4);
         }
-        mbar_init(acc_full, 1);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(acc_full(s), 1);
+            mbar_init(acc_empty(s), 4);
+        }
+        mbar_init(drained, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {       // one warp allocates all 512 TMEM columns of this SM
+    if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -150,182 +187,273 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const Args a)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // only now: a following kernel that took this SM's tensor memory first would wait for this one with it
+    pdl_launch_dependents();
     const uint32_t tmem = tmem_base_slot;
     volatile int* abortp = &abort_flag;
+    int never = 0;
 
     if (warp == 0) {
-        // ---------------- TMA producer: activations ----------------
-        if (lane == 0) {
-            for (int it = 0; it < nstages; it++) {
-                const int s = it % kBStages;
-                if (!mbar_wait(empty_b(s), ((it / kBStages) & 1) ^ 1, abortp)) { abort_flag = 1; break; }
-                mbar_expect_tx(full_b(s), kStageBytes);
-                const uint32_t dst = smem_u32(smem + (size_t)s * kStageBytes);
-                tma_load_2d(dst, &map_a, (it0 + it) * kStageK, m0, full_b(s));
-                tma_load_2d(dst + kBoxBytes, &map_a, (it0 + it) * kStageK + kBoxK, m0, full_b(s));
+        // ---------------- activations ----------------
+        const bool leader = elect_one();
+        pdl_wait();
+        Ring b;
+        bool ok = true;
+        for (int tile = first; ok && tile < a.tiles; tile += step) {
+            const int m0 = (tile % a.mt) * tm;
+            for (int it = 0; it < nst; it++) {
+                if (!(ok = mbar_wait(done(b.slot), b.phase ^ 1, abortp))) break;
+                const uint32_t dst = smem_u32(smem + b.slot * stage_bytes);
+                if (leader) {
+                    mbar_expect_tx(full(b.slot), stage_bytes);
+                    tma_load_2d(dst, &map_x, (it0 + it) * kGroup, m0, full(b.slot));
+                    tma_load_2d(dst + box_bytes, &map_x, (it0 + it) * kGroup + kBoxK, m0, full(b.slot));
+                }
+                b.step(nb);
             }
+        }
+        if (!ok) {
+            // The copies in flight land before the CTA leaves; a stage's barrier cannot tell that any more (its weights
+            // may never come), so a millisecond passes instead of their microseconds.
+            abort_flag = 1;
+            for (int i = 0; i < 1000; i++) __nanosleep(1000);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc<TM>();
-            for (int it = 0; it < nstages; it++) {
-                const int sb = it % kBStages, sa = it % kAStages;
-                if (!mbar_wait(full_b(sb), (it / kBStages) & 1, abortp) ||
-                    !mbar_wait(full_a(sa), (it / kAStages) & 1, abortp)) { abort_flag = 1; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t bsm = smem_u32(smem + (size_t)sb * kStageBytes);
-                const uint32_t a_t = tmem + kAccCols + sa * kAColsPerStage;
-#pragma unroll
-                for (int k = 0; k < kStageK / 16; k++) {
-                    // K step of 16: 32 bytes inside the 128-byte swizzled row; second box after 64 K
-                    const uint64_t bd = make_sw128_desc(bsm + (k >> 2) * kBoxBytes + (k & 3) * 32);
-                    mma_ts(tmem, a_t + k * 8, bd, idesc, (it > 0 || k > 0) ? 1u : 0u);
-                }
-                mma_commit(empty_b(sb));
-                mma_commit(empty_a(sa));
-            }
-            mma_commit(acc_full);
-        }
-    } else if (warp >= 4) {
-        // ---------------- weight expanders, then epilogue ----------------
-        const int row = tid - 128;                       // feature row inside the tile = TMEM lane
-        const int n = n0 + row;
-        const int rb = n >> 4, r16 = n & 15;             // 16-row block and row inside it
-        const int gq = r16 & 7, h = r16 >> 3;
-        const bool row_valid = rb < a.nrb;               // rows past the matrix expand to zeros
-        const uint8_t* tile0 = a.packed + ((size_t)(row_valid ? rb : 0) * a.groups + it0) * kTileBytes;
-        // this row's code words of MMA lane t: the pair (column halves j2 = 0, 1) at word index
-        // (gq*4 + t)*4 + 2h, i.e. one 64-bit load per t; each word holds all four 32-column steps
-        const int pair0 = (gq * 4) * 2 + h;              // in units of uint2; + t*2
-        const int spos = tile_scale_index(r16);
-        const uint32_t lane_base = tmem + ((uint32_t)(row & ~31) << 16);   // this warp's 32 TMEM lanes
-
-        uint2 cw[4];
-        uint32_t sbits = 0;
-        auto load_stage = [&](const uint8_t* tp) {
-            const uint2* p = reinterpret_cast<const uint2*>(tp) + pair0;
-#pragma unroll
-            for (int t = 0; t < 4; t++) cw[t] = __ldg(p + t * 2);
-            sbits = __half_as_ushort(__ldg(reinterpret_cast<const half*>(tp + kTileCodeBytes) + spos));
-        };
-        if (row_valid) load_stage(tile0);
+        const bool leader = elect_one();
+        pdl_wait();
+        const uint32_t idesc = make_idesc(tm);
+        Ring b, w, acc;
         bool ok = true;
-        for (int it = 0; it < nstages; it++) {
-            const int sa = it % kAStages;
-            // PRMT table of this stage: bytes 0,1 = -s (code 0), 2,3 = 0 (code 1), 4,5 = +s (code 2)
-            const uint32_t tab_lo = row_valid ? (sbits ^ 0x8000u) : 0u, tab_hi = row_valid ? sbits : 0u;
-            uint2 cur[4];
+        for (int tile = first; ok && tile < a.tiles; tile += step) {
+            if (!(ok = mbar_wait(acc_empty(acc.slot), acc.phase ^ 1, abortp))) break;
+            const uint32_t d = tmem + acc.slot * a.acc_stride;
+            for (int it = 0; it < nst; it++) {
+                if (!(ok = mbar_wait(full(b.slot), b.phase, abortp))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t d0 = make_sw128_desc(smem_u32(smem + b.slot * stage_bytes));
+                const uint64_t d1 = make_sw128_desc(smem_u32(smem + b.slot * stage_bytes) + box_bytes);
+                const uint32_t a_t = tmem + 2 * a.acc_stride + w.slot * kACols, more = it > 0 ? 1u : 0u;
+                if (leader) {
 #pragma unroll
-            for (int t = 0; t < 4; t++) cur[t] = cw[t];
-            if (it + 1 < nstages && row_valid) load_stage(tile0 + (size_t)(it + 1) * kTileBytes);   // prefetch the next group
-            if (!mbar_wait(empty_a(sa), ((it / kAStages) & 1) ^ 1, abortp)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a_t = lane_base + kAccCols + sa * kAColsPerStage;
-#pragma unroll
-            for (int m = 0; m < 4; m++) {                 // 32 K per step -> 16 columns; step m is code field m
-                uint32_t r[16];
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-#pragma unroll
-                    for (int j2 = 0; j2 < 2; j2++) {
-                        // four codes (K offsets 32m + 16*j2 + 4t .. +3) in the low two bits of each byte
-                        const uint32_t y = ((j2 ? cur[t].y : cur[t].x) >> (2 * m)) & 0x03030303u;
-                        // selector nibbles 2c, 2c+1 per weight: one PRMT makes an FP16 pair {-s,0,+s}
-                        r[8 * j2 + 2 * t] = prmt(tab_lo, tab_hi, y * 0x22u + 0x1010u);
-                        r[8 * j2 + 2 * t + 1] = prmt(tab_lo, tab_hi, (y >> 16) * 0x22u + 0x1010u);
-                    }
+                    for (int k = 0; k < kGroup / 16; k++)          // 32 bytes (2 in the descriptor) inside the 128-byte swizzled row
+                        mma_ts(d, a_t + k * 8, (k < 4 ? d0 : d1) + (k & 3) * 2, idesc, k ? 1u : more);
+                    mma_commit(done(b.slot));
                 }
-                tmem_st16(a_t + m * 16, r);
+                b.step(nb);
+                w.step(na);
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(full_a(sa));
+            if (leader) mma_commit(acc_full(acc.slot));
+            acc.step(2);
         }
         if (!ok) abort_flag = 1;
-
-        // ---------------- epilogue: accumulator -> C ----------------
-        const bool good = ok && mbar_wait(acc_full, 0, abortp);
-        const int tile_id = blockIdx.y * gridDim.x + blockIdx.x;
-        if (good) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float* wtile = a.ws + ((size_t)tile_id * ks + blockIdx.z) * kTileM * kTileN;
-#pragma unroll 1
-            for (int cchunk = 0; cchunk < kTileM / 32; cchunk++) {
-                if (m0 + cchunk * 32 >= a.M) break;       // uniform: no tokens left in this chunk
-                uint32_t v[32];
-                tmem_ld32(lane_base + cchunk * 32, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (ks == 1) {
-                    if (n < a.N) {
+        if (leader) mma_commit(drained);
+        __syncwarp();
+        mbar_wait(drained, 0, &never);
+    } else if (warp == 2) {
+        // ---------------- packed codes (constants: not behind the kernel before) ----------------
+        const bool leader = elect_one();
+        Ring c;
+        int used = 0;
+        bool ok = true;
+        for (int tile = first; ok && tile < a.tiles; tile += step) {
+            const int rb = tile / a.mt * rb_tile;
+            for (int it = 0; it < nst; it++) {
+                if (used == kCodes) pdl_wait();              // from here on a wait depends on the kernel before
+                if (!(ok = mbar_wait(empty_c(c.slot), c.phase ^ 1, abortp))) break;
+                const uint32_t dst = smem_u32(codes + c.slot * kCodeBytes);
+                if (leader) {
+                    mbar_expect_tx(full_c(c.slot), kCodeBytes);
+                    tma_load_2d(dst, &map_w, (it0 + it) * (kTileBytes / 4), rb, full_c(c.slot));
+                    if (a.glu) tma_load_2d(dst + kCodeBytes / 2, &map_w, (it0 + it) * (kTileBytes / 4), a.up_rb + rb, full_c(c.slot));
+                }
+                c.step(kCodes);
+                used = min(used + 1, kCodes);
+            }
+        }
+        if (!ok) abort_flag = 1;
+        for (; used > 0; used--) {                           // no copy outlives the CTA
+            c.slot = c.slot ? c.slot - 1 : kCodes - 1;
+            if (c.slot == kCodes - 1) c.phase ^= 1;
+            mbar_wait(full_c(c.slot), c.phase, &never);
+        }
+    } else if (warp >= 4 && warp < kOutWarp) {
+        // ---------------- expanders ----------------
+        const int set = (warp - 4) >> 2, row = (warp & 3) * 32 + lane;
+        // row block of the tile: with glu the quarter's 32 lanes are 16 gate rows and the up rows with the same numbers
+        const int rbl = a.glu ? (warp & 3) + 4 * (lane >> 4) : row >> 4, r16 = row & 15;
+        const int gq = r16 & 7, h = r16 >> 3;
+        // this row's code words of MMA lane t: the pair (column halves j2 = 0, 1) at word index
+        // (gq*4 + t)*4 + 2h, one 64-bit load per t; each word holds all four 32-column steps
+        const uint8_t* cp = codes + rbl * kTileBytes + gq * 64 + h * 8;
+        const uint8_t* sp = codes + rbl * kTileBytes + kTileCodeBytes + tile_scale_index(r16) * 2;
+        const uint32_t lane_base = tmem + ((uint32_t)(row & ~31) << 16) + 2 * a.acc_stride;   // this warp's 32 lanes
+        Ring c, w, f, past;                                  // codes; weight stage; stage; the stage that had the weight stage before
+        c.step(kCodes, set);
+        w.step(na, set);
+        f.step(nb, set);
+        past.slot = (set + kMaxA * kSets - na) % kSets;      // of the set's first scale group from na on (nb is at least 4)
+        bool ok = true;
+        int g = 0, turn = 0;                                 // scale groups of this CTA so far; whose the next one is
+        for (int tile = first; ok && tile < a.tiles; tile += step) {
+            for (int it = 0; it < nst; it++, g++) {
+                const bool mine = turn == set;
+                turn = turn + 1 == kSets ? 0 : turn + 1;
+                if (!mine) continue;
+                if (!(ok = mbar_wait(full_c(c.slot), c.phase, abortp))) break;
+                uint2 cur[4];
 #pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            const int m = m0 + cchunk * 32 + j;
-                            if (m < a.M) a.C[(size_t)m * a.N + n] = __float2half_rn(__uint_as_float(v[j]));
+                for (int t = 0; t < 4; t++) cur[t] = *reinterpret_cast<const uint2*>(cp + c.slot * kCodeBytes + t * 16);
+                const uint32_t sbits = *reinterpret_cast<const unsigned short*>(sp + c.slot * kCodeBytes);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty_c(c.slot));
+                c.step(kCodes, kSets);
+                // PRMT table of this row: bytes 0,1 = -s (code 0), 2,3 = 0 (code 1), 4,5 = +s (code 2)
+                const uint32_t tab_lo = sbits ^ 0x8000u, tab_hi = sbits;
+                if (g >= na) {
+                    if (g < na + kSets) pdl_wait();          // from here on a wait depends on the kernel before
+                    if (!(ok = mbar_wait(done(past.slot), past.phase, abortp))) break;
+                    past.step(nb, kSets);
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a_t = lane_base + w.slot * kACols;
+#pragma unroll
+                for (int m = 0; m < 4; m++) {                 // 32 K per step -> 16 columns; step m is code field m
+                    uint32_t r[16];
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+#pragma unroll
+                        for (int j2 = 0; j2 < 2; j2++) {
+                            // four codes (K offsets 32m + 16*j2 + 4t .. +3) in the low two bits of each byte;
+                            // selector nibbles 2c, 2c+1 per weight: one PRMT makes an FP16 pair {-s,0,+s}
+                            const uint32_t s = (((j2 ? cur[t].y : cur[t].x) >> (2 * m)) & 0x03030303u) * 0x22u + 0x10101010u;
+                            r[8 * j2 + 2 * t] = prmt(tab_lo, tab_hi, s);
+                            r[8 * j2 + 2 * t + 1] = prmt(tab_lo, tab_hi, s >> 16);
                         }
                     }
-                } else {
+                    tmem_st16(a_t + m * 16, r);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full(f.slot));
+                f.step(nb, kSets);
+                w.step(na, kSets);
+            }
+        }
+        if (!ok) abort_flag = 1;
+    } else if (warp >= kOutWarp) {
+        // ---------------- outputs ----------------
+        pdl_wait();
+        const int row = (warp & 3) * 32 + lane;
+        const uint32_t lane_base = tmem + ((uint32_t)(row & ~31) << 16);
+        Ring acc;
+        bool ok = true;
+        for (int tile = first; tile < a.tiles; tile += step) {
+            ok = mbar_wait(acc_full(acc.slot), acc.phase, abortp) && !*abortp;
+            if (!(ok = __all_sync(0xffffffffu, ok))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int m0 = (tile % a.mt) * tm, mv = min(tm, a.M - m0);
+            const int n = tile / a.mt * rb_tile * kTileRows + (a.glu ? (warp & 3) * 16 + (lane & 15) : row);
+            half* y = a.out[0].y;
+            int r0 = 0, rows = a.out[0].rows;
+#pragma unroll
+            for (int i = 1; i < TLLM_MAX_FUSED; i++)
+                if (n >= a.out[i].row0) {
+                    y = a.out[i].y;
+                    r0 = a.out[i].row0;
+                    rows = a.out[i].rows;
+                }
+            y += (size_t)m0 * rows + (n - r0);
+            float* part = reinterpret_cast<float*>(smem) + row;
+            const uint32_t d = lane_base + acc.slot * a.acc_stride;
+            for (int c = 0; c < mv; c += 32) {
+                uint32_t v[32];
+                tmem_ld32(d + c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (split > 1) {
 #pragma unroll
                     for (int j = 0; j < 32; j++)
-                        if (m0 + cchunk * 32 + j < a.M) wtile[(size_t)(cchunk * 32 + j) * kTileN + row] = __uint_as_float(v[j]);
+                        if (c + j < mv) part[(c + j) * kTileN] = __uint_as_float(v[j]);
+                } else if (a.glu) {
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {         // lanes below 16: even tokens, the others odd ones
+                        const bool low = lane < 16;
+                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(low ? v[j + 1] : v[j]), 16);
+                        const half o = low ? glu_out(__uint_as_float(v[j]), other) : glu_out(other, __uint_as_float(v[j + 1]));
+                        const int m = c + j + (low ? 0 : 1);
+                        if (m < mv && n < a.N) y[(size_t)m * rows] = o;
+                    }
+                } else if (n < a.N) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (c + j < mv) y[(size_t)(c + j) * rows] = __float2half_rn(__uint_as_float(v[j]));
                 }
             }
-        } else {
-            abort_flag = 1;
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty(acc.slot));
+            acc.step(2);
         }
-        if (ks > 1) {
-            // publish, count, and let the last CTA of the tile add the partials in z order (all 128
-            // epilogue threads take part in the two barriers whether or not their wait succeeded)
-            __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (row == 0) {
-                const unsigned prev = atomicAdd(a.counters + tile_id, 1u);
-                last_flag = (prev == (unsigned)ks - 1u) ? 1 : 0;
-                if (last_flag) a.counters[tile_id] = 0;
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
+        if (!ok) abort_flag = 1;
     }
-
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (ks > 1 && last_flag && !abort_flag) {
-        // The tile's last CTA adds the partial tiles in z order, all eight warps: lane l sums
-        // features 4l..4l+3 (one 16-byte load per partial), warps take tokens round-robin, eight
-        // tokens per trip so that 8 * ks loads are in flight per thread.
-        __threadfence();
-        const int tile_id = blockIdx.y * gridDim.x + blockIdx.x;
-        const int f4 = lane * 4;
-        const float* base = a.ws + (size_t)tile_id * ks * kTileM * kTileN + f4;
-        const int mt = min(kTileM, a.M - m0);
-        for (int mb = warp * 8; mb < mt; mb += 8 * (kThreads / 32)) {
-            float4 tot[8];
+    if (split > 1) {
+        // each CTA adds the cluster's sums for its share of the tile's tokens: a warp takes a token, a lane four rows
+        pdl_wait();
+        cluster_sync();
+        const int m0 = (first % a.mt) * tm, mv = min(tm, a.M - m0);
+        const int t0 = rank * mv / split, t1 = (rank + 1) * mv / split;
+        const int row = lane * 4;
+        const bool up = a.glu && ((lane >> 2) & 1);
+        const int n = first / a.mt * rb_tile * kTileRows + (a.glu ? (lane >> 3) * 16 + (row & 15) : row);
+        half* y = a.out[0].y;
+        int r0 = 0, rows = a.out[0].rows;
 #pragma unroll
-            for (int u = 0; u < 8; u++) tot[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int z = 0; z < ks; z++) {
-                float4 p[8];
+        for (int i = 1; i < TLLM_MAX_FUSED; i++)
+            if (n >= a.out[i].row0) {
+                y = a.out[i].y;
+                r0 = a.out[i].row0;
+                rows = a.out[i].rows;
+            }
+        for (int t = t0 + warp; t < t1; t += kThreads / 32) {
+            const uint32_t at = smem_u32(smem) + (uint32_t)(t * kTileN + row) * 4;
+            float4 p[kMaxSplit], v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    p[u] = (mb + u < mt) ? __ldcg(reinterpret_cast<const float4*>(base + ((size_t)z * kTileM + mb + u) * kTileN))
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    tot[u].x += p[u].x;
-                    tot[u].y += p[u].y;
-                    tot[u].z += p[u].z;
-                    tot[u].w += p[u].w;
+            for (int z = 0; z < kMaxSplit; z++)
+                if (z < split) {
+                    uint32_t peer;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(z));
+                    p[z] = ld_cluster(peer);
                 }
-            }
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                if (mb + u >= mt) continue;
-                half* cp = a.C + (size_t)(m0 + mb + u) * a.N + n0 + f4;
-                const float v[4] = {tot[u].x, tot[u].y, tot[u].z, tot[u].w};
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (n0 + f4 + j < a.N) cp[j] = __float2half_rn(v[j]);
+            for (int z = 0; z < kMaxSplit; z++)
+                if (z < split) {
+                    v.x += p[z].x;
+                    v.y += p[z].y;
+                    v.z += p[z].z;
+                    v.w += p[z].w;
+                }
+            half o[4];
+            if (a.glu) {
+                o[0] = glu_out(v.x, __shfl_xor_sync(0xffffffffu, v.x, 4));
+                o[1] = glu_out(v.y, __shfl_xor_sync(0xffffffffu, v.y, 4));
+                o[2] = glu_out(v.z, __shfl_xor_sync(0xffffffffu, v.z, 4));
+                o[3] = glu_out(v.w, __shfl_xor_sync(0xffffffffu, v.w, 4));
+            } else {
+                o[0] = __float2half_rn(v.x);
+                o[1] = __float2half_rn(v.y);
+                o[2] = __float2half_rn(v.z);
+                o[3] = __float2half_rn(v.w);
             }
+            half* yp = y + (size_t)(m0 + t) * rows + (n - r0);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (!up && n + j < a.N && !*abortp) yp[j] = o[j];
         }
+        cluster_sync();                                      // nobody leaves while its sums are still read
     }
     if (abort_flag && tid == 0) atomicExch(a.err, TLLM_ERR_TIMEOUT);
     if (warp == 1) {
@@ -334,112 +462,127 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const Args a)
     }
 }
 
-}  // namespace gemm
+struct Device {
+    int sms = 0;
+    int slots[kMaxSplit + 1] = {};       // CTAs that run at the same time in clusters of that size
+};
 
-
-bool gemm_tcgen05_supported(int M, int N, int K)
+static Device* device()
 {
-    (void)N;
-    return M >= 1 && K >= gemm::kStageK && K % gemm::kStageK == 0;
+    static Device devices[64];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    Device& d = devices[dev];
+    if (!d.sms) {
+        int sms = 0;
+        if (cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        for (int c = 1; c <= kMaxSplit; c++) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = c;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3((unsigned)(sms / c * c));
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = kSmem;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_kernel, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                n = 0;
+            }
+            d.slots[c] = n * c;
+        }
+        d.sms = sms;
+    }
+    return &d;
 }
 
-// Scratch of the split-K path: 4 regions handed out round-robin, so that launches on up to four
-// streams do not share one (launches on one stream are ordered).
-namespace gemm {
-constexpr size_t kSplitWsBytes = (size_t)24 << 20;
-constexpr int kSplitTickets = 4;
-constexpr int kSplitMaxTiles = 4096;
-struct SplitScratch {
-    float* ws = nullptr;
-    unsigned* counters = nullptr;
-    int sms = 0;
-    unsigned ticket = 0;
-    bool ready = false, failed = false;
-};
-static SplitScratch g_split[64];
-static std::mutex g_split_mu;
-}  // namespace gemm
-
-template <int TM>
-static int launch_tm(gemm::EncodeTiledFn enc, const half* A, const gemm::Args& a_in, cudaStream_t stream)
+// Tokens per tile and CTAs per tile: the least time in clocks of
+//   rounds of tiles x scale groups x (650 + 2.6 a token) + what a launch has around them
+// (first loads 2000, the last tile's outputs 10 a token, a cluster's sums 2000 + 4 a token).  A scale group's
+// time is measured: 770 clocks at 48 tokens, 950 at 128, 1150 at 192.
+static void choose(Args& a, int nt, const Device& d)
 {
-    using namespace gemm;
-    Args a = a_in;
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.K * sizeof(half)};
-    const cuuint32_t box[2] = {(cuuint32_t)kBoxK, (cuuint32_t)TM};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<half*>(A), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(TLLM_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with %d", (int)r);
-    static bool attr[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr[dev]) {
-        cudaFuncSetAttribute(gemm_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<TM>::kSmem);
-        cudaFuncSetAttribute(gemm_kernel<TM>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        attr[dev] = true;
-    }
-    dim3 grid((a.N + kTileN - 1) / kTileN, (a.M + TM - 1) / TM, 1);
-    // Too few tiles for the SMs: split K (at most four ways).
-    if (dev >= 0 && dev < 64) {
-        std::lock_guard<std::mutex> lk(g_split_mu);
-        SplitScratch& sc = g_split[dev];
-        if (!sc.sms) cudaDeviceGetAttribute(&sc.sms, cudaDevAttrMultiProcessorCount, dev);
-        const int tiles = (int)(grid.x * grid.y), slots = sc.sms * Cfg<TM>::kCtasPerSm;
-        int ks = 1;
-        if (tiles * 2 <= slots) ks = slots / tiles;
-        if (ks > a.groups / 8) ks = a.groups / 8;        // at least eight scale groups per split
-        if (ks > 4) ks = 4;
-        if (ks > 1 && tiles <= kSplitMaxTiles && (size_t)tiles * ks * TM * kTileN * sizeof(float) <= kSplitWsBytes && !sc.failed) {
-            if (!sc.ready) {
-                if (cudaMalloc(&sc.ws, kSplitWsBytes * kSplitTickets) != cudaSuccess ||
-                    cudaMalloc(&sc.counters, sizeof(unsigned) * kSplitMaxTiles * kSplitTickets) != cudaSuccess) {
-                    cudaGetLastError();
-                    sc.failed = true;
-                } else {
-                    cudaMemset(sc.counters, 0, sizeof(unsigned) * kSplitMaxTiles * kSplitTickets);
-                    sc.ready = true;
-                }
-            }
-            if (sc.ready) {
-                const unsigned t = sc.ticket++ % kSplitTickets;
-                a.ws = sc.ws + (size_t)t * (kSplitWsBytes / sizeof(float));
-                a.counters = sc.counters + (size_t)t * kSplitMaxTiles;
-                grid.z = ks;
+    long long best = LLONG_MAX;
+    for (int mt = (a.M + kMaxTm - 1) / kMaxTm, end = mt + 16; mt <= end; mt++) {
+        const int tm = ((a.M + mt - 1) / mt + 15) / 16 * 16;
+        if ((a.M + tm - 1) / tm != mt) continue;
+        const long long stage = 650 + 26 * tm / 10, tiles = (long long)nt * mt;
+        if (tiles > INT_MAX / kMaxSplit) break;
+        for (int c = 1; c <= kMaxSplit; c++) {
+            if (c > 1 && (tiles * c > d.slots[c] || a.groups < 2 * c)) continue;
+            const long long rounds = c > 1 ? 1 : (tiles + d.sms - 1) / d.sms;
+            const long long cost = rounds * ((a.groups + c - 1) / c) * stage + 2000 + 10 * tm + (c > 1 ? 2000 + 4 * tm : 0);
+            if (cost < best) {
+                best = cost;
+                a.mt = mt;
+                a.tm = tm;
+                a.tiles = (int)tiles;
+                a.split = c;
             }
         }
     }
-    gemm_kernel<TM><<<grid, kThreads, Cfg<TM>::kSmem, stream>>>(map, a);
-    return check_launch("gemm_tcgen05");
 }
 
-// A: half [M,K] row-major (16-byte aligned), packed: prepared weights of [N,K], C: half [M,N].
-int launch_gemm_tcgen05(const half* A, const uint8_t* packed, half* C, int M, int N, int K, cudaStream_t stream)
+static bool encode(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType type, const void* base, cuuint64_t inner, cuuint64_t outer,
+                   cuuint64_t stride, int box_inner, int box_outer, CUtensorMapSwizzle swizzle)
+{
+    const cuuint64_t dims[2] = {inner, outer}, strides[1] = {stride};
+    const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer}, estr[2] = {1, 1};
+    return enc(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace gemm
+
+// A: half [M,K] row-major (16-byte aligned), packed: prepared weights, possibly matrices packed back to back (every row
+// count but the last a multiple of 16); out[i]: rows row0 .. row0 + rows of them go to y[M, rows].  glu: one output, of
+// silu(gate) * up, where the up rows lie behind the gate's (rows of the gate a multiple of 16).
+int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out, int nout, bool glu, int M, int K, cudaStream_t stream)
 {
     using namespace gemm;
     EncodeTiledFn enc = encode_fn();
     if (!enc) return fail(TLLM_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from this driver");
     int* err = device_error_flag();
-    if (!err) return fail(TLLM_ERR_LAUNCH, "device scratch unavailable");
-    Args a;
-    a.packed = packed;
-    a.C = C;
+    Device* dev = device();
+    if (!err || !dev) return fail(TLLM_ERR_LAUNCH, "device scratch unavailable");
+    if (nout < 1 || nout > TLLM_MAX_FUSED || (glu && (nout != 1 || out[0].rows % kTileRows)))
+        return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: %d outputs", nout);
+    Args a = {};
+    for (int i = 0; i < TLLM_MAX_FUSED; i++) {
+        if (i < nout) a.out[i] = out[i];
+        else a.out[i].row0 = INT_MAX;
+    }
     a.M = M;
-    a.N = N;
-    a.K = K;
-    a.groups = K / kStageK;
-    a.nrb = (N + kTileRows - 1) / kTileRows;
+    a.N = out[nout - 1].row0 + out[nout - 1].rows;
+    a.groups = K / kGroup;
+    a.glu = glu ? 1 : 0;
+    const int nrb = (a.N + kTileRows - 1) / kTileRows;
+    a.up_rb = nrb;
+    const int tile_out = glu ? kTileN / 2 : kTileN;
+    choose(a, (a.N + tile_out - 1) / tile_out, *dev);
+    if (!a.split) return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: M=%d N=%d K=%d: too many tiles", M, a.N, K);
     a.err = err;
-    a.ws = nullptr;
-    a.counters = nullptr;
-    // token tile: the smallest that holds M, 256 for long prefills
-    if (M <= 32) return launch_tm<32>(enc, A, a, stream);
-    if (M <= 64) return launch_tm<64>(enc, A, a, stream);
-    if (M <= 128) return launch_tm<128>(enc, A, a, stream);
-    return launch_tm<256>(enc, A, a, stream);
+    a.acc_stride = (a.tm + 31) / 32 * 32;
+    a.na = (kTmemCols - 2 * a.acc_stride) / kACols;
+    if (a.na > kMaxA) a.na = kMaxA;
+    a.nb = (int)((kSmem - 1024 - kCodes * kCodeBytes) / (a.tm * kGroup * 2));
+    if (a.nb > kMaxB) a.nb = kMaxB;
+    CUtensorMap map_x, map_w;
+    if (!encode(enc, &map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, A, K, M, (cuuint64_t)K * sizeof(half), kBoxK, a.tm, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode(enc, &map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, packed, (cuuint64_t)a.groups * (kTileBytes / 4), glu ? 2 * nrb : nrb,
+                (cuuint64_t)a.groups * kTileBytes, kTileBytes / 4, glu ? kTileN / kTileRows / 2 : kTileN / kTileRows, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return fail(TLLM_ERR_LAUNCH, "cuTensorMapEncodeTiled failed");
+    const int grid = a.split > 1 ? a.tiles * a.split : (a.tiles < dev->sms ? a.tiles : dev->sms);
+    return launch_pdl_cluster("gemm_tcgen05", gemm_kernel, a.split, dim3((unsigned)grid), dim3(kThreads), kSmem, stream, map_x, map_w, a);
 }
 
 }  // namespace tllm

@@ -305,9 +305,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
 #pragma unroll
                 for (int t = 0; t < 4; t++) cur[t] = *reinterpret_cast<const uint2*>(cp + c.slot * kCodeBytes + t * 16);
                 const uint32_t sbits = *reinterpret_cast<const unsigned short*>(sp + c.slot * kCodeBytes);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(empty_c(c.slot));
-                c.step(kCodes, kSets);
                 // PRMT table of this row: bytes 0,1 = -s (code 0), 2,3 = 0 (code 1), 4,5 = +s (code 2)
                 const uint32_t tab_lo = sbits ^ 0x8000u, tab_hi = sbits;
                 if (g >= na) {
@@ -332,6 +329,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                         }
                     }
                     tmem_st16(a_t + m * 16, r);
+                    if (m == 0) {
+                        // the slot may be refilled now: this store's operands came from every load of it (an arrival behind
+                        // loads still in flight let the next group's codes overtake them)
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(empty_c(c.slot));
+                        c.step(kCodes, kSets);
+                    }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

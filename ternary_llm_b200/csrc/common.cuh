@@ -77,8 +77,8 @@ struct RowsOut {
     half* y;
     int row0, rows;
 };
-// tcgen05 prompt GEMM on prepared weights (gemm_tcgen05.cu); glu: y = silu(gate) * up of [gate|up].
-int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out, int nout, bool glu, int M, int K, cudaStream_t stream);
+// tcgen05 prompt GEMM on prepared weights (gemm_tcgen05.cu).
+int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out, int nout, int M, int K, cudaStream_t stream);
 
 // A few rows on prepared weights (gemm_rows.cu).
 int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream);

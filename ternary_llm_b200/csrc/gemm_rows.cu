@@ -309,7 +309,7 @@ bool linear_takes_rows(int m, int rows, int cols)
 int launch_linear_out(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream)
 {
     if (linear_takes_rows(m, out[nout - 1].row0 + out[nout - 1].rows, cols)) return launch_gemm_rows(packed, x, out, nout, m, cols, stream);
-    return launch_gemm_tcgen05(x, packed, out, nout, false, m, cols, stream);
+    return launch_gemm_tcgen05(x, packed, out, nout, m, cols, stream);
 }
 
 int launch_linear_f16(const uint8_t* packed, const half* x, half* y, int m, int rows, int cols, cudaStream_t stream)

@@ -65,10 +65,9 @@ constexpr int kMaxSplit = 8;
 
 struct Args {
     RowsOut out[TLLM_MAX_FUSED];     // row ranges of the matrix and where they go; unused ones start past every row
-    int M, N, groups;                // tokens; rows of W (of the gate where glu is set); K / 128
+    int M, N, groups;                // tokens; rows of W; K / 128
     int mt, tiles, split;            // token tiles; tiles; CTAs per tile
     int tm, acc_stride, na, nb;      // tokens per tile; columns between accumulators; weight and activation stages
-    int glu, up_rb;                  // rows n and 16 * up_rb + n are gate and up of output n
     int* err;
 };
 
@@ -108,8 +107,6 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ half glu_out(float g, float u) { return __float2half_rn(g / (1.0f + expf(-g)) * u); }
-
 // One lane of a converged warp.
 __device__ __forceinline__ bool elect_one()
 {
@@ -148,7 +145,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     const int it0 = (int)((long long)rank * a.groups / split);                       // scale groups of this CTA
     const int nst = (int)((long long)(rank + 1) * a.groups / split) - it0;
     const int box_bytes = tm * kBoxK * 2, stage_bytes = 2 * box_bytes;
-    const int rb_tile = a.glu ? kTileN / kTileRows / 2 : kTileN / kTileRows;           // row blocks of a tile (of the gate)
+    constexpr int rb_tile = kTileN / kTileRows;                                        // row blocks of a tile
     uint8_t* codes = smem + nb * stage_bytes;
 
     const uint32_t bar0 = smem_u32(bars);
@@ -265,7 +262,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                 if (leader) {
                     mbar_expect_tx(full_c(c.slot), kCodeBytes);
                     tma_load_2d(dst, &map_w, (it0 + it) * (kTileBytes / 4), rb, full_c(c.slot));
-                    if (a.glu) tma_load_2d(dst + kCodeBytes / 2, &map_w, (it0 + it) * (kTileBytes / 4), a.up_rb + rb, full_c(c.slot));
                 }
                 c.step(kCodes);
                 used = min(used + 1, kCodes);
@@ -280,8 +276,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     } else if (warp >= 4 && warp < kOutWarp) {
         // ---------------- expanders ----------------
         const int set = (warp - 4) >> 2, row = (warp & 3) * 32 + lane;
-        // row block of the tile: with glu the quarter's 32 lanes are 16 gate rows and the up rows with the same numbers
-        const int rbl = a.glu ? (warp & 3) + 4 * (lane >> 4) : row >> 4, r16 = row & 15;
+        const int rbl = row >> 4, r16 = row & 15;             // row block of the tile and row inside it
         const int gq = r16 & 7, h = r16 >> 3;
         // this row's code words of MMA lane t: the pair (column halves j2 = 0, 1) at word index
         // (gq*4 + t)*4 + 2h, one 64-bit load per t; each word holds all four 32-column steps
@@ -358,7 +353,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             if (!(ok = __all_sync(0xffffffffu, ok))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int m0 = (tile % a.mt) * tm, mv = min(tm, a.M - m0);
-            const int n = tile / a.mt * rb_tile * kTileRows + (a.glu ? (warp & 3) * 16 + (lane & 15) : row);
+            const int n = tile / a.mt * kTileN + row;
             half* y = a.out[0].y;
             int r0 = 0, rows = a.out[0].rows;
 #pragma unroll
@@ -379,15 +374,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
 #pragma unroll
                     for (int j = 0; j < 32; j++)
                         if (c + j < mv) part[(c + j) * kTileN] = __uint_as_float(v[j]);
-                } else if (a.glu) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 2) {         // lanes below 16: even tokens, the others odd ones
-                        const bool low = lane < 16;
-                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(low ? v[j + 1] : v[j]), 16);
-                        const half o = low ? glu_out(__uint_as_float(v[j]), other) : glu_out(other, __uint_as_float(v[j + 1]));
-                        const int m = c + j + (low ? 0 : 1);
-                        if (m < mv && n < a.N) y[(size_t)m * rows] = o;
-                    }
                 } else if (n < a.N) {
 #pragma unroll
                     for (int j = 0; j < 32; j++)
@@ -411,8 +397,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         const int m0 = (first % a.mt) * tm, mv = min(tm, a.M - m0);
         const int t0 = rank * mv / split, t1 = (rank + 1) * mv / split;
         const int row = lane * 4;
-        const bool up = a.glu && ((lane >> 2) & 1);
-        const int n = first / a.mt * rb_tile * kTileRows + (a.glu ? (lane >> 3) * 16 + (row & 15) : row);
+        const int n = first / a.mt * kTileN + row;
         half* y = a.out[0].y;
         int r0 = 0, rows = a.out[0].rows;
 #pragma unroll
@@ -440,22 +425,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                     v.z += p[z].z;
                     v.w += p[z].w;
                 }
-            half o[4];
-            if (a.glu) {
-                o[0] = glu_out(v.x, __shfl_xor_sync(0xffffffffu, v.x, 4));
-                o[1] = glu_out(v.y, __shfl_xor_sync(0xffffffffu, v.y, 4));
-                o[2] = glu_out(v.z, __shfl_xor_sync(0xffffffffu, v.z, 4));
-                o[3] = glu_out(v.w, __shfl_xor_sync(0xffffffffu, v.w, 4));
-            } else {
-                o[0] = __float2half_rn(v.x);
-                o[1] = __float2half_rn(v.y);
-                o[2] = __float2half_rn(v.z);
-                o[3] = __float2half_rn(v.w);
-            }
+            const half o[4] = {__float2half_rn(v.x), __float2half_rn(v.y), __float2half_rn(v.z), __float2half_rn(v.w)};
             half* yp = y + (size_t)(m0 + t) * rows + (n - r0);
 #pragma unroll
             for (int j = 0; j < 4; j++)
-                if (!up && n + j < a.N && !*abortp) yp[j] = o[j];
+                if (n + j < a.N && !*abortp) yp[j] = o[j];
         }
         cluster_sync();                                      // nobody leaves while its sums are still read
     }
@@ -548,9 +522,8 @@ static bool encode(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType type
 }  // namespace gemm
 
 // A: half [M,K] row-major (16-byte aligned), packed: prepared weights, possibly matrices packed back to back (every row
-// count but the last a multiple of 16); out[i]: rows row0 .. row0 + rows of them go to y[M, rows].  glu: one output, of
-// silu(gate) * up, where the up rows lie behind the gate's (rows of the gate a multiple of 16).
-int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out, int nout, bool glu, int M, int K, cudaStream_t stream)
+// count but the last a multiple of 16); out[i]: rows row0 .. row0 + rows of them go to y[M, rows].
+int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out, int nout, int M, int K, cudaStream_t stream)
 {
     using namespace gemm;
     EncodeTiledFn enc = encode_fn();
@@ -558,8 +531,7 @@ int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out
     int* err = device_error_flag();
     Device* dev = device();
     if (!err || !dev) return fail(TLLM_ERR_LAUNCH, "device scratch unavailable");
-    if (nout < 1 || nout > TLLM_MAX_FUSED || (glu && (nout != 1 || out[0].rows % kTileRows)))
-        return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: %d outputs", nout);
+    if (nout < 1 || nout > TLLM_MAX_FUSED) return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: %d outputs", nout);
     Args a = {};
     for (int i = 0; i < TLLM_MAX_FUSED; i++) {
         if (i < nout) a.out[i] = out[i];
@@ -568,11 +540,8 @@ int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out
     a.M = M;
     a.N = out[nout - 1].row0 + out[nout - 1].rows;
     a.groups = K / kGroup;
-    a.glu = glu ? 1 : 0;
     const int nrb = (a.N + kTileRows - 1) / kTileRows;
-    a.up_rb = nrb;
-    const int tile_out = glu ? kTileN / 2 : kTileN;
-    choose(a, (a.N + tile_out - 1) / tile_out, *dev);
+    choose(a, (a.N + kTileN - 1) / kTileN, *dev);
     if (!a.split) return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: M=%d N=%d K=%d: too many tiles", M, a.N, K);
     a.err = err;
     a.acc_stride = (a.tm + 31) / 32 * 32;
@@ -582,8 +551,8 @@ int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out
     if (a.nb > kMaxB) a.nb = kMaxB;
     CUtensorMap map_x, map_w;
     if (!encode(enc, &map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, A, K, M, (cuuint64_t)K * sizeof(half), kBoxK, a.tm, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !encode(enc, &map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, packed, (cuuint64_t)a.groups * (kTileBytes / 4), glu ? 2 * nrb : nrb,
-                (cuuint64_t)a.groups * kTileBytes, kTileBytes / 4, glu ? kTileN / kTileRows / 2 : kTileN / kTileRows, CU_TENSOR_MAP_SWIZZLE_NONE))
+        !encode(enc, &map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, packed, (cuuint64_t)a.groups * (kTileBytes / 4), nrb,
+                (cuuint64_t)a.groups * kTileBytes, kTileBytes / 4, kTileN / kTileRows, CU_TENSOR_MAP_SWIZZLE_NONE))
         return fail(TLLM_ERR_LAUNCH, "cuTensorMapEncodeTiled failed");
     const int grid = a.split > 1 ? a.tiles * a.split : (a.tiles < dev->sms ? a.tiles : dev->sms);
     return launch_pdl_cluster("gemm_tcgen05", gemm_kernel, a.split, dim3((unsigned)grid), dim3(kThreads), kSmem, stream, map_x, map_w, a);

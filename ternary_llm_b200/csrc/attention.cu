@@ -303,12 +303,13 @@ constexpr int kDecChunk = 64;
 constexpr int kDecMaxItems = 8;       // (head, channel pair) items per thread
 
 struct DecodeArgs {
-    half* q;                   // [n_heads, hd] of the new token, rotated in shared memory only
-    const half* k;             // [n_kv_heads, hd] new key (unrotated)
-    const half* v;             // [n_kv_heads, hd] new value
-    half* k_cache;
+    // one sequence per blockIdx.z
+    half* q;                   // [batch, n_heads, hd] of the new tokens, rotated in shared memory only
+    const half* k;             // [batch, n_kv_heads, hd] new keys (unrotated)
+    const half* v;             // [batch, n_kv_heads, hd] new values
+    half* k_cache;             // [batch, n_kv_heads, kv_len_max, hd]
     half* v_cache;
-    half* out;                 // [n_heads, hd]
+    half* out;                 // [batch, n_heads, hd]
     int n_heads, n_kv_heads, head_dim, kv_len_max;
     int pos;                   // position of the new token (pos_dev overrides)
     const int* pos_dev;
@@ -324,8 +325,19 @@ struct DecodeArgs {
 // quicker on short caches).
 template <bool kLong>
 __global__ void __launch_bounds__(kAttnThreads)
-attention_decode_kernel(const DecodeArgs a)
+attention_decode_kernel(DecodeArgs a)
 {
+    {
+        const size_t b = blockIdx.z, qo = b * a.n_heads * a.head_dim, ko = b * a.n_kv_heads * a.head_dim;
+        a.q += qo;
+        a.out += qo;
+        a.k += ko;
+        a.v += ko;
+        a.k_cache += ko * a.kv_len_max;
+        a.v_cache += ko * a.kv_len_max;
+        a.ws += b * a.n_kv_heads * a.nsplit * (a.n_heads / a.n_kv_heads) * (a.head_dim + 2);
+        a.counters += b * a.n_kv_heads;
+    }
     extern __shared__ __align__(16) float smem[];
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -686,17 +698,17 @@ attention_decode_kernel(const DecodeArgs a)
     }
 }
 
-size_t attention_decode_workspace_bytes(int n_heads, int n_kv_heads, int head_dim, int kv_len_max)
+size_t attention_decode_workspace_bytes(int batch, int n_heads, int n_kv_heads, int head_dim, int kv_len_max)
 {
     const int G = n_heads / n_kv_heads;
     const int nsplit = (kv_len_max + kDecChunk - 1) / kDecChunk;
-    return (size_t)n_kv_heads * nsplit * G * (head_dim + 2) * sizeof(float);
+    return (size_t)batch * n_kv_heads * nsplit * G * (head_dim + 2) * sizeof(float);
 }
 
-// One new token at position pos (or *pos_dev): q [n_heads, hd], k and v [n_kv_heads, hd] as
-// the projections wrote them; the rotated key and the value are appended to the caches.
-// ws: attention_decode_workspace_bytes; counters: n_kv_heads zero-initialised unsigned.
-int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache, half* v_cache, half* out, int n_heads,
+// One new token of each of `batch` sequences at position pos (or *pos_dev): q [batch, n_heads, hd], k and v
+// [batch, n_kv_heads, hd] as the projections wrote them; rotated keys and values are appended to the caches.
+// ws: attention_decode_workspace_bytes; counters: batch * n_kv_heads zero-initialised unsigned.
+int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache, half* v_cache, half* out, int batch, int n_heads,
                             int n_kv_heads, int head_dim, int kv_len_max, int pos, const int* pos_dev, float theta,
                             float* ws, unsigned* counters, cudaStream_t stream)
 {
@@ -722,7 +734,8 @@ int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache
     a.pos = pos;
     a.pos_dev = pos_dev;
     a.theta = theta;
-    a.nsplit = (kv_len_max + kDecChunk - 1) / kDecChunk;
+    // a position known here needs no CTAs beyond it
+    a.nsplit = ((pos_dev ? kv_len_max : pos + 1) + kDecChunk - 1) / kDecChunk;
     a.ws = ws;
     a.counters = counters;
     a.err = device_error_flag();
@@ -739,9 +752,9 @@ int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache
         attr[dev] = true;
     }
     if (a.nsplit > 16)
-        return launch_pdl("attention_decode", attention_decode_kernel<true>, dim3(a.nsplit, n_kv_heads), dim3(kAttnThreads),
+        return launch_pdl("attention_decode", attention_decode_kernel<true>, dim3(a.nsplit, n_kv_heads, batch), dim3(kAttnThreads),
                           smem, stream, a);
-    return launch_pdl("attention_decode", attention_decode_kernel<false>, dim3(a.nsplit, n_kv_heads), dim3(kAttnThreads), smem,
+    return launch_pdl("attention_decode", attention_decode_kernel<false>, dim3(a.nsplit, n_kv_heads, batch), dim3(kAttnThreads), smem,
                       stream, a);
 }
 

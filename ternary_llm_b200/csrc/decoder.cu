@@ -56,8 +56,7 @@ struct LlamaDecoder : Decoder {
     bool fused_ok = false;                     // every layer has concatenated q|k|v and gate|up
     int8_t* xq = nullptr;
     float* xscale = nullptr;
-    float* attn_ws = nullptr;
-    float* attn_ws2 = nullptr;     // split records of the fused single-token attention
+    float* attn_ws = nullptr;      // split records of the attention of single tokens
     unsigned* attn_counters = nullptr;
 
     int forward(const int* tokens, int n, int start_pos, const int* pos_dev, int seq, int batch, cudaStream_t s) override;
@@ -152,6 +151,15 @@ int linear_multi(LlamaDecoder* D, int count, const PackedW* const* w, half* cons
     return TLLM_OK;
 }
 
+// Widest model whose FP16 step makes the norm inside the GEMV: its staging holds the vector and its digits (6 bytes a
+// column) beside a ring, which fits up to 28000 columns; wider ones keep the norm's own launch.
+constexpr int kFusedNormMax = 16384;
+
+// Key/value heads of a lock-step token up to which the attention that splits a cache into ranges of 64 positions and
+// rotates by itself is taken; with more, rotation and ranges of 256 are quicker (a step of the 1B model, 8 heads: 2
+// sequences 1081 -> 916 us, 8: 832 -> 725; 24: 1174, there 1264; four 8B layers, 16 sequences: 550 -> 537).
+constexpr int kSplitHeads = 128;
+
 // One pass of the layer stack.
 //   batch == 0: n tokens of sequence `seq` at positions start_pos.. (pos_dev != nullptr: one
 //               token whose position is read from device memory, start_pos ignored);
@@ -173,9 +181,10 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
 #define TRY(x) do { if ((st = (x)) != TLLM_OK) return st; } while (0)
     TRY(launch_embedding(static_cast<const half*>(c.embedding_table), tokens, D->residual, n, hidden, s));
     half* res_cur = D->residual;
-    if (i8 && D->fused_ok) {
-        // Single token, INT8 activations: norm + quantise and SwiGLU + quantise happen inside the
-        // GEMVs' staging phase (7 launches per layer).  The residual alternates between two
+    if (n == 1 && D->fused_ok && (i8 || hidden <= kFusedNormMax)) {
+        // Single token: norm (INT8: + quantise) and, with INT8 activations, SwiGLU + quantise happen
+        // inside the GEMVs' staging phase, rotation and cache append inside the attention (5 launches
+        // per layer; 6 with FP16 activations).  The residual alternates between two
         // vectors because every CTA of a GEMV reads the old one while CTA 0 writes the new one.
         half* res_next = D->residual2;
         const size_t kvdim = (size_t)c.n_kv_heads * c.head_dim;
@@ -183,22 +192,30 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
             const LayerW& L = D->layers[l];
             const size_t kv_off = (size_t)l * kv_layer + kv_first;
             half *qb = D->qkv1, *kb = qb + qdim, *vb = kb + kvdim, *gb = D->gu1, *ub = gb + inter;
-            if (l == 0) {
-                TRY(launch_gemv_int8_packed_norm(L.qkv.p, res_cur, nullptr, L.attn_norm, nullptr, c.rms_norm_eps, qb,
-                                                 L.qkv.rows, L.qkv.cols, s));
-            } else {
-                TRY(launch_gemv_int8_packed_norm(L.qkv.p, D->ffn_out, res_cur, L.attn_norm, res_next, c.rms_norm_eps, qb,
-                                                 L.qkv.rows, L.qkv.cols, s));
-                std::swap(res_cur, res_next);
-            }
-            TRY(launch_attention_decode(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, c.n_heads,
+            // y = W . norm(a + b) * weight, the sum a + b to res_next
+            auto normed = [&](const PackedW& w, const half* a, const half* b, const half* weight, half* y) {
+                const uint8_t* p[1] = {w.p};
+                half* ys[1] = {y};
+                const int rows[1] = {w.rows};
+                half* out = b ? res_next : nullptr;
+                return i8 ? launch_gemv_int8_packed_norm(w.p, a, b, weight, out, c.rms_norm_eps, y, w.rows, w.cols, s)
+                          : launch_gemv_packed_multi_norm(1, p, ys, rows, w.cols, a, b, weight, out, c.rms_norm_eps, s);
+            };
+            TRY(normed(L.qkv, l ? D->ffn_out : res_cur, l ? res_cur : nullptr, L.attn_norm, qb));
+            if (l) std::swap(res_cur, res_next);
+            TRY(launch_attention_decode(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, 1, c.n_heads,
                                         c.n_kv_heads, c.head_dim, c.max_seq_len, start_pos, pos_dev, c.rope_theta,
-                                        D->attn_ws2, D->attn_counters, s));
-            TRY(launch_gemv_int8_packed_quant(L.o.p, D->attn_out, D->hidden2, L.o.rows, L.o.cols, s));
-            TRY(launch_gemv_int8_packed_norm(L.gate_up.p, D->hidden2, res_cur, L.ffn_norm, res_next, c.rms_norm_eps, gb,
-                                             L.gate_up.rows, L.gate_up.cols, s));
+                                        D->attn_ws, D->attn_counters, s));
+            if (i8) TRY(launch_gemv_int8_packed_quant(L.o.p, D->attn_out, D->hidden2, L.o.rows, L.o.cols, s));
+            else TRY(launch_gemv_packed(L.o.p, D->attn_out, D->hidden2, 1, L.o.rows, L.o.cols, s));
+            TRY(normed(L.gate_up, D->hidden2, res_cur, L.ffn_norm, gb));
             std::swap(res_cur, res_next);
-            TRY(launch_gemv_int8_packed_silu(L.down.p, gb, ub, D->ffn_out, L.down.rows, L.down.cols, s));
+            if (i8) {
+                TRY(launch_gemv_int8_packed_silu(L.down.p, gb, ub, D->ffn_out, L.down.rows, L.down.cols, s));
+            } else {
+                TRY(launch_silu_mul(gb, ub, gb, inter, nullptr, nullptr, s));
+                TRY(launch_gemv_packed(L.down.p, gb, D->ffn_out, 1, L.down.rows, L.down.cols, s));
+            }
         }
     } else
     for (int l = 0; l < c.n_layers; l++) {
@@ -223,14 +240,15 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
             half* y[3] = {qb, kb, vb};
             TRY(linear_multi(D, 3, w, y, D->hidden, i8, n, s, &L.qkv));
         }
-        TRY(launch_rope(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, bsz, seq_n, c.n_heads, c.n_kv_heads,
-                        c.head_dim, start_pos, pos_dev, c.rope_theta, c.max_seq_len, 1, s));
-        if (pos_dev)
-            TRY(launch_attention(qb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, 1, c.n_heads, c.n_kv_heads,
-                                 c.head_dim, 1, 1, c.max_seq_len, pos_dev, D->attn_ws, D->attn_counters, s));
-        else
-            TRY(launch_attention(qb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads,
-                                 c.head_dim, seq_n, start_pos + seq_n, c.max_seq_len, nullptr, D->attn_ws, D->attn_counters, s));
+        if (seq_n == 1 && (bsz == 1 || bsz * c.n_kv_heads <= kSplitHeads)) {        // rotation, append and attention of one token per sequence
+            TRY(launch_attention_decode(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads,
+                                        c.head_dim, c.max_seq_len, start_pos, pos_dev, c.rope_theta, D->attn_ws, D->attn_counters, s));
+        } else {
+            TRY(launch_rope(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, bsz, seq_n, c.n_heads, c.n_kv_heads, c.head_dim, start_pos,
+                            nullptr, c.rope_theta, c.max_seq_len, 1, s));
+            TRY(launch_attention(qb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads, c.head_dim, seq_n,
+                                 start_pos + seq_n, c.max_seq_len, nullptr, D->attn_ws, D->attn_counters, s));
+        }
         if (i8) TRY(launch_quantize_absmax_int8(D->attn_out, D->xq, D->xscale, qdim, s));
         {
             const PackedW* w[1] = {&L.o};
@@ -418,8 +436,12 @@ int tllm_b200_decoder_create_batched(const tllm_b200_model_desc* desc, int flags
     ALLOC(D->dev_alloc(&D->gu1, (size_t)2 * c.intermediate_dim, true));
     ALLOC(D->dev_alloc(&D->xq, maxdim, true));
     ALLOC(D->dev_alloc(&D->xscale, 4, true));
-    ALLOC(D->dev_alloc(&D->attn_ws, attention_workspace_bytes(max_batch, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len) / sizeof(float), true));
-    ALLOC(D->dev_alloc(&D->attn_ws2, attention_decode_workspace_bytes(c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len) / sizeof(float), true));
+    {
+        const size_t a = attention_workspace_bytes(max_batch, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len);
+        const int few = max_batch < kSplitHeads / c.n_kv_heads ? max_batch : kSplitHeads / c.n_kv_heads;
+        const size_t b = attention_decode_workspace_bytes(few < 1 ? 1 : few, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len);
+        ALLOC(D->dev_alloc(&D->attn_ws, (a > b ? a : b) / sizeof(float), true));
+    }
     ALLOC(D->dev_alloc(&D->attn_counters, (size_t)max_batch * c.n_kv_heads, true));
 #undef ALLOC
     if (cudaStreamSynchronize(D->stream) != cudaSuccess)

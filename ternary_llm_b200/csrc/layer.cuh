@@ -46,10 +46,10 @@ bool attention_prompt_supported(const half* q, const half* k_cache, const half* 
 int launch_attention_prompt(const half* q, const half* k_cache, const half* v_cache, half* out, int batch, int n_heads, int n_kv_heads,
                             int head_dim, int seq_len, int kv_len, int kv_len_max, cudaStream_t stream);
 
-// Single-token step: RoPE + cache append + attention in one launch (q is read unrotated and not
+// One token per sequence: RoPE + cache append + attention in one launch (q is read unrotated and not
 // modified; the rotated key and the value go to cache position pos, or *pos_dev).
-size_t attention_decode_workspace_bytes(int n_heads, int n_kv_heads, int head_dim, int kv_len_max);
-int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache, half* v_cache, half* out, int n_heads,
+size_t attention_decode_workspace_bytes(int batch, int n_heads, int n_kv_heads, int head_dim, int kv_len_max);
+int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache, half* v_cache, half* out, int batch, int n_heads,
                             int n_kv_heads, int head_dim, int kv_len_max, int pos, const int* pos_dev, float theta,
                             float* ws, unsigned* counters, cudaStream_t stream);
 

@@ -195,7 +195,7 @@ int launch_rmsnorm(const half* input, const half* weight, half* output, const ha
 // cache position start_pos + token.  start_pos comes from device memory when pos_dev != nullptr.
 // A CTA takes a token (and with few tokens a part of its heads); a thread's pair has one angle in all
 // heads, so power, sine and cosine are computed once per thread, not per (head, pair): those were
-// the time (2000 tokens, 32 + 8 heads of 128: 47 -> 14 us; 49 MB are 8 us).
+// the time (2000 tokens, 32 + 8 heads of 128, behind the projection: 67 -> 35 us a launch; 49 MB are 8 us).
 constexpr int kRopeThreads = 256;
 
 __global__ void __launch_bounds__(kRopeThreads)

@@ -366,18 +366,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             y += (size_t)m0 * rows + (n - r0);
             float* part = reinterpret_cast<float*>(smem) + row;
             const uint32_t d = lane_base + acc.slot * a.acc_stride;
-            for (int c = 0; c < mv; c += 32) {
-                uint32_t v[32];
-                tmem_ld32(d + c, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (split > 1) {
+            if (split > 1) {
+                for (int c = 0; c < mv; c += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(d + c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int j = 0; j < 32; j++)
                         if (c + j < mv) part[(c + j) * kTileN] = __uint_as_float(v[j]);
-                } else if (n < a.N) {
+                }
+            } else {
+                for (int c = 0; c < mv; c += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(d + c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (n >= a.N) continue;
+                    // whole chunks without a test per token, a running pointer: the stores' instructions bound short tiles
+                    // (16384 x 2048, 1000 tokens: 62.5 -> 53.9 us)
+                    half* yc = y + (size_t)c * rows;
+                    if (c + 32 <= mv) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (c + j < mv) y[(size_t)(c + j) * rows] = __float2half_rn(__uint_as_float(v[j]));
+                        for (int j = 0; j < 32; j++, yc += rows) *yc = __float2half_rn(__uint_as_float(v[j]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++, yc += rows)
+                            if (c + j < mv) *yc = __float2half_rn(__uint_as_float(v[j]));
+                    }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

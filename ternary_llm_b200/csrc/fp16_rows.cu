@@ -10,10 +10,11 @@
 //     may take its columns in any order, so the eight halves are slots of two MMAs as they come: MMA
 //     (q, j) contracts, in lane t, the columns 32q + 8t + 4j .. + 3, and the B fragment is the 8-byte piece
 //     of an activation row at the same place.
-//   * Two windows per warp are in flight (8 KB, 128 KB per SM), across the ends of blocks; the first two are
-//     requested before the wait on the previous kernel.  Loads in flight need room in the L1 cache, so this
-//     kernel asks for no more shared memory than its activations need: with the largest part, as its
-//     neighbours ask for it, about 25 KB of L1 remain and the stream stops at 3.7 TB/s whatever else is done.
+//   * Two windows per warp are in flight (8 KB, 128 KB per SM), across the ends of blocks; none is
+//     requested before the wait on the previous kernel, which may be the one that makes W.  Loads in flight
+//     need room in the L1 cache, so this kernel asks for no more shared memory than its activations need: with
+//     the largest part, as its neighbours ask for it, about 25 KB of L1 remain and the stream stops at 3.7 TB/s
+//     whatever else is done.
 //   * All activations lie in shared memory, so that no warp waits for another one.  Rows are padded by 64
 //     bytes: a fragment load touches every bank once.  Activations that do not fit are taken in as many
 //     passes as they need.
@@ -49,7 +50,7 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
 __device__ __forceinline__ uint4 ldg_stream(const half* p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 
@@ -86,10 +87,10 @@ fp16_rows_kernel(const Args a)
     };
     int cb = lb, cw = 0;                             // the window whose turn it is
     at_block();
+    pdl_wait();
     load(wr[0]);
     load(wr[1]);
 
-    pdl_wait();
     const int pieces = a.cols / 8;
     for (int n = 0; n < NB * 8; n++)
         for (int c = tid; c < pieces; c += kThreads) {

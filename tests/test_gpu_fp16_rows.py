@@ -46,3 +46,27 @@ def test_batch_equals_single_sequences(batch):
         assert (got[b].double() - one).norm() <= 1e-2 * one.norm()
     tl.check_device_errors()
     dec.close()
+
+
+@pytest.mark.parametrize("producer", ["gemm", "embedding"])
+def test_matrix_made_by_the_launch_before(producer):
+    """W is a tensor like any other: the operators that can make it let the next launch start early, and
+    that launch reads none of it before they have ended."""
+    rows, cols, k = 4736, 2048, 1024
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(cols, generator=gen, device="cuda").half()
+    a = (0.05 * torch.randn(2, rows, k, generator=gen, device="cuda")).half()
+    b = torch.randn(cols, k, generator=gen, device="cuda").half()
+    table = torch.randn(2 * rows, cols, generator=gen, device="cuda").half()
+    ids = torch.randperm(2 * rows, generator=gen, device="cuda").to(torch.int32).view(2, rows)
+    w, y = torch.zeros(rows, cols, dtype=torch.float16, device="cuda"), torch.empty(2, rows, dtype=torch.float16, device="cuda")
+    for i in range(8):
+        if producer == "gemm":
+            ops.fp16_gemm(a[i & 1], b, w, rows, cols, k)
+        else:
+            ops.embedding_lookup(table, ids[i & 1], w, rows, cols)
+        ops.fp16_gemv(w, x, y[i & 1], rows, cols)
+        want = w.double() @ x.double()
+        # as above
+        bound = cols * 2.0 ** -24 * (w.double().abs() @ x.double().abs()) + 2.0 ** -11 * want.abs() + 2.0 ** -25
+        assert ((y[i & 1].double() - want).abs() <= bound).all(), i

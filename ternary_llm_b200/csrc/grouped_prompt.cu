@@ -14,14 +14,16 @@
 // factor of 2^10, which the division by their sum takes out again: the largest is then between 2^10 and
 // 2^14, and a weight keeps 22 bits in its two parts down to 2^-13 of the largest (below that the parts
 // hold it to 2^-35 of the largest).  A position that a query does not see enters its product with the
-// weight 0, so a NaN or an infinity among the values of such a position in the query's last tile
-// reaches the query.
+// weight 0, which turns a NaN or an infinity among the values of such a position in the query's last tile
+// into a NaN of the query.  FP16 rows that are not finite at the end are therefore computed once more, over the
+// positions that they see alone (visible_row); with finite values this costs a comparison per output.
 //
 // FP16, 32 heads over 8 key/value heads, one launch among others, against the form with a CTA per query
 // and key/value head on the CUDA cores (attention.cu), which read every position once per query: 2000
 // queries 2210 -> 116 us (head size 64), 6733 -> 127 us (128); 300 queries 82 -> 15 and 256 -> 17 us;
 // 2 queries 6.8 -> 6.9 and 9.9 -> 8.2 us; 2 queries behind 1000 positions 35.7 -> 33.3 and 60 -> 36 us.
 // It is taken from two queries on.  All mbarrier waits are bounded (see dense_gemm.cu).
+#include <cfloat>
 #include <type_traits>
 
 #include "launch.cuh"
@@ -64,6 +66,7 @@ template <> struct Operand<half> {
 template <typename T>
 struct PromptArgs {
     T* out;
+    const T *q, *k, *v;                 // FP16: what the maps show, for rows that are computed once more
     int ld_out, per_kv, kv_heads, dim, vdim, n, pos0, chunk, cache_rows;
     int head_rows, k_cols, v_cols;
     float scale2, out_scale;
@@ -109,6 +112,53 @@ __device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.
 __device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+
+// One query by one warp over the positions that it sees, as attention.cu computes it.
+__device__ __forceinline__ void visible_row(const PromptArgs<half>& a, int h, int g, int seq, int qi, int lane)
+{
+    const size_t qo = ((size_t)seq * a.n + qi) * a.ld_out + (size_t)h * a.dim, head = (size_t)(seq * a.kv_heads + g) * a.head_rows * a.dim;
+    const half *kb = a.k + head, *vb = a.v + head;
+    const int len = a.pos0 + qi + 1, pairs = a.dim / 64;          // channel pairs lane, lane + 32 of the output
+    float m = -FLT_MAX, l = 0.f;
+    float2 o[2] = {};
+#pragma unroll 1
+    for (int p0 = 0; p0 < len; p0 += 32) {
+        const bool sees = p0 + lane < len;
+        float s = 0.f;
+#pragma unroll 1
+        for (int d = 0; sees && d < a.dim; d += 8) {
+            const uint4 x = *reinterpret_cast<const uint4*>(a.q + qo + d), y = *reinterpret_cast<const uint4*>(kb + (size_t)(p0 + lane) * a.dim + d);
+            const half2 *xh = reinterpret_cast<const half2*>(&x), *yh = reinterpret_cast<const half2*>(&y);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 u = __half22float2(xh[i]), w = __half22float2(yh[i]);
+                s = fmaf(u.x, w.x, fmaf(u.y, w.y, s));
+            }
+        }
+        s *= a.scale2;
+        const float m_new = fmaxf(m, warp_max(sees ? s : -FLT_MAX)), c = exp2_neg(m - m_new), p = sees ? exp2_neg(s - m_new) : 0.f;
+        l = l * c + p;
+        for (int i = 0; i < pairs; i++) o[i] = make_float2(o[i].x * c, o[i].y * c);
+#pragma unroll 1
+        for (int j = 0; j < min(32, len - p0); j++) {
+            const float pj = __shfl_sync(0xffffffffu, p, j);
+            const half2* vr = reinterpret_cast<const half2*>(vb + (size_t)(p0 + j) * a.dim) + lane;
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                if (i < pairs) {
+                    const float2 w = __half22float2(vr[32 * i]);
+                    o[i].x = fmaf(pj, w.x, o[i].x);
+                    o[i].y = fmaf(pj, w.y, o[i].y);
+                }
+        }
+        m = m_new;
+    }
+    l = warp_sum(l);
+    half2* out = reinterpret_cast<half2*>(a.out + qo) + lane;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        if (i < pairs) out[32 * i] = l > 0.f ? __floats2half2_rn(o[i].x / l, o[i].y / l) : __floats2half2_rn(0.f, 0.f);
+}
 
 enum Bar { kQFull, kKFull, kKEmpty, kVFull, kVEmpty, kSFull, kPReady, kPvDone, kBars };
 
@@ -297,6 +347,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             const bool zeros = std::is_same<T, half>::value && !(l > 0.f);
             const float f = zeros ? 1.f : a.out_scale / l;
             T* op = a.out + ((size_t)seq * a.n + q0 + tid) * a.ld_out + (size_t)h * a.vdim;
+            uint32_t largest = 0;                                             // exponents order infinities and NaN last
 #pragma unroll 1
             for (int c = 0; c < a.vdim; c += 32) {
                 uint32_t o[32];
@@ -308,6 +359,8 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
                 if (tid < nq) {
 #pragma unroll
+                    for (int j = 0; std::is_same<T, half>::value && j < 32; j++) largest = max(largest, o[j] & 0x7fffffffu);
+#pragma unroll
                     for (int j = 0; j < 4; j++) {
                         typename Op::Pair w[4];
 #pragma unroll
@@ -316,6 +369,11 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         *reinterpret_cast<uint4*>(op + c + 8 * j) = *reinterpret_cast<const uint4*>(w);
                     }
                 }
+            }
+            if constexpr (std::is_same<T, half>::value) {
+                __syncwarp();                                                 // the rows' first outputs lie before their second
+                for (uint32_t again = __ballot_sync(0xffffffffu, largest >= 0x7f800000u); again; again &= again - 1)
+                    visible_row(a, h, g, seq, q0 + warp * 32 + __ffs(again) - 1, lane);
             }
         } else {
             abort_flag = 1;
@@ -425,6 +483,9 @@ int launch_attention_prompt(const half* q, const half* k_cache, const half* v_ca
     if ((st = encode(enc, &mv, v_cache, head_dim, rows, head_dim))) return st;
     PromptArgs<half> p = {};
     p.out = out;
+    p.q = q;
+    p.k = k_cache;
+    p.v = v_cache;
     p.ld_out = n_heads * head_dim;
     p.per_kv = n_heads / n_kv_heads;
     p.kv_heads = n_kv_heads;

@@ -59,3 +59,33 @@ def test_scores_far_apart():
         want = exact(q, kc, vc, n)
         err = np.abs(out.cpu().numpy().astype(np.float64) - want)
         assert (err <= 2.0 ** -11 * np.abs(want) + 1e-4).all(), (hot, err.max())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("seq,kv_len", [(2, 2), (9, 140), (128, 128), (200, 333)])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_values_that_are_not_finite_do_not_travel_back(hd, seq, kv_len, value):
+    """A value of one position is in the outputs of the queries that see it and of no other, the queries
+    of its own tile in front of it included."""
+    rng = np.random.default_rng(seq + hd)
+    b, hq, hk, mx = 2, 4, 2, kv_len + 5
+    q = rng.standard_normal((b, seq, hq, hd)).astype(f16)
+    kc, vc = (rng.standard_normal((b, hk, mx, hd)).astype(f16) for _ in range(2))
+    kc[:, :, kv_len:], vc[:, :, kv_len:] = np.nan, np.nan
+    want = exact(q, kc, vc, kv_len)
+    bound = 2.0 ** -11 * np.abs(want) + 2e-5 * np.abs(vc[:, :, :kv_len].astype(np.float64)).max()     # as above
+    for first in (kv_len - 1, kv_len - seq + seq // 2):           # seen by the last query alone, by half of them
+        v, k = vc.copy(), kc.copy()
+        v[1, 1, first, 3] = value
+        if first == kv_len - 1:
+            k[1, 1, first] = value                                # its scores as well
+        out = torch.zeros(q.shape, dtype=torch.float16, device="cuda")
+        ops.attention_forward(*[torch.from_numpy(t).cuda() for t in (q, k, v)], out, b, hq, hk, hd, seq, kv_len, mx)
+        tl.check_device_errors()
+        got = out.cpu().numpy().astype(np.float64)
+        hit = np.zeros(q.shape, dtype=bool)
+        sees = np.arange(seq) >= first - (kv_len - seq)
+        hit[1, sees, 2:] = True if first == kv_len - 1 else np.arange(hd) == 3
+        assert (np.abs(got - want) <= bound)[~hit].all()
+        if first != kv_len - 1:
+            assert ((got[hit] == value) | (np.isnan(got[hit]) & np.isnan(value))).all()

@@ -53,7 +53,7 @@ struct LlamaDecoder : Decoder {
     half *k_cache = nullptr, *v_cache = nullptr;
     half *qkv1 = nullptr, *gu1 = nullptr;      // single-token outputs of the concatenated matrices
     half* residual2 = nullptr;                 // second residual vector of the fused single-token step
-    bool fused_ok = false;                     // every layer has concatenated q|k|v and gate|up
+    bool fused_ok = false;                     // every layer has concatenated q|k|v and gate|up, and norms on 16-byte boundaries
     int8_t* xq = nullptr;
     float* xscale = nullptr;
     float* attn_ws = nullptr;      // split records of the attention of single tokens
@@ -407,8 +407,11 @@ int tllm_b200_decoder_create_batched(const tllm_b200_model_desc* desc, int flags
         }
         if ((st = pack(D, w.o_proj, &L.o, D->stream)) || (st = pack(D, w.down_proj, &L.down, D->stream))) return bail(st);
     }
+    // the GEMVs that make the norm read its weight 16 bytes at a time; its own launch takes any address
+    auto aligned = [](const half* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     D->fused_ok = true;
-    for (const LayerW& L : D->layers) D->fused_ok = D->fused_ok && L.qkv.p && L.gate_up.p;
+    for (const LayerW& L : D->layers)
+        D->fused_ok = D->fused_ok && L.qkv.p && L.gate_up.p && aligned(L.attn_norm) && aligned(L.ffn_norm);
     D->d.layers = nullptr;      // the caller's array is not referenced after this call
     if (!c.lm_head_weight && (st = pack(D, c.lm_head_ternary, &D->lm_head, D->stream))) return bail(st);
 

@@ -102,6 +102,32 @@ def test_batched_lock_step_decode_matches_independent_sequences(batch):
     dec.close()
 
 
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("which", ["attn_norm", "ffn_norm"])
+def test_norm_weights_at_any_address(int8, which):
+    """Norm vectors that are views into a larger buffer, at odd elements of it: prompt, steps and the captured loop."""
+    cfg = cfg_small()
+    model = tf.random_model(cfg, seed=13)
+    ora = LO.Transformer(tf.random_model(cfg, seed=13), int8_decode=int8)
+    layer = model.layers[1]
+    buf = torch.zeros(cfg.hidden_dim + 8, dtype=torch.float16, device="cuda")
+    buf[3:3 + cfg.hidden_dim] = torch.from_numpy(np.array(layer[which])).cuda()
+    layer[which] = buf[3:3 + cfg.hidden_dim]
+    assert layer[which].data_ptr() % 16
+    dec = tl.Decoder(model, int8_decode=int8)
+    t = toks(12, cfg.vocab_size)
+    assert close(dec.forward(torch.from_numpy(t[:9]).cuda(), 0).float().cpu().numpy(), ora.forward(list(t[:9]), 0), 2e-2)
+    for i in range(9, 12):
+        got = dec.forward(torch.from_numpy(t[i:i + 1]).cuda(), i).float().cpu().numpy()
+        assert close(got, ora.forward([int(t[i])], i), 4e-2), f"step {i}"
+    want, tok = [], int(got.argmax())
+    for i in range(12, 16):
+        want.append(int(dec.forward(torch.tensor([tok if not want else want[-1]], dtype=torch.int32, device="cuda"), i).argmax()))
+    assert dec.generate(tok, 12, 4)[0] == want
+    tl.check_device_errors()
+    dec.close()
+
+
 def test_generate_replays_the_same_steps_as_forward():
     cfg = cfg_small(n_layers=3, max_seq_len=320)
     model = tf.random_model(cfg, seed=3)

@@ -388,7 +388,7 @@ int launch_embedding(const half* table, const int* indices, half* out, int n_tok
 // FP16 GEMV   y[r] = half(sum_c float(W[r, c]) * float(x[c]))    reference: kernels/elementwise.cu:158-201
 // ---------------------------------------------------------------------------
 // The lm_head of the 1B configuration is 525 MB of FP16, twice the ternary bytes of the
-// whole layer stack; columns in whole windows go to the tensor cores (fp16_rows.cu).  For the
+// whole layer stack; many rows of whole windows of columns go to the tensor cores (fp16_rows.cu).  For the
 // other shapes: x is staged in shared memory once per CTA, each warp streams whole rows with
 // 128-bit loads where the alignment allows, four loads in flight per lane, FP32 accumulation.
 constexpr int kFp16GemvWarps = 8;
@@ -452,7 +452,10 @@ int launch_fp16_gemv(const half* w, const half* x, half* y, int rows, int cols, 
     if (rows == 0) return TLLM_OK;
     const size_t smem = (size_t)cols * sizeof(half);
     if (smem > 200 * 1024) return fail(TLLM_ERR_SHAPE, "fp16_gemv: cols=%d exceeds %d", cols, 100 * 1024);
-    if (fp16_rows_supported(w, x, cols)) return launch_fp16_rows(w, x, y, 1, rows, cols, stream);
+    // The tensor-core form gives a warp 16 whole rows: up to 8192 rows leave most warps idle, and columns beyond 12288 leave its loads
+    // no room in the L1 cache.  us, here / there: 2048 x 2048 6.6 / 9.7, 4096 x 8192 24.6 / 37.4, 8192 x 4096 21.7 / 21.3 (behind a
+    // decoder's layer 46.7 / 50.2), 12288 x 4096 27.3 / 24.6, 16384 x 12288 84 / 79, 16384 x 14336 99 / 161.
+    if (rows > 8192 && cols <= 12288 && fp16_rows_supported(w, x, cols)) return launch_fp16_rows(w, x, y, 1, rows, cols, stream);
     static bool attr[64] = {};
     static int sms[64] = {};
     int dev = 0;
@@ -537,6 +540,7 @@ int launch_fp16_gemv_batched(const half* w, const half* x, half* y, int batch, i
     if (batch == 1) return launch_fp16_gemv(w, x, y, rows, cols, stream);
     const size_t smem = (size_t)kFp16GemvVecs * cols * sizeof(half);
     if (smem > 200 * 1024) return fail(TLLM_ERR_SHAPE, "fp16_gemv (batched): cols=%d exceeds %d", cols, 200 * 1024 / 16);
+    // any number of rows: 4096 x 4096 behind a layer, 2 vectors 78 / 69 us, 8 110 / 50, 24 272 / 65
     if (fp16_rows_supported(w, x, cols)) return launch_fp16_rows(w, x, y, batch, rows, cols, stream);
     static bool attr[64] = {};
     static int sms[64] = {};

@@ -1,5 +1,5 @@
-"""The dense FP16 head on the tensor cores (csrc/fp16_rows.cu): edges of the 16-row blocks, odd and even
-numbers of 128-column windows, one vector and batches that fill one, two and more column blocks of the MMA
+"""The dense FP16 head on the tensor cores (csrc/fp16_rows.cu) and, up to 8192 rows of one vector, on the CUDA
+cores: edges of the 16-row blocks, odd and even numbers of 128-column windows, one vector and batches that fill one, two and more column blocks of the MMA
 or need a second pass, against 64 bits."""
 import numpy as np
 import pytest
@@ -12,7 +12,7 @@ from ternary_llm_b200 import tllm_format as tf
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 15, 17, 2400, 40001])
+@pytest.mark.parametrize("rows", [1, 15, 17, 2400, 8192, 8193, 40001])
 @pytest.mark.parametrize("cols", [128, 384, 2048, 14336])
 def test_one_vector(rows, cols):
     gen = torch.Generator(device="cuda").manual_seed(rows + cols)
@@ -68,7 +68,7 @@ def test_products_of_one_sign(cols):
 def test_matrix_made_by_the_launch_before(producer):
     """W is a tensor like any other: the operators that can make it let the next launch start early, and
     that launch reads none of it before they have ended."""
-    rows, cols, k = 4736, 2048, 1024
+    rows, cols, k = 12304, 2048, 1024
     gen = torch.Generator(device="cuda").manual_seed(1)
     x = torch.randn(cols, generator=gen, device="cuda").half()
     a = (0.05 * torch.randn(2, rows, k, generator=gen, device="cuda")).half()

@@ -86,7 +86,7 @@ int tllm_b200_rope(void* q, void* k, int batch, int seq_len, int n_heads, int n_
     if (st || (st = check_device())) return st;
     if (misaligned(q, 4) || misaligned(k, 4)) return fail(TLLM_ERR_ALIGN, "rope: q and k must be 4-byte aligned");
     return launch_rope((half*)q, (half*)k, nullptr, nullptr, nullptr, batch, seq_len, n_heads, n_kv_heads, head_dim,
-                       start_pos, nullptr, theta, 0, 1, S(stream));
+                       start_pos, theta, 0, 1, S(stream));
 }
 
 int tllm_b200_copy_to_kv_cache(const void* k, const void* v, void* k_cache, void* v_cache, int batch, int n_kv_heads,
@@ -98,7 +98,7 @@ int tllm_b200_copy_to_kv_cache(const void* k, const void* v, void* k_cache, void
     if (misaligned(k, 4) || misaligned(v, 4) || misaligned(k_cache, 4) || misaligned(v_cache, 4))
         return fail(TLLM_ERR_ALIGN, "copy_to_kv_cache: pointers must be 4-byte aligned");
     return launch_rope(nullptr, (half*)k, (const half*)v, (half*)k_cache, (half*)v_cache, batch, seq_len, 0, n_kv_heads,
-                       head_dim, start_pos, nullptr, 1.0f, max_seq_len, 0, S(stream));
+                       head_dim, start_pos, 1.0f, max_seq_len, 0, S(stream));
 }
 
 int tllm_b200_rope_append(void* q, void* k, const void* v, void* k_cache, void* v_cache, int batch, int seq_len,
@@ -111,7 +111,7 @@ int tllm_b200_rope_append(void* q, void* k, const void* v, void* k_cache, void* 
     if (misaligned(q, 4) || misaligned(k, 4) || misaligned(v, 4) || misaligned(k_cache, 4) || misaligned(v_cache, 4))
         return fail(TLLM_ERR_ALIGN, "rope_append: pointers must be 4-byte aligned");
     return launch_rope((half*)q, (half*)k, (const half*)v, (half*)k_cache, (half*)v_cache, batch, seq_len, n_heads,
-                       n_kv_heads, head_dim, start_pos, nullptr, theta, max_seq_len, 1, S(stream));
+                       n_kv_heads, head_dim, start_pos, theta, max_seq_len, 1, S(stream));
 }
 
 int tllm_b200_attention(const void* q, const void* k_cache, const void* v_cache, void* output, int batch, int n_heads,

@@ -245,7 +245,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
                                         c.head_dim, c.max_seq_len, start_pos, pos_dev, c.rope_theta, D->attn_ws, D->attn_counters, s));
         } else {
             TRY(launch_rope(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, bsz, seq_n, c.n_heads, c.n_kv_heads, c.head_dim, start_pos,
-                            nullptr, c.rope_theta, c.max_seq_len, 1, s));
+                            c.rope_theta, c.max_seq_len, 1, s));
             TRY(launch_attention(qb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads, c.head_dim, seq_n,
                                  start_pos + seq_n, c.max_seq_len, nullptr, D->attn_ws, D->attn_counters, s));
         }

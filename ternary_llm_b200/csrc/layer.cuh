@@ -10,11 +10,9 @@ namespace tllm {
 // add-then-normalise sequence computes) instead of the unrounded one.
 int launch_rmsnorm(const half* input, const half* weight, half* output, const half* residual, half* residual_out,
                    int8_t* q, float* q_scale, int batch, int dim, float eps, int round_first, cudaStream_t stream);
-// pos_dev: start_pos is read from device memory when not null.  Caches may be null (rotation
-// only); do_rope == 0 appends without rotating.
+// Caches may be null (rotation only); do_rope == 0 appends without rotating.
 int launch_rope(half* q, half* k, const half* v, half* k_cache, half* v_cache, int batch, int seq_len, int n_heads,
-                int n_kv_heads, int head_dim, int start_pos, const int* pos_dev, float theta, int max_seq_len,
-                int do_rope, cudaStream_t stream);
+                int n_kv_heads, int head_dim, int start_pos, float theta, int max_seq_len, int do_rope, cudaStream_t stream);
 // q / q_scale not null: one vector, output also quantised.
 int launch_silu_mul(const half* gate, const half* up, half* out, long long size, int8_t* q, float* q_scale,
                     cudaStream_t stream);

@@ -9,6 +9,7 @@
 // launch, and positions / scales read from device memory so that a whole decode step
 // replays as one CUDA graph without a host round trip.
 #include <cfloat>
+#include <climits>
 
 #include "launch.cuh"
 #include "layer.cuh"
@@ -192,67 +193,81 @@ int launch_rmsnorm(const half* input, const half* weight, half* output, const ha
 //   [batch, n_kv_heads, max_seq_len, head_dim], positions beyond the cache dropped)
 // ---------------------------------------------------------------------------
 // q and k are rotated in place; when caches are given the rotated k pair and the v pair of kv heads go to
-// cache position start_pos + token.  start_pos comes from device memory when pos_dev != nullptr.
-// A CTA takes a token (and with few tokens a part of its heads); a thread's pair has one angle in all
-// heads, so power, sine and cosine are computed once per thread, not per (head, pair): those were
-// the time (2000 tokens, 32 + 8 heads of 128, behind the projection: 67 -> 35 us a launch; 49 MB are 8 us).
+// cache position start_pos + token.
+// A thread's pair has one angle in all heads, and power, sine and cosine are the time as soon as there are more threads than run at
+// once.  So a thread takes as many heads as it needs for all threads to run at once, up to 24, and where that is not enough a third
+// of up to 48 heads or 16.  us a launch, a thread per (head, pair) / now: 32 + 8 heads of 128, 24 tokens 2.1 / 2.0, 300: 7.0 / 4.0, 600:
+// 13.4 / 5.5, 2000: 42.9 / 14.8 (98 MB read and written: 15 at the copy rate); 32 + 8 of 64, 300: 4.0 / 3.5, 2000: 22.8 / 8.5; 64 + 8
+// of 128, 100: 4.9 / 3.4, 2000: 82.7 / 22.3 (16 heads a thread in one CTA a token: 20.6, but 300 tokens 14.8 in place of 5.0).
 constexpr int kRopeThreads = 256;
+constexpr long long kRopeResident = 148 * 1536;      // threads at the same time
 
+template <bool kMany>
 __global__ void __launch_bounds__(kRopeThreads)
 rope_kernel(half* __restrict__ q, half* __restrict__ k, const half* __restrict__ v, half* __restrict__ k_cache,
-            half* __restrict__ v_cache, int seq_len, int n_heads, int n_kv_heads, int head_dim,
-            int start_pos, const int* __restrict__ pos_dev, float theta, int max_seq_len, int do_rope)
+            half* __restrict__ v_cache, int batch, int seq_len, int n_heads, int n_kv_heads, int head_dim,
+            int start_pos, float theta, int max_seq_len, int do_rope, int slots)
 {
     pdl_launch_dependents();
-    const int half_dim = head_dim >> 1, lanes = max(1, kRopeThreads / half_dim);
-    const int b = blockIdx.x / seq_len, s = blockIdx.x - b * seq_len;
+    const int half_dim = head_dim >> 1;
     const int max_heads = max(n_heads, n_kv_heads);
-    for (int i = threadIdx.x; i < half_dim * lanes; i += kRopeThreads) {
-        const int pair = i % half_dim;
-        const float freq = 1.0f / powf(theta, (2.0f * (float)pair) / (float)head_dim);
-        pdl_wait();
-        const int pos = (pos_dev ? *pos_dev : start_pos) + s;
-        float sn = 0.f, cs = 1.f;
-        if (do_rope) sincosf((float)pos * freq, &sn, &cs);
-        auto turn = [&](half2 h) {
-            const float2 x = __half22float2(h);
-            return __halves2half2(__float2half_rn(x.x * cs - x.y * sn), __float2half_rn(x.x * sn + x.y * cs));
-        };
-#pragma unroll 4
-        for (int head = i / half_dim + blockIdx.y * lanes; head < max_heads; head += lanes * gridDim.y) {
-            if (head < n_heads && do_rope) {
-                half2* p = reinterpret_cast<half2*>(q + ((size_t)blockIdx.x * n_heads + head) * head_dim) + pair;
-                *p = turn(*p);
+    const long long idx = (long long)blockIdx.x * kRopeThreads + threadIdx.x;
+    if (idx >= (long long)batch * seq_len * slots * half_dim) return;
+    int pair, slot, b, pos;
+    size_t t;                                         // token
+    auto place = [&](auto i) {
+        pair = (int)(i % half_dim);
+        i /= half_dim;
+        slot = (int)(i % slots);
+        i /= slots;
+        t = i;
+        b = (int)(i / seq_len);
+        pos = start_pos + (int)(i % seq_len);
+    };
+    if (gridDim.x <= INT_MAX / kRopeThreads) place((unsigned)idx);        // divisions of 32 bits
+    else place((unsigned long long)idx);
+    const float freq = 1.0f / powf(theta, (2.0f * (float)pair) / (float)head_dim);
+    float sn = 0.f, cs = 1.f;
+    if (do_rope) sincosf((float)pos * freq, &sn, &cs);
+    pdl_wait();
+    auto turn = [&](half2 h) {
+        const float2 x = __half22float2(h);
+        return __halves2half2(__float2half_rn(x.x * cs - x.y * sn), __float2half_rn(x.x * sn + x.y * cs));
+    };
+#pragma unroll(kMany ? 4 : 1)
+    for (int head = slot; head < (kMany ? max_heads : slot + 1); head += slots) {
+        if (head < n_heads && do_rope) {
+            half2* p = reinterpret_cast<half2*>(q + (t * n_heads + head) * head_dim) + pair;
+            *p = turn(*p);
+        }
+        if (head < n_kv_heads) {
+            const size_t src = (t * n_kv_heads + head) * head_dim;
+            half2 kr = *(reinterpret_cast<const half2*>(k + src) + pair);
+            if (do_rope) {
+                kr = turn(kr);
+                *(reinterpret_cast<half2*>(k + src) + pair) = kr;
             }
-            if (head < n_kv_heads) {
-                const size_t src = ((size_t)blockIdx.x * n_kv_heads + head) * head_dim;
-                half2 kr = *(reinterpret_cast<const half2*>(k + src) + pair);
-                if (do_rope) {
-                    kr = turn(kr);
-                    *(reinterpret_cast<half2*>(k + src) + pair) = kr;
-                }
-                if (k_cache && pos < max_seq_len) {
-                    const size_t dst = (((size_t)b * n_kv_heads + head) * max_seq_len + pos) * head_dim;
-                    *(reinterpret_cast<half2*>(k_cache + dst) + pair) = kr;
-                    *(reinterpret_cast<half2*>(v_cache + dst) + pair) = *(reinterpret_cast<const half2*>(v + src) + pair);
-                }
+            if (k_cache && pos < max_seq_len) {
+                const size_t dst = (((size_t)b * n_kv_heads + head) * max_seq_len + pos) * head_dim;
+                *(reinterpret_cast<half2*>(k_cache + dst) + pair) = kr;
+                *(reinterpret_cast<half2*>(v_cache + dst) + pair) = *(reinterpret_cast<const half2*>(v + src) + pair);
             }
         }
     }
 }
 
 int launch_rope(half* q, half* k, const half* v, half* k_cache, half* v_cache, int batch, int seq_len, int n_heads,
-                int n_kv_heads, int head_dim, int start_pos, const int* pos_dev, float theta, int max_seq_len,
-                int do_rope, cudaStream_t stream)
+                int n_kv_heads, int head_dim, int start_pos, float theta, int max_seq_len, int do_rope, cudaStream_t stream)
 {
     const int max_heads = n_heads > n_kv_heads ? n_heads : n_kv_heads;
-    const long long tokens = (long long)batch * seq_len;
-    if (tokens == 0 || max_heads == 0 || head_dim < 2) return TLLM_OK;
-    const int lanes = head_dim / 2 < kRopeThreads ? kRopeThreads / (head_dim / 2) : 1;
-    int parts = tokens < 592 ? (max_heads + lanes - 1) / lanes : 1;          // four CTAs per SM without parts
-    if (parts > 65535) parts = 65535;
-    return launch_pdl("rope", rope_kernel, dim3((unsigned)tokens, parts), dim3(kRopeThreads), 0, stream, q, k, v, k_cache, v_cache, seq_len,
-                      n_heads, n_kv_heads, head_dim, start_pos, pos_dev, theta, max_seq_len, do_rope);
+    const long long pairs = (long long)batch * seq_len * (head_dim / 2);
+    if (pairs * max_heads == 0) return TLLM_OK;
+    long long slots = kRopeResident / pairs;
+    if (slots < (max_heads + 23) / 24) slots = max_heads > 48 ? (max_heads + 15) / 16 : 3;
+    if (slots > max_heads) slots = max_heads;
+    const unsigned grid = (unsigned)((pairs * slots + kRopeThreads - 1) / kRopeThreads);
+    return launch_pdl("rope", slots < max_heads ? rope_kernel<true> : rope_kernel<false>, dim3(grid), dim3(kRopeThreads), 0, stream, q, k, v, k_cache,
+                      v_cache, batch, seq_len, n_heads, n_kv_heads, head_dim, start_pos, theta, max_seq_len, do_rope, (int)slots);
 }
 
 // ---------------------------------------------------------------------------

@@ -94,6 +94,21 @@ def test_rope_and_cache_append(seq, start, hq, hk, hd):
         assert np.abs(host(q3).astype(np.float32) - host(qd).astype(np.float32)).max() <= 2e-2
 
 
+@pytest.mark.parametrize("n,hq,hk,hd", [(110, 32, 8, 128), (112, 32, 8, 128), (600, 12, 12, 96), (1200, 32, 8, 128), (1900, 5, 1, 64), (4000, 64, 8, 64)])
+def test_rope_of_many_tokens_is_that_of_few(n, hq, hk, hd):
+    """A thread takes one head of few tokens and up to 24 of many: the same arithmetic, to the last bit."""
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    q, k, v = (torch.randn(n, h, hd, generator=gen, device=DEV).half() for h in (hq, hk, hk))
+    whole, parts = ([q.clone(), k.clone()] + [torch.zeros(hk, n, hd, dtype=torch.float16, device=DEV) for _ in range(2)] for _ in range(2))
+    ops.rope_append(whole[0], whole[1], v, whole[2], whole[3], 1, n, hq, hk, hd, 0, 1e4, n)
+    for i in range(0, n, 50):
+        m = min(50, n - i)
+        ops.rope_append(parts[0][i:i + m], parts[1][i:i + m], v[i:i + m], parts[2], parts[3], 1, m, hq, hk, hd, i, 1e4, n)
+    for a, b in zip(whole, parts):
+        assert torch.equal(a, b)
+    assert not torch.equal(whole[0], q)
+
+
 def test_cache_append_drops_positions_past_the_end():
     b, hk, hd, mx = 1, 2, 64, 8
     k = torch.ones((b, 4, hk, hd), dtype=torch.float16, device=DEV)

@@ -780,7 +780,7 @@ int launch_attention(const half* q, const half* k_cache, const half* v_cache, ha
                     head_dim, G);
     if (!kv_len_dev && (kv_len < seq_len || kv_len > kv_len_max))
         return fail(TLLM_ERR_SHAPE, "attention: kv_len=%d seq_len=%d kv_len_max=%d", kv_len, seq_len, kv_len_max);
-    if (!kv_len_dev && attention_prompt_supported(q, k_cache, v_cache, out, batch, n_kv_heads, head_dim, seq_len, kv_len_max))
+    if (!kv_len_dev && attention_prompt_supported(q, k_cache, v_cache, out, batch, n_heads, n_kv_heads, head_dim, seq_len, kv_len, kv_len_max))
         return launch_attention_prompt(q, k_cache, v_cache, out, batch, n_heads, n_kv_heads, head_dim, seq_len, kv_len, kv_len_max, stream);
     AttnArgs a = {};
     a.q = q;

@@ -21,8 +21,8 @@
 // FP16, 32 heads over 8 key/value heads, one launch among others, against the form with a CTA per query
 // and key/value head on the CUDA cores (attention.cu), which read every position once per query: 2000
 // queries 2210 -> 116 us (head size 64), 6733 -> 127 us (128); 300 queries 82 -> 15 and 256 -> 17 us;
-// 2 queries 6.8 -> 6.9 and 9.9 -> 8.2 us; 2 queries behind 1000 positions 35.7 -> 33.3 and 60 -> 36 us.
-// It is taken from two queries on.  All mbarrier waits are bounded (see dense_gemm.cu).
+// 2 queries behind 1000 positions 35.7 -> 33.3 and 60 -> 36 us.  few_queries has the calls that stay there.
+// All mbarrier waits are bounded (see dense_gemm.cu).
 #include <cfloat>
 #include <type_traits>
 
@@ -39,7 +39,6 @@ using namespace gemm;
 
 constexpr int kTile = 128, kThreads = 192;
 constexpr int kBlock = kTile * 128;                 // bytes of 64 columns of a tile: 128-byte rows
-constexpr int kMinQueries = 2;                      // FP16; one query splits the positions (attention.cu)
 constexpr uint32_t kTmemCols = 256;                 // S and the weights: 128, O: 128
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -460,11 +459,31 @@ int launch_grouped_prompt_tcgen05(const GroupedArgs<bf16>& a, cudaStream_t strea
     return launch(p, mq, mk, mv, a.heads, 1, stream);
 }
 
-bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_kv_heads, int head_dim,
-                                int seq_len, int kv_len_max)
+// Few queries over few channels: a CTA per query and key/value head on the CUDA cores (attention.cu) is quicker than a tile of
+// 128 queries.  Its chunk of 256 positions grows with the channels of a group (one head of 64: 5.7 us, two 6.2, four 8.2; one
+// of 128: 8.1), a pair of tiles here takes 6.7 (64) and 7.8 us (128), and the launch around them 1 to 1.5 us more.  So it stays
+//   * while its CTAs run at the same time: three an SM, of head size 128 one;
+//   * up to 32 positions (2 or 3 queries: 64), where the launch is all: four heads of 64, 2 queries of 8 sequences: 7.2, here 9.1;
+//   * never up to 128 positions, one tile here: one head, 8 queries behind 100: 6.8, here 6.2;
+//   * up to 256 positions, one chunk there and two tiles here: three heads, 8 queries behind 200: 9.3, here 10.6;
+//   * behind more for one or two heads of 64 alone: 8 queries behind 1000: 26.4 and 28.4, here 29.8 and 31.4; three heads,
+//     8 queries: 31.8, here 32.2; and while an SM has one CTA: 32 x 1 heads, 4 queries: 30.2, here 32.7; 5: 35, here 32.6.
+static bool few_queries(int batch, int group, int n_kv_heads, int head_dim, int seq_len, int kv_len)
 {
-    // rows of a map are addressed with 32-bit coordinates
-    return (head_dim == 64 || head_dim == 128) && seq_len >= kMinQueries && (long long)batch * n_kv_heads * kv_len_max < (1ll << 30) &&
+    const long long ctas = (long long)batch * n_kv_heads * seq_len;
+    const int channels = group * head_dim;
+    if ((seq_len > 12 && seq_len * group > 16) || ctas > (head_dim == 64 ? 444 : 148) || channels > 256) return false;
+    if (kv_len > 256) return head_dim == 64 && channels <= 128 && ctas <= 128;
+    if (kv_len > (seq_len <= 3 ? 64 : 32) && kv_len <= 128) return false;
+    return (head_dim == 64 || group == 1) && (channels <= 192 || (kv_len <= 32 && seq_len <= 8));
+}
+
+bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_heads, int n_kv_heads,
+                                int head_dim, int seq_len, int kv_len, int kv_len_max)
+{
+    // rows of a map are addressed with 32-bit coordinates; one query splits the positions (attention.cu)
+    return (head_dim == 64 || head_dim == 128) && seq_len >= 2 && !few_queries(batch, n_heads / n_kv_heads, n_kv_heads, head_dim, seq_len, kv_len) &&
+           (long long)batch * n_kv_heads * kv_len_max < (1ll << 30) &&
            (long long)batch * seq_len < (1ll << 30) && batch <= 65535 &&
            ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) |
              reinterpret_cast<uintptr_t>(out)) & 15) == 0;

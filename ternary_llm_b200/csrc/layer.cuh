@@ -38,9 +38,9 @@ int launch_attention(const half* q, const half* k_cache, const half* v_cache, ha
                      int n_kv_heads, int head_dim, int seq_len, int kv_len, int kv_len_max, const int* kv_len_dev,
                      float* ws, unsigned* counters, cudaStream_t stream);
 
-// Several queries on tcgen05 (grouped_prompt.cu); launch_attention takes it where it is supported.
-bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_kv_heads, int head_dim,
-                                int seq_len, int kv_len_max);
+// Several queries on tcgen05 (grouped_prompt.cu); launch_attention takes it where it is supported and quicker.
+bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_heads, int n_kv_heads,
+                                int head_dim, int seq_len, int kv_len, int kv_len_max);
 int launch_attention_prompt(const half* q, const half* k_cache, const half* v_cache, half* out, int batch, int n_heads, int n_kv_heads,
                             int head_dim, int seq_len, int kv_len, int kv_len_max, cudaStream_t stream);
 

@@ -46,6 +46,23 @@ def test_prompt_attention(b, hq, hk, hd, seq, kv_len, mx):
     assert (err <= 2.0 ** -11 * np.abs(want) + 2e-5 * np.abs(vc[:, :, :kv_len].astype(np.float64)).max()).all(), err.max()
 
 
+@pytest.mark.parametrize("b,hq,hk,hd,seq,kv_len", [
+    (1, 8, 8, 64, 16, 16), (1, 8, 8, 64, 17, 17), (1, 16, 8, 64, 12, 300), (1, 16, 8, 64, 13, 300), (1, 4, 4, 64, 3, 64), (1, 4, 4, 64, 3, 65),
+    (1, 4, 4, 64, 4, 32), (1, 4, 4, 64, 4, 33), (1, 6, 2, 64, 5, 128), (1, 6, 2, 64, 5, 129), (1, 6, 2, 64, 5, 256), (1, 6, 2, 64, 5, 257),
+    (1, 4, 4, 128, 5, 256), (1, 4, 4, 128, 5, 257), (1, 8, 2, 64, 8, 8), (1, 8, 2, 64, 9, 9), (2, 32, 32, 64, 2, 300), (2, 32, 32, 64, 3, 300),
+    (8, 28, 7, 64, 7, 7), (8, 32, 8, 64, 7, 7)])
+def test_both_sides_of_the_lines_for_few_queries(b, hq, hk, hd, seq, kv_len):
+    """Few queries stay with the form on the CUDA cores up to lines of their own; on either side of each the result is the same."""
+    rng = np.random.default_rng(seq + kv_len)
+    q, kc, vc = (rng.standard_normal(s).astype(f16) for s in ((b, seq, hq, hd), (b, hk, kv_len, hd), (b, hk, kv_len, hd)))
+    out = torch.zeros(q.shape, dtype=torch.float16, device="cuda")
+    ops.attention_forward(*[torch.from_numpy(t).cuda() for t in (q, kc, vc)], out, b, hq, hk, hd, seq, kv_len, kv_len)
+    tl.check_device_errors()
+    want = exact(q, kc, vc, kv_len)
+    # as above
+    assert (np.abs(out.cpu().numpy().astype(np.float64) - want) <= 2.0 ** -11 * np.abs(want) + 2e-5 * np.abs(vc.astype(np.float64)).max()).all()
+
+
 def test_scores_far_apart():
     """One position's score far above the others', first, last or in between: the running maximum
     moves, and the weights of the others are nothing."""

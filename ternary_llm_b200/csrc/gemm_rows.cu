@@ -30,6 +30,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kStages = 3;
+constexpr int kRowWarps = 2, kGroupWarps = 4;        // RG and KW
 
 struct RowsArgs {
     const uint8_t* packed;
@@ -241,25 +242,40 @@ gemm_rows_kernel(const RowsArgs a)
     }
 }
 
-template <int NB, int RG, int KW>
+// CTAs that run at the same time on the current device, two per SM; 0 without one.
+int cta_slots()
+{
+    static int sms[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+    return 2 * sms[dev];
+}
+
+// CTAs that share the scale groups of a tile: as many, a power of two, as run at the same time and have two of them per warp.
+int split_of(int tiles, int groups, int slots)
+{
+    int split = 1;
+    while (split < 8 && tiles * split * 2 <= slots && groups >= split * 2 * kGroupWarps) split *= 2;
+    return split;
+}
+
+template <int NB>
 int launch(RowsArgs a, cudaStream_t stream)
 {
-    using S = Shape<NB, RG, KW>;
+    using S = Shape<NB, kRowWarps, kGroupWarps>;
+    auto kernel = gemm_rows_kernel<NB, kRowWarps, kGroupWarps>;
     static bool attr[64] = {};
-    static int sms[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
     if (!attr[dev]) {
-        cudaFuncSetAttribute(gemm_rows_kernel<NB, RG, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
-        cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
         attr[dev] = true;
     }
-    const int tiles = (a.nrb + RG * S::kR - 1) / (RG * S::kR), slots = 2 * sms[dev];
-    a.split = 1;
-    while (a.split < 8 && tiles * a.split * 2 <= slots && a.groups >= a.split * 2 * KW) a.split *= 2;
-    return launch_pdl_cluster("gemm_rows", gemm_rows_kernel<NB, RG, KW>, a.split, dim3((unsigned)(tiles * a.split)), dim3(kThreads),
-                              S::kSmem, stream, a);
+    const int tiles = (a.nrb + S::kRows / kTileRows - 1) / (S::kRows / kTileRows);
+    a.split = split_of(tiles, a.groups, cta_slots());
+    return launch_pdl_cluster("gemm_rows", kernel, a.split, dim3((unsigned)(tiles * a.split)), dim3(kThreads), S::kSmem, stream, a);
 }
 
 }  // namespace
@@ -280,29 +296,41 @@ int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, i
     a.groups = cols / kGroup;
     a.nrb = (out[nout - 1].row0 + out[nout - 1].rows + kTileRows - 1) / kTileRows;
     switch ((m + 7) / 8) {
-        case 1: return launch<1, 2, 4>(a, stream);
-        case 2: return launch<2, 2, 4>(a, stream);
-        case 3: return launch<3, 2, 4>(a, stream);
-        default: return launch<4, 2, 4>(a, stream);
+        case 1: return launch<1>(a, stream);
+        case 2: return launch<2>(a, stream);
+        case 3: return launch<3>(a, stream);
+        default: return launch<4>(a, stream);
     }
 }
 
-// Where the lines lie (us among launches of the same kind, weights larger than L2):
-//   m = 1..3: one GEMV pass is as quick (2048 x 2048, m = 3: 5.6, here 3.2; 14336 x 4096: 7.9, here 12.5),
-//     and its block fixed point answers a non-finite activation with NaN in every output
-//   m = 4: one GEMV pass reads 24 tiles per warp before its staging is paid back, and long rows lengthen
-//     that staging: 4096 x 4096 6.9, here 5.3; 4096 x 14336 13.4, here 12.5; 16384 x 2048 6.5, here 7.1
-//   m = 5..8: two GEMV passes: 4096 x 4096, m = 8: 13.5, here 5.6; 28672 x 4096, m = 8: 21.3, here 24.3
-//   m = 9..32: the tcgen05 kernel (here / there): 2048 x 2048, m = 32 6.4 / 6.5; 4096 x 4096, m = 24 7.9 / 8.8;
-//     16384 x 2048, m = 16 9.7 / 8.8; 28672 x 4096, m = 9 29.8 / 25.0; 4096 x 14336, m = 16 15.4 / 16.2, m = 24
-//     18.1 / 16.5
+// Where the lines lie.  A CTA here walks its share of the scale groups, one after the other (0.35 us each beside 3 us a launch for
+// 8 rows, 0.42 for 16): the time is steps = groups / split x rounds of CTAs, and the split falls from eight to one as the rows grow past
+// 2368, 4736 and 9472.  The GEMV and the tcgen05 kernel divide their work more evenly.  us among launches of the same kind, weights
+// larger than L2, other / here:
+//   m = 1..3: one GEMV pass is as quick (2048 x 2048, m = 3: 5.6 / 3.2; 14336 x 4096: 7.9 / 12.5), and its block fixed point answers
+//     a non-finite activation with NaN in every output
+//   m = 4, one GEMV pass: with four or more CTAs a tile 4096 x 2048 5.7 / 3.9, 4096 x 8192 9.1 / 8.2, 4096 x 14336 13.9 / 12.9; with
+//     fewer up to eight steps 8192 x 2048 5.5 / 5.2, 16384 x 1024 4.7 / 4.2, behind them 6144 x 4096 7.2 / 7.6, 8192 x 14336
+//     17.1 / 22.9, 14336 x 14336 21.8 / 42.0; longer rows than 20480 leave the GEMV passes of two vectors: 8192 x 24576 64 / 37
+//   m = 5..8, two GEMV passes: two or more CTAs a tile 8192 x 4096 14.2 / 8.3, 8192 x 14336 31.9 / 23.2; one and up to 32 steps 16384 x
+//     4096 17.0 / 13.6; more: 10240 x 6144, m = 5 16.6 / 18.3; 28672 x 4096, m = 8 21.3 / 24.3
+//   m = 9..16, tcgen05: eight CTAs a tile 2048 x 28672 18.1 / 15.9; two or four up to 16 steps 8192 x 4096 10.8 / 9.7, 4096 x 8192 11.3 /
+//     9.8; more 3072 x 14336 13.5 / 14.6, 3072 x 28672 21.4 / 26.3; one up to 8 steps 16384 x 1024 6.1 / 5.1, 16 steps 10240 x 2048
+//     8.0 / 8.4
+//   m = 17..24: eight CTAs a tile, or up to 8 steps in two: 4096 x 4096 9.0 / 8.0; 4096 x 8192 11.8 / 12.1
+//   m = 25..32: up to 8 steps in four: 2048 x 2048 6.6 / 6.5; 6144 x 4096 10.7 / 13.9
 bool linear_takes_rows(int m, int rows, int cols)
 {
-    const long long tiles = (long long)((rows + kTileRows - 1) / kTileRows) * (cols / kGroup);
     if (m < 4 || m > kRowsMax) return false;
-    if (m == 4) return tiles <= 12288 || cols >= 12288;
-    if (m <= 8) return tiles <= 40000;
-    return tiles <= 12288 || (m <= 16 && cols >= 8192 && rows <= 4096);
+    const int slots = cta_slots(), groups = cols / kGroup, per = Shape<1, kRowWarps, kGroupWarps>::kRows, tiles = (rows + per - 1) / per;
+    if (!slots || !groups) return false;
+    const int split = split_of(tiles, groups, slots);
+    const long long rounds = ((long long)tiles * split + slots - 1) / slots, steps = (groups + split - 1) / split * rounds;
+    if (m == 4) return split >= 4 || steps <= 8 || cols > 20480;
+    if (m <= 8) return split >= 2 || steps <= 32 || cols > 20480;
+    if (m <= 16) return split == 8 || steps <= (split > 1 ? 16 : 8);
+    if (m <= 24) return split == 8 || (split > 1 && steps <= 8);
+    return split >= 4 && steps <= 8;
 }
 
 // Matrices packed back to back on this kernel or the tcgen05 GEMM (m > 8, or where this one is taken).

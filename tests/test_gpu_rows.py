@@ -26,3 +26,24 @@ def test_rows(m, n, k):
     # products are exact; K sums in FP32, each rounded once: K * 2^-24 of the sum of magnitudes, then FP16
     bound = k * 2.0 ** -24 * oracle.tolerance_bound(nz, sg, sc, x) / 2e-3 + 2.0 ** -11 * np.abs(y64) + 2.0 ** -25
     assert (np.abs(got[:m] - y64) <= bound).all(), np.max(np.abs(got[:m] - y64) / bound)
+
+
+@pytest.mark.parametrize("n", [2368, 2369, 4736, 4737, 9472, 9473])
+def test_both_sides_of_the_lines(n):
+    """Where a tile's CTAs go from eight to four, two and one, and with them the kernel of a number of vectors."""
+    k, ms = 4096, (3, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33)
+    nz, sg, sc, x = oracle.make_case(n, k, seed=n, batch=max(ms))
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (nz, sg, sc, x)]
+    w = tl.PreparedWeight(*dev[:3], n, k, register=False)
+    wd = torch.from_numpy(oracle.unpack_bitmasks(nz, sg).astype(np.float32) * np.repeat(sc.astype(np.float32), 128, axis=1)).cuda().double()
+    want, size = dev[3].double() @ wd.T, dev[3].double().abs() @ wd.T.abs()
+    for m in ms:
+        y = torch.full((m + 1, n), 7.0, dtype=torch.float16, device="cuda")
+        tl.ternary_gemm_packed(dev[3][:m].contiguous(), w, y, m)
+        assert (y[m] == 7.0).all()
+        # products are exact; K sums cut or rounded to FP32, then FP16
+        bound = k * 2.0 ** -23 * size[:m] + 2.0 ** -11 * want[:m].abs() + 2.0 ** -25
+        if m <= 8:       # the GEMV holds 3 and 4 vectors in steps of 2^-14 of a group's largest magnitude or less, each off by half a step
+            bound = bound + 2.0 ** -15 * dev[3][:m].double().abs().amax(1, keepdim=True) * wd.abs().sum(1)
+        assert ((y[:m].double() - want[:m]).abs() <= bound).all(), m
+    tl.check_device_errors()

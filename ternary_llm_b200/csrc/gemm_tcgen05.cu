@@ -6,8 +6,8 @@
 // FP32 accumulation rounding.
 //
 // Bound: the tensor pipe for long prompts (4 clocks a token of a tile and scale group); the chain of
-// expansion, MMA and hand-overs, about 700 clocks a scale group, for tiles of few tokens.  A tile is
-// 128 features x TM tokens, TM any multiple of 16 up to 192: the launch picks the TM (and a split of K)
+// expansion, MMA and hand-overs, about 600 clocks a scale group, for tiles of few tokens.  A tile is
+// 128 features x TM tokens, TM any multiple of 16 up to 256: the launch picks the TM (and a split of K)
 // with which the tiles come out even over the SMs.  One persistent CTA per SM, whose warps run ahead
 // of one another over the tiles' scale groups:
 //   * one warp loads the activations by TMA, a scale group (two boxes of 64 columns, 128-byte swizzled rows) a
@@ -19,13 +19,13 @@
 //     The codes c = t + 1 of two weights are the selector of one PRMT into the byte table {-s, 0, +s}, which
 //     yields the FP16 pair; tcgen05.st writes it.  The expanded weights are the MMA's A operand in TENSOR
 //     MEMORY and never touch shared memory.
-//   * one warp issues tcgen05.mma (kind::f16, M=128, N=TM, K=16) into one of two accumulators.  A stage is one
+//   * one warp issues tcgen05.mma (kind::f16, M=128, N=TM, K=16) into one of two accumulators (one beyond 192 tokens).  A stage is one
 //     wait (activations and weights arrive on one barrier), eight MMAs and one commit, and the warp's loop is
 //     uniform with an elected lane for the MMAs: as the loop of one thread, with a barrier and a commit for
 //     either operand, the issue alone took 2000 clocks a stage;
 //   * four warps empty the other accumulator with tcgen05.ld and store C (a lane is an output feature, so a
 //     warp stores 32 adjacent features of one token at a time).
-// Tensor memory: two accumulators of TM columns (a multiple of 32 apart), then two to four weight
+// Tensor memory: the accumulators of TM columns (a multiple of 32 apart), then two to four weight
 // stages of 64 columns.
 // Too few tiles for the SMs: K is split over the CTAs of a cluster; each leaves its FP32 sums in its
 // shared memory, and each adds all of them, in rank order, for its share of the tokens.
@@ -50,7 +50,8 @@ namespace gemm {
 constexpr int kTileN = 128;          // features per tile (MMA M, TMEM lanes)
 constexpr int kBoxK = 64;            // columns per activation box (128 bytes of FP16)
 constexpr int kACols = kGroup / 2;   // tensor-memory columns of a weight stage (FP16 pairs)
-constexpr int kMaxTm = 192;
+constexpr int kMaxTm = 256;
+constexpr int kMaxTm2 = 192;         // of two accumulators beside the weights
 constexpr int kMaxB = 8;             // activation stages, upper bound
 constexpr int kMaxA = 4;             // weight stages, upper bound
 constexpr int kCodes = 6;            // scale groups of codes in shared memory
@@ -67,7 +68,8 @@ struct Args {
     RowsOut out[TLLM_MAX_FUSED];     // row ranges of the matrix and where they go; unused ones start past every row
     int M, N, groups;                // tokens; rows of W; K / 128
     int mt, tiles, split;            // token tiles; tiles; CTAs per tile
-    int tm, acc_stride, na, nb;      // tokens per tile; columns between accumulators; weight and activation stages
+    int tm, acc_stride, na, nb;      // tokens per tile; columns between accumulators; weight and activation stages (na <= nb)
+    int accs;                        // accumulators: two, or one for tiles of more than kMaxTm2 tokens
     int* err;
 };
 
@@ -230,7 +232,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t d0 = make_sw128_desc(smem_u32(smem + b.slot * stage_bytes));
                 const uint64_t d1 = make_sw128_desc(smem_u32(smem + b.slot * stage_bytes) + box_bytes);
-                const uint32_t a_t = tmem + 2 * a.acc_stride + w.slot * kACols, more = it > 0 ? 1u : 0u;
+                const uint32_t a_t = tmem + a.accs * a.acc_stride + w.slot * kACols, more = it > 0 ? 1u : 0u;
                 if (leader) {
 #pragma unroll
                     for (int k = 0; k < kGroup / 16; k++)          // 32 bytes (2 in the descriptor) inside the 128-byte swizzled row
@@ -241,7 +243,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                 w.step(na);
             }
             if (leader) mma_commit(acc_full(acc.slot));
-            acc.step(2);
+            acc.step(a.accs);
         }
         if (!ok) abort_flag = 1;
         if (leader) mma_commit(drained);
@@ -282,12 +284,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         // (gq*4 + t)*4 + 2h, one 64-bit load per t; each word holds all four 32-column steps
         const uint8_t* cp = codes + rbl * kTileBytes + gq * 64 + h * 8;
         const uint8_t* sp = codes + rbl * kTileBytes + kTileCodeBytes + tile_scale_index(r16) * 2;
-        const uint32_t lane_base = tmem + ((uint32_t)(row & ~31) << 16) + 2 * a.acc_stride;   // this warp's 32 lanes
+        const uint32_t lane_base = tmem + ((uint32_t)(row & ~31) << 16) + a.accs * a.acc_stride;   // this warp's 32 lanes
         Ring c, w, f, past;                                  // codes; weight stage; stage; the stage that had the weight stage before
         c.step(kCodes, set);
         w.step(na, set);
         f.step(nb, set);
-        past.slot = (set + kMaxA * kSets - na) % kSets;      // of the set's first scale group from na on (nb is at least 4)
+        past.slot = (set + kMaxA * kSets - na) % kSets;      // of the set's first scale group from na on (nb is at least 3)
         bool ok = true;
         int g = 0, turn = 0;                                 // scale groups of this CTA so far; whose the next one is
         for (int tile = first; ok && tile < a.tiles; tile += step) {
@@ -397,7 +399,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty(acc.slot));
-            acc.step(2);
+            acc.step(a.accs);
         }
         if (!ok) abort_flag = 1;
     }
@@ -498,21 +500,28 @@ static Device* device()
 }
 
 // Tokens per tile and CTAs per tile: the least time in clocks of
-//   rounds of tiles x scale groups x (650 + 2.6 a token) + what a launch has around them
-// (first loads 2000, the last tile's outputs 10 a token, a cluster's sums 2000 + 4 a token).  A scale group's
-// time is measured: 770 clocks at 48 tokens, 950 at 128, 1150 at 192.
+//   rounds of tiles x scale groups x the largest of 580 and 500 + 2.45 a token (chain) and 4.6 a token (MMA)
+//   + 31 a CTA (they start one after the other) + what a launch has around them: first loads 3000, the last tile's outputs 16 a
+//     token, those of every tile 21 a token where one accumulator has to be emptied first, a cluster's sums 3000 + 33 a token
+//     (beyond 192 tokens 1000 more).
+// Fitted to 1949 times of 231 products (14 matrices, 33 to 2048 tokens): what it takes is within 4 % of the quickest of them but
+// for five products of 512 or 3072 features (10 %).  With tiles of up to 192 tokens alone 4096 x 4096, 1024 tokens, needed two
+// rounds of 128-token tiles, 32.9 us in place of 27.3; 2048 x 8192, 2048 tokens 58.5, now 45.6; 14336 x 14336, 256 tokens 97, now 77.
 static void choose(Args& a, int nt, const Device& d)
 {
     long long best = LLONG_MAX;
-    for (int mt = (a.M + kMaxTm - 1) / kMaxTm, end = mt + 16; mt <= end; mt++) {
+    for (int mt = (a.M + kMaxTm - 1) / kMaxTm, end = (a.M + kMaxTm2 - 1) / kMaxTm2 + 16; mt <= end; mt++) {
         const int tm = ((a.M + mt - 1) / mt + 15) / 16 * 16;
         if ((a.M + tm - 1) / tm != mt) continue;
-        const long long stage = 650 + 26 * tm / 10, tiles = (long long)nt * mt;
+        const bool one = tm > kMaxTm2;
+        const long long chain = 500 + 49 * tm / 20, mma = 23 * tm / 5, stage = mma > chain ? mma : chain > 580 ? chain : 580;
+        const long long tiles = (long long)nt * mt;
         if (tiles > INT_MAX / kMaxSplit) break;
         for (int c = 1; c <= kMaxSplit; c++) {
             if (c > 1 && (tiles * c > d.slots[c] || a.groups < 2 * c)) continue;
-            const long long rounds = c > 1 ? 1 : (tiles + d.sms - 1) / d.sms;
-            const long long cost = rounds * ((a.groups + c - 1) / c) * stage + 2000 + 10 * tm + (c > 1 ? 2000 + 4 * tm : 0);
+            const long long rounds = c > 1 ? 1 : (tiles + d.sms - 1) / d.sms, ctas = tiles * c < d.sms ? tiles * c : d.sms;
+            const long long cost = rounds * ((a.groups + c - 1) / c) * stage + 31 * ctas + 3000 + 16 * tm + (one ? (rounds - 1) * 21 * tm : 0) +
+                                   (c > 1 ? 3000 + 33 * tm + (one ? 1000 : 0) : 0);
             if (cost < best) {
                 best = cost;
                 a.mt = mt;
@@ -559,10 +568,12 @@ int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out
     if (!a.split) return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: M=%d N=%d K=%d: too many tiles", M, a.N, K);
     a.err = err;
     a.acc_stride = (a.tm + 31) / 32 * 32;
-    a.na = (kTmemCols - 2 * a.acc_stride) / kACols;
+    a.accs = a.tm > kMaxTm2 ? 1 : 2;
+    a.na = (kTmemCols - a.accs * a.acc_stride) / kACols;
     if (a.na > kMaxA) a.na = kMaxA;
     a.nb = (int)((kSmem - 1024 - kCodes * kCodeBytes) / (a.tm * kGroup * 2));
     if (a.nb > kMaxB) a.nb = kMaxB;
+    if (a.na > a.nb) a.na = a.nb;        // weights of a scale group are announced on its stage's barrier
     CUtensorMap map_x, map_w;
     if (!encode(enc, &map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, A, K, M, (cuuint64_t)K * sizeof(half), kBoxK, a.tm, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode(enc, &map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, packed, (cuuint64_t)a.groups * (kTileBytes / 4), nrb,

@@ -1,5 +1,5 @@
-"""The tcgen05 prompt GEMM over its free token tiles (csrc/gemm_tcgen05.cu): token counts around every
-multiple of 16 and the largest tile, one to many tiles per SM, splits of K over clusters with uneven shares
+"""The tcgen05 prompt GEMM over its free token tiles (csrc/gemm_tcgen05.cu): token counts around
+multiples of 16 and the largest tiles, one to many tiles per SM, splits of K over clusters with uneven shares
 (and fewer scale groups than stages), ragged features, against 64 bits."""
 import numpy as np
 import pytest
@@ -15,6 +15,16 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m", [33, 48, 65, 113, 161, 192, 193, 385, 700])
 @pytest.mark.parametrize("n,k", [(1, 128), (127, 384), (130, 2176), (1000, 640), (4112, 1152)])
 def test_tiles(m, n, k):
+    product(m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(1000, 4112, 1152), (2000, 2000, 1152), (2000, 3456, 2304), (1999, 3460, 2304), (201, 3200, 6144), (205, 3070, 6144)])
+def test_tiles_of_one_accumulator(m, n, k):
+    """Tiles of more than 192 tokens: one and two rounds of them, whole and ragged, and K split over a cluster."""
+    product(m, n, k)
+
+
+def product(m, n, k):
     nz, sg, sc, x = oracle.make_case(n, k, seed=m + n + k, batch=m)
     dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (nz, sg, sc, x)]
     w = tl.PreparedWeight(*dev[:3], n, k, register=False)

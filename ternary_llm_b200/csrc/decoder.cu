@@ -155,10 +155,18 @@ int linear_multi(LlamaDecoder* D, int count, const PackedW* const* w, half* cons
 // column) beside a ring, which fits up to 28000 columns; wider ones keep the norm's own launch.
 constexpr int kFusedNormMax = 16384;
 
-// Key/value heads of a lock-step token up to which the attention that splits a cache into ranges of 64 positions and
-// rotates by itself is taken; with more, rotation and ranges of 256 are quicker (a step of the 1B model, 8 heads: 2
-// sequences 1081 -> 916 us, 8: 832 -> 725; 24: 1174, there 1264; four 8B layers, 16 sequences: 550 -> 537).
-constexpr int kSplitHeads = 128;
+// Whether a lock-step token takes the attention that splits each cache into ranges of 64 positions and rotates by itself, or
+// rotation and ranges of 256.  The former saves a launch and has more CTAs, which pays while they are few: a merge of more than
+// 16 ranges of head size 64 and more CTAs than run at the same time cost more than that.  A step, 8 key/value heads, us, by itself /
+// rotation first: 1B model (head size 64) behind 300 positions 4 sequences 753 / 917, 16 (640 CTAs) 1064 / 1075; behind 500 12 (768)
+// 1075 / 1069; behind 1500 2 sequences (24 ranges) 1175 / 1121, 16 2188 / 1389.  Four 8B layers (128): behind 1500 4 sequences
+// (768) 559 / 594, 6 (1152) 613 / 628, 16 (3072) 944 / 909; behind 1000 8 (1024) 609 / 607.
+constexpr int kSplitHeads = 128;              // heads that its workspace is made for
+static bool splits_by_itself(int heads, int head_dim, int kv_len)
+{
+    const int ranges = (kv_len + 63) / 64;
+    return heads <= kSplitHeads && (head_dim == 128 ? heads * ranges <= 1024 : ranges <= 16 && heads * ranges <= 640);
+}
 
 // One pass of the layer stack.
 //   batch == 0: n tokens of sequence `seq` at positions start_pos.. (pos_dev != nullptr: one
@@ -240,7 +248,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
             half* y[3] = {qb, kb, vb};
             TRY(linear_multi(D, 3, w, y, D->hidden, i8, n, s, &L.qkv));
         }
-        if (seq_n == 1 && (bsz == 1 || bsz * c.n_kv_heads <= kSplitHeads)) {        // rotation, append and attention of one token per sequence
+        if (seq_n == 1 && (bsz == 1 || splits_by_itself(bsz * c.n_kv_heads, c.head_dim, start_pos + 1))) {        // a token per sequence
             TRY(launch_attention_decode(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads,
                                         c.head_dim, c.max_seq_len, start_pos, pos_dev, c.rope_theta, D->attn_ws, D->attn_counters, s));
         } else {

@@ -102,6 +102,32 @@ def test_batched_lock_step_decode_matches_independent_sequences(batch):
     dec.close()
 
 
+def near(got, want):
+    """One layer in FP16: two roundings per operator, on kernels that sum in another order."""
+    return np.linalg.norm(got.astype(np.float64) - want) <= 1e-2 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("batch,context", [(3, 62), (2, 63), (3, 64), (2, 300), (2, 1022), (2, 1100), (32, 100), (32, 319), (33, 63), (33, 300)])
+def test_lock_step_behind_contexts(batch, context):
+    """Lock-step tokens behind contexts of one and several ranges of positions, each sequence with one of its own, two in a
+    row, on the launch that rotates and splits by itself and, with more heads or positions, on rotation and attention."""
+    cfg = cfg_small(vocab_size=256, intermediate_dim=256, n_layers=1, n_heads=8, n_kv_heads=4, max_seq_len=1152)
+    model = tf.random_model(cfg, seed=31)
+    dec = tl.Decoder(model, int8_decode=False, max_batch=batch)
+    prompts = [toks(context, cfg.vocab_size, seed=b) for b in range(batch)]
+    for b in range(batch):
+        dec.forward_seq(b, torch.from_numpy(prompts[b]).cuda(), 0)
+    nxt = np.stack([toks(batch, cfg.vocab_size, seed=900 + i) for i in range(2)])
+    got = [dec.forward_batch(torch.from_numpy(nxt[i]).cuda(), context + i).double().cpu().numpy() for i in range(2)]
+    for b in sorted({0, batch // 2, batch - 1}):
+        ora = LO.Transformer(model, int8_decode=False)
+        ora.forward(list(prompts[b]), 0)
+        for i in range(2):
+            assert near(got[i][b], ora.forward([int(nxt[i][b])], context + i).astype(np.float64)), (b, i)
+    tl.check_device_errors()
+    dec.close()
+
+
 @pytest.mark.parametrize("int8", [False, True])
 @pytest.mark.parametrize("which", ["attn_norm", "ffn_norm"])
 def test_norm_weights_at_any_address(int8, which):

@@ -589,6 +589,7 @@ attention_decode_kernel(DecodeArgs a)
     }
     const bool writer_all = (pgroups == 1);
     half* op = a.out + (size_t)kvh * G * hd;
+    const half2 zero = __half2half2(__ushort_as_half(0));          // of a head whose sum is not positive (NaN), as from attention_kernel
     const int rec = G * (hd + 2);
     float* my = a.ws + ((size_t)kvh * a.nsplit + split) * rec;
 #pragma unroll
@@ -598,10 +599,9 @@ attention_decode_kernel(DecodeArgs a)
         if (mine) {
             const int g = item / hp, pr = item - g * hp;
             if (nactive == 1) {
-                const float l = l_run[g];
-                const float inv = l > 0.f ? 1.0f / l : 0.f;
+                const float l = l_run[g], inv = 1.0f / l;
                 *(reinterpret_cast<half2*>(op + (size_t)g * hd) + pr) =
-                    __halves2half2(__float2half_rn(o[e].x * inv), __float2half_rn(o[e].y * inv));
+                    l > 0.f ? __halves2half2(__float2half_rn(o[e].x * inv), __float2half_rn(o[e].y * inv)) : zero;
             } else {
                 *reinterpret_cast<float2*>(my + (size_t)g * hd + 2 * pr) = o[e];
             }
@@ -659,10 +659,10 @@ attention_decode_kernel(DecodeArgs a)
                     }
                 }
             }
-            const float inv = den > 0.f ? 1.0f / den : 0.f;
+            const float inv = 1.0f / den;
             half2* o2 = reinterpret_cast<half2*>(op + (size_t)(i4 << 2));
-            o2[0] = __halves2half2(__float2half_rn(num.x * inv), __float2half_rn(num.y * inv));
-            o2[1] = __halves2half2(__float2half_rn(num.z * inv), __float2half_rn(num.w * inv));
+            o2[0] = den > 0.f ? __halves2half2(__float2half_rn(num.x * inv), __float2half_rn(num.y * inv)) : zero;
+            o2[1] = den > 0.f ? __halves2half2(__float2half_rn(num.z * inv), __float2half_rn(num.w * inv)) : zero;
         }
         return;
     }

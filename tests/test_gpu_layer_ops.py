@@ -167,6 +167,29 @@ def test_fused_single_token_attention_entry_point(hq, hk, hd, pos, mx):
     tl.check_device_errors()
 
 
+@pytest.mark.parametrize("pos", [10, 63, 64, 300, 1100])
+def test_scores_that_are_not_numbers_give_zeros(pos):
+    """A head whose softmax has no positive sum is zero in every form: one range of positions, ranges merged at
+    once and in stages, the operator without the append, several queries; the other heads are as ever."""
+    hq, hk, hd, mx = 4, 2, 64, 1152
+    rng = np.random.default_rng(pos)
+    kc, vc = (dev(rng.standard_normal((hk, mx, hd)).astype(f16)) for _ in range(2))
+    q, k, v = (dev(rng.standard_normal((h, hd)).astype(f16)) for h in (hq, hk, hk))
+    outs = []
+    for bad in (0.0, np.nan):
+        kc[0, 3, 0] = bad
+        fused, split = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
+        ops.attention_decode(q, k, v, kc, vc, fused, hq, hk, hd, pos, 1e4, mx)
+        qr, kr = q.clone(), k.clone()
+        ops.rope_append(qr, kr, v, kc, vc, 1, 1, hq, hk, hd, pos, 1e4, mx)
+        ops.attention_forward(qr, kc, vc, split, 1, hq, hk, hd, 1, pos + 1, mx)
+        two = torch.full((2, hq, hd), 7.0, dtype=torch.float16, device=DEV)
+        ops.attention_forward(torch.stack([qr, qr]), kc, vc, two, 1, hq, hk, hd, 2, pos + 1, mx)
+        outs.append([host(t) for t in (fused, split, two[1])])
+    for good, bad in zip(*outs):
+        assert (bad[:2] == 0).all() and np.array_equal(bad[2:], good[2:]) and (np.abs(good) < 7).all()
+
+
 @pytest.mark.parametrize("seq,kv_len", [(2, 2), (33, 33), (16, 300)])
 def test_attention_several_tokens_is_causal_softmax(seq, kv_len):
     rng = np.random.default_rng(seq)

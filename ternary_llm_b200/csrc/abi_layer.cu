@@ -134,7 +134,7 @@ int tllm_b200_attention(const void* q, const void* k_cache, const void* v_cache,
         if (st) return st;
     }
     return launch_attention((const half*)q, (const half*)k_cache, (const half*)v_cache, (half*)output, batch, n_heads,
-                            n_kv_heads, head_dim, seq_len, kv_len, kv_len_max, nullptr, ws, counters, S(stream));
+                            n_kv_heads, head_dim, seq_len, kv_len, kv_len_max, ws, counters, S(stream));
 }
 
 int tllm_b200_attention_decode(void* q, const void* k, const void* v, void* k_cache, void* v_cache, void* output,

@@ -24,7 +24,7 @@
 // Decode (seq_len == 1) splits the cache positions over several CTAs (one chunk each);
 // each writes (max, sum, unnormalised output) and the CTA that arrives last on a counter
 // merges them in split order and resets the counter, so replays of a captured graph need
-// no host-side clearing.  The cache length can come from device memory for that case.
+// no host-side clearing.
 #include <cfloat>
 
 #include "launch.cuh"
@@ -58,7 +58,6 @@ struct AttnArgs {
     const half* v_cache;
     half* out;
     int n_heads, n_kv_heads, head_dim, seq_len, kv_len, kv_len_max;
-    const int* kv_len_dev;     // decode: kv_len = *kv_len_dev + kv_len when not null
     int nsplit;                // decode: CTAs per (batch, kv head); 1 otherwise
     float* ws;                 // [batch * n_kv_heads][nsplit][group * (head_dim + 2)]
     unsigned* counters;        // [batch * n_kv_heads]
@@ -96,9 +95,7 @@ attention_kernel(const AttnArgs a)
     }
 
     pdl_wait();
-    int kv_len = a.kv_len;
-    if (a.kv_len_dev) kv_len += *a.kv_len_dev;
-    const int limit = kv_len - a.seq_len + s_idx + 1;          // positions [0, limit) are visible
+    const int limit = a.kv_len - a.seq_len + s_idx + 1;          // positions [0, limit) are visible
     int lo = 0, hi = limit, nactive = 1;
     if (decode) {
         nactive = (limit + kAttnChunk - 1) / kAttnChunk;
@@ -768,8 +765,7 @@ size_t attention_workspace_bytes(int batch, int n_heads, int n_kv_heads, int hea
 // ws / counters: decode scratch (attention_workspace_bytes; counters zero-initialised,
 // batch * n_kv_heads unsigned).  With ws == nullptr decode runs as one CTA per KV head.
 int launch_attention(const half* q, const half* k_cache, const half* v_cache, half* out, int batch, int n_heads,
-                     int n_kv_heads, int head_dim, int seq_len, int kv_len, int kv_len_max, const int* kv_len_dev,
-                     float* ws, unsigned* counters, cudaStream_t stream)
+                     int n_kv_heads, int head_dim, int seq_len, int kv_len, int kv_len_max, float* ws, unsigned* counters, cudaStream_t stream)
 {
     if (batch == 0 || seq_len == 0) return TLLM_OK;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads) return fail(TLLM_ERR_SHAPE, "attention: n_heads=%d n_kv_heads=%d", n_heads, n_kv_heads);
@@ -778,9 +774,9 @@ int launch_attention(const half* q, const half* k_cache, const half* v_cache, ha
     if (head_dim % 8 || head_dim > 128 || G * head_dim > kAttnMaxElems * kAttnThreads)
         return fail(TLLM_ERR_SHAPE, "attention: head_dim=%d (a multiple of 8 up to 128) with %d heads per group is not supported",
                     head_dim, G);
-    if (!kv_len_dev && (kv_len < seq_len || kv_len > kv_len_max))
+    if (kv_len < seq_len || kv_len > kv_len_max)
         return fail(TLLM_ERR_SHAPE, "attention: kv_len=%d seq_len=%d kv_len_max=%d", kv_len, seq_len, kv_len_max);
-    if (!kv_len_dev && attention_prompt_supported(q, k_cache, v_cache, out, batch, n_heads, n_kv_heads, head_dim, seq_len, kv_len, kv_len_max))
+    if (attention_prompt_supported(q, k_cache, v_cache, out, batch, n_heads, n_kv_heads, head_dim, seq_len, kv_len, kv_len_max))
         return launch_attention_prompt(q, k_cache, v_cache, out, batch, n_heads, n_kv_heads, head_dim, seq_len, kv_len, kv_len_max, stream);
     AttnArgs a = {};
     a.q = q;
@@ -793,7 +789,6 @@ int launch_attention(const half* q, const half* k_cache, const half* v_cache, ha
     a.seq_len = seq_len;
     a.kv_len = kv_len;
     a.kv_len_max = kv_len_max;
-    a.kv_len_dev = kv_len_dev;
     a.ws = ws;
     a.counters = counters;
     const bool decode = (seq_len == 1);

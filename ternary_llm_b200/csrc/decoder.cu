@@ -255,7 +255,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
             TRY(launch_rope(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, bsz, seq_n, c.n_heads, c.n_kv_heads, c.head_dim, start_pos,
                             c.rope_theta, c.max_seq_len, 1, s));
             TRY(launch_attention(qb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads, c.head_dim, seq_n,
-                                 start_pos + seq_n, c.max_seq_len, nullptr, D->attn_ws, D->attn_counters, s));
+                                 start_pos + seq_n, c.max_seq_len, D->attn_ws, D->attn_counters, s));
         }
         if (i8) TRY(launch_quantize_absmax_int8(D->attn_out, D->xq, D->xscale, qdim, s));
         {

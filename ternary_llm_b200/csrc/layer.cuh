@@ -33,10 +33,9 @@ int launch_argmax(const float* logits, int n, int* out, int* history, int* step,
                   unsigned* counter, int* pos, cudaStream_t stream);
 
 size_t attention_workspace_bytes(int batch, int n_heads, int n_kv_heads, int head_dim, int kv_len_max);
-// kv_len_dev: decode only, kv_len = kv_len + *kv_len_dev.  ws / counters: decode split scratch or null.
+// ws / counters: decode split scratch or null.
 int launch_attention(const half* q, const half* k_cache, const half* v_cache, half* out, int batch, int n_heads,
-                     int n_kv_heads, int head_dim, int seq_len, int kv_len, int kv_len_max, const int* kv_len_dev,
-                     float* ws, unsigned* counters, cudaStream_t stream);
+                     int n_kv_heads, int head_dim, int seq_len, int kv_len, int kv_len_max, float* ws, unsigned* counters, cudaStream_t stream);
 
 // Several queries on tcgen05 (grouped_prompt.cu); launch_attention takes it where it is supported and quicker.
 bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_heads, int n_kv_heads,

@@ -77,8 +77,8 @@ def test_fused_decode_attention_geometries(heads, kv_heads, head_dim):
 
 @pytest.mark.parametrize("batch", [2, 5, 9])
 def test_batched_lock_step_decode_matches_independent_sequences(batch):
-    """B sequences with their own KV caches decoded in lock step (GEMV passes up to 6 sequences,
-    the tcgen05 GEMM above) against the oracle run once per sequence (FP16 activations)."""
+    """B sequences with their own KV caches decoded in lock step (two on GEMV passes, more on the products of few
+    rows) against the oracle run once per sequence (FP16 activations)."""
     cfg = cfg_small(max_seq_len=64)
     model = tf.random_model(cfg, seed=21)
     dec = tl.Decoder(model, int8_decode=True, max_batch=batch)
@@ -124,6 +124,25 @@ def test_lock_step_behind_contexts(batch, context):
         ora.forward(list(prompts[b]), 0)
         for i in range(2):
             assert near(got[i][b], ora.forward([int(nxt[i][b])], context + i).astype(np.float64)), (b, i)
+    tl.check_device_errors()
+    dec.close()
+
+
+def test_fp16_steps_and_loop_across_a_range_of_positions():
+    """FP16 steps with the norms in the GEMVs and rotation in the attention, given and captured, over the edge of 64 positions."""
+    cfg = cfg_small(n_layers=1)
+    model = tf.random_model(cfg, seed=41)
+    dec, ora = tl.Decoder(model, int8_decode=False), LO.Transformer(model, int8_decode=False)
+    t = toks(61, cfg.vocab_size)
+    got, want = dec.forward(torch.from_numpy(t).cuda(), 0), ora.forward(list(t), 0)
+    first = tok = int(got.argmax())
+    out = []
+    for i in range(61, 69):
+        got, want = dec.forward(torch.tensor([tok], dtype=torch.int32, device="cuda"), i), ora.forward([tok], i)
+        assert near(got.double().cpu().numpy(), want.astype(np.float64)), i
+        tok = int(got.argmax())
+        out.append(tok)
+    assert dec.generate(first, 61, 8)[0] == out
     tl.check_device_errors()
     dec.close()
 

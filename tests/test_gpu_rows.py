@@ -1,12 +1,13 @@
-"""Products of a few rows (csrc/gemm_rows.cu) through ternary_gemm_packed and, for matrices packed back to
-back, through the decoder: edges of the 16-row blocks, the 64-feature tiles, the groups and their
-split over clusters, against the oracle in 64 bits."""
+"""Products of a few rows (csrc/gemm_rows.cu) through ternary_gemm_packed: edges of the 16-row blocks, the
+64-feature tiles, the groups and their split over clusters, against the oracle in 64 bits; matrices packed back to
+back, here and in the tcgen05 GEMM, through the decoder."""
 import numpy as np
 import pytest
 import torch
 
 import ternary_llm_b200 as tl
-from oracle import oracle
+from oracle import layer_oracle, oracle
+from ternary_llm_b200 import tllm_format as tf
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +48,20 @@ def test_both_sides_of_the_lines(n):
             bound = bound + 2.0 ** -15 * dev[3][:m].double().abs().amax(1, keepdim=True) * wd.abs().sum(1)
         assert ((y[:m].double() - want[:m]).abs() <= bound).all(), m
     tl.check_device_errors()
+
+
+@pytest.mark.parametrize("n", [4, 5, 8, 9, 16, 17, 32, 33, 65])
+def test_matrices_packed_back_to_back(n):
+    """q|k|v and gate|up of a prompt in one launch each, k and v of 48 rows, whose borders fall inside the tiles of 64
+    and 128 features: the logits show every row of every output, through the attention and the gate."""
+    cfg = tf.TllmConfig(vocab_size=512, hidden_dim=384, intermediate_dim=640, n_layers=1, n_heads=24, n_kv_heads=3, head_dim=16,
+                        max_seq_len=80, rope_theta=10000.0, rms_norm_eps=1e-5)
+    model = tf.random_model(cfg, seed=n)
+    dec = tl.Decoder(model, int8_decode=False)
+    t = np.random.default_rng(n).integers(0, cfg.vocab_size, n).astype(np.int32)
+    got = dec.forward(torch.from_numpy(t).cuda(), 0).double().cpu().numpy()
+    want = layer_oracle.Transformer(model, int8_decode=False).forward(list(t), 0).astype(np.float64)
+    tl.check_device_errors()
+    # one layer in FP16: two roundings per operator, on kernels that sum in another order
+    assert np.linalg.norm(got - want) <= 1e-2 * np.linalg.norm(want)
+    dec.close()

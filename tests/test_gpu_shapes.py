@@ -72,7 +72,7 @@ def test_gemv_batched_at_8b_shapes(name, batch):
     torch.cuda.synchronize()
     tl.check_device_errors()
     _check_rows(y.cpu().numpy(), nz, sg, sc, _sample_rows(n, seed=batch), x, f"gemv {name} batch {batch}")
-    if batch <= 8:      # the integer-MMA GEMV: scaling by two only shifts the block exponent
+    if batch <= 8:      # the integer-MMA GEMV, where scaling by two only shifts the block exponent, or FP16 products in FP32
         # (exact wherever the FP16 result is a normal number; a subnormal one rounds on a fixed grid)
         normal = y.float().abs() >= 2.0 ** -13
         assert torch.equal(y2.float()[normal], y.float()[normal] * 2), "W(2x) != 2 W(x)"
@@ -87,8 +87,8 @@ GEMM_CASES = [(m, s) for s in ("gate/up", "down") for m in (128, 512, 2048)] + [
 
 @pytest.mark.parametrize("m,name", GEMM_CASES)
 def test_gemm_at_8b_shapes(m, name):
-    """The tcgen05 GEMM at the prefill sizes of the benchmark definition (k/v at 2048 tokens
-    takes the split-K path), sampled tokens x sampled features against the oracle."""
+    """The tcgen05 GEMM at the prefill sizes of the benchmark definition (down at 128 tokens
+    splits K over clusters), sampled tokens x sampled features against the oracle."""
     n, k = SHAPES_8B[name]
     nz, sg, sc, w = _weights(n, k, seed=2000 + n + k)
     a = torch.randn(m, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(m)).half()

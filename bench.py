@@ -454,7 +454,7 @@ def run_tp(args, torch, dist, tl, synth, rank, world, local, dev):
             ms32 = timed(fn32, reps) / reps
             batch32 = {"ms_per_step": ms32, "tok_per_s": B * 1000.0 / ms32, "allreduce": "NCCL, FP16 [32, 8192]",
                        "launch": mode32, "finite": finite,
-                       "gemv_route": "tcgen05 GEMM kernel (more than 8 vectors)"}
+                       "gemv_route": "tcgen05 GEMM kernel, mma.sync for small matrices"}
             g32 = None
             s32 = None
         except Exception as e:          # reported, never fatal for the headline
@@ -530,7 +530,7 @@ class ColdTimer:
 def gemv_batch_rows(torch, tl, synth, prepared, dev, stream, cold):
     """Configuration "GEMV sweep at batch 1/4/16" shape by shape, and the single-GEMV
     configuration (8192 x 2048): each row is one launch per distinct matrix (32 of them) as a
-    CUDA graph, weights cold.  Batch 16 runs on the tcgen05 kernel (the library's routing)."""
+    CUDA graph, weights cold.  The library chooses the kernel by batch and matrix."""
     rows = []
     per_layer = len(SHAPES_8B)
     cases = [("q", 0), ("k/v", 1), ("o", 3), ("gate/up", 4), ("down", 6)]
@@ -946,7 +946,7 @@ def run_ours(args):
         }
         if batch_rows is not None:
             out["gemv_batch"] = {"note": "one launch per distinct matrix (32), CUDA graph, L2 flushed before every timed replay, median of 5; "
-                                         "batch <= 8 is the streaming GEMV (one or two vectors on 24-bit block fixed point; three and four vectors per weight pass on 16-bit block fixed point, within the 2e-3 bound for any input), batch 16 the tcgen05 kernel",
+                                         "one or two vectors are a pass of the streaming GEMV on 24-bit block fixed point, four one on 16 bits (within the 2e-3 bound for any input) or the FP16 mma.sync kernel, 16 that kernel or the tcgen05 GEMM, by the matrix",
                                  "rows": batch_rows}
         if ref_cuda is not None:
             out["reference_cuda"] = ref_cuda

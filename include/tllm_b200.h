@@ -160,7 +160,8 @@ int tllm_b200_weight_unregister(const uint32_t* nonzero_masks);
  * one or two vectors per call, 16 bits for passes of three or four vectors (their
  * rounding error per output is at most 2^-17 * sum over groups of scale * 128 *
  * max|x| of the group, under half of the 2e-3 * sum|scale * x| bound for any
- * input); nine vectors and more run on the tcgen05 GEMM kernel in FP16.
+ * input).  Four vectors and more run in FP16 on the tensor cores where the matrix
+ * makes that quicker, nine and more always (see tllm_b200_gemm_packed).
  */
 int tllm_b200_gemv_packed(const void* packed, const void* x, void* y,
                           int batch, int rows, int cols, void* stream);
@@ -256,10 +257,11 @@ int tllm_b200_gemv_packed_noalloc_status(void* stream);
 
 /*
  * Prefill GEMM on prepared weights: C[M,N] = A[M,K] . W^T, same contract as
- * tllm_b200_gemm.  M > 8 runs the tcgen05 tensor-core kernel (weights expanded to
- * exact FP16 {-s,0,+s} in tensor memory, FP32 accumulation in TMEM; token tile 32, 64,
- * 128 or 256 by M); smaller M runs passes of the streaming GEMV.  tllm_b200_gemm reaches the same kernels when
- * the weight pointer has been registered.
+ * tllm_b200_gemm.  Up to 3 rows, and up to 8 of a large matrix, are passes of the streaming
+ * GEMV; 4 to 32 rows of a matrix small enough that a launch's latencies count run on
+ * mma.sync; everything else runs the tcgen05 tensor-core kernel (weights expanded to exact
+ * FP16 {-s,0,+s} in tensor memory, FP32 accumulation in TMEM; token tiles of 16 to 256).
+ * tllm_b200_gemm reaches the same kernels when the weight pointer has been registered.
  */
 int tllm_b200_gemm_packed(const void* A, const void* packed, void* C, int M, int N, int K, void* stream);
 

@@ -155,8 +155,8 @@ int tllm_b200_decoder_forward_seq(void* decoder, int seq, const int* token_ids, 
                                   void** logits, void* stream);
 
 /* One decode step of `batch` sequences in lock step: token_ids[b] is the next token of
- * sequence b, all at cache position pos; the weights are read once for the whole batch (FP16
- * activations: passes of the streaming GEMV up to 6 sequences, the tcgen05 GEMM above).
+ * sequence b, all at cache position pos, FP16 activations; the weights are read once for the
+ * whole batch (the kernels of tllm_b200_gemm_packed).
  * *logits: half [batch, vocab]. */
 int tllm_b200_decoder_forward_batch(void* decoder, const int* token_ids, int batch, int pos, void** logits,
                                     void* stream);

@@ -11,7 +11,7 @@
 // with which the tiles come out even over the SMs.  One persistent CTA per SM, whose warps run ahead
 // of one another over the tiles' scale groups:
 //   * one warp loads the activations by TMA, a scale group (two boxes of 64 columns, 128-byte swizzled rows) a
-//     stage, four to eight stages; another one the packed codes, one box of 8 row blocks x 544 bytes per scale
+//     stage, three to eight stages; another one the packed codes, one box of 8 row blocks x 544 bytes per scale
 //     group, six ahead.  (Read by the expanders from global memory one group ahead, a group took a
 //     microsecond whatever the tile, the latency of a load from HBM.)
 //   * twelve warps expand: one thread per feature row = one lane of tensor memory, three warps per
@@ -32,9 +32,9 @@
 // All mbarrier waits are bounded; a wait that gives up sets the device error flag, every role waits for
 // its own copies and MMAs (bounded again) and falls through to the common exit.
 //
-// us, of tiles of 128 x 256 or fewer tokens without all this and now (weights from HBM): 4096 x 4096, 37 tokens
-// 13.3 -> 9.3, 300: 26.5 -> 16.3; 4096 x 14336, 37: 29.8 -> 17.0, 300: 60 -> 34.2; 28672 x 4096, 300: 104 -> 62, 2048:
-// 333 (1445 TFLOP/s); 2048 x 8192, 300: 29.2 -> 16.8.
+// us among a few launches (weights from HBM), with a CTA a tile of 32 to 256 tokens and without all this -> now: 4096 x 4096, 40 tokens
+// 13.8 -> 9.4, 300: 26.5 -> 15.2, 1024: 29.6 -> 26.8; 4096 x 14336, 40: 30.1 -> 17.1, 300: 60 -> 33.7; 28672 x 4096, 300: 103 -> 60,
+// 2048: 372 -> 335 (1436 TFLOP/s; single launches 320 to 330); 2048 x 8192, 300: 29.3 -> 16.1, 2048: 53.8 -> 46.2.
 #include <climits>
 #include <mutex>
 

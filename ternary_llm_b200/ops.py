@@ -292,7 +292,7 @@ def ternary_gemv_packed_allreduce(w: PreparedWeight, input, output, ar: FusedAll
 
 
 def ternary_gemm_packed(A, w: PreparedWeight, C, M: int) -> None:
-    """C[M,N] = A[M,K] . W^T on prepared weights (tcgen05 kernel for M > 8)."""
+    """C[M,N] = A[M,K] . W^T on prepared weights, on the kernel for M and the matrix."""
     _dims(w.rows, w.cols, M)
     _lib.check(_lib.lib().tllm_b200_gemm_packed(_chk(A, torch.float16, "A", M * w.cols),
                                                 _chk(w.packed, torch.uint8, "packed weights"),

@@ -122,7 +122,7 @@ class TpLayerStack:
 
     def _matmul(self, w, x, y):
         if self.batch <= 16:
-            ops.ternary_gemv_packed(w, x, y, self.batch)     # up to 8 vectors: streaming GEMV; above: tcgen05 kernel
+            ops.ternary_gemv_packed(w, x, y, self.batch)
         else:
             ops.ternary_gemm_packed(x, w, y, self.batch)
 

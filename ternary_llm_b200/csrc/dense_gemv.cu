@@ -121,6 +121,53 @@ __device__ __forceinline__ void stage_norm(const GemvNorm& f, int m, int K, T* x
     __syncthreads();             // the next vector's sums reuse sh
 }
 
+// ---- what becomes of a row's sum (or of the two sums of a gated pair) -------------------------
+// every lane of the group holds the row's new input v; lane j weighs carried input j (hist), lane
+// taps - 1 the new one
+template <typename T>
+__device__ __forceinline__ void conv_tail(const GemvTail<T>& t, int ch, int width, int m, int l, int lanes_per_row, bool conv, float v, float hist,
+                                          float tw)
+{
+    v = to_f<T>(from_f<T>(v));
+    float s = 0.f;
+    if (conv) s = l + 1 < t.taps ? tw * hist : l + 1 == t.taps ? tw * v : 0.f;
+    for (int o = lanes_per_row >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (!conv) return;
+    T* cr = t.carried + (size_t)(t.first_slot + m) * t.slot_stride + ch;
+    if (l > 0 && l + 1 < t.taps) cr[(size_t)(l - 1) * width] = from_f<T>(hist);
+    if (l + 1 == t.taps && t.taps > 1) cr[(size_t)(t.taps - 2) * width] = from_f<T>(v);
+    if (l == 0) t.out[(size_t)m * t.ld_out + ch] = from_f<T>(apply_act(t.act, s + (t.bias ? t.bias[ch] : 0.f)));
+}
+
+template <typename T>
+__device__ __forceinline__ void gate_tail(const LinearArgs<T>& a, const GemvTail<T>& t, int z, int n, int ch, int m, float r0, float r1, float hist,
+                                          float tw, T x)
+{
+    const float* b = a.bias + (size_t)z * 2 * a.N;
+    const float r = sigmoid_f(r0 + b[n]), i = sigmoid_f(r1 + b[a.N + n]);
+    const float log_a = tw * r, A = decay_exp(log_a, expf(log_a));
+    const float S = fmaf(A, hist, sqrtf(one_minus_exp(2.f * log_a, A * A)) * i * to_f<T>(x));
+    t.state[(size_t)(t.first_slot + m) * t.slot_stride + ch] = S;
+    t.out[(size_t)m * t.ld_out + ch] = from_f<T>(S * apply_act(t.act, to_f<T>(t.y[(size_t)m * t.ld_y + ch])));
+}
+
+// m: row of the vectors, row: row of y
+template <typename T>
+__device__ __forceinline__ void store_output(const LinearArgs<T>& a, int z, int n, int m, int row, float v, float up)
+{
+    if (a.bias) v += a.bias[(size_t)z * a.N + n];
+    if (n >= a.f32_from) {
+        a.y2[(size_t)m * a.ldy2 + n - a.f32_from] = v;
+        return;
+    }
+    if (n >= a.act_lo && n < a.act_hi) v = apply_act(a.act, v, a.act_param);
+    if (a.glu) v *= up;
+    if (a.gate) v *= sigmoid_f(to_f<T>(a.gate[(size_t)m * a.gate_ld + z]));
+    const size_t o = (size_t)row * a.ldy + (size_t)z * a.y_batch + n;
+    if (a.y_f32) static_cast<float*>(a.y)[o] = v;
+    else static_cast<T*>(a.y)[o] = from_f<T>(v);
+}
+
 enum Route { kRouteNone = 0, kRouteEach = 1, kRouteSum = 2 };
 
 // ROUTE (one vector per CTA, blockIdx.y = place in y): the entries of w are chosen from the row's
@@ -277,48 +324,237 @@ dense_gemv_kernel(const LinearArgs<T> a, const GemvNorm f, const GemvTail<T> t, 
             }
         }
         if (TAIL == kTailConv) {
-            // every lane of the group holds the row's new input; lane j weighs carried input j,
-            // lane taps - 1 the new one
 #pragma unroll
-            for (int m = 0; m < MB; m++) {
-                const float v = to_f<T>(from_f<T>(res[0][m] + ((a.bias && valid) ? a.bias[n] : 0.f)));
-                float s = 0.f;
-                if (conv && m < mb) s = l + 1 < t.taps ? tw * hist[m] : l + 1 == t.taps ? tw * v : 0.f;
-                for (int o = lanes_per_row >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (conv && m < mb) {
-                    T* cr = t.carried + (size_t)(t.first_slot + m) * t.slot_stride + ch;
-                    if (l > 0 && l + 1 < t.taps) cr[(size_t)(l - 1) * width] = from_f<T>(hist[m]);
-                    if (l + 1 == t.taps && t.taps > 1) cr[(size_t)(t.taps - 2) * width] = from_f<T>(v);
-                    if (l == 0) t.out[(size_t)m * t.ld_out + ch] = from_f<T>(apply_act(t.act, s + (t.bias ? t.bias[ch] : 0.f)));
-                }
-            }
+            for (int m = 0; m < MB; m++)
+                conv_tail(t, ch, width, m, l, lanes_per_row, conv && m < mb, res[0][m] + ((a.bias && valid) ? a.bias[n] : 0.f), hist[m], tw);
             if (conv) continue;
         }
         if (!valid) continue;
 #pragma unroll
         for (int m = 0; m < MB; m++) {
             if (m >= mb || l != m % lanes_per_row) continue;     // one lane of the group per vector
-            if (TAIL == kTailGate) {
-                const float* b = a.bias + (size_t)z * 2 * a.N;
-                const float r = sigmoid_f(res[0][m] + b[n]), i = sigmoid_f(res[1][m] + b[a.N + n]);
-                const float log_a = tw * r, A = decay_exp(log_a, expf(log_a));
-                const float S = fmaf(A, hist[m], sqrtf(one_minus_exp(2.f * log_a, A * A)) * i * to_f<T>(xs[(size_t)m * a.K + n]));
-                t.state[(size_t)(t.first_slot + m) * t.slot_stride + ch] = S;
-                t.out[(size_t)m * t.ld_out + ch] = from_f<T>(S * apply_act(t.act, to_f<T>(t.y[(size_t)m * t.ld_y + ch])));
-                continue;
+            if (TAIL == kTailGate) gate_tail(a, t, z, n, ch, m, res[0][m], res[1][m], hist[m], tw, xs[(size_t)m * a.K + n]);
+            else store_output(a, z, n, m0 + m, ROUTE ? (int)blockIdx.y : m0 + m, res[0][m], res[1][m]);
+        }
+    }
+}
+
+// ---- one vector ---------------------------------------------------------------------------------
+// The kernel above takes 73 instructions for a piece (eight BF16 weights of a lane) of one vector, which
+// is more than the stream leaves time for, and finishes a row in one lane while its warp waits.  Here a warp
+// walks R rows at once on one read of x (the two rows of a gated pair, or two neighbours) in groups of
+// kPieces pieces that need no test for the end of a row, and multiplies two weights per instruction.
+// A CTA owns neighbouring rows, evenly over the grid; their sums go to shared memory, and once all are there a
+// thread finishes a row.  Bound by HBM: BF16 launches on cold weights in a chain, us, kernel above / here: 2048 x 2048 3.4 / 2.8,
+// 16384 x 2048 16 / 11.7 = 5.8 TB/s, 2048 x 8192 8.5 / 6.8; gate and up of 8192 x 2048 with two norms in the staging 19.6 / 14.3, 8448 x
+// 2048 with a convolution at its end 15.1 / 10.5.  Tried: K split over the warps of a CTA (rows come out even, but every four pieces
+// end in a sum over lanes: 17 us for the gate and up), and the rest of the rows brought to L2 before the wait (no gain).
+__device__ __forceinline__ unsigned long long pair_f32(uint32_t lo, uint32_t hi)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum_pair(unsigned long long v)
+{
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+    return __uint_as_float(lo) + __uint_as_float(hi);
+}
+// 16 bytes of T as pairs of floats
+template <typename T> __device__ __forceinline__ void unpack_pairs(const uint4& v, unsigned long long* p);
+template <> __device__ __forceinline__ void unpack_pairs<bf16>(const uint4& v, unsigned long long* p)
+{
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[i] = pair_f32(w[i] << 16, w[i] & 0xffff0000u);
+}
+template <> __device__ __forceinline__ void unpack_pairs<float>(const uint4& v, unsigned long long* p)
+{
+    p[0] = pair_f32(v.x, v.y);
+    p[1] = pair_f32(v.z, v.w);
+}
+
+constexpr int kHist = 4;       // carried inputs of a channel that are requested before the rows
+
+template <typename T, int R, bool NORM, int TAIL, int ROUTE>
+__global__ void __launch_bounds__(kWarps * 32)
+dense_row_kernel(const LinearArgs<T> a, const GemvNorm f, const GemvTail<T> t)
+{
+    constexpr int V = Vec16<T>::n, kSteps = kPieces / R, kP = V / 2;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ float sh[3 * kWarps];
+    // ring, the vectors, with NORM the norm weights, with ROUTE the choice, the rows' sums
+    T* xs = reinterpret_cast<T*>(smem_raw + kRingBytes);
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int z = ROUTE ? 0 : blockIdx.y;
+    const int xr = ROUTE == kRouteEach ? blockIdx.y / a.route.top : blockIdx.y;
+    const int nv = a.K / V;
+    const bool pairs = R == 2 && (TAIL == kTailGate || a.glu);        // a unit is rows n and N + n, else R neighbours
+    const int width = pairs ? 1 : R, all = (a.N + width - 1) / width;
+    const int n0 = (int)((long long)all * blockIdx.x / gridDim.x) * width;
+    const int n1 = min(a.N, (int)((long long)all * (blockIdx.x + 1) / gridDim.x) * width), rows = n1 - n0;
+    const int parts = ROUTE == kRouteSum ? a.route.top : 1;
+    const int norms = NORM ? (f.w_next != nullptr) + (f.w_post != nullptr) + (f.w_sum != nullptr) : 0;
+    float* wn = reinterpret_cast<float*>(xs + (size_t)parts * a.K);
+    float* wgt = wn + (size_t)norms * a.K;
+    int* idx = reinterpret_cast<int*>(wgt + (ROUTE ? a.route.top : 0));
+    float* sums = reinterpret_cast<float*>(idx + (ROUTE ? a.route.top : 0));
+
+    // piece i of group s of this lane at ring + (s * kPieces + i) * threads
+    const uint4* ring = reinterpret_cast<const uint4*>(smem_raw) + threadIdx.x;
+    const uint32_t ring32 = (uint32_t)__cvta_generic_to_shared(ring);
+    const size_t pitch = (size_t)a.ldw * sizeof(T);
+    const int row_bytes = a.K * (int)sizeof(T);
+    const uint8_t* wz = reinterpret_cast<const uint8_t*>(a.w + (size_t)z * a.w_rows * a.ldw) + lane * 16;
+    // what is requested next: from byte f_off on of part f_part of the unit at row f_n
+    int f_n = n0 + warp * width, f_part = 0, f_off = 0;
+    uint32_t f_dst = ring32;
+    const uint8_t *f_row0 = nullptr, *f_row1 = nullptr;
+    auto request = [&]() {
+        if (f_n < n1) {
+            if (f_off == 0) {
+                const size_t r = ROUTE == kRouteSum ? (size_t)idx[f_part] * a.w_rows + f_n : (size_t)f_n;
+                f_row0 = wz + r * pitch;
+                if (R == 2) f_row1 = f_row0 + (pairs ? (size_t)a.N * pitch : f_n + 1 < n1 ? pitch : 0);    // no second row: the first again
             }
-            float v = res[0][m];
-            if (a.bias) v += a.bias[(size_t)z * a.N + n];
-            if (n >= a.f32_from) {
-                a.y2[(size_t)(m0 + m) * a.ldy2 + n - a.f32_from] = v;
-                continue;
+#pragma unroll
+            for (int u = 0; u < kSteps; u++)
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(f_dst + (uint32_t)((u * R + r) * kWarps * 32 * 16)),
+                                 "l"((r ? f_row1 : f_row0) + f_off + u * 512) : "memory");
+            f_off += kSteps * 512;
+            if (f_off == row_bytes) {
+                f_off = 0;
+                if (++f_part == parts) {
+                    f_part = 0;
+                    f_n += kWarps * width;
+                }
             }
-            if (n >= a.act_lo && n < a.act_hi) v = apply_act(a.act, v, a.act_param);
-            if (a.glu) v *= res[1][m];
-            if (a.gate) v *= sigmoid_f(to_f<T>(a.gate[(size_t)(m0 + m) * a.gate_ld + z]));
-            const size_t o = (size_t)(ROUTE ? (int)blockIdx.y : m0 + m) * a.ldy + (size_t)z * a.y_batch + n;
-            if (a.y_f32) static_cast<float*>(a.y)[o] = v;
-            else static_cast<T*>(a.y)[o] = from_f<T>(v);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        f_dst += kPieces * kWarps * 32 * 16;
+        if (f_dst == ring32 + (uint32_t)kRingBytes) f_dst = ring32;
+    };
+    if (!ROUTE) {
+#pragma unroll
+        for (int g = 0; g < kGroups; g++) request();
+    }
+    if (NORM) {
+        const float* w[3] = {f.w_next, f.w_post, f.w_sum};
+        float* d = wn;
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            if (!w[p]) continue;
+            for (int i = threadIdx.x; i < a.K / 4; i += kWarps * 32) reinterpret_cast<float4*>(d)[i] = gemv_ld4(w[p], i);
+            d += a.K;
+        }
+    }
+
+    pdl_wait();
+    if (ROUTE) {
+        if (warp == 0) choose_experts(a.route.z + (size_t)xr * a.route.ld_z, a.route.experts, a.route.top, idx, wgt);
+        const int n16 = parts * nv;
+        for (int i = (int)threadIdx.x - 32; i < n16; i += (kWarps - 1) * 32)
+            if (i >= 0) reinterpret_cast<uint4*>(xs)[i] = *(reinterpret_cast<const uint4*>(a.x + (size_t)xr * a.ldx) + i);
+        __syncthreads();
+        if (ROUTE == kRouteEach) wz += (size_t)idx[blockIdx.y - xr * a.route.top] * a.w_rows * pitch;
+#pragma unroll
+        for (int g = 0; g < kGroups; g++) request();
+    } else if (NORM) {
+        const float* wp = wn + (f.w_next ? a.K : 0);
+        stage_norm<T>(f, 0, a.K, xs, wp, wp + (f.w_post ? a.K : 0), wn, sh);
+    } else {
+        const uint4* src = reinterpret_cast<const uint4*>(a.x + (size_t)z * a.x_batch);
+        for (int i = threadIdx.x; i < nv; i += kWarps * 32) reinterpret_cast<uint4*>(xs)[i] = src[i];
+    }
+    // what the tail of this thread's first row needs
+    const bool fresh = TAIL != kTailNone && (t.pos_dev ? *t.pos_dev : t.start_pos) == 0;
+    float hist[kHist];
+    const int mine = n0 + (int)threadIdx.x;
+    if (TAIL == kTailConv) {
+#pragma unroll
+        for (int j = 0; j < kHist; j++)
+            hist[j] = (mine < n1 && mine >= t.lo && mine < t.hi && j + 1 < t.taps && !fresh)
+                          ? to_f<T>(t.carried[(size_t)t.first_slot * t.slot_stride + (size_t)j * (t.hi - t.lo) + mine - t.lo]) : 0.f;
+    } else if (TAIL == kTailGate) {
+        hist[0] = (mine < n1 && !fresh) ? t.state[(size_t)t.first_slot * t.slot_stride + (size_t)z * a.N + mine] : 0.f;
+    }
+    __syncthreads();
+
+    const int trips = row_bytes / (kSteps * 512);
+    const uint4* rs = ring;
+    for (int n = n0 + warp * width; n < n1; n += kWarps * width) {
+        float res[R], sum = 0.f;
+        for (int part = 0; part < parts; part++) {
+            unsigned long long acc[R][2];
+#pragma unroll
+            for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = 0ull;
+            const uint4* xp = reinterpret_cast<const uint4*>(xs + (size_t)part * a.K) + lane;
+            for (int i = 0; i < trips; i++) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kGroups - 1) : "memory");
+#pragma unroll
+                for (int s = 0; s < kSteps; s++) {
+                    unsigned long long xf[kP], wf[kP];
+                    unpack_pairs<T>(xp[s * 32], xf);
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        unpack_pairs<T>(rs[(s * R + r) * kWarps * 32], wf);
+#pragma unroll
+                        for (int j = 0; j < kP; j++) fma_pair(acc[r][j & 1], wf[j], xf[j]);
+                    }
+                }
+                request();
+                xp += kSteps * 32;
+                rs += kPieces * kWarps * 32;
+                if (rs == ring + kRingBytes / 16) rs = ring;
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) res[r] = sum_pair(acc[r][0]) + sum_pair(acc[r][1]);
+            if (ROUTE == kRouteSum) res[0] = sum = fmaf(wgt[part], res[0], sum);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int r = 0; r < R; r++) res[r] += __shfl_xor_sync(0xffffffffu, res[r], o);
+        if (lane == 0) {
+            sums[n - n0] = res[0];
+            if (R == 2 && (pairs || n + 1 < n1)) sums[n - n0 + (pairs ? rows : 1)] = res[R - 1];
+        }
+    }
+    __syncthreads();
+
+    for (int n = mine; n < n1; n += kWarps * 32) {
+        const int i = n - n0;
+        const float v = sums[i], up = pairs ? sums[rows + i] : 0.f;
+        if (TAIL == kTailConv && n >= t.lo && n < t.hi) {
+            const int ch = n - t.lo, width = t.hi - t.lo;
+            const T rounded = from_f<T>(v + (a.bias ? a.bias[n] : 0.f));
+            T* cr = t.carried + (size_t)t.first_slot * t.slot_stride + ch;
+            const float* tw = t.w + (size_t)ch * t.taps;
+            float s = t.bias ? t.bias[ch] : 0.f;
+            for (int j = 0; j + 1 < t.taps; j++) {
+                float h;
+                if (j < kHist && n == mine) h = hist[j];
+                else h = fresh ? 0.f : to_f<T>(cr[(size_t)j * width]);
+                s = fmaf(tw[j], h, s);
+                if (j > 0) cr[(size_t)(j - 1) * width] = from_f<T>(h);
+            }
+            s = fmaf(tw[t.taps - 1], to_f<T>(rounded), s);
+            if (t.taps > 1) cr[(size_t)(t.taps - 2) * width] = rounded;
+            t.out[ch] = from_f<T>(apply_act(t.act, s));
+        } else if (TAIL == kTailGate) {
+            const int ch = z * a.N + n;
+            const float h = n == mine ? hist[0] : fresh ? 0.f : t.state[(size_t)t.first_slot * t.slot_stride + ch];
+            gate_tail(a, t, z, n, ch, 0, v, up, h, -t.decay * t.soft_lam[ch], xs[n]);
+        } else {
+            store_output(a, z, n, 0, ROUTE ? (int)blockIdx.y : 0, v, up);
         }
     }
 }
@@ -333,6 +569,46 @@ int row_lanes(int k)
 }
 
 constexpr size_t kSmemLimit = 220 * 1024;
+
+// Returns false where rows are no whole groups of the ring or shared memory does not hold the launch.
+template <typename T, int R, bool NORM, int TAIL, int ROUTE>
+bool launch_rows(const LinearArgs<T>& a, const GemvNorm& f, const GemvTail<T>& t, int ny, cudaStream_t stream, int* st)
+{
+    if (a.K % (kPieces / R * 32 * Vec16<T>::n)) return false;
+    static bool attr[64] = {};
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const auto kernel = dense_row_kernel<T, R, NORM, TAIL, ROUTE>;
+    if (!attr[dev]) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+        cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+        attr[dev] = true;
+    }
+    const bool pairs = TAIL == kTailGate || a.glu;
+    const int units = (R == 2 && !pairs) ? (a.N + 1) / 2 : a.N;
+    int grid = (2 * sms[dev] + ny - 1) / ny;
+    if (grid > units) grid = units;
+    const int norms = NORM ? (f.w_next != nullptr) + (f.w_post != nullptr) + (f.w_sum != nullptr) : 0;
+    const size_t sums = (size_t)((units + grid - 1) / grid) * R * sizeof(float);
+    const size_t smem = kRingBytes + (size_t)(ROUTE == kRouteSum ? a.route.top : 1) * a.K * sizeof(T) + (size_t)norms * a.K * sizeof(float) +
+                        (ROUTE ? (size_t)a.route.top * 8 : 0) + sums;
+    if (smem > kSmemLimit || (NORM && a.K > kNormMaxK)) return false;
+    *st = launch_pdl("dense_gemv", kernel, dim3(grid, ny), dim3(kWarps * 32), smem, stream, a, f, t);
+    return true;
+}
+
+// One vector.  Gated pairs take two rows a warp; other matrices one, which is as quick where both fit (16384 x 2048 BF16 11.7 us, two
+// rows 12.0; 28672 x 4096 38.5 / 39.2; 2048 to 8192 rows equal), and two where K is an odd number of half groups.
+template <typename T, bool NORM, int TAIL, int ROUTE>
+bool launch_one(const LinearArgs<T>& a, const GemvNorm& f, const GemvTail<T>& t, int ny, cudaStream_t stream, int* st)
+{
+    const bool pairs = TAIL == kTailGate || a.glu;
+    if constexpr (TAIL != kTailGate)
+        if (!pairs && launch_rows<T, 1, NORM, TAIL, ROUTE>(a, f, t, ny, stream, st)) return true;
+    if constexpr (ROUTE != kRouteSum) return launch_rows<T, 2, NORM, TAIL, ROUTE>(a, f, t, ny, stream, st);
+    return false;
+}
 
 template <typename T, int MB, bool NORM, int TAIL>
 int launch_mb(const LinearArgs<T>& a, const GemvNorm& f, const GemvTail<T>& t, int m0, cudaStream_t stream)
@@ -355,6 +631,8 @@ int launch_mb(const LinearArgs<T>& a, const GemvNorm& f, const GemvTail<T>& t, i
     const int norms = NORM ? (f.w_next != nullptr) + (f.w_post != nullptr) + (f.w_sum != nullptr) : 0;
     const size_t smem = kRingBytes + (size_t)MB * a.K * sizeof(T) + (size_t)norms * a.K * sizeof(float);
     if (smem > kSmemLimit || (NORM && a.K > kNormMaxK)) return fail(TLLM_ERR_SHAPE, "dense_gemv: %d vectors of %d", MB, a.K);
+    int st = TLLM_OK;
+    if (MB == 1 && a.M == 1 && launch_one<T, NORM, TAIL, kRouteNone>(a, f, t, a.batch, stream, &st)) return st;
     return launch_pdl("dense_gemv", dense_gemv_kernel<T, MB, NORM, TAIL>, dim3(grid, a.batch), dim3(kWarps * 32), smem, stream, a, f, t, lpr, m0);
 }
 
@@ -378,6 +656,8 @@ int launch_routed(const LinearArgs<T>& a, cudaStream_t stream)
     const int lpr = row_lanes<T>(a.K), rows_per_cta = kWarps * (32 / lpr), ny = ROUTE == kRouteSum ? a.M : a.M * a.route.top;
     int grid = (a.N + rows_per_cta - 1) / rows_per_cta;
     const int cap = (2 * sms[dev] + ny - 1) / ny;
+    int st = TLLM_OK;
+    if (launch_one<T, false, kTailNone, ROUTE>(a, GemvNorm(), GemvTail<T>(), ny, stream, &st)) return st;
     if (grid > cap) grid = cap;
     return launch_pdl("dense_gemv_routed", kernel, dim3(grid, ny), dim3(kWarps * 32), smem, stream, a, GemvNorm(), GemvTail<T>(), lpr, 0);
 }

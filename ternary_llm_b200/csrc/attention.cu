@@ -717,6 +717,8 @@ int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache
         items > kDecMaxItems * kAttnThreads || G * head_dim / 2 > 4 * kAttnThreads)
         return fail(TLLM_ERR_SHAPE, "attention: head_dim=%d with %d heads per group is not supported", head_dim, G);
     if (!pos_dev && (pos < 0 || pos >= kv_len_max)) return fail(TLLM_ERR_SHAPE, "attention: pos=%d kv_len_max=%d", pos, kv_len_max);
+    if (attention_step_supported(q, k, v, k_cache, v_cache, n_heads, n_kv_heads, head_dim))
+        return launch_attention_step(q, k, v, k_cache, v_cache, out, batch, n_heads, n_kv_heads, head_dim, kv_len_max, pos, pos_dev, theta, stream);
     DecodeArgs a = {};
     a.q = q;
     a.k = k;

@@ -157,12 +157,12 @@ int linear_multi(LlamaDecoder* D, int count, const PackedW* const* w, half* cons
 // 16384 44.8 / 33.7.
 constexpr int kFusedNormMax = 16384;
 
-// Whether a lock-step token takes the attention that splits each cache into ranges of 64 positions and rotates by itself, or
-// rotation and ranges of 256.  The former saves a launch and has more CTAs, which pays while they are few: a merge of more than
-// 16 ranges of head size 64 and more CTAs than run at the same time cost more than that.  A step, 8 key/value heads, us, by itself /
-// rotation first: 1B model (head size 64) behind 300 positions 4 sequences 753 / 917, 16 (640 CTAs) 1064 / 1075; behind 500 12 (768)
-// 1075 / 1069; behind 1500 2 sequences (24 ranges) 1175 / 1121, 16 2188 / 1389.  Four 8B layers (128): behind 1500 4 sequences
-// (768) 559 / 594, 6 (1152) 613 / 628, 16 (3072) 944 / 909; behind 1000 8 (1024) 609 / 607.
+// Whether a lock-step token of a head size or group that attention_step.cu does not take goes through the attention that splits each
+// cache into ranges of 64 positions and rotates by itself, or through rotation and ranges of 256.  The former saves a launch and has
+// more CTAs, which pays while they are few: a merge of more than 16 ranges of head size 64 and more CTAs than run at the same time
+// cost more than that.  A step, 8 key/value heads of 64, us, by itself / rotation first: behind 300 positions 4 sequences 753 / 917, 16
+// (640 CTAs) 1064 / 1075; behind 500 12 (768) 1075 / 1069; behind 1500 2 sequences (24 ranges) 1175 / 1121, 16 2188 / 1389.  Heads of
+// 128, four layers: behind 1500 4 sequences (768) 559 / 594, 6 (1152) 613 / 628, 16 (3072) 944 / 909; behind 1000 8 (1024) 609 / 607.
 constexpr int kSplitHeads = 128;              // heads that its workspace is made for
 static bool splits_by_itself(int heads, int head_dim, int kv_len)
 {
@@ -250,7 +250,9 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
             half* y[3] = {qb, kb, vb};
             TRY(linear_multi(D, 3, w, y, D->hidden, i8, n, s, &L.qkv));
         }
-        if (seq_n == 1 && (bsz == 1 || splits_by_itself(bsz * c.n_kv_heads, c.head_dim, start_pos + 1))) {        // a token per sequence
+        const bool by_itself = seq_n == 1 && (bsz == 1 || attention_step_supported(qb, kb, vb, D->k_cache, D->v_cache, c.n_heads, c.n_kv_heads, c.head_dim) ||
+                                              splits_by_itself(bsz * c.n_kv_heads, c.head_dim, start_pos + 1));
+        if (by_itself) {        // a token per sequence
             TRY(launch_attention_decode(qb, kb, vb, D->k_cache + kv_off, D->v_cache + kv_off, D->attn_out, bsz, c.n_heads, c.n_kv_heads,
                                         c.head_dim, c.max_seq_len, start_pos, pos_dev, c.rope_theta, D->attn_ws, D->attn_counters, s));
         } else {

@@ -10,6 +10,7 @@
 // before the wait on the previous kernel -- weights depend on nothing in the stream -- and a
 // launch leaves room on the SM for the next one to do the same.
 #include "dense.cuh"
+#include "f32x2.cuh"
 #include "launch.cuh"
 #include "route.cuh"
 
@@ -349,31 +350,15 @@ dense_gemv_kernel(const LinearArgs<T> a, const GemvNorm f, const GemvTail<T> t, 
 // 16384 x 2048 16 / 11.7 = 5.8 TB/s, 2048 x 8192 8.5 / 6.8; gate and up of 8192 x 2048 with two norms in the staging 19.6 / 14.3, 8448 x
 // 2048 with a convolution at its end 15.1 / 10.5.  Tried: K split over the warps of a CTA (rows come out even, but every four pieces
 // end in a sum over lanes: 17 us for the gate and up), and the rest of the rows brought to L2 before the wait (no gain).
-__device__ __forceinline__ unsigned long long pair_f32(uint32_t lo, uint32_t hi)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float sum_pair(unsigned long long v)
-{
-    uint32_t lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-    return __uint_as_float(lo) + __uint_as_float(hi);
-}
 // 16 bytes of T as pairs of floats
-template <typename T> __device__ __forceinline__ void unpack_pairs(const uint4& v, unsigned long long* p);
-template <> __device__ __forceinline__ void unpack_pairs<bf16>(const uint4& v, unsigned long long* p)
+template <typename T> __device__ __forceinline__ void unpack_pairs(const uint4& v, f32x2* p);
+template <> __device__ __forceinline__ void unpack_pairs<bf16>(const uint4& v, f32x2* p)
 {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; i++) p[i] = pair_f32(w[i] << 16, w[i] & 0xffff0000u);
 }
-template <> __device__ __forceinline__ void unpack_pairs<float>(const uint4& v, unsigned long long* p)
+template <> __device__ __forceinline__ void unpack_pairs<float>(const uint4& v, f32x2* p)
 {
     p[0] = pair_f32(v.x, v.y);
     p[1] = pair_f32(v.z, v.w);
@@ -493,7 +478,7 @@ dense_row_kernel(const LinearArgs<T> a, const GemvNorm f, const GemvTail<T> t)
     for (int n = n0 + warp * width; n < n1; n += kWarps * width) {
         float res[R], sum = 0.f;
         for (int part = 0; part < parts; part++) {
-            unsigned long long acc[R][2];
+            f32x2 acc[R][2];
 #pragma unroll
             for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = 0ull;
             const uint4* xp = reinterpret_cast<const uint4*>(xs + (size_t)part * a.K) + lane;
@@ -501,7 +486,7 @@ dense_row_kernel(const LinearArgs<T> a, const GemvNorm f, const GemvTail<T> t)
                 asm volatile("cp.async.wait_group %0;" ::"n"(kGroups - 1) : "memory");
 #pragma unroll
                 for (int s = 0; s < kSteps; s++) {
-                    unsigned long long xf[kP], wf[kP];
+                    f32x2 xf[kP], wf[kP];
                     unpack_pairs<T>(xp[s * 32], xf);
 #pragma unroll
                     for (int r = 0; r < R; r++) {

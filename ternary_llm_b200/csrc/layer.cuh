@@ -50,4 +50,10 @@ int launch_attention_decode(half* q, const half* k, const half* v, half* k_cache
                             int n_kv_heads, int head_dim, int kv_len_max, int pos, const int* pos_dev, float theta,
                             float* ws, unsigned* counters, cudaStream_t stream);
 
+// The same on clusters (attention_step.cu), without scratch; launch_attention_decode takes it where it is supported.
+bool attention_step_supported(const half* q, const half* k, const half* v, const half* k_cache, const half* v_cache, int n_heads, int n_kv_heads,
+                              int head_dim);
+int launch_attention_step(const half* q, const half* k, const half* v, half* k_cache, half* v_cache, half* out, int batch, int n_heads, int n_kv_heads,
+                          int head_dim, int kv_len_max, int pos, const int* pos_dev, float theta, cudaStream_t stream);
+
 }  // namespace tllm

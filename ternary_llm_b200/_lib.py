@@ -146,6 +146,24 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native module csrc/hostcall.c with this library's functions in it."""
+    global _host
+    if _host is None:
+        import torch
+
+        from . import _hostcall
+        h = lib()
+        address = [ctypes.cast(getattr(h, name), _vp).value for name in
+                   ("tllm_b200_gemv_packed", "tllm_b200_gemv_int8_packed", "tllm_b200_gemm_packed")]
+        _hostcall.bind(*address, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, torch.float16, torch.int8, torch.uint8)
+        _host = _hostcall
+    return _host
+
+
 def check(status: int) -> None:
     if status != 0:
         h = lib()

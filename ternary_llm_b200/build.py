@@ -9,7 +9,8 @@ load it instead of the regular library.
 
 The library is a single shared object built from every .cu file under csrc/, each compiled to
 an object of its own (build/, in parallel, only what changed).  nvcc cross-compiles without a
-GPU, so this runs on a CPU-only build machine.
+GPU, so this runs on a CPU-only build machine.  Beside it goes _hostcall.so, the Python module
+of csrc/hostcall.c.
 """
 from __future__ import annotations
 
@@ -18,11 +19,13 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libtllm_b200.so")
+HOST_SRC, HOST_LIB = os.path.join(PKG, "csrc", "hostcall.c"), os.path.join(PKG, "_hostcall.so")
 OBJ_DIR = os.path.join(ROOT, "build")
 
 NVCC_FLAGS = [
@@ -47,7 +50,7 @@ def _older(target: str, deps) -> bool:
 
 
 def _stale() -> bool:
-    return _older(LIB, sources() + headers())
+    return _older(LIB, sources() + headers()) or _older(HOST_LIB, [HOST_SRC])
 
 
 def build(force: bool = False, verbose: bool = False, timeline: bool = False) -> str:
@@ -76,6 +79,10 @@ def build(force: bool = False, verbose: bool = False, timeline: bool = False) ->
         part = out + ".part"
         subprocess.check_call(["nvcc"] + NVCC_FLAGS[:2] + ["-shared", "-o", part] + [obj for _, obj in jobs])
         os.replace(part, out)
+        if force or _older(HOST_LIB, [HOST_SRC]):
+            part = HOST_LIB + ".part"
+            subprocess.check_call(["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-o", part, HOST_SRC])
+            os.replace(part, HOST_LIB)
     return out
 
 

@@ -18,7 +18,8 @@ MAX_BATCH = 16
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # torch.cuda.current_stream().cuda_stream without the object, which takes 3 us to make
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _chk(t: torch.Tensor, dtype, name: str, numel: int | None = None) -> int:
@@ -188,6 +189,9 @@ def prepare_group(weights, register: bool = False, keep_source: bool = False):
 
 def ternary_gemv_packed(w: PreparedWeight, input, output, batch: int = 1) -> None:
     """y[b] = W x[b] on prepared weights, FP16 activations, 1..16 vectors."""
+    status = _lib.host().gemv_packed(w.packed, w.rows, w.cols, input, output, batch)
+    if status is not None:
+        return _lib.check(status)
     _dims(w.rows, w.cols, batch)
     _lib.check(_lib.lib().tllm_b200_gemv_packed(_chk(w.packed, torch.uint8, "packed weights"),
                                                 _chk(input, torch.float16, "input", batch * w.cols),
@@ -197,6 +201,9 @@ def ternary_gemv_packed(w: PreparedWeight, input, output, batch: int = 1) -> Non
 
 def ternary_gemv_int8_packed(w: PreparedWeight, input_int8, input_scale: float, output) -> None:
     """INT8-activation GEMV on prepared weights."""
+    status = _lib.host().gemv_int8_packed(w.packed, w.rows, w.cols, input_int8, input_scale, output)
+    if status is not None:
+        return _lib.check(status)
     _lib.check(_lib.lib().tllm_b200_gemv_int8_packed(_chk(w.packed, torch.uint8, "packed weights"),
                                                      _chk(input_int8, torch.int8, "input_int8", w.cols),
                                                      float(input_scale), _chk(output, torch.float16, "output", w.rows),
@@ -293,6 +300,9 @@ def ternary_gemv_packed_allreduce(w: PreparedWeight, input, output, ar: FusedAll
 
 def ternary_gemm_packed(A, w: PreparedWeight, C, M: int) -> None:
     """C[M,N] = A[M,K] . W^T on prepared weights, on the kernel for M and the matrix."""
+    status = _lib.host().gemm_packed(A, w.packed, w.rows, w.cols, C, M)
+    if status is not None:
+        return _lib.check(status)
     _dims(w.rows, w.cols, M)
     _lib.check(_lib.lib().tllm_b200_gemm_packed(_chk(A, torch.float16, "A", M * w.cols),
                                                 _chk(w.packed, torch.uint8, "packed weights"),

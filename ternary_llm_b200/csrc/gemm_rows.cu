@@ -14,11 +14,15 @@
 //     4t..4t+3 in lane t's four slots, and the B fragment is one 8-byte piece of an activation row.
 //   * Codes and scales go from global memory into registers, D groups ahead, and the first D are
 //     requested before the wait on the previous kernel.
+//   * A code becomes -1, 0 or +1 in FP16 by one logical and one FP16 instruction for two weights (code_f16),
+//     without the scale: the group's sums are multiplied by it in FP32 when they join the others.  (As a byte table
+//     of -s, 0, +s, ten instructions of the slower integer pipe for eight weights instead of five, the pipe was the
+//     bound: 4096 x 14336, four rows, 12.7 us; 9.6 here = 1.6 TB/s of weights.)
 //   * Activations pass through shared memory in stages of KW groups, cp.async, three stages; rows are
 //     padded by 32 bytes so that a fragment load touches every bank once.
 //   * The KW partial sums of a CTA meet in shared memory.  Where there are too few row blocks for the
-//     SMs, a cluster of C CTAs splits the groups; its CTAs add one another's sums over the cluster's
-//     shared memory, in rank order, each for a share of the outputs.
+//     SMs, a cluster of C CTAs splits the groups; a CTA sends its sums to the CTAs that finish them, one barrier
+//     of the cluster later they are added in rank order.
 #include <climits>
 
 #include "launch.cuh"
@@ -36,7 +40,9 @@ struct RowsArgs {
     const uint8_t* packed;
     const half* x;                           // [m, cols]
     RowsOut out[TLLM_MAX_FUSED];             // row ranges of the matrix and where they go; unused ones start past every row
-    int m, cols, groups, nrb, split;
+    int m, cols, groups, nrb;
+    int split, share;                        // CTAs that share a tile's groups; features that one of them finishes, at most
+    uint32_t over_split, over_share;         // 2^32 over the two, rounded up: the upper word of a product with it is a quotient
 };
 
 __device__ __forceinline__ uint32_t sm32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -46,15 +52,26 @@ __device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel)
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(lo), "r"(hi), "r"(sel));
     return r;
 }
+// Two codes of 0, 1, 2 in the field f of a word's halves as the FP16 numbers -1, 0, +1: placed in the mantissa of 1024 they are
+// 1024 + 4^f c, from which one multiplication and addition without rounding makes c - 1.
+template <int SHIFT>
+__device__ __forceinline__ uint32_t code_f16(uint32_t w, int f)
+{
+    uint32_t v;                                              // one instruction for and, or: the compiler makes two of the constants
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(w >> SHIFT), "r"(0x00030003u << (2 * f)), "r"(0x64006400u));
+    const float m = 1.0f / (float)(1 << (2 * f));
+    const half2 r = __hfma2(*reinterpret_cast<const half2*>(&v), __float2half2_rn(m), __float2half2_rn(-1024.0f * m - 1.0f));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid)
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ uint4 ldg_stream(const void* p)
 {
@@ -71,14 +88,16 @@ __device__ __forceinline__ uint32_t ldg_word(const void* p)
 
 template <int NB, int RG, int KW> struct Shape {
     static constexpr int kR = 2;                                     // row blocks per warp
-    static constexpr int kAhead = 3;                                 // groups per warp whose weights are in flight
+    static constexpr int kAhead = NB == 4 ? 2 : 3;                   // groups per warp whose weights are in flight (registers)
     static constexpr int kRows = RG * kR * kTileRows;                // features per CTA
     static constexpr int kLd = KW * kGroup + 16;                     // halves per staged activation row
     static constexpr int kStage = NB * 8 * kLd;                      // halves per stage
     static constexpr int kLdRed = kRows + 4;                         // floats per vector of the partial sums
     static constexpr size_t kX = (size_t)kStages * kStage * sizeof(half);
-    static constexpr size_t kRed = (size_t)(KW + 1) * NB * 8 * kLdRed * sizeof(float);
-    static constexpr size_t kSmem = kX > kRed ? kX : kRed;
+    static constexpr size_t kRed = (size_t)KW * NB * 8 * kLdRed * sizeof(float);
+    static constexpr size_t kMain = kX > kRed ? kX : kRed;
+    static constexpr size_t kSmem = kMain + (size_t)NB * 8 * (kRows + 8) * sizeof(float);   // and what the cluster's CTAs send
+
     static_assert(RG * KW * 32 == kThreads, "eight warps");
 };
 
@@ -92,10 +111,12 @@ gemm_rows_kernel(const RowsArgs a)
     half* xs = reinterpret_cast<half*>(smem_raw);
     float* red = reinterpret_cast<float*>(smem_raw);                 // after the last group
     pdl_launch_dependents();
+    if (a.split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3;
     const int kw = warp % KW, rg = warp / KW;
-    const int rank = blockIdx.x % a.split, tile = blockIdx.x / a.split;
-    const int g0 = (int)((long long)rank * a.groups / a.split), ng = (int)((long long)(rank + 1) * a.groups / a.split) - g0;
+    const int rank = blockIdx.x, tile = blockIdx.y;
+    const int g0 = a.split > 1 ? __umulhi(rank * a.groups, a.over_split) : 0;
+    const int ng = (a.split > 1 ? __umulhi((rank + 1) * a.groups, a.over_split) : a.groups) - g0;
     const int nst = (ng + KW - 1) / KW, mine = (ng - kw + KW - 1) / KW;        // stages; groups of this warp
     const int rb0 = (tile * RG + rg) * R;
 
@@ -127,22 +148,31 @@ gemm_rows_kernel(const RowsArgs a)
             for (int e = 0; e < 4; e++) acc[r][n][e] = 0.f;
 
     pdl_wait();
-    auto stage = [&](int i) {
-        if (i < nst) {
-            const uint32_t dst = sm32(xs + (i % kStages) * S::kStage);
-            const int c0 = (g0 + i * KW) * kGroup, cend = (g0 + ng) * kGroup;
-            constexpr int kPieces = KW * kGroup / 8;
-            for (int p = tid; p < NB * 8 * kPieces; p += kThreads) {
-                const int n = p / kPieces, c = (p - n * kPieces) * 8;
-                const bool v = n < a.m && c0 + c < cend;
-                copy16(dst + (n * S::kLd + c) * 2, v ? a.x + (size_t)n * a.cols + c0 + c : a.x, v);
-            }
+    // a thread's piece (8 columns) of every fourth row; what lies behind the rows and the groups is left as it is, its sums go nowhere
+    constexpr int kPieces = KW * kGroup / 8, kPass = kThreads / kPieces;
+    static_assert(kThreads % kPieces == 0 && kPass == 4, "whole rows");
+    const int piece = tid % kPieces, n0 = tid / kPieces;
+    const half* src = a.x + (size_t)n0 * a.cols + g0 * kGroup + piece * 8;
+    int left = ng * kGroup - piece * 8;                  // columns from this piece on
+    const uint32_t dst0 = sm32(xs) + (uint32_t)(n0 * S::kLd + piece * 8) * 2;
+    uint32_t slot = 0;
+    const size_t pass = (size_t)kPass * a.cols;
+    auto stage = [&]() {
+        if (left > 0) {
+            const half* p = src;
+#pragma unroll
+            for (int u = 0; u < NB * 8 / kPass; u++, p += pass)
+                if (n0 + u * kPass < a.m) copy16(dst0 + slot + u * (kPass * S::kLd * 2), p);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        src += KW * kGroup;
+        left -= KW * kGroup;
+        slot = slot == (kStages - 1) * S::kStage * 2 ? 0 : slot + S::kStage * 2;
     };
 #pragma unroll
-    for (int i = 0; i < kStages - 1; i++) stage(i);
+    for (int i = 0; i < kStages - 1; i++) stage();
 
+    int at = 0;                                          // of stage i in shared memory
     for (int i0 = 0; i0 < nst; i0 += kAhead) {
 #pragma unroll
         for (int d = 0; d < kAhead; d++) {
@@ -150,36 +180,51 @@ gemm_rows_kernel(const RowsArgs a)
             if (i >= nst) break;
             asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
             __syncthreads();                             // stage i is here, stage i - 1 is free
-            stage(i + kStages - 1);
+            stage();
             if (i < mine) {
-                const half* xr = xs + (i % kStages) * S::kStage + gq * S::kLd + kw * kGroup + 4 * t;
-                uint32_t lo[R][2], hi[R][2];
+                const half* xr = xs + at + gq * S::kLd + kw * kGroup + 4 * t;
+                float sum[R][NB][4];
 #pragma unroll
-                for (int r = 0; r < R; r++) {            // byte table of a row: -s, 0, +s for the codes 0, 1, 2
-                    lo[r][0] = (sw[d][r] & 0xffffu) ^ 0x8000u;
-                    hi[r][0] = sw[d][r];
-                    hi[r][1] = sw[d][r] >> 16;
-                    lo[r][1] = hi[r][1] ^ 0x8000u;
+                for (int r = 0; r < R; r++)
+#pragma unroll
+                    for (int n = 0; n < NB; n++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) sum[r][n][e] = 0.f;
+                // bytes 0, 2, 1, 3: columns 4t, 4t + 1 at the same bits of a word's halves, 4t + 2 and 4t + 3 eight bits above
+                uint32_t w[R][4];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    w[r][0] = prmt(cw[d][r].x, 0, 0x3120);
+                    w[r][1] = prmt(cw[d][r].y, 0, 0x3120);
+                    w[r][2] = prmt(cw[d][r].z, 0, 0x3120);
+                    w[r][3] = prmt(cw[d][r].w, 0, 0x3120);
                 }
 #pragma unroll
-                for (int f = 0; f < 4; f++)
+                for (int j2 = 0; j2 < 2; j2++)
 #pragma unroll
-                    for (int j2 = 0; j2 < 2; j2++) {
+                    for (int f = 0; f < 4; f++) {
                         uint2 b[NB];
 #pragma unroll
                         for (int n = 0; n < NB; n++) b[n] = *reinterpret_cast<const uint2*>(xr + n * 8 * S::kLd + 32 * f + 16 * j2);
 #pragma unroll
                         for (int r = 0; r < R; r++) {
-                            const uint32_t s0 = (((j2 ? cw[d][r].y : cw[d][r].x) >> (2 * f)) & 0x03030303u) * 0x22u + 0x10101010u;
-                            const uint32_t s1 = (((j2 ? cw[d][r].w : cw[d][r].z) >> (2 * f)) & 0x03030303u) * 0x22u + 0x10101010u;
-                            const uint32_t fr[4] = {prmt(lo[r][0], hi[r][0], s0), prmt(lo[r][1], hi[r][1], s1),
-                                                    prmt(lo[r][0], hi[r][0], s0 >> 16), prmt(lo[r][1], hi[r][1], s1 >> 16)};
+                            const uint32_t fr[4] = {code_f16<0>(w[r][j2], f), code_f16<0>(w[r][2 + j2], f), code_f16<8>(w[r][j2], f),
+                                                    code_f16<8>(w[r][2 + j2], f)};
 #pragma unroll
-                            for (int n = 0; n < NB; n++) mma_f16(acc[r][n], fr, b[n].x, b[n].y);
+                            for (int n = 0; n < NB; n++) mma_f16(sum[r][n], fr, b[n].x, b[n].y);
                         }
                     }
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const float2 sc = __half22float2(*reinterpret_cast<const half2*>(&sw[d][r]));     // rows gq, gq + 8
+#pragma unroll
+                    for (int n = 0; n < NB; n++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) acc[r][n][e] = fmaf(e < 2 ? sc.x : sc.y, sum[r][n][e], acc[r][n][e]);
+                }
             }
             load(i + kAhead, cw[d], sw[d]);
+            at = at == (kStages - 1) * S::kStage ? 0 : at + S::kStage;
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -194,10 +239,9 @@ gemm_rows_kernel(const RowsArgs a)
             for (int e = 0; e < 4; e++)
                 red[((size_t)kw * NB * 8 + n * 8 + 2 * t + (e & 1)) * S::kLdRed + (rg * R + r) * kTileRows + gq + 8 * (e >> 1)] = acc[r][n][e];
     __syncthreads();
-    float* part = red + KW * NB * 8 * S::kLdRed;
     const int row0 = tile * S::kRows;
-    auto store = [&](int e, float v) {
-        const int n = e / S::kRows, row = row0 + e - n * S::kRows;
+    auto store = [&](int n, int r, float v) {
+        const int row = row0 + r;
         half* y = a.out[0].y;
         int first = 0, rows = a.out[0].rows;
 #pragma unroll
@@ -209,73 +253,115 @@ gemm_rows_kernel(const RowsArgs a)
             }
         if (row - first < rows) y[(size_t)n * rows + row - first] = __float2half_rn(v);
     };
-    for (int e = tid; e < a.m * S::kRows; e += kThreads) {
-        const int n = e / S::kRows, row = e - n * S::kRows;
+    // CTA z of the cluster finishes the features f of all rows with f * split / kRows == z: from first(z) on
+    float* sent = reinterpret_cast<float*>(smem_raw + S::kMain);      // [CTA of the cluster][row][feature of the share]
+    auto first = [&](int z) { return (int)__umulhi(z * S::kRows + a.split - 1, a.over_split); };
+    if (a.split > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // all of them run
+    const int share = a.share;
+    static_assert(kThreads % S::kRows == 0, "a thread's feature is the same in every pass");
+    const int row = tid % S::kRows, to = row * a.split / S::kRows;
+    uint32_t peer = 0;
+    if (a.split > 1) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(sm32(sent + rank * (NB * 8) * share + row - first(to))), "r"(to));
+    for (int n = tid / S::kRows; n < a.m; n += kThreads / S::kRows) {
         float v = 0.f;
 #pragma unroll
         for (int k = 0; k < KW; k++) v += red[((size_t)k * NB * 8 + n) * S::kLdRed + row];
-        if (a.split == 1) store(e, v);
-        else part[n * S::kLdRed + row] = v;
+        if (a.split == 1) store(n, row, v);
+        else asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer + n * share * 4), "f"(v) : "memory");
     }
     if (a.split > 1) {
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        for (int e = rank * kThreads + tid; e < a.m * S::kRows; e += a.split * kThreads) {
-            const int n = e / S::kRows, row = e - n * S::kRows;
-            const uint32_t at = sm32(part + n * S::kLdRed + row);
-            float p[8], v = 0.f;
-#pragma unroll
-            for (int z = 0; z < 8; z++) {
-                p[z] = 0.f;
-                if (z < a.split) {
-                    uint32_t peer;
-                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(z));
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(p[z]) : "r"(peer) : "memory");
-                }
-            }
-#pragma unroll
-            for (int z = 0; z < 8; z++)
-                if (z < a.split) v += p[z];
-            store(e, v);
+        const int f0 = first(rank), mine_f = first(rank + 1) - f0;
+        for (int e = tid; e < a.m * share; e += kThreads) {
+            const int n = __umulhi(e, a.over_share), f = e - n * share;
+            if (f >= mine_f) continue;
+            float v = 0.f;
+            for (int z = 0; z < a.split; z++) v += sent[z * (NB * 8) * share + e];
+            store(n, f0 + f, v);
         }
-        // nobody leaves while its sums are still read
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
 
-// CTAs that run at the same time on the current device, two per SM; 0 without one.
-int cta_slots()
-{
-    static int sms[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    return 2 * sms[dev];
-}
+constexpr int kMaxSplit = 8;
 
-// CTAs that share the scale groups of a tile: as many, a power of two, as run at the same time and have two of them per warp.
-int split_of(int tiles, int groups, int slots)
+// How a product is cut: CTAs that share the scale groups of a tile, and the groups that one of them walks in all rounds of CTAs.
+struct Cut {
+    int split = 0, steps = 0;
+};
+
+// Clusters come in GPCs, so fewer CTAs run at once the larger the cluster; a second round of them costs more than a split saves.
+// Among the splits that run at once, the fewest stages of kGroupWarps groups, of which the exchange in a cluster takes as long as one
+// and a half (1024 x 1024: one CTA and two stages 2.3 us, two CTAs and one 2.7; 512 x 2048: two and two 3.1, four and one 2.6; 8192 x 2048:
+// one and four 5.2, two and two 4.1), then the fewest CTAs.
+template <int NB>
+int cut(int rows, int groups, Cut* c)
 {
-    int split = 1;
-    while (split < 8 && tiles * split * 2 <= slots && groups >= split * 2 * kGroupWarps) split *= 2;
-    return split;
+    using S = Shape<NB, kRowWarps, kGroupWarps>;
+    const auto kernel = gemm_rows_kernel<NB, kRowWarps, kGroupWarps>;
+    static int slots[64][kMaxSplit + 1] = {};            // CTAs that run at once
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
+    if (!slots[dev][1]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
+        }
+        prefer_max_shared(reinterpret_cast<const void*>(kernel));
+        for (int split = kMaxSplit; split >= 1; split--) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at = {};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = split;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(split * 1024);
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = S::kSmem;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+                cudaGetLastError();
+                return fail(TLLM_ERR_LAUNCH, "gemm_rows: clusters of %d do not run", split);
+            }
+            slots[dev][split] = n * split;
+        }
+    }
+    const int tiles = (rows + S::kRows - 1) / S::kRows;
+    int best = INT_MAX;
+    for (int split = 1; split <= kMaxSplit; split++) {
+        if (split > 1 && (tiles * split > slots[dev][split] || groups < split * kGroupWarps)) continue;
+        const int per = (groups + split - 1) / split, cost = 2 * ((per + kGroupWarps - 1) / kGroupWarps) + (split > 1 ? 3 : 0);
+        if (cost >= best) continue;
+        best = cost;
+        c->split = split;
+        c->steps = per * ((tiles * split + slots[dev][split] - 1) / slots[dev][split]);
+    }
+    return TLLM_OK;
+}
+int cut_for(int m, int rows, int groups, Cut* c)
+{
+    switch ((m + 7) / 8) {
+        case 1: return cut<1>(rows, groups, c);
+        case 2: return cut<2>(rows, groups, c);
+        case 3: return cut<3>(rows, groups, c);
+        default: return cut<4>(rows, groups, c);
+    }
 }
 
 template <int NB>
 int launch(RowsArgs a, cudaStream_t stream)
 {
     using S = Shape<NB, kRowWarps, kGroupWarps>;
-    auto kernel = gemm_rows_kernel<NB, kRowWarps, kGroupWarps>;
-    static bool attr[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
-    if (!attr[dev]) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
-        attr[dev] = true;
-    }
-    const int tiles = (a.nrb + S::kRows / kTileRows - 1) / (S::kRows / kTileRows);
-    a.split = split_of(tiles, a.groups, cta_slots());
-    return launch_pdl_cluster("gemm_rows", kernel, a.split, dim3((unsigned)(tiles * a.split)), dim3(kThreads), S::kSmem, stream, a);
+    Cut c;
+    const int st = cut<NB>(a.nrb * kTileRows, a.groups, &c);
+    if (st) return st;
+    a.split = c.split;
+    a.share = (S::kRows + a.split - 1) / a.split;
+    a.over_split = (uint32_t)((0x100000000ull + a.split - 1) / a.split);         // of one CTA not used
+    a.over_share = (uint32_t)((0x100000000ull + a.share - 1) / a.share);
+    const int tiles = (a.nrb * kTileRows + S::kRows - 1) / S::kRows;
+    return launch_pdl_cluster("gemm_rows", gemm_rows_kernel<NB, kRowWarps, kGroupWarps>, a.split, dim3(a.split, tiles), dim3(kThreads),
+                              S::kSmem, stream, a);
 }
 
 }  // namespace
@@ -303,34 +389,33 @@ int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, i
     }
 }
 
-// Where the lines lie.  A CTA here walks its share of the scale groups, one after the other (0.35 us each beside 3 us a launch for
-// 8 rows, 0.42 for 16): the time is steps = groups / split x rounds of CTAs, and the split falls from eight to one as the rows grow past
-// 2368, 4736 and 9472.  The GEMV and the tcgen05 kernel divide their work more evenly.  us among launches of the same kind, weights
-// larger than L2, other / here:
-//   m = 1..3: one GEMV pass is as quick (2048 x 2048, m = 3: 5.6 / 3.2; 14336 x 4096: 7.9 / 12.5), and its block fixed point answers
-//     a non-finite activation with NaN in every output
-//   m = 4, one GEMV pass: with four or more CTAs a tile 4096 x 2048 5.7 / 3.9, 4096 x 8192 9.1 / 8.2, 4096 x 14336 13.9 / 12.9; with
-//     fewer up to eight steps 8192 x 2048 5.5 / 5.2, 16384 x 1024 4.7 / 4.2, behind them 6144 x 4096 7.2 / 7.6, 8192 x 14336
-//     17.1 / 22.9, 14336 x 14336 21.8 / 42.0; longer rows than 20480 leave the GEMV passes of two vectors: 8192 x 24576 64 / 37
-//   m = 5..8, two GEMV passes: two or more CTAs a tile 8192 x 4096 14.2 / 8.3, 8192 x 14336 31.9 / 23.2; one and up to 32 steps 16384 x
-//     4096 17.0 / 13.6; more: 10240 x 6144, m = 5 16.6 / 18.3; 28672 x 4096, m = 8 21.3 / 24.3
-//   m = 9..16, tcgen05: eight CTAs a tile 2048 x 28672 18.1 / 15.9; two or four up to 16 steps 8192 x 4096 10.8 / 9.7, 4096 x 8192 11.3 /
-//     9.8; more 3072 x 14336 13.5 / 14.6, 3072 x 28672 21.4 / 26.3; one up to 8 steps 16384 x 1024 6.1 / 5.1, 16 steps 10240 x 2048
-//     8.0 / 8.4
-//   m = 17..24: eight CTAs a tile, or up to 8 steps in two: 4096 x 4096 9.0 / 8.0; 4096 x 8192 11.8 / 12.1
-//   m = 25..32: up to 8 steps in four: 2048 x 2048 6.6 / 6.5; 6144 x 4096 10.7 / 13.9
+// Where the lines lie.  A CTA here walks its share of the scale groups in stages of four (0.9 us for 8 rows, 1.2 for 16, 1.8 for 24, two CTAs
+// on an SM) beside 2.5 us a launch; the split falls from eight to one as the rows grow past 2112, 4544 and 9472.  The GEMV and the
+// tcgen05 kernel divide their work more evenly.  us among launches of the same kind, weights larger than L2, other / here:
+//   m = 1..3: one GEMV pass is as quick (14336 x 4096: 7.9 / 10), and its block fixed point answers a non-finite activation
+//     with NaN in every output
+//   m = 4, one GEMV pass: 4096 x 2048 5.7 / 3.0, 4096 x 14336 13.9 / 9.6, 6144 x 4096 7.0 / 6.0, 16384 x 2048 6.7 / 5.8, 16384 x 3072 (24
+//     steps) 7.8 / 7.9, 14336 x 4096 (32) 8.4 / 10.2, 8192 x 14336 (56) 16.9 / 17.3; longer rows than 20480 leave the GEMV passes of two
+//     vectors: 8192 x 24576 64 / 37 before these figures
+//   m = 5..8, two GEMV passes: quicker everywhere, 512 x 2048 9.6 / 2.6, 28672 x 4096 22.1 / 19.8, 14336 x 14336 41 / 33
+//   m = 9..16, tcgen05: 2048 x 14336 11.7 / 8.2, 8192 x 14336 (two CTAs, 56 steps) 25.1 / 22.8, 14336 x 4096 (one, 32) 13.7 / 13.1 - 13.4, 28672
+//     x 4096 (one, 64) 24.0 / 24.1 - 25.3, 14336 x 1280 (one, 10) 6.4 / 5.6 - 6.1, 12800 x 1664 (one, 13) 7.2 / 7.1 - 7.7
+//   m = 17..24: 2048 x 14336 12.0 / 10.3, 4096 x 14336 (four CTAs, 28 steps) 16.0 / 15.1 - 16.0, 8192 x 2048 (two, 8) 7.2 / 6.8, 6144 x 4096
+//     (two, 16) 10.4 / 10.1 - 10.7, 4600 x 8192 (three, 22) 12.9 / 13.3 - 14.2, 1024 x 1024 (one, 8) 4.4 / 3.6 - 4.0, 10240 x 1024 5.5 / 5.4 - 6.0
+//   m = 25..32: 2048 x 8192 (eight, 8) 9.3 / 8.6, 4096 x 4096 (four, 8) 8.9 / 7.4 - 7.8, 2048 x 14336 (eight, 14) 12.0 / 12.6, 1024 x
+//     1024 4.4 / 4.7
 bool linear_takes_rows(int m, int rows, int cols)
 {
     if (m < 4 || m > kRowsMax) return false;
-    const int slots = cta_slots(), groups = cols / kGroup, per = Shape<1, kRowWarps, kGroupWarps>::kRows, tiles = (rows + per - 1) / per;
-    if (!slots || !groups) return false;
-    const int split = split_of(tiles, groups, slots);
-    const long long rounds = ((long long)tiles * split + slots - 1) / slots, steps = (groups + split - 1) / split * rounds;
-    if (m == 4) return split >= 4 || steps <= 8 || cols > 20480;
-    if (m <= 8) return split >= 2 || steps <= 32 || cols > 20480;
-    if (m <= 16) return split == 8 || steps <= (split > 1 ? 16 : 8);
-    if (m <= 24) return split == 8 || (split > 1 && steps <= 8);
-    return split >= 4 && steps <= 8;
+    const int groups = cols / kGroup;
+    Cut c;
+    if (!groups || cut_for(m, rows, groups, &c)) return false;
+    const int split = c.split, steps = c.steps;
+    if (m == 4) return split >= 4 || steps <= 20 || cols > 20480;
+    if (m <= 8) return true;
+    if (m <= 16) return split > 1 || steps <= (m <= 12 ? 32 : 10);
+    if (m <= 24) return split >= 7 || (split >= 4 && steps <= 28) || (steps <= 8 && (split > 1 || rows <= 4736));
+    return split >= 3 && steps <= 12;
 }
 
 // Matrices packed back to back on this kernel or the tcgen05 GEMM (m > 8, or where this one is taken).

@@ -29,6 +29,24 @@ def test_rows(m, n, k):
     assert (np.abs(got[:m] - y64) <= bound).all(), np.max(np.abs(got[:m] - y64) / bound)
 
 
+@pytest.mark.parametrize("k", [7168, 6784])
+@pytest.mark.parametrize("n", [500, 2113, 2700, 3300, 4544, 5800, 9472])
+def test_clusters_of_all_sizes(n, k):
+    """Eight to one CTAs that share 56 or 53 groups of a tile, whose shares of the groups and of the 64 features are uneven."""
+    nz, sg, sc, x = oracle.make_case(n, k, seed=n + k, batch=32)
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (nz, sg, sc, x)]
+    w = tl.PreparedWeight(*dev[:3], n, k, register=False)
+    wd = torch.from_numpy(oracle.unpack_bitmasks(nz, sg).astype(np.float32) * np.repeat(sc.astype(np.float32), 128, axis=1)).cuda().double()
+    want, size = dev[3].double() @ wd.T, dev[3].double().abs() @ wd.T.abs()
+    for m in (4, 7, 13, 24, 32):
+        y = torch.full((m + 1, n), 7.0, dtype=torch.float16, device="cuda")
+        tl.ternary_gemm_packed(dev[3], w, y, m)
+        assert (y[m] == 7.0).all()
+        bound = k * 2.0 ** -24 * size[:m] + 2.0 ** -11 * want[:m].abs() + 2.0 ** -25      # as above
+        assert ((y[:m].double() - want[:m]).abs() <= bound).all(), m
+    tl.check_device_errors()
+
+
 @pytest.mark.parametrize("n", [2368, 2369, 4736, 4737, 9472, 9473])
 def test_both_sides_of_the_lines(n):
     """Where a tile's CTAs go from eight to four, two and one, and with them the kernel of a number of vectors."""

@@ -26,6 +26,12 @@ __device__ __forceinline__ f32x2 mul_pair(f32x2 a, f32x2 b)
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ f32x2 add_pair(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ float sum_pair(f32x2 v)
 {
     const float2 f = split_f32(v);

@@ -109,14 +109,6 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// One lane of a converged warp.
-__device__ __forceinline__ bool elect_one()
-{
-    uint32_t p;
-    asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
-    return p != 0;
-}
-
 // A place in a ring of n slots: the slot and the parity of its uses.
 struct Ring {
     int slot = 0;

@@ -20,12 +20,16 @@
 //
 // FP16, 32 heads over 8 key/value heads, one launch among others, against the form with a CTA per query
 // and key/value head on the CUDA cores (attention.cu), which read every position once per query: 2000
-// queries 2210 -> 116 us (head size 64), 6733 -> 127 us (128); 300 queries 82 -> 15 and 256 -> 17 us;
-// 2 queries behind 1000 positions 35.7 -> 33.3 and 60 -> 36 us.  few_queries has the calls that stay there.
+// queries 2210 -> 76 us (head size 64), 6733 -> 90 us (128); 300 queries 82 -> 12.6 and 256 -> 15.7 us.  few_queries has the calls
+// that stay there.  Bound by the chain of a tile (product, softmax, product, 3.5 us), which two CTAs an SM hide in part.  Its
+// longest link is the softmax, a row per thread: two scores per instruction where there is one for it and no mask but in the tiles that
+// need one; with a mask in every tile and one score at a time 2000 queries took 117 and 130 us, 300 16.1 and 17.9.  The MMAs and
+// copies are issued by an elected lane of a warp that runs the loop together (2000 queries 85 -> 76, 96 -> 90).
 // All mbarrier waits are bounded (see dense_gemm.cu).
 #include <cfloat>
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "launch.cuh"
 #include "layer.cuh"
 #include "mixers.cuh"
@@ -106,6 +110,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
                  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
                  "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
                  "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -201,18 +211,19 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
     if (warp == 4) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int issued = 0;                                     // tiles whose copies were issued: keys, then values
-            const int head_row = (seq * a.kv_heads + g) * a.head_rows;
+        const bool leader = elect_one();
+        int issued = 0;                                         // tiles whose copies were issued: keys, then values
+        bool ok = true;
+        const int head_row = (seq * a.kv_heads + g) * a.head_rows;
+        if (leader) {
             mbar_expect_tx(bar(kQFull), nd * kBlock);
             for (int j = 0; j < nd; j++) tma_load_2d(qs + j * kBlock, &map_q, h * a.dim + j * 64, seq * a.n + q0, bar(kQFull));
-            for (int i = 0; i < 2 * tiles; i++, issued++) {
-                const int t = i >> 1, row = head_row + (lo + t * kTile) % a.cache_rows;
-                const bool v = i & 1;
-                if (!mbar_wait(bar(v ? kVEmpty : kKEmpty), (t & 1) ^ 1, abortp)) {
-                    abort_flag = 1;
-                    break;
-                }
+        }
+        for (int i = 0; i < 2 * tiles; i++, issued++) {
+            const int t = i >> 1, row = head_row + (lo + t * kTile) % a.cache_rows;
+            const bool v = i & 1;
+            if (!(ok = mbar_wait(bar(v ? kVEmpty : kKEmpty), (t & 1) ^ 1, abortp))) break;
+            if (leader) {
                 const int blocks = v ? ne : nd;
                 mbar_expect_tx(bar(v ? kVFull : kKFull), blocks * kBlock);
                 for (int j = 0; j < blocks; j++) {
@@ -220,46 +231,57 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     else tma_load_2d(ks + j * kBlock, &map_k, g * a.k_cols + j * 64, row, bar(kKFull));
                 }
             }
-            // after an abort the copies still in flight must land before the shared memory goes away
-            if (*abortp) {
-                mbar_wait(bar(kQFull), 0, &never);
-                if (issued > 0) mbar_wait(bar(kKFull), ((issued - 1) >> 1) & 1, &never);
-                if (issued > 1) mbar_wait(bar(kVFull), ((issued - 2) >> 1) & 1, &never);
-            }
+        }
+        if (!ok) abort_flag = 1;
+        __syncwarp();
+        // after an abort the copies still in flight must land before the shared memory goes away
+        if (*abortp) {
+            mbar_wait(bar(kQFull), 0, &never);
+            if (issued > 0) mbar_wait(bar(kKFull), ((issued - 1) >> 1) & 1, &never);
+            if (issued > 1) mbar_wait(bar(kVFull), ((issued - 2) >> 1) & 1, &never);
         }
     } else if (warp == 5) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t id_s = idesc<T>(kTile, false), id_o = idesc<T>(a.vdim, true);
-            bool ok = mbar_wait(bar(kQFull), 0, abortp);
-            int done = 0;                                       // tiles whose last product was issued
-            for (int t = 0; ok && t < tiles; t++) {
-                // the weights of the tile before lie where S goes
-                ok = (t == 0 || mbar_wait(bar(kPvDone), (t - 1) & 1, abortp)) && mbar_wait(bar(kKFull), t & 1, abortp);
-                if (!ok) break;
-                fence_after();
-                for (int k = 0; k < a.dim / 16; k++) {
-                    const uint32_t o = (k >> 2) * kBlock + (k & 3) * 32;
-                    mma_ss(tmem, make_sw128_desc(qs + o), make_sw128_desc(ks + o), id_s, k > 0);
-                }
+        const bool leader = elect_one();
+        const uint32_t id_s = idesc<T>(kTile, false), id_o = idesc<T>(a.vdim, true);
+        const uint64_t qd = make_sw128_desc(qs), kd = make_sw128_desc(ks), vd = feature_major_desc(vs);
+        bool ok = mbar_wait(bar(kQFull), 0, abortp);
+        int done = 0;                                           // tiles whose last product was issued
+        for (int t = 0; ok && t < tiles; t++) {
+            // the weights of the tile before lie where S goes
+            ok = (t == 0 || mbar_wait(bar(kPvDone), (t - 1) & 1, abortp)) && mbar_wait(bar(kKFull), t & 1, abortp);
+            if (!ok) break;
+            fence_after();
+            if (leader) {
+                for (int j = 0; j < nd; j++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {               // 32 bytes (2 in the descriptor) inside the swizzled row
+                        const uint32_t o = j * (kBlock >> 4) + k * 2;
+                        mma_ss(tmem, qd + o, kd + o, id_s, j > 0 || k > 0);
+                    }
                 mma_commit(bar(kKEmpty));
                 mma_commit(bar(kSFull));
-                ok = mbar_wait(bar(kVFull), t & 1, abortp) && mbar_wait(bar(kPReady), t & 1, abortp);
-                if (!ok) break;
-                fence_after();
+            }
+            ok = mbar_wait(bar(kVFull), t & 1, abortp) && mbar_wait(bar(kPReady), t & 1, abortp);
+            if (!ok) break;
+            fence_after();
+            if (leader) {
+#pragma unroll
                 for (int part = 0; part < 2; part++)
+#pragma unroll
                     for (int k = 0; k < kTile / 16; k++)
-                        mma_ts(tmem_o, tmem + part * 64 + k * 8, feature_major_desc(vs + k * 2048), id_o, t > 0 || part > 0 || k > 0);
+                        mma_ts(tmem_o, tmem + part * 64 + k * 8, vd + k * (2048 >> 4), id_o, t > 0 || part > 0 || k > 0);
                 mma_commit(bar(kVEmpty));
                 mma_commit(bar(kPvDone));
-                done++;
             }
-            if (!ok) {
-                abort_flag = 1;
-                // what was issued completes before the memory is given up
-                mma_commit(bar(kPvDone));
-                mbar_wait(bar(kPvDone), done & 1, &never);
-            }
+            done++;
+        }
+        if (!ok) {
+            abort_flag = 1;
+            // what was issued completes before the memory is given up
+            if (leader) mma_commit(bar(kPvDone));
+            __syncwarp();
+            mbar_wait(bar(kPvDone), done & 1, &never);
         }
     } else if (warp < 4) {
         // ---------------- softmax: a row per thread ----------------
@@ -272,23 +294,30 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             ok = __all_sync(0xffffffffu, mbar_wait(bar(kSFull), t & 1, abortp));
             if (!ok) break;
             fence_after();
-            uint32_t s[4][32];
+            uint32_t raw[4][32];
             __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 4; i++) tmem_ld32(row_s + i * 32, s[i]);
+            for (int i = 0; i < 4; i++) tmem_ld32(row_s + i * 32, raw[i]);
             wait_ld();
-            const bool edge = k0 + kTile > first + 1 || k0 < lo_last;         // some (query, position) pair of the tile is masked
-            float mx = -INFINITY;
+            f32x2 s[64];                                                      // scores of two positions each
+            const f32x2 scale = pair_f32(a.scale2, a.scale2);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 64; i++) s[i] = mul_pair(pair_f32(raw[i >> 4][2 * (i & 15)], raw[i >> 4][2 * (i & 15) + 1]), scale);
+            if (k0 + kTile > first + 1 || k0 < lo_last) {                     // some (query, position) pair of the tile is masked
+                const int seen = pos - k0, unseen = from - k0;                // the last and the first that this row sees
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    float v = __uint_as_float(s[i][j]) * a.scale2;
-                    const int p = k0 + i * 32 + j;
-                    if (edge && (p > pos || p < from)) v = -INFINITY;
-                    s[i][j] = __float_as_uint(v);
-                    mx = fmaxf(mx, v);
+                for (int i = 0; i < 64; i++) {
+                    const float2 v = split_f32(s[i]);
+                    s[i] = pair_f32(2 * i > seen || 2 * i < unseen ? -INFINITY : v.x, 2 * i + 1 > seen || 2 * i + 1 < unseen ? -INFINITY : v.y);
                 }
+            }
+            float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int i = 0; i < 64; i++) {
+                const float2 v = split_f32(s[i]);
+                top[i & 3] = fmaxf(top[i & 3], fmaxf(v.x, v.y));
+            }
+            const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
             const bool grows = mx > m + Op::kSlack || (m == -INFINITY && mx > m);
             if (__any_sync(0xffffffffu, grows)) {
                 const float f = grows ? exp2_neg(m - mx) : 1.f;               // 0 where nothing was seen before
@@ -308,24 +337,29 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     }
                 }
             }
-            const float ref = (m == -INFINITY ? 0.f : m) - Op::kLift;
+            const float ref = Op::kLift - (m == -INFINITY ? 0.f : m);
+            const f32x2 off = pair_f32(ref, ref);
+            f32x2 sum[2] = {0ull, 0ull};
 #pragma unroll
-            for (int half = 0; half < 2; half++) {                            // 64 positions: 32 words of high, 32 of low parts
-                uint32_t ph[32], pl[32];
+            for (int part = 0; part < 4; part++) {                            // 32 positions: 16 words of high, 16 of low parts
+                uint32_t ph[16], pl[16];
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const float p0 = exp2_neg(__uint_as_float(s[2 * half + (j >> 4)][2 * (j & 15)]) - ref);
-                    const float p1 = exp2_neg(__uint_as_float(s[2 * half + (j >> 4)][2 * (j & 15) + 1]) - ref);
-                    l += p0 + p1;
-                    const typename Op::Pair b = Op::pair(p0, p1);
+                for (int j = 0; j < 16; j++) {
+                    const float2 e = split_f32(add_pair(s[part * 16 + j], off));
+                    const f32x2 p = pair_f32(exp2_neg(e.x), exp2_neg(e.y));
+                    sum[j & 1] = add_pair(sum[j & 1], p);
+                    const float2 pf = split_f32(p);
+                    const typename Op::Pair b = Op::pair(pf.x, pf.y);
                     const float2 r = Op::floats(b);
-                    const typename Op::Pair c = Op::pair(p0 - r.x, p1 - r.y);
+                    const float2 low = split_f32(add_pair(p, pair_f32(-r.x, -r.y)));
+                    const typename Op::Pair c = Op::pair(low.x, low.y);
                     ph[j] = *reinterpret_cast<const uint32_t*>(&b);
                     pl[j] = *reinterpret_cast<const uint32_t*>(&c);
                 }
-                tmem_st32(row_s + half * 32, ph);
-                tmem_st32(row_s + 64 + half * 32, pl);
+                tmem_st16(row_s + part * 16, ph);
+                tmem_st16(row_s + 64 + part * 16, pl);
             }
+            l += sum_pair(add_pair(sum[0], sum[1]));
             if (k0 + kTile > hi) {
                 // rows of the cache behind the last query hold anything: their weights are 0, their values become 0
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(kVFull), t & 1, abortp));

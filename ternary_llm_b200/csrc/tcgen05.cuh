@@ -43,6 +43,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return false;
 }
 
+// One lane of the warp.  A role that issues copies or MMAs runs its loop with all lanes and lets this one issue: the loop of a
+// single thread keeps descriptors in its own registers, and moving them to the issuing unit costs some 80 clocks an MMA.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar)
 {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"

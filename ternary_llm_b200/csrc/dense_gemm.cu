@@ -2,7 +2,14 @@
 // with FP32 accumulation in tensor memory and the element-wise tail of the operator (bias,
 // activation, gated product, per-head gate) in the epilogue.
 //
-// A tile is 128 tokens x TN features.  One persistent CTA per SM walks tiles with three roles
+// A tile is 128 tokens x TN features, or 256 tokens x TN features of a pair of CTAs (PAIR,
+// cta_group::2): each loads its 128 tokens and half of the features' weights and keeps the sums of
+// its tokens, the first one issues the MMAs of both.  What bounds a tile is the copies of its operands into
+// shared memory (64 bytes a clock and SM): 48 KB for 64 columns of K and 256 features, 32 KB a CTA of a
+// pair.  Gate and up of 8192 x 2048, 2000 tokens: 92 -> 81 us = 1.66 PFLOP/s in a prompt; in tiles of 64
+// and 128 features what bounded was the loop of one thread that issued the MMAs (2048 x 8192, 100 tokens
+// 40.5 -> 29.2 us with the loop run by a warp and one elected lane).
+// One persistent CTA per SM walks tiles with three roles
 // that run ahead of one another: a TMA producer (K-major tiles of 64 columns, 128-byte swizzle;
 // out-of-range rows and columns read as zero, so no size needs to divide a tile), one thread
 // that issues tcgen05.mma kind::f16 (M = 128, N = TN, K = 16) into one of two accumulators in
@@ -32,12 +39,12 @@ constexpr int kThr = 128 + 32 * kEpiWarps;
 
 constexpr int kStageLd = 20;         // words per row of an epilogue warp's tile: 16 of data (16 FP32 or 32 BF16 columns)
 
-template <int TN>
+template <int TN, bool PAIR>
 struct DCfg {
     static constexpr int kXBytes = kTok * kBlkK * 2;
-    static constexpr int kWBytes = TN * kBlkK * 2;
+    static constexpr int kWBytes = TN * kBlkK * 2 / (PAIR ? 2 : 1);
     static constexpr int kStage = kXBytes + kWBytes;
-    static constexpr int kStages = (TN == 256) ? 4 : (TN == 128) ? 6 : 8;
+    static constexpr int kStages = PAIR ? (TN == 256 ? 6 : 8) : (TN == 256) ? 4 : (TN == 128) ? 6 : 8;
     static constexpr int kEpiBytes = kEpiWarps * 32 * kStageLd * 4;
     static constexpr size_t kSmem = (size_t)kStages * kStage + kEpiBytes + 1024;
 };
@@ -57,25 +64,71 @@ struct DenseEpi {
     int* err;
 };
 
-template <int TN>
+template <int TN, bool PAIR>
 __device__ __forceinline__ uint32_t idesc_bf16()
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kTok >> 4) << 24);
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)((PAIR ? 2 * kTok : kTok) >> 4) << 24);
 }
 
+template <bool PAIR>
 __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
 {
-    asm volatile(
-        "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }"
+            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+    else
+        asm volatile(
+            "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
+            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+// arrives, once everything issued so far is complete, at this barrier of the CTA, or of both CTAs of the pair
+template <bool PAIR>
+__device__ __forceinline__ void commit(uint32_t bar)
+{
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else
+        mma_commit(bar);
+}
+// the copy's bytes count on `bar`, of the pair's first CTA for both
+template <bool PAIR>
+__device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar)
+{
+    if constexpr (PAIR)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+    else
+        tma_load_2d(dst, map, x, y, bar);
+}
+__device__ __forceinline__ uint32_t in_first_cta(uint32_t addr)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// all threads of the CTA, or of the pair
+template <bool PAIR>
+__device__ __forceinline__ void sync_all()
+{
+    __syncwarp();
+    if constexpr (PAIR) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
 }
 
-template <int TN>
+template <int TN, bool PAIR>
 __global__ void __launch_bounds__(kThr, 1)
 dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const DenseEpi a)
 {
-    constexpr int kStages = DCfg<TN>::kStages, kStage = DCfg<TN>::kStage, kXBytes = DCfg<TN>::kXBytes;
+    using Cfg = DCfg<TN, PAIR>;
+    constexpr int kStages = Cfg::kStages, kStage = Cfg::kStage, kXBytes = Cfg::kXBytes;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
@@ -84,6 +137,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int outs = a.glu ? TN / 2 : TN;              // output features of a tile
+    const int rank = PAIR ? blockIdx.x & 1 : 0;        // CTA of the pair: its half of the tile's tokens and of its rows of W
+    const int first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x, step_tiles = PAIR ? gridDim.x >> 1 : gridDim.x;
     const int nk = (a.K + kBlkK - 1) / kBlkK;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * s; };
@@ -98,19 +153,25 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(acc_full(i), 1);
-            mbar_init(acc_empty(i), 32 * kEpiWarps);
+            mbar_init(acc_empty(i), PAIR ? 2 * kEpiWarps : 32 * kEpiWarps);
         }
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_slot)), "r"(2 * TN) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(&tmem_slot)), "r"(2 * TN) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(&tmem_slot)), "r"(2 * TN) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    sync_all<PAIR>();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
     volatile int* abortp = &abort_flag;
@@ -129,7 +190,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             entry = g[0];
             return;
         }
-        m0 = (tile % a.mt) * kTok;
+        m0 = (tile % a.mt) * (PAIR ? 2 * kTok : kTok) + rank * kTok;
         tile /= a.mt;
         n0 = (tile % a.nt) * outs;
         entry = z = tile / a.nt;
@@ -137,67 +198,77 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int it = 0;                                  // stages filled so far, over all tiles
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-                int m0, n0, z, entry;
-                where(tile, m0, n0, z, entry);
-                const int wr0 = entry * a.w_rows + n0, wr1 = a.glu ? wr0 + a.N : wr0 + TN / 2;
-                for (int k = 0; k < nk; k++, it++) {
-                    const int s = it % kStages;
-                    if (!mbar_wait(empty(s), ((it / kStages) & 1) ^ 1, abortp)) {
-                        abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    mbar_expect_tx(full(s), kStage);
-                    const uint32_t dst = smem_u32(smem + (size_t)s * kStage);
-                    tma_load_2d(dst, &map_x, z * a.x_batch + k * kBlkK, m0, full(s));
-                    tma_load_2d(dst + kXBytes, &map_w, k * kBlkK, wr0, full(s));
-                    tma_load_2d(dst + kXBytes + TN / 2 * kBlkK * 2, &map_w, k * kBlkK, wr1, full(s));
+        const bool leader = elect_one();
+        int s = 0, phase = 1, used = 0;                  // stage, parity that means empty; stages filled, up to all of them
+        bool ok = true;
+        for (int tile = first_tile; ok && tile < tiles; tile += step_tiles) {
+            int m0, n0, z, entry;
+            where(tile, m0, n0, z, entry);
+            const int wr0 = entry * a.w_rows + n0, wr1 = a.glu ? wr0 + a.N : wr0 + TN / 2, x0 = z * a.x_batch;
+            for (int k = 0; k < nk; k++) {
+                if (!(ok = mbar_wait(empty(s), phase, abortp))) break;
+                if (leader) {
+                    if (rank == 0) mbar_expect_tx(full(s), PAIR ? 2 * kStage : kStage);
+                    const uint32_t dst = smem_u32(smem + (size_t)s * kStage), bar = PAIR ? in_first_cta(full(s)) : full(s);
+                    load_tile<PAIR>(dst, &map_x, x0 + k * kBlkK, m0, bar);
+                    load_tile<PAIR>(dst + kXBytes, &map_w, k * kBlkK, rank ? wr1 : wr0, bar);
+                    if (!PAIR) load_tile<PAIR>(dst + kXBytes + TN / 2 * kBlkK * 2, &map_w, k * kBlkK, wr1, bar);
+                }
+                used = min(used + 1, kStages);
+                if (++s == kStages) {
+                    s = 0;
+                    phase ^= 1;
                 }
             }
-            // normally the MMAs consume every stage; after an abort the copies still in flight
-            // must land before the shared memory goes away
-            if (*abortp)
-                for (int j = it > kStages ? it - kStages : 0; j < it; j++) mbar_wait(full(j % kStages), (j / kStages) & 1, &never);
         }
-    } else if (warp == 1) {
+        if (!ok) abort_flag = 1;
+        __syncwarp();
+        // normally the MMAs consume every stage; after an abort the copies still in flight
+        // must land before the shared memory goes away
+        if (*abortp && rank) __nanosleep(1000000);       // they count on the other CTA's barriers, which waits for them
+        if (*abortp && rank == 0)
+            for (; used > 0; used--) {
+                if (--s < 0) {
+                    s = kStages - 1;
+                    phase ^= 1;
+                }
+                mbar_wait(full(s), phase ^ 1, &never);
+            }
+    } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16<TN>();
-            int it = 0, i = 0;                           // i: tiles of this CTA so far
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, i++) {
-                const int buf = i & 1;
-                if (!mbar_wait(acc_empty(buf), ((i >> 1) & 1) ^ 1, abortp)) {
-                    abort_flag = 1;
-                    break;
-                }
+        const bool leader = elect_one();
+        const uint32_t idesc = idesc_bf16<TN, PAIR>();
+        int s = 0, phase = 0, i = 0;                     // i: tiles of this CTA so far
+        bool ok = true;
+        for (int tile = first_tile; ok && tile < tiles; tile += step_tiles, i++) {
+            const int buf = i & 1;
+            if (!(ok = mbar_wait(acc_empty(buf), ((i >> 1) & 1) ^ 1, abortp))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem + buf * TN;
+            for (int k = 0; k < nk; k++) {
+                if (!(ok = mbar_wait(full(s), phase, abortp))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + buf * TN;
-                for (int k = 0; k < nk; k++, it++) {
-                    const int s = it % kStages;
-                    if (!mbar_wait(full(s), (it / kStages) & 1, abortp)) {
-                        abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t xb = smem_u32(smem + (size_t)s * kStage), wb = xb + kXBytes;
+                const uint64_t xd = make_sw128_desc(smem_u32(smem + (size_t)s * kStage)), wd = make_sw128_desc(smem_u32(smem + (size_t)s * kStage + kXBytes));
+                const uint32_t more = k > 0;
+                if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < kBlkK / 16; kk++)
-                        mma_ss(acc, make_sw128_desc(xb + kk * 32), make_sw128_desc(wb + kk * 32), idesc, (k > 0 || kk > 0) ? 1u : 0u);
-                    mma_commit(empty(s));
+                    for (int kk = 0; kk < kBlkK / 16; kk++)          // 32 bytes (2 in the descriptor) inside the swizzled row
+                        mma_ss<PAIR>(acc, xd + kk * 2, wd + kk * 2, idesc, kk ? 1u : more);
+                    commit<PAIR>(empty(s));
                 }
-                // arrives after everything issued so far, on the abort path too
-                mma_commit(acc_full(buf));
+                if (++s == kStages) {
+                    s = 0;
+                    phase ^= 1;
+                }
             }
-            // the last accumulators complete before TMEM and shared memory are given up
-            for (int j = i > 2 ? i - 2 : 0; j < i; j++)
-                if (!mbar_wait(acc_full(j & 1), (j >> 1) & 1, &never)) abort_flag = 1;
+            // arrives after everything issued so far, on the abort path too
+            if (leader) commit<PAIR>(acc_full(buf));
         }
+        if (!ok) abort_flag = 1;
+        __syncwarp();
+        // the last accumulators complete before TMEM and shared memory are given up
+        for (int j = i > 2 ? i - 2 : 0; j < i; j++)
+            if (!mbar_wait(acc_full(j & 1), (j >> 1) & 1, &never)) abort_flag = 1;
     } else if (warp >= 4) {
         // ---------------- epilogue ----------------
         const int ew = warp - 4, row0 = (ew & 3) * 32, half = ew >> 2;
@@ -205,7 +276,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         uint32_t* st = reinterpret_cast<uint32_t*>(smem + (size_t)kStages * kStage) + ew * 32 * kStageLd;
         const int sr = lane >> 2, sw = (lane & 3) * 4;   // row (of eight) and words this lane stores
         int i = 0;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, i++) {
+        for (int tile = first_tile; tile < tiles; tile += step_tiles, i++) {
             const int buf = i & 1;
             if (!__all_sync(0xffffffffu, mbar_wait(acc_full(buf), (i >> 1) & 1, abortp))) {
                 abort_flag = 1;
@@ -311,15 +382,21 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(acc_empty(buf));
+            if constexpr (PAIR) {
+                __syncwarp();
+                if (lane == 0) arrive_cluster(in_first_cta(acc_empty(buf)));
+            } else {
+                mbar_arrive(acc_empty(buf));
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    sync_all<PAIR>();                                    // of a pair: nothing of one CTA is used by the other any more
     if (abort_flag && tid == 0) atomicExch(a.err, TLLM_ERR_TIMEOUT);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
     }
 }
 
@@ -336,7 +413,7 @@ int encode(EncodeTiledFn enc, CUtensorMap* map, const bf16* p, int cols, int row
     return TLLM_OK;
 }
 
-template <int TN>
+template <int TN, bool PAIR>
 int launch_tn(EncodeTiledFn enc, const LinearArgs<bf16>& l, DenseEpi e, int sms, cudaStream_t stream)
 {
     CUtensorMap mx, mw;
@@ -347,14 +424,16 @@ int launch_tn(EncodeTiledFn enc, const LinearArgs<bf16>& l, DenseEpi e, int sms,
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr[dev]) {
-        cudaFuncSetAttribute(dense_gemm_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DCfg<TN>::kSmem);
+        cudaFuncSetAttribute(dense_gemm_kernel<TN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DCfg<TN, PAIR>::kSmem);
         attr[dev] = true;
     }
     const int outs = l.glu ? TN / 2 : TN;
-    e.mt = (l.M + kTok - 1) / kTok;
+    const int tokens = PAIR ? 2 * kTok : kTok, per = PAIR ? 2 : 1;
+    e.mt = (l.M + tokens - 1) / tokens;
     e.nt = (l.N + outs - 1) / outs;
     e.tiles = e.mt * e.nt * l.batch;
-    return launch_pdl("dense_gemm", dense_gemm_kernel<TN>, dim3(e.tiles < sms ? e.tiles : sms), dim3(kThr), DCfg<TN>::kSmem, stream, mx, mw, e);
+    const int grid = (e.tiles < sms / per ? e.tiles : sms / per) * per;
+    return launch_pdl_cluster("dense_gemm", dense_gemm_kernel<TN, PAIR>, per, dim3(grid), dim3(kThr), DCfg<TN, PAIR>::kSmem, stream, mx, mw, e);
 }
 
 }  // namespace
@@ -408,15 +487,39 @@ int launch_dense_gemm_tcgen05(const LinearArgs<bf16>& l, cudaStream_t stream)
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "dense_gemm: no current device");
     if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    // the widest tile that still gives most SMs one
     const long long mt = (l.M + kTok - 1) / kTok;
-    auto tiles = [&](int tn) {
+    auto tiles = [&](int tn, long long m) {
         const int outs = l.glu ? tn / 2 : tn;
-        return mt * ((l.N + outs - 1) / outs) * l.batch;
+        return m * ((l.N + outs - 1) / outs) * l.batch;
     };
-    if (tiles(256) * 10 >= 7LL * sms[dev]) return launch_tn<256>(enc, l, e, sms[dev], stream);
-    if (tiles(128) * 10 >= 7LL * sms[dev]) return launch_tn<128>(enc, l, e, sms[dev], stream);
-    return launch_tn<64>(enc, l, e, sms[dev], stream);
+    int tn = 64;
+    bool pair = false;
+    if (l.group) {                           // their number is known on the device alone: the widest tile that still gives most SMs one
+        tn = tiles(256, mt) * 10 >= 7LL * sms[dev] ? 256 : tiles(128, mt) * 10 >= 7LL * sms[dev] ? 128 : 64;
+    } else {
+        // The quickest by rounds of tiles: 64 columns of K take 0.21, 0.27, 0.39 us in a tile of 64, 128, 256 features (its operands' 24,
+        // 32, 48 KB through 64 bytes a clock), 0.235 and 0.36 in a pair's tile of 128 and 256 (24 and 32 KB a CTA); the outputs of a tile
+        // 0.8 and 0.02 a feature, beside the next tile's product; a launch 2.5, of pairs 4.  us measured with 64, 128, 256, pair 128, pair
+        // 256, the one taken in brackets: 2000 tokens 2048 x 2048 31 22 (20) 20 21, 8192 x 2048 gated 183 116 96 107 (89), 4096 x 128
+        // 16.2 16.2 (15.2) 18.8 17.0; 1000 tokens 2048 x 8192 55 35 53 (31) 48; 300 tokens 4096 x 4096 30 21 32 (19) 30, 14336 x 4096 gated
+        // 128 85 (83) 95 89; 100 tokens 8192 x 2048 (12.3) 14.4 20.7 14.3 19.8.
+        const struct { int tn; bool pair; double step; } way[] = {{64, false, 0.21}, {128, false, 0.27}, {256, false, 0.39}, {128, true, 0.235}, {256, true, 0.36}};
+        double best = 0.;
+        for (const auto& w : way) {
+            if (w.pair && mt == 1) continue;
+            const long long at_once = w.pair ? sms[dev] / 2 : sms[dev], n = tiles(w.tn, w.pair ? (mt + 1) / 2 : mt);
+            const double product = (l.K + kBlkK - 1) / kBlkK * w.step, output = 0.8 + 0.02 * w.tn;
+            const double t = (double)((n + at_once - 1) / at_once) * (product > output ? product : output) + (product > output ? output : product) + (w.pair ? 4. : 2.5);
+            if (best == 0. || t < best) {
+                best = t;
+                tn = w.tn;
+                pair = w.pair;
+            }
+        }
+    }
+    if (tn == 256) return pair ? launch_tn<256, true>(enc, l, e, sms[dev], stream) : launch_tn<256, false>(enc, l, e, sms[dev], stream);
+    if (tn == 128) return pair ? launch_tn<128, true>(enc, l, e, sms[dev], stream) : launch_tn<128, false>(enc, l, e, sms[dev], stream);
+    return launch_tn<64, false>(enc, l, e, sms[dev], stream);
 }
 
 }  // namespace tllm

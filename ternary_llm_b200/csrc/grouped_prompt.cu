@@ -493,23 +493,13 @@ int launch_grouped_prompt_tcgen05(const GroupedArgs<bf16>& a, cudaStream_t strea
     return launch(p, mq, mk, mv, a.heads, 1, stream);
 }
 
-// Few queries over few channels: a CTA per query and key/value head on the CUDA cores (attention.cu) is quicker than a tile of
-// 128 queries.  Its chunk of 256 positions grows with the channels of a group (one head of 64: 5.7 us, two 6.2, four 8.2; one
-// of 128: 8.1), a pair of tiles here takes 6.7 (64) and 7.8 us (128), and the launch around them 1 to 1.5 us more.  So it stays
-//   * while its CTAs run at the same time: three an SM, of head size 128 one;
-//   * up to 32 positions (2 or 3 queries: 64), where the launch is all: four heads of 64, 2 queries of 8 sequences: 7.2, here 9.1;
-//   * never up to 128 positions, one tile here: one head, 8 queries behind 100: 6.8, here 6.2;
-//   * up to 256 positions, one chunk there and two tiles here: three heads, 8 queries behind 200: 9.3, here 10.6;
-//   * behind more for one or two heads of 64 alone: 8 queries behind 1000: 26.4 and 28.4, here 29.8 and 31.4; three heads,
-//     8 queries: 31.8, here 32.2; and while an SM has one CTA: 32 x 1 heads, 4 queries: 30.2, here 32.7; 5: 35, here 32.6.
+// Two or three queries of single heads of 64 behind a few positions: a CTA per query and key/value head on the CUDA cores
+// (attention.cu) has the shorter launch while all CTAs run at once.  us there / here: 32 heads, 2 queries of 16 positions 5.9 / 6.5, of 32
+// 6.0 / 6.6, of 48 6.2 / 6.7, of 64 equal; one head, 2 of 16 5.6 / 5.9.  Elsewhere a tile is as quick or quicker: 8 queries of one head behind
+// 256 8.1 / 7.4, behind 1000 25.4 / 19.8; 32 heads over 8, 2 queries behind 400 13.6 / 12.0.
 static bool few_queries(int batch, int group, int n_kv_heads, int head_dim, int seq_len, int kv_len)
 {
-    const long long ctas = (long long)batch * n_kv_heads * seq_len;
-    const int channels = group * head_dim;
-    if ((seq_len > 12 && seq_len * group > 16) || ctas > (head_dim == 64 ? 444 : 148) || channels > 256) return false;
-    if (kv_len > 256) return head_dim == 64 && channels <= 128 && ctas <= 128;
-    if (kv_len > (seq_len <= 3 ? 64 : 32) && kv_len <= 128) return false;
-    return (head_dim == 64 || group == 1) && (channels <= 192 || (kv_len <= 32 && seq_len <= 8));
+    return head_dim == 64 && group == 1 && seq_len <= 3 && kv_len <= 48 && (long long)batch * n_kv_heads * seq_len <= 444;
 }
 
 bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_heads, int n_kv_heads,

@@ -83,6 +83,19 @@ int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out
 // A few rows on prepared weights (gemm_rows.cu).
 int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream);
 
+// One vector made inside the launch from FP16 inputs on 16-byte boundaries (gemm_rows.cu):
+//   kRowPlain: x = a;  kRowNorm: x = half(rmsnorm(s) * w) with s = a, or half(a + b), which goes to res_out, a different
+//   vector than a and b;  kRowSilu: x = half(silu(a) * b)
+// row_supported: sizes where this is quicker than the streaming GEMV behind the operator's own launch.
+enum RowInput { kRowPlain = 0, kRowNorm = 1, kRowSilu = 2 };
+struct RowVector {
+    const half *a, *b, *w;
+    half* res_out;
+    float eps;
+};
+bool row_supported(RowInput input, int rows, int cols);
+int launch_gemm_row(const uint8_t* packed, RowInput input, const RowVector& x, half* y, int rows, int cols, cudaStream_t stream);
+
 // y[m, rows] = x[m, cols] . W^T, FP16 activations, on the kernel for these sizes: passes of the
 // streaming GEMV (four vectors share one over the weights), gemm_rows.cu, or the tcgen05 GEMM.
 constexpr int kRowsMax = 32;

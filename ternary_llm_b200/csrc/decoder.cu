@@ -194,7 +194,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
     if (n == 1 && D->fused_ok && (i8 || hidden <= kFusedNormMax)) {
         // Single token: norm (INT8: + quantise) and, with INT8 activations, SwiGLU + quantise happen
         // inside the GEMVs' staging phase, rotation and cache append inside the attention (5 launches
-        // per layer; 6 with FP16 activations).  The residual alternates between two
+        // per layer; 6 with FP16 activations where row_supported leaves SwiGLU a launch of its own).  The residual alternates between two
         // vectors because every CTA of a GEMV reads the old one while CTA 0 writes the new one.
         half* res_next = D->residual2;
         const size_t kvdim = (size_t)c.n_kv_heads * c.head_dim;
@@ -208,6 +208,7 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
                 half* ys[1] = {y};
                 const int rows[1] = {w.rows};
                 half* out = b ? res_next : nullptr;
+                if (!i8 && row_supported(kRowNorm, w.rows, w.cols)) return launch_gemm_row(w.p, kRowNorm, {a, b, weight, out, c.rms_norm_eps}, y, w.rows, w.cols, s);
                 return i8 ? launch_gemv_int8_packed_norm(w.p, a, b, weight, out, c.rms_norm_eps, y, w.rows, w.cols, s)
                           : launch_gemv_packed_multi_norm(1, p, ys, rows, w.cols, a, b, weight, out, c.rms_norm_eps, s);
             };
@@ -217,11 +218,15 @@ int LlamaDecoder::forward(const int* tokens, int n, int start_pos, const int* po
                                         c.n_kv_heads, c.head_dim, c.max_seq_len, start_pos, pos_dev, c.rope_theta,
                                         D->attn_ws, D->attn_counters, s));
             if (i8) TRY(launch_gemv_int8_packed_quant(L.o.p, D->attn_out, D->hidden2, L.o.rows, L.o.cols, s));
+            else if (row_supported(kRowPlain, L.o.rows, L.o.cols))
+                TRY(launch_gemm_row(L.o.p, kRowPlain, {D->attn_out}, D->hidden2, L.o.rows, L.o.cols, s));
             else TRY(launch_gemv_packed(L.o.p, D->attn_out, D->hidden2, 1, L.o.rows, L.o.cols, s));
             TRY(normed(L.gate_up, D->hidden2, res_cur, L.ffn_norm, gb));
             std::swap(res_cur, res_next);
             if (i8) {
                 TRY(launch_gemv_int8_packed_silu(L.down.p, gb, ub, D->ffn_out, L.down.rows, L.down.cols, s));
+            } else if (row_supported(kRowSilu, L.down.rows, L.down.cols)) {
+                TRY(launch_gemm_row(L.down.p, kRowSilu, {gb, ub}, D->ffn_out, L.down.rows, L.down.cols, s));
             } else {
                 TRY(launch_silu_mul(gb, ub, gb, inter, nullptr, nullptr, s));
                 TRY(launch_gemv_packed(L.down.p, gb, D->ffn_out, 1, L.down.rows, L.down.cols, s));

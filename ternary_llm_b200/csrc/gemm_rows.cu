@@ -26,6 +26,7 @@
 #include <climits>
 
 #include "launch.cuh"
+#include "layer.cuh"
 #include "packed_layout.cuh"
 
 namespace tllm {
@@ -283,6 +284,188 @@ gemm_rows_kernel(const RowsArgs a)
 }
 
 constexpr int kMaxSplit = 8;
+// ---- one vector ---------------------------------------------------------------------------------
+// A decode step's products of one vector on the same codes and cuts.  The whole share of the vector lies in shared memory before the
+// first group, made there from what the step has (RowInput), so that there is no barrier between the groups and no launch for a norm
+// or a SwiGLU; all lanes of a quarter read the same activations, and the MMA's eight columns are the same.
+struct OneArgs {
+    const uint8_t* packed;
+    RowVector x;
+    half* y;
+    int rows, cols, groups, nrb, split, share;
+    uint32_t over_split;
+};
+
+constexpr int kOneAhead = 4;
+constexpr size_t kOneSmem = 40 * 1024;                 // shared memory that needs no attribute
+
+template <int INPUT>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_row_kernel(const OneArgs a)
+{
+    constexpr int R = 2, RG = kRowWarps, KW = kGroupWarps, kRows = RG * R * kTileRows;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    half* xs = reinterpret_cast<half*>(smem_raw);        // the vector (kRowNorm), or its share
+    __shared__ float red[KW][kRows], sent[kMaxSplit * kRows], sums[kThreads / 32];
+    pdl_launch_dependents();
+    if (a.split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3;
+    const int kw = warp % KW, rg = warp / KW;
+    const int rank = blockIdx.x, tile = blockIdx.y;
+    const int g0 = a.split > 1 ? __umulhi(rank * a.groups, a.over_split) : 0;
+    const int ng = (a.split > 1 ? __umulhi((rank + 1) * a.groups, a.over_split) : a.groups) - g0;
+    const int mine = (ng - kw + KW - 1) / KW;
+    const int rb0 = (tile * RG + rg) * R;
+
+    const uint8_t* wp[R];
+#pragma unroll
+    for (int r = 0; r < R; r++)      // row blocks past the matrix repeat the last one and are not stored
+        wp[r] = a.packed + ((size_t)min(rb0 + r, a.nrb - 1) * a.groups + g0 + kw) * kTileBytes;
+    uint4 cw[kOneAhead][R];
+    uint32_t sw[kOneAhead][R];
+    auto load = [&](int i, uint4 (&c)[R], uint32_t (&s)[R]) {
+        if (i < mine) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint8_t* p = wp[r] + (size_t)i * (KW * kTileBytes);
+                c[r] = ldg_stream(p + lane * 16);
+                s[r] = ldg_word(p + kTileCodeBytes + gq * 4);
+            }
+        }
+    };
+#pragma unroll
+    for (int d = 0; d < kOneAhead; d++) load(d, cw[d], sw[d]);
+
+    pdl_wait();
+    const uint4 *xa = reinterpret_cast<const uint4*>(a.x.a), *xb = reinterpret_cast<const uint4*>(a.x.b);
+    uint4* x8 = reinterpret_cast<uint4*>(xs);
+    const half* mine_x = xs;                             // of the first group
+    if (INPUT == kRowNorm) {
+        // the arithmetic of the norm operator: sum rounded to FP16, mean of squares and scaling in FP32, one rounding of the result
+        const int n8 = a.cols >> 3;
+        const bool keeps = a.x.res_out && rank == 0 && tile == 0;
+        float ss = 0.f;
+        for (int i = tid; i < n8; i += kThreads) {
+            uint4 v = xa[i];
+            half* vh = reinterpret_cast<half*>(&v);
+            if (xb) {
+                const uint4 br = xb[i];
+                const half* bh = reinterpret_cast<const half*>(&br);
+#pragma unroll
+                for (int j = 0; j < 8; j++) vh[j] = __float2half_rn(__half2float(vh[j]) + __half2float(bh[j]));
+                if (keeps) reinterpret_cast<uint4*>(a.x.res_out)[i] = v;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float f = __half2float(vh[j]);
+                ss += f * f;
+            }
+            x8[i] = v;
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) sums[warp] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; i++) ss += sums[i];
+        const float rinv = rsqrtf(ss / (float)a.cols + a.x.eps);
+        for (int i = tid; i < n8; i += kThreads) {
+            uint4 v = x8[i];
+            const uint4 wr = reinterpret_cast<const uint4*>(a.x.w)[i];
+            half* vh = reinterpret_cast<half*>(&v);
+            const half* wh = reinterpret_cast<const half*>(&wr);
+#pragma unroll
+            for (int j = 0; j < 8; j++) vh[j] = __float2half_rn(__half2float(vh[j]) * rinv * __half2float(wh[j]));
+            x8[i] = v;
+        }
+        mine_x += g0 * kGroup;
+    } else {
+        const int first = g0 * (kGroup / 8), n8 = ng * (kGroup / 8);
+        for (int i = tid; i < n8; i += kThreads) {
+            uint4 v = xa[first + i];
+            if (INPUT == kRowSilu) {
+                const uint4 ur = xb[first + i];
+                half* vh = reinterpret_cast<half*>(&v);
+                const half* uh = reinterpret_cast<const half*>(&ur);
+#pragma unroll
+                for (int j = 0; j < 8; j++) vh[j] = __float2half_rn(silu_mul(__half2float(vh[j]), __half2float(uh[j])));
+            }
+            x8[i] = v;
+        }
+    }
+    __syncthreads();
+
+    float acc[R][2] = {};                                // rows gq, gq + 8
+    for (int i0 = 0; i0 < mine; i0 += kOneAhead) {
+#pragma unroll
+        for (int d = 0; d < kOneAhead; d++) {
+            const int i = i0 + d;
+            if (i >= mine) break;
+            const half* xr = mine_x + (i * KW + kw) * kGroup + 4 * t;
+            float sum[R][2][4] = {};                     // two chains of MMAs
+            uint32_t w[R][4];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                w[r][0] = prmt(cw[d][r].x, 0, 0x3120);
+                w[r][1] = prmt(cw[d][r].y, 0, 0x3120);
+                w[r][2] = prmt(cw[d][r].z, 0, 0x3120);
+                w[r][3] = prmt(cw[d][r].w, 0, 0x3120);
+            }
+#pragma unroll
+            for (int f = 0; f < 4; f++)
+#pragma unroll
+                for (int j2 = 0; j2 < 2; j2++) {
+                    const uint2 b = *reinterpret_cast<const uint2*>(xr + 32 * f + 16 * j2);
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const uint32_t fr[4] = {code_f16<0>(w[r][j2], f), code_f16<0>(w[r][2 + j2], f), code_f16<8>(w[r][j2], f),
+                                                code_f16<8>(w[r][2 + j2], f)};
+                        mma_f16(sum[r][j2], fr, b.x, b.y);
+                    }
+                }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const float2 sc = __half22float2(*reinterpret_cast<const half2*>(&sw[d][r]));
+                acc[r][0] = fmaf(sc.x, sum[r][0][0] + sum[r][1][0], acc[r][0]);
+                acc[r][1] = fmaf(sc.y, sum[r][0][2] + sum[r][1][2], acc[r][1]);
+            }
+            load(i + kOneAhead, cw[d], sw[d]);
+        }
+    }
+    if (t == 0)
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            red[kw][(rg * R + r) * kTileRows + gq] = acc[r][0];
+            red[kw][(rg * R + r) * kTileRows + gq + 8] = acc[r][1];
+        }
+    __syncthreads();
+    const int row0 = tile * kRows;
+    auto first = [&](int z) { return (int)__umulhi(z * kRows + a.split - 1, a.over_split); };
+    if (a.split > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // all of them run
+    if (tid < kRows) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < KW; k++) v += red[k][tid];
+        if (a.split == 1) {
+            if (row0 + tid < a.rows) a.y[row0 + tid] = __float2half_rn(v);
+        } else {
+            const int to = tid * a.split / kRows;
+            uint32_t peer;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(sm32(sent + rank * a.share + tid - first(to))), "r"(to));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer), "f"(v) : "memory");
+        }
+    }
+    if (a.split > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int f0 = first(rank);
+        if (tid < first(rank + 1) - f0 && row0 + f0 + tid < a.rows) {
+            float v = 0.f;
+            for (int z = 0; z < a.split; z++) v += sent[z * a.share + tid];
+            a.y[row0 + f0 + tid] = __float2half_rn(v);
+        }
+    }
+}
+
 
 // How a product is cut: CTAs that share the scale groups of a tile, and the groups that one of them walks in all rounds of CTAs.
 struct Cut {
@@ -364,7 +547,53 @@ int launch(RowsArgs a, cudaStream_t stream)
                               S::kSmem, stream, a);
 }
 
+template <int INPUT>
+int launch_one(OneArgs a, cudaStream_t stream)
+{
+    using S = Shape<1, kRowWarps, kGroupWarps>;
+    Cut c;
+    const int st = cut<1>(a.rows, a.groups, &c);         // its shared memory is no larger than the other kernel's
+    if (st) return st;
+    a.split = c.split;
+    a.share = (S::kRows + a.split - 1) / a.split;
+    a.over_split = (uint32_t)((0x100000000ull + a.split - 1) / a.split);         // of one CTA not used
+    const int per = (a.groups + a.split - 1) / a.split;
+    const size_t smem = (size_t)(INPUT == kRowNorm ? a.cols : per * kGroup) * sizeof(half);
+    if (smem > kOneSmem) return fail(TLLM_ERR_SHAPE, "gemm_row: %d columns", a.cols);
+    const int tiles = (a.rows + S::kRows - 1) / S::kRows;
+    return launch_pdl_cluster("gemm_row", gemm_row_kernel<INPUT>, a.split, dim3(a.split, tiles), dim3(kThreads), smem, stream, a);
+}
+
 }  // namespace
+
+// us in the chain of a step, streaming GEMV (SwiGLU's launch included) / here: plain 1024 x 1024 3.3 / 2.0, 2048 x 2048 4.1 / 3.0, 4096 x
+// 4096 5.4 / 3.6, 8192 x 8192 11.2 / 9.0; SwiGLU 2048 x 8192 6.6 / 4.4, 4096 x 14336 11.8 / 9.2, 8192 x 28672 30.9 / 29.4; norm 3072 x 2048
+// 5.5 / 3.9, 16384 x 2048 7.2 / 6.1, 12288 x 4096 (32 steps) 9.3 / 9.3, 10240 x 8192 (64) 16.1 / 16.5, 28672 x 4096 (64) 15.7 / 18.2.
+bool row_supported(RowInput input, int rows, int cols)
+{
+    Cut c;
+    const int groups = cols / kGroup;
+    if (!groups || cut<1>(rows, groups, &c)) return false;
+    return (size_t)(input == kRowNorm ? cols : (groups + c.split - 1) / c.split * kGroup) * sizeof(half) <= kOneSmem &&
+           (input != kRowNorm || c.steps <= 32);
+}
+
+int launch_gemm_row(const uint8_t* packed, RowInput input, const RowVector& x, half* y, int rows, int cols, cudaStream_t stream)
+{
+    OneArgs a = {};
+    a.packed = packed;
+    a.x = x;
+    a.y = y;
+    a.rows = rows;
+    a.cols = cols;
+    a.groups = cols / kGroup;
+    a.nrb = (rows + kTileRows - 1) / kTileRows;
+    switch (input) {
+        case kRowNorm: return launch_one<kRowNorm>(a, stream);
+        case kRowSilu: return launch_one<kRowSilu>(a, stream);
+        default: return launch_one<kRowPlain>(a, stream);
+    }
+}
 
 // Matrices packed back to back (every row count but the last a multiple of 16) as one.
 int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, int nout, int m, int cols, cudaStream_t stream)

@@ -5,6 +5,8 @@
 
 namespace tllm {
 
+__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + expf(-g)) * u; }
+
 // q / q_scale: when not null the normalised vector is also quantised (one scale per row).
 // round_first: the variance is taken over the FP16-rounded sum (what a separate
 // add-then-normalise sequence computes) instead of the unrounded one.

@@ -347,8 +347,6 @@ int launch_rope(half* q, half* k, const half* v, half* k_cache, half* v_cache, i
 // ---------------------------------------------------------------------------
 // SwiGLU   out = half(g / (1 + exp(-g)) * u)       reference: kernels/activations.cu:18-74
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + expf(-g)) * u; }
-
 // Eight elements a thread (whole 16-byte pieces): bound by the exponential and the division, so that what an element costs
 // beside them counts.  us a launch, two elements a thread / eight: 2000 x 14336 63 / 32, 300 x 8192 5.7 / 3.7, 24 x 8192 1.8 / 3.1: two
 // while all threads run at once.

@@ -83,3 +83,25 @@ def test_matrices_packed_back_to_back(n):
     # one layer in FP16: two roundings per operator, on kernels that sum in another order
     assert np.linalg.norm(got - want) <= 1e-2 * np.linalg.norm(want)
     dec.close()
+
+
+@pytest.mark.parametrize("hidden,inter,heads,kv_heads", [(128, 128, 2, 1), (1152, 3200, 18, 9), (2304, 6784, 36, 12), (4096, 11008, 64, 8)])
+def test_step_of_one_vector(hidden, inter, heads, kv_heads):
+    """FP16 steps, whose products make their vector (norm with and without a residual, SwiGLU) inside the launch: one and uneven
+    numbers of groups, one to eight CTAs a tile, matrices that stay with the GEMV; against the oracle, with the limits of the
+    decoder's tests, and against the same token in lock step, which takes the other kernels."""
+    cfg = tf.TllmConfig(vocab_size=777, hidden_dim=hidden, intermediate_dim=inter, n_layers=2, n_heads=heads, n_kv_heads=kv_heads, head_dim=64,
+                        max_seq_len=16, rope_theta=10000.0, rms_norm_eps=1e-5)
+    model = tf.random_model(cfg, seed=hidden)
+    dec, ora = tl.Decoder(model, int8_decode=False, max_batch=5), layer_oracle.Transformer(model, int8_decode=False)
+    tokens = np.random.default_rng(hidden).integers(0, cfg.vocab_size, 3).astype(np.int32)
+    for i, token in enumerate(tokens):
+        ids = torch.from_numpy(np.repeat(token, 5).astype(np.int32)).cuda()
+        both = dec.forward_batch(ids, i).clone()
+        got = dec.forward(ids[:1], i).float()
+        want = torch.from_numpy(np.asarray(ora.forward([int(token)], i), np.float32)).cuda()
+        scale = max(1.0, want.abs().max().item())
+        assert (got - want).abs().max().item() <= 2e-2 * scale, f"step {i}"
+        assert (got - both[0].float()).abs().max().item() <= 2e-2 * scale, f"step {i}, lock step"
+    tl.check_device_errors()
+    dec.close()

@@ -9,6 +9,8 @@
 // pair.  Gate and up of 8192 x 2048, 2000 tokens: 92 -> 81 us = 1.66 PFLOP/s in a prompt; in tiles of 64
 // and 128 features what bounded was the loop of one thread that issued the MMAs (2048 x 8192, 100 tokens
 // 40.5 -> 29.2 us with the loop run by a warp and one elected lane).
+// Where tiles are few, the CTAs of a cluster share one, each a part of K (SPLIT); they send one another
+// their sums of the tokens that the other finishes, and add them in rank order.
 // One persistent CTA per SM walks tiles with three roles
 // that run ahead of one another: a TMA producer (K-major tiles of 64 columns, 128-byte swizzle;
 // out-of-range rows and columns read as zero, so no size needs to divide a tile), one thread
@@ -39,14 +41,18 @@ constexpr int kThr = 128 + 32 * kEpiWarps;
 
 constexpr int kStageLd = 20;         // words per row of an epilogue warp's tile: 16 of data (16 FP32 or 32 BF16 columns)
 
-template <int TN, bool PAIR>
+enum Way { kSingle, kPair, kSplit };      // a CTA a tile; two CTAs a tile of 256 tokens; K of a tile over the CTAs of a cluster
+
+template <int TN, Way WAY>
 struct DCfg {
+    static constexpr bool PAIR = WAY == kPair;
     static constexpr int kXBytes = kTok * kBlkK * 2;
     static constexpr int kWBytes = TN * kBlkK * 2 / (PAIR ? 2 : 1);
     static constexpr int kStage = kXBytes + kWBytes;
-    static constexpr int kStages = PAIR ? (TN == 256 ? 6 : 8) : (TN == 256) ? 4 : (TN == 128) ? 6 : 8;
+    static constexpr int kStages = PAIR ? (TN == 256 ? 6 : 8) : WAY == kSplit ? 6 : (TN == 256) ? 4 : (TN == 128) ? 6 : 8;
     static constexpr int kEpiBytes = kEpiWarps * 32 * kStageLd * 4;
-    static constexpr size_t kSmem = (size_t)kStages * kStage + kEpiBytes + 1024;
+    static constexpr size_t kSums = WAY == kSplit ? (size_t)TN * kTok * 4 : 0;      // what the cluster's CTAs send
+    static constexpr size_t kSmem = (size_t)kStages * kStage + kEpiBytes + kSums + 1024;
 };
 
 struct DenseEpi {
@@ -56,6 +62,7 @@ struct DenseEpi {
     int ldy, y_batch, gate_ld;
     int M, N, K, x_batch, w_rows;
     int mt, nt, tiles;             // tiles along the tokens, along the features, in all
+    int split;                     // CTAs that share a tile's K, a power of two
     int act, glu, y_f32, vec, bias_vec;
     float act_param;
     int act_lo, act_hi, f32_from, ldy2, vec2;
@@ -123,11 +130,12 @@ __device__ __forceinline__ void sync_all()
     else __syncthreads();
 }
 
-template <int TN, bool PAIR>
+template <int TN, Way WAY>
 __global__ void __launch_bounds__(kThr, 1)
 dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const DenseEpi a)
 {
-    using Cfg = DCfg<TN, PAIR>;
+    constexpr bool PAIR = WAY == kPair, SPLIT = WAY == kSplit;
+    using Cfg = DCfg<TN, WAY>;
     constexpr int kStages = Cfg::kStages, kStage = Cfg::kStage, kXBytes = Cfg::kXBytes;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -138,8 +146,12 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int outs = a.glu ? TN / 2 : TN;              // output features of a tile
     const int rank = PAIR ? blockIdx.x & 1 : 0;        // CTA of the pair: its half of the tile's tokens and of its rows of W
-    const int first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x, step_tiles = PAIR ? gridDim.x >> 1 : gridDim.x;
-    const int nk = (a.K + kBlkK - 1) / kBlkK;
+    const int first_tile = PAIR ? blockIdx.x >> 1 : SPLIT ? blockIdx.x / a.split : blockIdx.x;
+    const int step_tiles = PAIR ? gridDim.x >> 1 : gridDim.x;                  // SPLIT: one tile
+    const int nk_all = (a.K + kBlkK - 1) / kBlkK;
+    // SPLIT: this CTA's part of K and, of its tile's tokens, those that it finishes
+    const int part = SPLIT ? blockIdx.x & (a.split - 1) : 0, k0 = SPLIT ? part * nk_all / a.split : 0;
+    const int nk = (SPLIT ? (part + 1) * nk_all / a.split : nk_all) - k0;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (kStages + s); };
@@ -147,6 +159,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     auto acc_empty = [&](int i) { return bar0 + 8u * (2 * kStages + 2 + i); };
 
     if (tid == 0) {
+        prefetch_map(&map_x);
+        prefetch_map(&map_w);
         for (int s = 0; s < kStages; s++) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
@@ -171,7 +185,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    sync_all<PAIR>();
+    sync_all<PAIR || SPLIT>();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
     volatile int* abortp = &abort_flag;
@@ -196,6 +210,98 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         entry = z = tile / a.nt;
     };
 
+    float* sums = reinterpret_cast<float*>(smem + (size_t)kStages * kStage + Cfg::kEpiBytes);       // SPLIT
+    auto head_gate = [&](int mrow, int z) {
+        return (a.gate && mrow + lane < a.M) ? sigmoid_f(__bfloat162float(a.gate[(size_t)(mrow + lane) * a.gate_ld + z])) : 1.f;
+    };
+    // Epilogue of 32 columns from column c of a tile on (features n0 + c ..), whose sums `read` gives for this lane's row, mrow + lane
+    // of the nrows from mrow on; st: a tile of this warp in shared memory.
+    const int ew = warp - 4;
+    uint32_t* st = reinterpret_cast<uint32_t*>(smem + (size_t)kStages * kStage) + ew * 32 * kStageLd;
+    const int sr = lane >> 2, sw = (lane & 3) * 4;       // row (of eight) and words this lane stores
+    auto finish = [&](int c, int ncols, int n0, int z, int mrow, int nrows, float hg, auto read) {
+        // 32 columns go one way: the limits of the activation and of y2 are multiples of 64
+        const bool second = n0 + c >= a.f32_from, y_f32 = a.y_f32 || second;
+        const int act = n0 + c >= a.act_lo && n0 + c < a.act_hi && !second ? a.act : kActNone;
+        const int wcols = y_f32 ? 1 : 2;         // columns per staged word
+        float f[32];
+        read(c, f);
+        if (a.glu) {
+            float u[32];
+            read(TN / 2 + c, u);
+            apply_act_n<32>(act, f);
+#pragma unroll
+            for (int j = 0; j < 32; j++) f[j] *= u[j];
+        } else {
+            if (a.bias) {
+                const float* bp = a.bias + (size_t)z * a.N + n0 + c;
+                if (a.bias_vec && c + 32 <= ncols) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const float4 t = __ldg(reinterpret_cast<const float4*>(bp) + j);
+                        f[4 * j] += t.x;
+                        f[4 * j + 1] += t.y;
+                        f[4 * j + 2] += t.z;
+                        f[4 * j + 3] += t.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (c + j < ncols) f[j] += __ldg(bp + j);
+                }
+            }
+            apply_act_n<32>(act, f, a.act_param);
+            if (a.gate) {
+#pragma unroll
+                for (int j = 0; j < 32; j++) f[j] *= hg;
+            }
+        }
+        // through shared memory, 16 words of a row at a time: FP32 in two halves, BF16 at once
+#pragma unroll
+        for (int part = 0; part < 2; part++) {
+            if (part == 1 && !y_f32) break;
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                uint32_t w[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int e = 4 * j + q;
+                    if (y_f32) {
+                        w[q] = __float_as_uint(f[part * 16 + e]);
+                    } else {
+                        const __nv_bfloat162 t = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+                        w[q] = *reinterpret_cast<const uint32_t*>(&t);
+                    }
+                }
+                *reinterpret_cast<uint4*>(st + lane * kStageLd + 4 * j) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            __syncwarp();
+            const int col = c + part * 16 + sw * wcols;      // first of this lane's columns inside the tile
+            if (col < ncols) {
+                const bool vec = (second ? a.vec2 : a.vec) && col + 4 * wcols <= ncols;
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int rr = r * 8 + sr, m = mrow + rr;
+                    if (m >= a.M || rr >= nrows) break;
+                    const uint4 t = *reinterpret_cast<const uint4*>(st + rr * kStageLd + sw);
+                    const size_t o = second ? (size_t)m * a.ldy2 + n0 + col - a.f32_from
+                                            : (size_t)m * a.ldy + (size_t)z * a.y_batch + n0 + col;
+                    if (vec) {
+                        if (y_f32) *reinterpret_cast<uint4*>((second ? a.y2 : static_cast<float*>(a.y)) + o) = t;
+                        else *reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + o) = t;
+                    } else {
+                        const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+                        for (int q = 0; q < 4 * wcols && col + q < ncols; q++) {
+                            if (y_f32) (second ? a.y2 : static_cast<float*>(a.y))[o + q] = __uint_as_float(w[q]);
+                            else static_cast<uint16_t*>(a.y)[o + q] = (uint16_t)(w[q >> 1] >> ((q & 1) * 16));
+                        }
+                    }
+                }
+            }
+        }
+    };
+
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         const bool leader = elect_one();
@@ -210,9 +316,9 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 if (leader) {
                     if (rank == 0) mbar_expect_tx(full(s), PAIR ? 2 * kStage : kStage);
                     const uint32_t dst = smem_u32(smem + (size_t)s * kStage), bar = PAIR ? in_first_cta(full(s)) : full(s);
-                    load_tile<PAIR>(dst, &map_x, x0 + k * kBlkK, m0, bar);
-                    load_tile<PAIR>(dst + kXBytes, &map_w, k * kBlkK, rank ? wr1 : wr0, bar);
-                    if (!PAIR) load_tile<PAIR>(dst + kXBytes + TN / 2 * kBlkK * 2, &map_w, k * kBlkK, wr1, bar);
+                    load_tile<PAIR>(dst, &map_x, x0 + (k0 + k) * kBlkK, m0, bar);
+                    load_tile<PAIR>(dst + kXBytes, &map_w, (k0 + k) * kBlkK, rank ? wr1 : wr0, bar);
+                    if (!PAIR) load_tile<PAIR>(dst + kXBytes + TN / 2 * kBlkK * 2, &map_w, (k0 + k) * kBlkK, wr1, bar);
                 }
                 used = min(used + 1, kStages);
                 if (++s == kStages) {
@@ -271,10 +377,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             if (!mbar_wait(acc_full(j & 1), (j >> 1) & 1, &never)) abort_flag = 1;
     } else if (warp >= 4) {
         // ---------------- epilogue ----------------
-        const int ew = warp - 4, row0 = (ew & 3) * 32, half = ew >> 2;
+        const int row0 = (ew & 3) * 32, half = ew >> 2;
         const uint32_t lane_base = tmem + ((uint32_t)row0 << 16);
-        uint32_t* st = reinterpret_cast<uint32_t*>(smem + (size_t)kStages * kStage) + ew * 32 * kStageLd;
-        const int sr = lane >> 2, sw = (lane & 3) * 4;   // row (of eight) and words this lane stores
         int i = 0;
         for (int tile = first_tile; tile < tiles; tile += step_tiles, i++) {
             const int buf = i & 1;
@@ -286,101 +390,35 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             int m0, n0, z, entry;
             where(tile, m0, n0, z, entry);
             const int mrow = m0 + row0;
-            const float hg = (a.gate && mrow + lane < a.M) ? sigmoid_f(__bfloat162float(a.gate[(size_t)(mrow + lane) * a.gate_ld + z])) : 1.f;
-            const int ncols = min(outs, a.N - n0);
             const uint32_t acc = lane_base + buf * TN;
-            if (mrow < a.M)
-#pragma unroll 1
-            for (int c = half * 32; c < ncols; c += 64) {
-                // 32 columns go one way: the limits of the activation and of y2 are multiples of 64
-                const bool second = n0 + c >= a.f32_from, y_f32 = a.y_f32 || second;
-                const int act = n0 + c >= a.act_lo && n0 + c < a.act_hi && !second ? a.act : kActNone;
-                const int wcols = y_f32 ? 1 : 2;         // columns per staged word
+            auto read = [&](int c, float (&f)[32]) {
                 uint32_t v[32];
                 __syncwarp();
                 tmem_ld32(acc + c, v);
-                float f[32];
-                if (a.glu) {
-                    uint32_t u[32];
-                    tmem_ld32(acc + TN / 2 + c, u);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < 32; j++) f[j] = __uint_as_float(v[j]);
-                    apply_act_n<32>(act, f);
+                for (int j = 0; j < 32; j++) f[j] = __uint_as_float(v[j]);
+            };
+            if constexpr (SPLIT) {
+                // this CTA's sums of a row to the CTA that finishes it: [CTA][column][row]
+                const int rows = kTok / a.split, to = (row0 + lane) / rows;
+                uint32_t peer;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(smem_u32(sums + part * TN * rows + (row0 + lane) % rows)), "r"(to));
+                if (mrow < a.M)
+                    for (int c = half * 32; c < TN; c += 64) {
+                        float f[32];
+                        read(c, f);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) f[j] *= __uint_as_float(u[j]);
-                } else {
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int j = 0; j < 32; j++) f[j] = __uint_as_float(v[j]);
-                    if (a.bias) {
-                        const float* bp = a.bias + (size_t)z * a.N + n0 + c;
-                        if (a.bias_vec && c + 32 <= ncols) {
-#pragma unroll
-                            for (int j = 0; j < 8; j++) {
-                                const float4 t = __ldg(reinterpret_cast<const float4*>(bp) + j);
-                                f[4 * j] += t.x;
-                                f[4 * j + 1] += t.y;
-                                f[4 * j + 2] += t.z;
-                                f[4 * j + 3] += t.w;
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; j++)
-                                if (c + j < ncols) f[j] += __ldg(bp + j);
-                        }
+                        for (int j = 0; j < 32; j++)
+                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer + (uint32_t)((c + j) * rows * 4)), "f"(f[j]) : "memory");
                     }
-                    apply_act_n<32>(act, f, a.act_param);
-                    if (a.gate) {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) f[j] *= hg;
-                    }
-                }
-                // through shared memory, 16 words of a row at a time: FP32 in two halves, BF16 at once
-#pragma unroll
-                for (int part = 0; part < 2; part++) {
-                    if (part == 1 && !y_f32) break;
-                    __syncwarp();
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const int e = 4 * j + q;
-                            if (y_f32) {
-                                w[q] = __float_as_uint(f[part * 16 + e]);
-                            } else {
-                                const __nv_bfloat162 t = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
-                                w[q] = *reinterpret_cast<const uint32_t*>(&t);
-                            }
-                        }
-                        *reinterpret_cast<uint4*>(st + lane * kStageLd + 4 * j) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                    __syncwarp();
-                    const int col = c + part * 16 + sw * wcols;      // first of this lane's columns inside the tile
-                    if (col < ncols) {
-                        const bool vec = (second ? a.vec2 : a.vec) && col + 4 * wcols <= ncols;
-#pragma unroll
-                        for (int r = 0; r < 4; r++) {
-                            const int rr = r * 8 + sr, m = mrow + rr;
-                            if (m >= a.M) break;
-                            const uint4 t = *reinterpret_cast<const uint4*>(st + rr * kStageLd + sw);
-                            const size_t o = second ? (size_t)m * a.ldy2 + n0 + col - a.f32_from
-                                                    : (size_t)m * a.ldy + (size_t)z * a.y_batch + n0 + col;
-                            if (vec) {
-                                if (y_f32) *reinterpret_cast<uint4*>((second ? a.y2 : static_cast<float*>(a.y)) + o) = t;
-                                else *reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + o) = t;
-                            } else {
-                                const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-                                for (int q = 0; q < 4 * wcols && col + q < ncols; q++) {
-                                    if (y_f32) (second ? a.y2 : static_cast<float*>(a.y))[o + q] = __uint_as_float(w[q]);
-                                    else static_cast<uint16_t*>(a.y)[o + q] = (uint16_t)(w[q >> 1] >> ((q & 1) * 16));
-                                }
-                            }
-                        }
-                    }
-                }
+                break;
             }
+            const float hg = head_gate(mrow, z);
+            const int ncols = min(outs, a.N - n0);
+            if (mrow < a.M)
+#pragma unroll 1
+                for (int c = half * 32; c < ncols; c += 64) finish(c, ncols, n0, z, mrow, 32, hg, read);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             if constexpr (PAIR) {
                 __syncwarp();
@@ -391,7 +429,27 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    sync_all<PAIR>();                                    // of a pair: nothing of one CTA is used by the other any more
+    sync_all<PAIR || SPLIT>();                           // of a pair: nothing of one CTA is used by the other any more
+    if constexpr (SPLIT) {
+        if (warp >= 4 && !abort_flag) {
+            const int rows = kTok / a.split, nrows = min(32, rows), groups = rows / nrows, per = (outs + 31) / 32;
+            int m0, n0, z, entry;
+            where(first_tile, m0, n0, z, entry);
+            const int ncols = min(outs, a.N - n0);
+            for (int i = ew; i < groups * per; i += kEpiWarps) {
+                const int c = i / groups * 32, r0 = i % groups * 32, mrow = m0 + part * rows + r0;
+                if (c >= ncols || mrow >= a.M) continue;
+                finish(c, ncols, n0, z, mrow, nrows, head_gate(mrow, z), [&](int col, float (&f)[32]) {
+                    const float* p = sums + col * rows + r0 + lane % nrows;
+#pragma unroll
+                    for (int j = 0; j < 32; j++) f[j] = 0.f;
+                    for (int q = 0; q < a.split; q++, p += TN * rows)
+#pragma unroll
+                        for (int j = 0; j < 32; j++) f[j] += p[j * rows];
+                });
+            }
+        }
+    }
     if (abort_flag && tid == 0) atomicExch(a.err, TLLM_ERR_TIMEOUT);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -413,7 +471,7 @@ int encode(EncodeTiledFn enc, CUtensorMap* map, const bf16* p, int cols, int row
     return TLLM_OK;
 }
 
-template <int TN, bool PAIR>
+template <int TN, Way WAY>
 int launch_tn(EncodeTiledFn enc, const LinearArgs<bf16>& l, DenseEpi e, int sms, cudaStream_t stream)
 {
     CUtensorMap mx, mw;
@@ -424,16 +482,16 @@ int launch_tn(EncodeTiledFn enc, const LinearArgs<bf16>& l, DenseEpi e, int sms,
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr[dev]) {
-        cudaFuncSetAttribute(dense_gemm_kernel<TN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DCfg<TN, PAIR>::kSmem);
+        cudaFuncSetAttribute(dense_gemm_kernel<TN, WAY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DCfg<TN, WAY>::kSmem);
         attr[dev] = true;
     }
     const int outs = l.glu ? TN / 2 : TN;
-    const int tokens = PAIR ? 2 * kTok : kTok, per = PAIR ? 2 : 1;
+    const int tokens = WAY == kPair ? 2 * kTok : kTok, per = WAY == kPair ? 2 : WAY == kSplit ? e.split : 1;
     e.mt = (l.M + tokens - 1) / tokens;
     e.nt = (l.N + outs - 1) / outs;
     e.tiles = e.mt * e.nt * l.batch;
-    const int grid = (e.tiles < sms / per ? e.tiles : sms / per) * per;
-    return launch_pdl_cluster("dense_gemm", dense_gemm_kernel<TN, PAIR>, per, dim3(grid), dim3(kThr), DCfg<TN, PAIR>::kSmem, stream, mx, mw, e);
+    const int grid = (WAY == kSplit || e.tiles < sms / per ? e.tiles : sms / per) * per;
+    return launch_pdl_cluster("dense_gemm", dense_gemm_kernel<TN, WAY>, per, dim3(grid), dim3(kThr), DCfg<TN, WAY>::kSmem, stream, mx, mw, e);
 }
 
 }  // namespace
@@ -516,10 +574,25 @@ int launch_dense_gemm_tcgen05(const LinearArgs<bf16>& l, cudaStream_t stream)
                 pair = w.pair;
             }
         }
+        // Few tiles: K over a cluster's CTAs while all of them run at once; exchanging the sums takes 3.7 us.  One CTA a tile / so, 100
+        // tokens: 2048 x 8192 29 / 15, 4096 x 14336 48 / 32, 2048 x 2048 10.6 / 9.7, 2048 x 1024 7.5 / 8.6.
+        const long long n = tiles(64, mt), most[3] = {sms[dev], sms[dev] * 8 / 9, sms[dev] * 4 / 5};
+        for (int i = 0, split = 2; i < 3 && n * split <= most[i]; i++, split *= 2) {
+            const int steps = (l.K + kBlkK - 1) / kBlkK;
+            if (steps < split) break;
+            const double t = (steps + split - 1) / split * 0.21 + 0.8 + 0.02 * 64 + 2.5 + 3.7;
+            if (t < best) {
+                best = t;
+                tn = 64;
+                pair = false;
+                e.split = split;
+            }
+        }
     }
-    if (tn == 256) return pair ? launch_tn<256, true>(enc, l, e, sms[dev], stream) : launch_tn<256, false>(enc, l, e, sms[dev], stream);
-    if (tn == 128) return pair ? launch_tn<128, true>(enc, l, e, sms[dev], stream) : launch_tn<128, false>(enc, l, e, sms[dev], stream);
-    return launch_tn<64, false>(enc, l, e, sms[dev], stream);
+    if (tn == 256) return pair ? launch_tn<256, kPair>(enc, l, e, sms[dev], stream) : launch_tn<256, kSingle>(enc, l, e, sms[dev], stream);
+    if (tn == 128) return pair ? launch_tn<128, kPair>(enc, l, e, sms[dev], stream) : launch_tn<128, kSingle>(enc, l, e, sms[dev], stream);
+    if (e.split > 1) return launch_tn<64, kSplit>(enc, l, e, sms[dev], stream);
+    return launch_tn<64, kSingle>(enc, l, e, sms[dev], stream);
 }
 
 }  // namespace tllm

@@ -68,6 +68,7 @@ struct Args {
     RowsOut out[TLLM_MAX_FUSED];     // row ranges of the matrix and where they go; unused ones start past every row
     int M, N, groups;                // tokens; rows of W; K / 128
     int mt, tiles, split;            // token tiles; tiles; CTAs per tile
+    uint32_t over_split;             // 2^32 / split rounded up: the upper word of a product with it is a quotient
     int tm, acc_stride, na, nb;      // tokens per tile; columns between accumulators; weight and activation stages (na <= nb)
     int accs;                        // accumulators: two, or one for tiles of more than kMaxTm2 tokens
     int* err;
@@ -109,6 +110,17 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+enum Special { kClusterRank, kClusterId, kClusters };
+template <Special S>
+__device__ __forceinline__ uint32_t special_register()
+{
+    uint32_t r;
+    if constexpr (S == kClusterRank) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    else if constexpr (S == kClusterId) asm("mov.u32 %0, %%clusterid.x;" : "=r"(r));
+    else asm("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
+    return r;
+}
+
 // A place in a ring of n slots: the slot and the parity of its uses.
 struct Ring {
     int slot = 0;
@@ -135,9 +147,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tm = a.tm, nb = a.nb, na = a.na;
-    const int split = a.split, rank = blockIdx.x % split, first = blockIdx.x / split, step = gridDim.x / split;
-    const int it0 = (int)((long long)rank * a.groups / split);                       // scale groups of this CTA
-    const int nst = (int)((long long)(rank + 1) * a.groups / split) - it0;
+    // the CTAs of a cluster share a tile; from registers and by a multiplication, because divisions here are in front of everything
+    const int split = a.split, rank = (int)special_register<kClusterRank>(), first = (int)special_register<kClusterId>();
+    const int step = (int)special_register<kClusters>();
+    const int it0 = split > 1 ? (int)__umulhi(rank * a.groups, a.over_split) : 0;    // scale groups of this CTA
+    const int nst = (split > 1 ? (int)__umulhi((rank + 1) * a.groups, a.over_split) : a.groups) - it0;
     const int box_bytes = tm * kBoxK * 2, stage_bytes = 2 * box_bytes;
     constexpr int rb_tile = kTileN / kTileRows;                                        // row blocks of a tile
     uint8_t* codes = smem + nb * stage_bytes;
@@ -153,6 +167,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     const uint32_t drained = bar0 + 8u * (2 * kMaxB + 2 * kCodes + 4);
 
     if (tid == 0) {
+        prefetch_map(&map_w);
+        prefetch_map(&map_x);
         for (int s = 0; s < kMaxB; s++) {
             mbar_init(full(s), 5);
             mbar_init(done(s), 1);
@@ -558,6 +574,7 @@ int launch_gemm_tcgen05(const half* A, const uint8_t* packed, const RowsOut* out
     const int nrb = (a.N + kTileRows - 1) / kTileRows;
     choose(a, (a.N + kTileN - 1) / kTileN, *dev);
     if (!a.split) return fail(TLLM_ERR_SHAPE, "gemm_tcgen05: M=%d N=%d K=%d: too many tiles", M, a.N, K);
+    a.over_split = (uint32_t)((0x100000000ull + a.split - 1) / a.split);         // of one CTA not used
     a.err = err;
     a.acc_stride = (a.tm + 31) / 32 * 32;
     a.accs = a.tm > kMaxTm2 ? 1 : 2;

@@ -194,6 +194,9 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     int never = 0;
 
     if (tid == 0) {
+        prefetch_map(&map_q);
+        prefetch_map(&map_k);
+        prefetch_map(&map_v);
         for (int i = 0; i < kBars; i++) mbar_init(bar(i), i == kPReady ? kTile : 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

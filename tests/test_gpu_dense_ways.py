@@ -1,5 +1,5 @@
-"""The dense GEMM of prompts (csrc/dense_gemm.cu) at sizes that take each of its tiles, 64, 128 and 256 features of one CTA and
-128 and 256 of a pair: whole and ragged rows, features and columns, one round of tiles and several, against 64 bits."""
+"""The dense GEMM of prompts (csrc/dense_gemm.cu) at sizes that take each of its tiles, 64, 128 and 256 features of one CTA,
+128 and 256 of a pair, 64 of two, four and eight CTAs that share K: whole and ragged rows, features and columns, one round of tiles and several, against 64 bits."""
 import pytest
 import torch
 
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m", [9, 128, 129, 256, 257, 300, 385, 1000])
-@pytest.mark.parametrize("n,k", [(64, 64), (2048, 512), (2050, 4104), (4096, 2048), (4100, 72), (9000, 1032)])
+@pytest.mark.parametrize("n,k", [(64, 64), (500, 4104), (1000, 2056), (2048, 512), (2050, 4104), (4096, 2048), (4100, 72), (9000, 1032)])
 @pytest.mark.parametrize("glu", [False, True])
 def test_product(m, n, k, glu):
     gen = torch.Generator(device="cuda").manual_seed(m + n + k)

@@ -25,8 +25,14 @@
 // longest link is the softmax, a row per thread: two scores per instruction where there is one for it and no mask but in the tiles that
 // need one; with a mask in every tile and one score at a time 2000 queries took 117 and 130 us, 300 16.1 and 17.9.  The MMAs and
 // copies are issued by an elected lane of a warp that runs the loop together (2000 queries 85 -> 76, 96 -> 90).
+//
+// Latent attention over expanded keys and values (BF16, key parts and values in pieces of 64) is the same walk with a key of two
+// parts; its operands leave room for one CTA an SM.  16 heads of 128 + 64, 2000 tokens: 192 -> 75 us a launch against
+// mma.sync on 64 queries (latent_attention.cu, which keeps the other sizes).  Tried: the scores read from tensor memory twice, 64 at a time,
+// which leaves no spills: 75 -> 85, 90 -> 100 (FP16, 128).
 // All mbarrier waits are bounded (see dense_gemm.cu).
 #include <cfloat>
+#include <climits>
 #include <type_traits>
 
 #include "f32x2.cuh"
@@ -74,6 +80,18 @@ struct PromptArgs {
     int head_rows, k_cols, v_cols;
     float scale2, out_scale;
     int* err;
+};
+
+// Latent attention: a head's keys are dim columns of its own and rot columns that all heads share (columns shared_col .. of rows of
+// ld_shared); q has rows of ld_q with dim + rot columns a head, k and v of heads * dim and heads * vdim.  The other kernels take the
+// empty one, so that nothing of it is in their parameters.
+template <bool LATENT> struct LatentPart {};
+template <> struct LatentPart<true> {
+    CUtensorMap map_r;                  // the shared columns
+    const bf16* shared;
+    const float* sink;                  // [heads] or null: exp(sink) joins the sum of the weights
+    const bf16* gate;                   // out *= sigmoid(gate[row * gate_ld + head]), or null
+    int rot, ld_q, ld_shared, shared_col, gate_ld;
 };
 
 __device__ __forceinline__ int chunk_start(int pos, int chunk) { return chunk > 0 ? pos / chunk * chunk : 0; }
@@ -169,12 +187,58 @@ __device__ __forceinline__ void visible_row(const PromptArgs<half>& a, int h, in
         if (i < pairs) out[32 * i] = l > 0.f ? __floats2half2_rn(o[i].x / l, o[i].y / l) : __floats2half2_rn(0.f, 0.f);
 }
 
+// The same for latent attention in BF16: a lane has vdim / 32 neighbouring outputs (two or four).
+__device__ __forceinline__ void visible_row(const PromptArgs<bf16>& a, const LatentPart<true>& x, int h, int qi, int lane)
+{
+    const int dq = a.dim + x.rot, heads = gridDim.y, len = a.pos0 + qi + 1, per = a.vdim / 32;
+    const bf16 *q = a.q + (size_t)qi * x.ld_q + (size_t)h * dq, *vb = a.v + (size_t)h * a.vdim + lane * per;
+    float m = -FLT_MAX, l = 0.f, o[4] = {};
+#pragma unroll 1
+    for (int p0 = 0; p0 < len; p0 += 32) {
+        const int p = p0 + lane;
+        const bool sees = p < len;
+        float s = 0.f;
+#pragma unroll 1
+        for (int d = 0; sees && d < dq; d += 8) {
+            const bf16* k = d < a.dim ? a.k + ((size_t)p * heads + h) * a.dim + d : x.shared + (size_t)p * x.ld_shared + x.shared_col + d - a.dim;
+            float u[8], w8[8];
+            Vec16<bf16>::unpack(*reinterpret_cast<const uint4*>(q + d), u);
+            Vec16<bf16>::unpack(*reinterpret_cast<const uint4*>(k), w8);
+#pragma unroll
+            for (int i = 0; i < 8; i++) s = fmaf(u[i], w8[i], s);
+        }
+        s *= a.scale2;
+        const float m_new = fmaxf(m, warp_max(sees ? s : -FLT_MAX)), c = exp2_neg(m - m_new), w = sees ? exp2_neg(s - m_new) : 0.f;
+        l = l * c + w;
+#pragma unroll
+        for (int i = 0; i < 4; i++) o[i] *= c;
+#pragma unroll 1
+        for (int j = 0; j < min(32, len - p0); j++) {
+            const float wj = __shfl_sync(0xffffffffu, w, j);
+            const bf16* v = vb + (size_t)(p0 + j) * heads * a.vdim;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (i < per) o[i] = fmaf(wj, to_f<bf16>(v[i]), o[i]);
+        }
+        m = m_new;
+    }
+    l = warp_sum(l);
+    if (x.sink) l += exp2f(x.sink[h] * kLog2e - m);
+    float f = a.out_scale / l;
+    if (x.gate) f *= sigmoid_f(to_f<bf16>(x.gate[(size_t)qi * x.gate_ld + h]));
+    bf16* out = a.out + (size_t)qi * a.ld_out + (size_t)h * a.vdim + lane * per;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (i < per) out[i] = from_f<bf16>(o[i] * f);
+}
+
 enum Bar { kQFull, kKFull, kKEmpty, kVFull, kVEmpty, kSFull, kPReady, kPvDone, kBars };
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2)
+// LATENT: keys of two parts, a sink and a gate per head
+template <typename T, bool LATENT>
+__global__ void __launch_bounds__(kThreads, LATENT ? 1 : 2)
 grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                         const __grid_constant__ CUtensorMap map_v, const PromptArgs<T> a)
+                         const __grid_constant__ CUtensorMap map_v, const PromptArgs<T> a, const __grid_constant__ LatentPart<LATENT> x)
 {
     using Op = Operand<T>;
     extern __shared__ uint8_t smem_raw[];
@@ -187,7 +251,9 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int h = blockIdx.y, g = h / a.per_kv, seq = blockIdx.z, q0 = (gridDim.x - 1 - blockIdx.x) * kTile;       // longest first
     const int nq = min(kTile, a.n - q0), first = a.pos0 + q0, hi = first + nq;                    // positions of the queries
     const int lo = chunk_start(first, a.chunk) & ~(kTile - 1), lo_last = chunk_start(hi - 1, a.chunk);
-    const int tiles = (hi - lo + kTile - 1) / kTile, nd = a.dim / 64, ne = a.vdim / 64;
+    const int tiles = (hi - lo + kTile - 1) / kTile, ne = a.vdim / 64;
+    int nd = a.dim / 64;
+    if constexpr (LATENT) nd += x.rot / 64;
     const uint32_t qs = smem_u32(smem), ks = qs + nd * kBlock, vs = ks + nd * kBlock, bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * i; };
     volatile int* abortp = &abort_flag;
@@ -197,6 +263,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         prefetch_map(&map_q);
         prefetch_map(&map_k);
         prefetch_map(&map_v);
+        if constexpr (LATENT) prefetch_map(&x.map_r);
         for (int i = 0; i < kBars; i++) mbar_init(bar(i), i == kPReady ? kTile : 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -220,7 +287,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         const int head_row = (seq * a.kv_heads + g) * a.head_rows;
         if (leader) {
             mbar_expect_tx(bar(kQFull), nd * kBlock);
-            for (int j = 0; j < nd; j++) tma_load_2d(qs + j * kBlock, &map_q, h * a.dim + j * 64, seq * a.n + q0, bar(kQFull));
+            for (int j = 0; j < nd; j++) tma_load_2d(qs + j * kBlock, &map_q, h * (LATENT ? nd * 64 : a.dim) + j * 64, seq * a.n + q0, bar(kQFull));
         }
         for (int i = 0; i < 2 * tiles; i++, issued++) {
             const int t = i >> 1, row = head_row + (lo + t * kTile) % a.cache_rows;
@@ -231,7 +298,14 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 mbar_expect_tx(bar(v ? kVFull : kKFull), blocks * kBlock);
                 for (int j = 0; j < blocks; j++) {
                     if (v) tma_load_2d(vs + j * kBlock, &map_v, g * a.v_cols + j * 64, row, bar(kVFull));
-                    else tma_load_2d(ks + j * kBlock, &map_k, g * a.k_cols + j * 64, row, bar(kKFull));
+                    else {
+                        if constexpr (LATENT)
+                            if (j * 64 >= a.dim) {
+                                tma_load_2d(ks + j * kBlock, &x.map_r, x.shared_col + j * 64 - a.dim, row, bar(kKFull));
+                                continue;
+                            }
+                        tma_load_2d(ks + j * kBlock, &map_k, g * a.k_cols + j * 64, row, bar(kKFull));
+                    }
                 }
             }
         }
@@ -381,7 +455,14 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             fence_after();
             // a row without a positive sum: zeros from the FP16 operator, as from its decode form
             const bool zeros = std::is_same<T, half>::value && !(l > 0.f);
-            const float f = zeros ? 1.f : a.out_scale / l;
+            float f;
+            if constexpr (LATENT) {
+                if (x.sink) l += exp2f(x.sink[h] * kLog2e - m);
+                f = a.out_scale / l;
+                if (x.gate && tid < nq) f *= sigmoid_f(to_f<T>(x.gate[(size_t)(q0 + tid) * x.gate_ld + h]));
+            } else {
+                f = zeros ? 1.f : a.out_scale / l;
+            }
             T* op = a.out + ((size_t)seq * a.n + q0 + tid) * a.ld_out + (size_t)h * a.vdim;
             uint32_t largest = 0;                                             // exponents order infinities and NaN last
 #pragma unroll 1
@@ -395,7 +476,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
                 if (tid < nq) {
 #pragma unroll
-                    for (int j = 0; std::is_same<T, half>::value && j < 32; j++) largest = max(largest, o[j] & 0x7fffffffu);
+                    for (int j = 0; (std::is_same<T, half>::value || LATENT) && j < 32; j++) largest = max(largest, o[j] & 0x7fffffffu);
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         typename Op::Pair w[4];
@@ -406,10 +487,13 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     }
                 }
             }
-            if constexpr (std::is_same<T, half>::value) {
+            if constexpr (std::is_same<T, half>::value || LATENT) {
                 __syncwarp();                                                 // the rows' first outputs lie before their second
-                for (uint32_t again = __ballot_sync(0xffffffffu, largest >= 0x7f800000u); again; again &= again - 1)
-                    visible_row(a, h, g, seq, q0 + warp * 32 + __ffs(again) - 1, lane);
+                for (uint32_t again = __ballot_sync(0xffffffffu, largest >= 0x7f800000u); again; again &= again - 1) {
+                    const int qi = q0 + warp * 32 + __ffs(again) - 1;
+                    if constexpr (LATENT) visible_row(a, x, h, qi, lane);
+                    else visible_row(a, h, g, seq, qi, lane);
+                }
             }
         } else {
             abort_flag = 1;
@@ -424,6 +508,7 @@ grouped_prompt_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
 }
 
+constexpr size_t kLatentSmem = 220 * 1024;
 size_t smem_bytes(int dim, int vdim) { return (size_t)(2 * (dim / 64) + vdim / 64) * kBlock + 1024; }
 
 template <typename T>
@@ -439,8 +524,9 @@ int encode(EncodeTiledFn enc, CUtensorMap* map, const T* p, int cols, size_t row
     return TLLM_OK;
 }
 
-template <typename T>
-int launch(PromptArgs<T>& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, int heads, int batch, cudaStream_t stream)
+template <typename T, bool LATENT = false>
+int launch(PromptArgs<T>& p, const LatentPart<LATENT>& x, int columns, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, int heads,
+           int batch, cudaStream_t stream)
 {
     p.err = device_error_flag();
     if (!p.err) return fail(TLLM_ERR_LAUNCH, "device scratch unavailable");
@@ -448,12 +534,13 @@ int launch(PromptArgs<T>& p, const CUtensorMap& mq, const CUtensorMap& mk, const
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "grouped_prompt: no current device");
+    const auto kernel = grouped_prompt_tc_kernel<T, LATENT>;
     if (!attr[dev]) {
-        cudaFuncSetAttribute(grouped_prompt_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(128, 128));
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(LATENT ? kLatentSmem : smem_bytes(128, 128)));
         attr[dev] = true;
     }
-    return launch_pdl("grouped_prompt", grouped_prompt_tc_kernel<T>, dim3((p.n + kTile - 1) / kTile, heads, batch), dim3(kThreads),
-                      smem_bytes(p.dim, p.vdim), stream, mq, mk, mv, p);
+    return launch_pdl("grouped_prompt", kernel, dim3((p.n + kTile - 1) / kTile, heads, batch), dim3(kThreads),
+                      smem_bytes(columns, p.vdim), stream, mq, mk, mv, p, x);
 }
 
 }  // namespace
@@ -493,7 +580,56 @@ int launch_grouped_prompt_tcgen05(const GroupedArgs<bf16>& a, cudaStream_t strea
     p.v_cols = a.vdim;
     p.scale2 = a.scale * kLog2e;
     p.out_scale = a.out_scale;
-    return launch(p, mq, mk, mv, a.heads, 1, stream);
+    return launch(p, LatentPart<false>(), p.dim, mq, mk, mv, a.heads, 1, stream);
+}
+
+bool latent_prompt_tcgen05_supported(const LatentArgs<bf16>& a)
+{
+    return a.dim > 0 && a.dim % 64 == 0 && a.rot % 64 == 0 && (a.vdim == 64 || a.vdim == 128) && smem_bytes(a.dim + a.rot, a.vdim) <= kLatentSmem &&
+           a.g.n_seq == 1 && !a.g.pos_dev && a.q_off % 8 == 0 && a.ld % 8 == 0 && a.rank % 8 == 0 && a.slot_stride % 8 == 0 && a.heads <= 65535 &&
+           ((reinterpret_cast<uintptr_t>(a.proj) | reinterpret_cast<uintptr_t>(a.cache)) & 15) == 0;
+}
+
+// kx [context][heads][dim], vx [context][heads][vdim], out [rows][heads][vdim], all on 16-byte boundaries
+int launch_latent_prompt_tcgen05(const LatentArgs<bf16>& a, const bf16* kx, const bf16* vx, bf16* out, cudaStream_t stream)
+{
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return fail(TLLM_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from this driver");
+    const int ctx = a.g.start_pos + a.g.seq_len, dq = a.dim + a.rot, ldc = a.rank + a.rot;
+    const bf16* cache = a.cache + (size_t)a.g.first_slot * a.slot_stride;
+    CUtensorMap mq, mk, mv;
+    LatentPart<true> x = {};
+    int st;
+    if ((st = encode(enc, &mq, a.proj + a.q_off, a.heads * dq, a.g.seq_len, a.ld))) return st;
+    if ((st = encode(enc, &mk, kx, a.heads * a.dim, ctx, (size_t)a.heads * a.dim))) return st;
+    if ((st = encode(enc, &mv, vx, a.heads * a.vdim, ctx, (size_t)a.heads * a.vdim))) return st;
+    if ((st = encode(enc, &x.map_r, cache, ldc, ctx, ldc))) return st;
+    PromptArgs<bf16> p = {};
+    p.out = out;
+    p.ld_out = a.heads * a.vdim;
+    p.q = a.proj + a.q_off;
+    p.k = kx;
+    p.v = vx;
+    p.per_kv = 1;
+    p.kv_heads = a.heads;
+    p.dim = a.dim;
+    p.vdim = a.vdim;
+    p.n = a.g.seq_len;
+    p.pos0 = a.g.start_pos;
+    p.cache_rows = INT_MAX;
+    p.k_cols = a.dim;
+    p.v_cols = a.vdim;
+    p.scale2 = a.scale * kLog2e;
+    p.out_scale = 1.f;
+    x.rot = a.rot;
+    x.ld_q = a.ld;
+    x.ld_shared = ldc;
+    x.shared_col = a.rank;
+    x.shared = cache;
+    x.sink = a.sink;
+    x.gate = a.gate;
+    x.gate_ld = a.gate_ld;
+    return launch<bf16, true>(p, x, dq, mq, mk, mv, a.heads, 1, stream);
 }
 
 // Two or three queries of single heads of 64 behind a few positions: a CTA per query and key/value head on the CUDA cores
@@ -541,7 +677,7 @@ int launch_attention_prompt(const half* q, const half* k_cache, const half* v_ca
     p.cache_rows = p.head_rows = kv_len_max;
     p.scale2 = kLog2e / sqrtf((float)head_dim);
     p.out_scale = 1.f;
-    return launch(p, mq, mk, mv, n_heads, batch, stream);
+    return launch(p, LatentPart<false>(), p.dim, mq, mk, mv, n_heads, batch, stream);
 }
 
 }  // namespace tllm

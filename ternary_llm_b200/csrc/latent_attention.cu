@@ -701,6 +701,9 @@ int launch_latent_expanded(const LatentArgs<bf16>& a, const bf16* kx, const bf16
     int st = check_latent(a);
     if (st) return st;
     if (!latent_expanded_supported(a)) return fail(TLLM_ERR_SHAPE, "latent attention: no expanded form for dim=%d rot=%d vdim=%d", a.dim, a.rot, a.vdim);
+    if (latent_prompt_tcgen05_supported(a) &&
+        ((reinterpret_cast<uintptr_t>(kx) | reinterpret_cast<uintptr_t>(vx) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+        return launch_latent_prompt_tcgen05(a, kx, vx, out, stream);
     const dim3 grid((a.g.seq_len + kExpQ - 1) / kExpQ, a.heads), block(kExpThreads);
     const size_t smem = expanded_smem(a.dim + a.rot, a.vdim);
 #define TLLM_CASE(N)                                                                                                     \

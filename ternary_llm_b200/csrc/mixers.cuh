@@ -152,6 +152,9 @@ int launch_latent_absorbed(const LatentArgs<T>& a, const T* q_abs, T* o_lat, flo
 // [heads][dim], vx [context][heads][vdim], out [rows][heads][vdim] times the output gate.
 bool latent_expanded_supported(const LatentArgs<bf16>& a);
 int launch_latent_expanded(const LatentArgs<bf16>& a, const bf16* kx, const bf16* vx, bf16* out, cudaStream_t stream);
+// the same on tcgen05 (grouped_prompt.cu), which launch_latent_expanded takes where it is supported
+bool latent_prompt_tcgen05_supported(const LatentArgs<bf16>& a);
+int launch_latent_prompt_tcgen05(const LatentArgs<bf16>& a, const bf16* kx, const bf16* vx, bf16* out, cudaStream_t stream);
 
 // ---- grouped-query attention --------------------------------------------------------------
 // Query head h reads key/value head h / (heads / kv_heads); per-head RMS norm of queries and keys

@@ -147,7 +147,7 @@ norm_chain_kernel(const NormArgs<T> a)
 // ---------------------------------------------------------------------------
 // Causal convolution per channel
 // ---------------------------------------------------------------------------
-constexpr int kConvThreads = 128, kConvChunk = 32;
+constexpr int kConvThreads = 128, kConvChunk = 16;
 
 template <typename T> struct Pair;
 template <> struct Pair<bf16> { using type = __nv_bfloat162; };
@@ -156,6 +156,12 @@ __device__ __forceinline__ float2 ld2(const bf16* p) { return __bfloat1622float2
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void st2(bf16* p, float2 v) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v.x, v.y); }
 __device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+// two adjacent values as they lie in memory, for loads that run ahead
+template <typename T> struct Two;
+template <> struct Two<bf16> { using type = uint32_t; };
+template <> struct Two<float> { using type = float2; };
+__device__ __forceinline__ float2 two(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+__device__ __forceinline__ float2 two(float2 v) { return v; }
 
 // A thread owns two adjacent channels and one time chunk; only the threads of the first chunk
 // read the carried inputs, and they also write the new ones.  TAPS = 0: any number of taps.
@@ -188,20 +194,28 @@ causal_conv_kernel(const ConvArgs<T> a, int chunk)
         }
 #pragma unroll
         for (int j = 1; j < TAPS; j++) win[j] = input(t0 - TAPS + j);
-        // Eight tokens at a time: their inputs are requested before the first output is stored (the compiler does not know that the two
-        // lie apart), and the activation is chosen once for all.  Four taps, us, a token at a time / so: 2000 x
-        // 4096 25 / 20, 2000 x 2048 17 / 14.
+        // Eight tokens at a time, the next eight as they lie in memory on their way: the compiler does not move a load over a store, nor
+        // a conversion away from its load, and bound by latency each of these costs a round trip.  Four taps, Petulix prompt of 2000
+        // tokens, us a launch: a token at a time 21, eight without the next ones and chunks of 32 16.8, now 11.6 (its bytes take 5).
         constexpr int kTokens = 8;
+        using Raw = typename Two<T>::type;
+        Raw next[kTokens];
+        auto request = [&](int t) {
+#pragma unroll
+            for (int u = 0; u < kTokens; u++) next[u] = t + u < t1 ? *reinterpret_cast<const Raw*>(x + (size_t)(t + u) * a.ldx) : Raw();
+        };
+        request(t0);
         for (int t = t0; t < t1; t += kTokens) {
-            float2 in[kTokens];
+            Raw in[kTokens];
             float v[2 * kTokens];
 #pragma unroll
-            for (int u = 0; u < kTokens; u++) in[u] = t + u < t1 ? ld2(x + (size_t)(t + u) * a.ldx) : make_float2(0.f, 0.f);
+            for (int u = 0; u < kTokens; u++) in[u] = next[u];
+            request(t + kTokens);
 #pragma unroll
             for (int u = 0; u < kTokens; u++) {
 #pragma unroll
                 for (int j = 0; j + 1 < TAPS; j++) win[j] = win[j + 1];
-                win[TAPS - 1] = in[u];
+                win[TAPS - 1] = two(in[u]);
                 v[2 * u] = b0;
                 v[2 * u + 1] = b1;
 #pragma unroll
@@ -593,13 +607,17 @@ int scan16_passes(const ScanArgs<float>&, int, cudaStream_t) { return TLLM_ERR_S
 // ---------------------------------------------------------------------------
 // Real-gated linear recurrence: one thread per channel and time chunk
 // ---------------------------------------------------------------------------
+// Bound by the latency of its loads, so a thread has those of TT tokens under way at once: 16 in the first pass, 8 in the second, which
+// carries the outputs' gate too (16 there cost 38 us: fewer threads fit).  A Petulix prompt of 2000 tokens, us: first pass 35.5 with 8
+// tokens and each load converted where it stands, 25.0 with the conversions behind, 17.4 with 16 tokens; second 36.2 -> 29.7.  Requesting
+// a tile ahead of the sums was slower in every form (32 and 41 with tiles of 4, 33 and 62 with 8).
 constexpr int kGateThreads = 64;
 
 template <typename T, bool OUT>
-__global__ void __launch_bounds__(kGateThreads)
+__global__ void __launch_bounds__(kGateThreads, 1)
 gated_scan_kernel(const GatedScanArgs<T> a, int nchunk)
 {
-    constexpr int TT = 8;
+    constexpr int TT = OUT ? 8 : 16;
     pdl_launch_dependents();
     const int c = blockIdx.x * kGateThreads + threadIdx.x, chunk = blockIdx.y, b = blockIdx.z;
     const int n = a.g.seq_len, len = (n + nchunk - 1) / nchunk, t0 = min(n, chunk * len), t1 = min(n, t0 + len);
@@ -624,15 +642,26 @@ gated_scan_kernel(const GatedScanArgs<T> a, int nchunk)
 #pragma unroll 8
         for (int k = 0; k < chunk; k++) S = fmaf(expf(rec_log[(size_t)k * CH]), S, rec[(size_t)k * CH]);
     }
-    for (int t = t0; t < t1; t += TT) {
-        float r[TT], i[TT], u[TT], y[OUT ? TT : 1];
+    // as they lie in memory: every load is under way before the first is used
+    float r_raw[TT], i_raw[TT];
+    T u_raw[TT], y_raw[OUT ? TT : 1];
+    auto request = [&](int t) {
 #pragma unroll
         for (int j = 0; j < TT; j++) {
             const bool in = t + j < t1;                        // past the end r = u = 0: the state stays
-            r[j] = in ? rp[(size_t)(t + j) * 2 * CH] : 0.f;
-            i[j] = in ? rp[(size_t)(t + j) * 2 * CH + a.block] : 0.f;
-            u[j] = in ? to_f<T>(up[(size_t)(t + j) * CH]) : 0.f;
-            if (OUT) y[j] = in ? to_f<T>(yp[(size_t)(t + j) * a.ld_y]) : 0.f;
+            r_raw[j] = in ? rp[(size_t)(t + j) * 2 * CH] : 0.f;
+            i_raw[j] = in ? rp[(size_t)(t + j) * 2 * CH + a.block] : 0.f;
+            u_raw[j] = in ? up[(size_t)(t + j) * CH] : T(0.f);
+            if (OUT) y_raw[j] = in ? yp[(size_t)(t + j) * a.ld_y] : T(0.f);
+        }
+    };
+    for (int t = t0; t < t1; t += TT) {
+        float r[TT], i[TT], u[TT], y[OUT ? TT : 1];
+        request(t);
+#pragma unroll
+        for (int j = 0; j < TT; j++) {
+            r[j] = r_raw[j], i[j] = i_raw[j], u[j] = to_f<T>(u_raw[j]);
+            if (OUT) y[j] = to_f<T>(y_raw[j]);
         }
         if (OUT) apply_act_n(a.act, y);
 #pragma unroll
@@ -674,8 +703,12 @@ int launch_causal_conv(const ConvArgs<T>& a, cudaStream_t stream)
 {
     if (a.g.rows() == 0) return TLLM_OK;
     if (a.channels % 2 || a.ldx % 2 || a.taps < 1) return fail(TLLM_ERR_SHAPE, "causal_conv: channels=%d ldx=%d taps=%d", a.channels, a.ldx, a.taps);
-    const int chunk = a.taps - 1 > kConvChunk ? a.taps - 1 : kConvChunk;
-    const dim3 grid((a.channels / 2 + kConvThreads - 1) / kConvThreads, (a.g.seq_len + chunk - 1) / chunk, a.g.n_seq), block(kConvThreads);
+    // a chunk reads taps - 1 tokens before it again; chunks of 8 where 16 would leave SMs without one (us, chunks of 8 / 16 / 32: Petulix
+    // 2000 tokens 12.9 / 10.9 / 12.6, 100 tokens 4.8 / 6.3 / 8.9, Femolix 1000 tokens 9.6 / 8.4 / 13.8)
+    const int gx = (a.channels / 2 + kConvThreads - 1) / kConvThreads;
+    const int fill = (long long)gx * a.g.n_seq * ((a.g.seq_len + kConvChunk - 1) / kConvChunk) < 148 ? kConvChunk / 2 : kConvChunk;
+    const int chunk = a.taps - 1 > fill ? a.taps - 1 : fill;
+    const dim3 grid(gx, (a.g.seq_len + chunk - 1) / chunk, a.g.n_seq), block(kConvThreads);
     switch (a.taps) {
         case 2: return launch_pdl("causal_conv", causal_conv_kernel<T, 2>, grid, block, 0, stream, a, chunk);
         case 3: return launch_pdl("causal_conv", causal_conv_kernel<T, 3>, grid, block, 0, stream, a, chunk);

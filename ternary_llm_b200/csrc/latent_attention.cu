@@ -8,7 +8,9 @@
 //     the result.  The cache row is read once for 16 (token, head) pairs, which is what a decode
 //     step wants: the positions are split over CTAs, partial results are merged afterwards.
 //   expanded -- keys and values of the whole context are computed once and a tile of 64 queries
-//     of one head walks over them: fewer operations per (query, key) pair, for prompts.
+//     of one head walks over them: fewer operations per (query, key) pair, for prompts.  Values
+//     of 64 or 128 entries and key parts of whole 64s take the tcgen05 kernel of grouped_prompt.cu
+//     instead of the one here.
 // The BF16 kernels run on mma.sync with FP32 scores; the softmax weights enter the second
 // product as the sum of two BF16 numbers (high part and remainder), so they keep 16 bits.
 // The exact 32-bit mode uses the plain kernel below, which also takes latents wider than the
@@ -167,14 +169,18 @@ constexpr int kAbsThreads = 256, kAbsWarps = kAbsThreads / 32, kAbsRows = 16;
 constexpr int kAbsMaxSplit = 64, kAbsTargetCtas = 2 * 148;
 
 struct SplitPlan {
-    int row_tiles, nsplit;
+    int row_tiles, nsplit, tile;
 };
-SplitPlan split_plan(int n_seq, int seq_len, int heads, int keys)
+// `tile`: positions of a CTA's tile, and what a split is a multiple of.  A step is the chain of one tile, so tiles of 32 where tiles of 64
+// would leave SMs without one (16 heads, rank 512, steps behind 100 / 1900 tokens: 8.0 / 8.6 -> 6.3 / 7.7 us, the merge of twice the
+// records 3.3 / 4.7 -> 3.3 / 5.0); with every SM busy a tile of 64 has half of the barriers.
+SplitPlan split_plan(int n_seq, int seq_len, int heads, int keys, bool fits64)
 {
     SplitPlan p;
     p.row_tiles = (seq_len * heads + kAbsRows - 1) / kAbsRows;
+    p.tile = fits64 && (long long)p.row_tiles * n_seq * ((keys + 63) / 64) > 148 ? 64 : 32;
     int s = kAbsTargetCtas / (p.row_tiles * n_seq);
-    const int most = (keys + 63) / 64;
+    const int most = (keys + p.tile - 1) / p.tile;
     if (s > most) s = most;
     if (s > kAbsMaxSplit) s = kAbsMaxSplit;
     p.nsplit = s < 1 ? 1 : s;
@@ -182,7 +188,7 @@ SplitPlan split_plan(int n_seq, int seq_len, int heads, int keys)
 }
 
 // positions per split when `total` positions exist
-__device__ __forceinline__ int split_len(int total, int nsplit) { return ((total + nsplit - 1) / nsplit + 63) & ~63; }
+__device__ __forceinline__ int split_len(int total, int nsplit, int tile) { return ((total + nsplit - 1) / nsplit + tile - 1) & -tile; }
 
 // ws record of (sequence, row, split): rank unnormalised sums, then maximum (base-2) and sum
 template <int TK, int NTW>
@@ -215,25 +221,35 @@ latent_absorbed_mma_kernel(const LatentArgs<bf16> a, const bf16* __restrict__ q_
     pdl_wait();
     const int pos0 = a.g.pos_dev ? *a.g.pos_dev : a.g.start_pos;
     const int total = min(pos0 + a.g.seq_len, a.max_seq);
-    const int len = split_len(total, nsplit), lo = split * len;
+    const int len = split_len(total, nsplit, TK), lo = split * len;
     if (lo >= total) return;
     const int last_row = min(r0 + kAbsRows, rows) - 1;
     const int hi = min(min(total, lo + len), pos0 + last_row / a.heads + 1);   // positions some row of the tile sees
     const bf16* cache = a.cache + (size_t)(a.g.first_slot + b) * a.slot_stride;
     const int pieces = dk / 8;
     const bf16* q = q_abs + ((size_t)b * rows + r0) * dk;
-    for (int i = tid; i < kAbsRows * pieces; i += kAbsThreads) {
-        const int r = i / pieces, c = i - r * pieces;
+    // 16-byte pieces of the tiles' rows, a division a thread instead of one a piece
+    const int row_first = tid / pieces, c_first = tid - row_first * pieces, row_step = kAbsThreads / pieces, c_step = kAbsThreads - row_step * pieces;
+    auto pieces_of = [&](int n, auto&& copy) {
+        for (int r = row_first, c = c_first; r < n; r += row_step) {
+            copy(r, c * 8);
+            c += c_step;
+            if (c >= pieces) {
+                c -= pieces;
+                r++;
+            }
+        }
+    };
+    pieces_of(kAbsRows, [&](int r, int c) {
         const bool v = r0 + r < rows;
-        cp16(qs + r * ldk + c * 8, v ? q + (size_t)r * dk + c * 8 : q_abs, v);
-    }
+        cp16(qs + r * ldk + c, v ? q + (size_t)r * dk + c : q_abs, v);
+    });
     auto load_tile = [&](int k0, int stage) {
         bf16* dst = ks + (size_t)stage * TK * ldk;
-        for (int i = tid; i < TK * pieces; i += kAbsThreads) {
-            const int r = i / pieces, c = i - r * pieces;
+        pieces_of(TK, [&](int r, int c) {
             const bool v = k0 + r < hi;
-            cp16(dst + r * ldk + c * 8, v ? cache + (size_t)(k0 + r) * dk + c * 8 : cache, v);
-        }
+            cp16(dst + r * ldk + c, v ? cache + (size_t)(k0 + r) * dk + c : cache, v);
+        });
         cp_commit();
     };
     float acc[NTW][4];
@@ -354,7 +370,7 @@ latent_absorbed_mma_kernel(const LatentArgs<bf16> a, const bf16* __restrict__ q_
 constexpr int kMergeThreads = 64;
 
 __global__ void __launch_bounds__(kMergeThreads)
-latent_merge_kernel(const LatentArgs<bf16> a, const float* __restrict__ ws, bf16* __restrict__ o_lat, int nsplit)
+latent_merge_kernel(const LatentArgs<bf16> a, const float* __restrict__ ws, bf16* __restrict__ o_lat, int nsplit, int tile)
 {
     __shared__ float wgt[kAbsMaxSplit];
     pdl_launch_dependents();
@@ -362,7 +378,7 @@ latent_merge_kernel(const LatentArgs<bf16> a, const float* __restrict__ ws, bf16
     const int c = blockIdx.y * kMergeThreads + threadIdx.x;
     pdl_wait();
     const int total = min((a.g.pos_dev ? *a.g.pos_dev : a.g.start_pos) + a.g.seq_len, a.max_seq);
-    const int len = split_len(total, nsplit), active = (total + len - 1) / len, rec = a.rank + 2;
+    const int len = split_len(total, nsplit, tile), active = (total + len - 1) / len, rec = a.rank + 2;
     const float* base = ws + (size_t)row * nsplit * rec;
     // the first half of the partial sums is requested before the weights are known
     constexpr int kAtOnce = kAbsMaxSplit / 2;
@@ -651,11 +667,11 @@ int absorbed(const LatentArgs<bf16>& a, const bf16* q_abs, bf16* o_lat, float* w
     const int dk = a.rank + a.rot;
     const bool fits64 = absorbed_smem(64, dk) <= kSmemLimit, fits32 = absorbed_smem(32, dk) <= kSmemLimit;
     if (!fits32 || a.rank > 8 * kAbsWarps * 16) return launch_plain<bf16>(a, q_abs, o_lat, stream);
-    const SplitPlan p = split_plan(a.g.n_seq, a.g.seq_len, a.heads, a.g.pos_dev ? a.max_seq : a.g.start_pos + a.g.seq_len);
-    int st = fits64 ? launch_absorbed_tk<64>(a, q_abs, ws, p, stream) : launch_absorbed_tk<32>(a, q_abs, ws, p, stream);
+    const SplitPlan p = split_plan(a.g.n_seq, a.g.seq_len, a.heads, a.g.pos_dev ? a.max_seq : a.g.start_pos + a.g.seq_len, fits64);
+    int st = p.tile == 64 ? launch_absorbed_tk<64>(a, q_abs, ws, p, stream) : launch_absorbed_tk<32>(a, q_abs, ws, p, stream);
     if (st) return st;
     return launch_pdl("latent_merge", latent_merge_kernel, dim3(a.g.rows() * a.heads, (a.rank + kMergeThreads - 1) / kMergeThreads),
-                      dim3(kMergeThreads), 0, stream, a, ws, o_lat, p.nsplit);
+                      dim3(kMergeThreads), 0, stream, a, ws, o_lat, p.nsplit, p.tile);
 }
 
 }  // namespace

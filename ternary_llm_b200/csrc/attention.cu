@@ -21,8 +21,9 @@
 //             of a shared-memory phase on different banks;
 //   softmax - one warp per query head over the chunk's 256 scores;
 //   P.V     - one thread per (query head, channel), V rows read from shared memory.
-// Decode (seq_len == 1) splits the cache positions over several CTAs (one chunk each);
-// each writes (max, sum, unnormalised output) and the CTA that arrives last on a counter
+// A single token of head sizes 64 and 128 is served by the clusters of attention_step.cu, prompts of
+// those sizes by the tcgen05 kernel of grouped_prompt.cu.  Other single tokens split the cache
+// positions over several CTAs (one chunk each); each writes (max, sum, unnormalised output) and the CTA that arrives last on a counter
 // merges them in split order and resets the counter, so replays of a captured graph need
 // no host-side clearing.
 #include <cfloat>

@@ -9,6 +9,8 @@
 //   cache) | o GEMV with the quantiser in its staging |
 //   [gate|up] GEMV with add + RMSNorm + quantise in its staging |
 //   down GEMV with SwiGLU + quantise in its staging
+// FP16 activations take the same five launches with the products on the few-row kernel
+// (gemm_rows.cu) where that is quicker (row_supported).
 // The activation scale stays in device memory (the reference copies it to the host before
 // every GEMV, src/transformer.cpp:132-136), the position and the token live in device
 // memory too, and greedy sampling runs on the device, so that one decode step can be

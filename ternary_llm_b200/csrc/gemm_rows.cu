@@ -1,4 +1,4 @@
-// Products of a few activation rows (4..32) with a ternary matrix, C[M, N] = A[M, K] . W^T.
+// Products of a few activation rows (4..32; one in a decode step) with a ternary matrix, C[M, N] = A[M, K] . W^T.
 //
 // Bound: the weight stream and, at these sizes, the latencies of a launch.  A tcgen05 tile of 128
 // features walks its weights through tensor memory one scale group at a time, a chain of about a

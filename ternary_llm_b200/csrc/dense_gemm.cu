@@ -21,11 +21,14 @@
 // tile, so both factors of a product meet in the same thread.  Tiles also run over the entries
 // of a block-diagonal or per-head product (column offset in X and Y, row offset in W).  All
 // mbarrier waits are bounded; a wait that gives up sets the device error flag, the roles wait
-// for their own copies and MMAs (bounded again), and TMEM is freed.
+// for their own copies and MMAs (bounded again), and TMEM is freed.  The CTAs of a pair give up together: the
+// copies of both count on the first one's barriers, so it waits for what either has issued (pair_drain.cuh)
+// before both leave.
 #include <mutex>
 
 #include "dense.cuh"
 #include "launch.cuh"
+#include "pair_drain.cuh"
 #include "tcgen05.cuh"
 
 namespace tllm {
@@ -111,11 +114,18 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, 
     else
         tma_load_2d(dst, map, x, y, bar);
 }
-__device__ __forceinline__ uint32_t in_first_cta(uint32_t addr)
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, int rank)
 {
     uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
+}
+__device__ __forceinline__ uint32_t in_first_cta(uint32_t addr) { return in_cta(addr, 0); }
+__device__ __forceinline__ void store_cluster(uint32_t addr, int v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+// counts bytes that no copy will bring
+__device__ __forceinline__ void complete_tx(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void arrive_cluster(uint32_t bar)
 {
@@ -141,7 +151,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
     __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, other_count;            // of a pair: stages that the second CTA filled, tiles that the first one committed
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int outs = a.glu ? TN / 2 : TN;              // output features of a tile
@@ -189,6 +199,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
     volatile int* abortp = &abort_flag;
+    int fills = 0;                                     // stages that this warp's producer filled
+    auto give_up = [&]() {
+        abort_flag = 1;
+        if constexpr (PAIR) store_cluster(in_cta(smem_u32(&abort_flag), rank ^ 1), 1);
+    };
     int never = 0;
     pdl_wait();
     // tile -> first token, first feature, batch entry, entry of W; tokens vary fastest (neighbours
@@ -305,7 +320,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         const bool leader = elect_one();
-        int s = 0, phase = 1, used = 0;                  // stage, parity that means empty; stages filled, up to all of them
+        int s = 0, phase = 1;                            // stage, parity that means empty
         bool ok = true;
         for (int tile = first_tile; ok && tile < tiles; tile += step_tiles) {
             int m0, n0, z, entry;
@@ -320,26 +335,22 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                     load_tile<PAIR>(dst + kXBytes, &map_w, (k0 + k) * kBlkK, rank ? wr1 : wr0, bar);
                     if (!PAIR) load_tile<PAIR>(dst + kXBytes + TN / 2 * kBlkK * 2, &map_w, (k0 + k) * kBlkK, wr1, bar);
                 }
-                used = min(used + 1, kStages);
+                fills++;
                 if (++s == kStages) {
                     s = 0;
                     phase ^= 1;
                 }
             }
         }
-        if (!ok) abort_flag = 1;
+        if (!ok) give_up();
         __syncwarp();
         // normally the MMAs consume every stage; after an abort the copies still in flight
-        // must land before the shared memory goes away
-        if (*abortp && rank) __nanosleep(1000000);       // they count on the other CTA's barriers, which waits for them
-        if (*abortp && rank == 0)
-            for (; used > 0; used--) {
-                if (--s < 0) {
-                    s = kStages - 1;
-                    phase ^= 1;
-                }
-                mbar_wait(full(s), phase ^ 1, &never);
-            }
+        // must land before the shared memory goes away (of a pair: below, for both CTAs)
+        if constexpr (PAIR) {
+            if (leader && rank) store_cluster(in_cta(smem_u32(&other_count), 0), fills);
+        } else if (*abortp) {
+            for (int f = max(0, fills - kStages); f < fills; f++) mbar_wait(full(f % kStages), (f / kStages) & 1, &never);
+        }
     } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer ----------------
         const bool leader = elect_one();
@@ -370,11 +381,13 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             // arrives after everything issued so far, on the abort path too
             if (leader) commit<PAIR>(acc_full(buf));
         }
-        if (!ok) abort_flag = 1;
+        if (!ok) give_up();
+        if constexpr (PAIR)
+            if (leader) store_cluster(in_cta(smem_u32(&other_count), 1), i);
         __syncwarp();
         // the last accumulators complete before TMEM and shared memory are given up
         for (int j = i > 2 ? i - 2 : 0; j < i; j++)
-            if (!mbar_wait(acc_full(j & 1), (j >> 1) & 1, &never)) abort_flag = 1;
+            if (!mbar_wait(acc_full(j & 1), (j >> 1) & 1, &never)) give_up();
     } else if (warp >= 4) {
         // ---------------- epilogue ----------------
         const int row0 = (ew & 3) * 32, half = ew >> 2;
@@ -383,7 +396,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int tile = first_tile; tile < tiles; tile += step_tiles, i++) {
             const int buf = i & 1;
             if (!__all_sync(0xffffffffu, mbar_wait(acc_full(buf), (i >> 1) & 1, abortp))) {
-                abort_flag = 1;
+                give_up();
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -430,6 +443,21 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     sync_all<PAIR || SPLIT>();                           // of a pair: nothing of one CTA is used by the other any more
+    if constexpr (PAIR) {
+        if (abort_flag) {                                // of both CTAs: the copies of either and the last arrivals come before they leave
+            if (rank == 0 && warp == 0) {
+                for (int f = pair_fills_begin(fills, other_count, kStages); f < pair_fills_end(fills, other_count); f++) {
+                    const PairFill p = pair_fill(f, fills, other_count, kStages);
+                    if (lane == 0 && p.unarmed) mbar_expect_tx(full(p.stage), kStage);
+                    if (lane == 0 && p.lacks) complete_tx(full(p.stage), kStage);
+                    mbar_wait(full(p.stage), p.parity, &never);
+                }
+            } else if (rank == 1 && warp == 1) {
+                for (int j = max(0, other_count - 2); j < other_count; j++) mbar_wait(acc_full(j & 1), (j >> 1) & 1, &never);
+            }
+            sync_all<true>();
+        }
+    }
     if constexpr (SPLIT) {
         if (warp >= 4 && !abort_flag) {
             const int rows = kTok / a.split, nrows = min(32, rows), groups = rows / nrows, per = (outs + 31) / 32;

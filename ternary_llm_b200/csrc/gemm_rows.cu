@@ -37,6 +37,14 @@ constexpr int kThreads = 256;
 constexpr int kStages = 3;
 constexpr int kRowWarps = 2, kGroupWarps = 4;        // RG and KW
 
+// A cluster's CTAs along x, the tiles along y and, where they are more than a grid may be high, z: of the few that this is too many
+// nothing is stored.
+dim3 grid_of(int split, int tiles)
+{
+    const int nz = (tiles + 65534) / 65535;
+    return dim3(split, (tiles + nz - 1) / nz, nz);
+}
+
 struct RowsArgs {
     const uint8_t* packed;
     const half* x;                           // [m, cols]
@@ -115,7 +123,7 @@ gemm_rows_kernel(const RowsArgs a)
     if (a.split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3;
     const int kw = warp % KW, rg = warp / KW;
-    const int rank = blockIdx.x, tile = blockIdx.y;
+    const int rank = blockIdx.x, tile = blockIdx.z * gridDim.y + blockIdx.y;
     const int g0 = a.split > 1 ? __umulhi(rank * a.groups, a.over_split) : 0;
     const int ng = (a.split > 1 ? __umulhi((rank + 1) * a.groups, a.over_split) : a.groups) - g0;
     const int nst = (ng + KW - 1) / KW, mine = (ng - kw + KW - 1) / KW;        // stages; groups of this warp
@@ -311,7 +319,7 @@ gemm_row_kernel(const OneArgs a)
     if (a.split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3;
     const int kw = warp % KW, rg = warp / KW;
-    const int rank = blockIdx.x, tile = blockIdx.y;
+    const int rank = blockIdx.x, tile = blockIdx.z * gridDim.y + blockIdx.y;
     const int g0 = a.split > 1 ? __umulhi(rank * a.groups, a.over_split) : 0;
     const int ng = (a.split > 1 ? __umulhi((rank + 1) * a.groups, a.over_split) : a.groups) - g0;
     const int mine = (ng - kw + KW - 1) / KW;
@@ -543,7 +551,7 @@ int launch(RowsArgs a, cudaStream_t stream)
     a.over_split = (uint32_t)((0x100000000ull + a.split - 1) / a.split);         // of one CTA not used
     a.over_share = (uint32_t)((0x100000000ull + a.share - 1) / a.share);
     const int tiles = (a.nrb * kTileRows + S::kRows - 1) / S::kRows;
-    return launch_pdl_cluster("gemm_rows", gemm_rows_kernel<NB, kRowWarps, kGroupWarps>, a.split, dim3(a.split, tiles), dim3(kThreads),
+    return launch_pdl_cluster("gemm_rows", gemm_rows_kernel<NB, kRowWarps, kGroupWarps>, a.split, grid_of(a.split, tiles), dim3(kThreads),
                               S::kSmem, stream, a);
 }
 
@@ -561,7 +569,7 @@ int launch_one(OneArgs a, cudaStream_t stream)
     const size_t smem = (size_t)(INPUT == kRowNorm ? a.cols : per * kGroup) * sizeof(half);
     if (smem > kOneSmem) return fail(TLLM_ERR_SHAPE, "gemm_row: %d columns", a.cols);
     const int tiles = (a.rows + S::kRows - 1) / S::kRows;
-    return launch_pdl_cluster("gemm_row", gemm_row_kernel<INPUT>, a.split, dim3(a.split, tiles), dim3(kThreads), smem, stream, a);
+    return launch_pdl_cluster("gemm_row", gemm_row_kernel<INPUT>, a.split, grid_of(a.split, tiles), dim3(kThreads), smem, stream, a);
 }
 
 }  // namespace

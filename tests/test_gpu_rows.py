@@ -105,3 +105,25 @@ def test_step_of_one_vector(hidden, inter, heads, kv_heads):
         assert (got - both[0].float()).abs().max().item() <= 2e-2 * scale, f"step {i}, lock step"
     tl.check_device_errors()
     dec.close()
+
+
+@pytest.mark.parametrize("m", [5, 8, 9])
+def test_more_tiles_than_a_grid_is_high(m):
+    """65537 tiles of 64 features and a ragged one: more than the second or third dimension of a grid holds."""
+    n, k = 65536 * 64 + 69, 128
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    words = lambda: torch.randint(-2 ** 31, 2 ** 31, (n, k // 32), generator=gen, device="cuda", dtype=torch.int64).to(torch.int32)
+    nz = words()
+    sg, sc = words() & nz, (torch.rand(n, 1, generator=gen, device="cuda") + 0.5).half()
+    w = tl.PreparedWeight(nz, sg, sc, n, k, register=False, keep_source=False)
+    x = torch.randn(m, k, generator=gen, device="cuda").half()
+    y = torch.full((m, n), 9.0, device="cuda", dtype=torch.float16)
+    tl.ternary_gemv_packed(w, x, y, batch=m)
+    shift = torch.arange(32, device="cuda", dtype=torch.int32)
+    for rows in (slice(0, 130), slice(n // 2, n // 2 + 130), slice(n - 200, n)):
+        t = (((nz[rows, :, None] >> shift) & 1) * (2 * ((sg[rows, :, None] >> shift) & 1) - 1)).reshape(-1, k).double()
+        want = (x.double() @ t.T) * sc[rows, 0].double()
+        # 128 exact products, their sums in FP32, each cut or rounded once, and one rounding to FP16
+        size = (x.double().abs() @ t.abs().T) * sc[rows, 0].double()
+        assert ((y[:, rows].double() - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -16 * size + 1e-7).all()
+    tl.check_device_errors()

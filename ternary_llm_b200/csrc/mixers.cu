@@ -228,6 +228,7 @@ norm_rows_kernel(const NormArgs<T> a)
 // Causal convolution per channel
 // ---------------------------------------------------------------------------
 constexpr int kConvThreads = 128, kConvChunk = 16;
+constexpr int kMaxGridY = 65535;
 
 template <typename T> struct Pair;
 template <> struct Pair<bf16> { using type = __nv_bfloat162; };
@@ -792,7 +793,9 @@ int launch_causal_conv(const ConvArgs<T>& a, cudaStream_t stream)
     // 2000 tokens 12.9 / 10.9 / 12.6, 100 tokens 4.8 / 6.3 / 8.9, Femolix 1000 tokens 9.6 / 8.4 / 13.8)
     const int gx = (a.channels / 2 + kConvThreads - 1) / kConvThreads;
     const int fill = (long long)gx * a.g.n_seq * ((a.g.seq_len + kConvChunk - 1) / kConvChunk) < 148 ? kConvChunk / 2 : kConvChunk;
-    const int chunk = a.taps - 1 > fill ? a.taps - 1 : fill;
+    int chunk = a.taps - 1 > fill ? a.taps - 1 : fill;
+    const int least = (a.g.seq_len + kMaxGridY - 1) / kMaxGridY;       // of a grid that can be launched
+    if (chunk < least) chunk = least;
     const dim3 grid(gx, (a.g.seq_len + chunk - 1) / chunk, a.g.n_seq), block(kConvThreads);
     switch (a.taps) {
         case 2: return launch_pdl("causal_conv", causal_conv_kernel<T, 2>, grid, block, 0, stream, a, chunk);

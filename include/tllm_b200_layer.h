@@ -71,6 +71,11 @@ int tllm_b200_attention_decode(void* q, const void* k, const void* v, void* k_ca
                                int n_heads, int n_kv_heads, int head_dim, int pos, float theta, int max_seq_len,
                                void* stream);
 
+/* How one token of each of `batch` sequences at position pos is spread for head sizes 64 and 128 with 1, 2, 4 or 8
+ * query heads to a KV head: the CTAs that share a KV head, and how many CTAs of such clusters the current device runs at
+ * once.  Nothing is launched. */
+int tllm_b200_attention_step_plan(int n_heads, int n_kv_heads, int head_dim, int batch, int pos, int* parts, int* at_once);
+
 /* silu_mul_forward, include/kernels.cuh:60-62 (kernels/activations.cu:18-74). */
 int tllm_b200_silu_mul(const void* gate, const void* up, void* output, int size, void* stream);
 

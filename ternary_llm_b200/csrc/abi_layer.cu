@@ -157,6 +157,15 @@ int tllm_b200_attention_decode(void* q, const void* k, const void* v, void* k_ca
                                    n_heads, n_kv_heads, head_dim, max_seq_len, pos, nullptr, theta, ws, counters, S(stream));
 }
 
+int tllm_b200_attention_step_plan(int n_heads, int n_kv_heads, int head_dim, int batch, int pos, int* parts, int* at_once)
+{
+    if (!parts || !at_once) return fail(TLLM_ERR_NULL, "attention_step_plan: null pointer");
+    if (batch < 1 || pos < 0 || !attention_step_supported(nullptr, nullptr, nullptr, nullptr, nullptr, n_heads, n_kv_heads, head_dim))
+        return fail(TLLM_ERR_SHAPE, "attention_step_plan: heads=%d/%d head_dim=%d batch=%d pos=%d", n_heads, n_kv_heads, head_dim, batch, pos);
+    const int st = check_device();
+    return st ? st : attention_step_plan(n_heads, n_kv_heads, head_dim, batch * n_kv_heads, pos + 1, parts, at_once);
+}
+
 int tllm_b200_silu_mul(const void* gate, const void* up, void* output, int size, void* stream)
 {
     if (!gate || !up || !output) return fail(TLLM_ERR_NULL, "silu_mul: null pointer");

@@ -33,10 +33,15 @@ namespace cg = cooperative_groups;
 constexpr int kThreads = 256, kWarps = kThreads / 32;
 constexpr int kPasses = 8;             // passes over a warp's positions between two softmax updates
 constexpr int kMaxCluster = 8;
-// A cluster grows while all CTAs run at once, two to an SM, and a CTA keeps more than 64 positions.  A step, us: 8 sequences of the
-// 1B model (64 heads) behind 1800 positions 4 parts 762, 2 parts 871; behind 500 666 / 696; 24 sequences (192) behind 300 one part
-// 869, two 952; 8 of four 8B layers behind 200 4 parts 455, 8 parts 504.
-constexpr int kMaxCtas = 296, kLeast = 64;
+// A cluster grows while all CTAs run at once and a CTA keeps more than 32 positions, or 64 where an SM has more than two of them.  How
+// many run at once is asked of each instantiation and cluster size: a group of eight has one CTA an SM (registers), of four two, of two
+// and one three, and clusters leave some SMs out (264 CTAs of a group of four in clusters of eight).  A launch among others, us, CTAs
+// to 296 for all / so: heads of 128 in groups of eight, 32 key/value heads, behind 400 22.9 / 9.2, behind 2000 39.6 / 22.0, 64 heads behind
+// 2000 43.3 / 37.9; groups of four, 37 heads behind 400 13.4 / 8.2; groups of one, 80 heads behind 2000 30.6 / 19.8; with 32 positions in three
+// CTAs an SM 48 heads of 64 in groups of two, behind 400, 8.5 instead of 6.3.  A step: 8 sequences of the 1B model (64 heads) behind 1800
+// positions 4 parts 762, 2 parts 871; behind 500 666 / 696; 24 sequences (192) behind 300 one part 869, two 952; 8 of four 8B layers
+// behind 200 4 parts 455, 8 parts 504.
+constexpr int kLeast = 64;
 
 struct StepArgs {
     const half *q, *k, *v;             // [batch, heads, hd] of the new token, not rotated
@@ -333,28 +338,68 @@ attention_step_kernel(StepArgs a)
     }
 }
 
+struct Plan {
+    int parts, at_once;                // CTAs of a head; CTAs of such clusters that run at once
+};
+
 template <int HD, int G>
-int launch(const StepArgs& a, int parts, int batch, cudaStream_t stream)
+int plan(int heads, int longest, Plan* p)
 {
-    static bool attr[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
     const auto kernel = attention_step_kernel<HD, G>;
-    if (!attr[dev]) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared<HD, G>));
-        attr[dev] = true;
+    static int slots[64][kMaxCluster + 1] = {};          // CTAs that run at once in clusters of 1, 2, 4, 8
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "attention_step: no current device");
+    if (!slots[dev][1]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared<HD, G>)) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(TLLM_ERR_LAUNCH, "attention_step: no current device");
+        }
+        prefer_max_shared(reinterpret_cast<const void*>(kernel));
+        for (int c = kMaxCluster; c >= 1; c /= 2) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at = {};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = c;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(c * 1024);
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = sizeof(Shared<HD, G>);
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                n = 0;
+            }
+            slots[dev][c] = c == 1 && n < 1 ? 1 : n * c;
+        }
     }
-    return launch_pdl_cluster("attention_step", kernel, parts, dim3(parts, a.n_kv_heads, batch), dim3(kThreads), sizeof(Shared<HD, G>), stream, a);
+    p->parts = 1;
+    while (p->parts < kMaxCluster && heads * p->parts * 2 <= slots[dev][2 * p->parts] &&
+           longest > p->parts * (heads * p->parts * 2 > 2 * 148 ? 2 * kLeast : kLeast))
+        p->parts *= 2;
+    p->at_once = slots[dev][p->parts];
+    return TLLM_OK;
+}
+
+// batch 0: the plan alone
+template <int HD, int G>
+int launch(const StepArgs& a, int heads, int longest, int batch, cudaStream_t stream, Plan* p)
+{
+    const int st = plan<HD, G>(heads, longest, p);
+    if (st || !batch) return st;
+    return launch_pdl_cluster("attention_step", attention_step_kernel<HD, G>, p->parts, dim3(p->parts, a.n_kv_heads, batch), dim3(kThreads),
+                              sizeof(Shared<HD, G>), stream, a);
 }
 
 template <int HD>
-int launch_group(const StepArgs& a, int group, int parts, int batch, cudaStream_t stream)
+int launch_group(const StepArgs& a, int group, int heads, int longest, int batch, cudaStream_t stream, Plan* p)
 {
     switch (group) {
-        case 8: return launch<HD, 8>(a, parts, batch, stream);
-        case 4: return launch<HD, 4>(a, parts, batch, stream);
-        case 2: return launch<HD, 2>(a, parts, batch, stream);
-        default: return launch<HD, 1>(a, parts, batch, stream);
+        case 8: return launch<HD, 8>(a, heads, longest, batch, stream, p);
+        case 4: return launch<HD, 4>(a, heads, longest, batch, stream, p);
+        case 2: return launch<HD, 2>(a, heads, longest, batch, stream, p);
+        default: return launch<HD, 1>(a, heads, longest, batch, stream, p);
     }
 }
 
@@ -374,10 +419,20 @@ int launch_attention_step(const half* q, const half* k, const half* v, half* k_c
 {
     const StepArgs a = {q, k, v, k_cache, v_cache, out, n_kv_heads, kv_len_max, pos, pos_dev, theta};
     const int heads = batch * n_kv_heads, longest = pos_dev ? kv_len_max : pos + 1;
-    int parts = 1;
-    while (parts < kMaxCluster && heads * parts * 2 <= kMaxCtas && longest > parts * kLeast) parts *= 2;
-    return head_dim == 64 ? launch_group<64>(a, n_heads / n_kv_heads, parts, batch, stream)
-                          : launch_group<128>(a, n_heads / n_kv_heads, parts, batch, stream);
+    Plan p;
+    return head_dim == 64 ? launch_group<64>(a, n_heads / n_kv_heads, heads, longest, batch, stream, &p)
+                          : launch_group<128>(a, n_heads / n_kv_heads, heads, longest, batch, stream, &p);
+}
+
+int attention_step_plan(int n_heads, int n_kv_heads, int head_dim, int heads, int longest, int* parts, int* at_once)
+{
+    const StepArgs a = {};
+    Plan p = {};
+    const int st = head_dim == 64 ? launch_group<64>(a, n_heads / n_kv_heads, heads, longest, 0, nullptr, &p)
+                                  : launch_group<128>(a, n_heads / n_kv_heads, heads, longest, 0, nullptr, &p);
+    *parts = p.parts;
+    *at_once = p.at_once;
+    return st;
 }
 
 }  // namespace tllm

@@ -57,5 +57,8 @@ bool attention_step_supported(const half* q, const half* k, const half* v, const
                               int head_dim);
 int launch_attention_step(const half* q, const half* k, const half* v, half* k_cache, half* v_cache, half* out, int batch, int n_heads, int n_kv_heads,
                           int head_dim, int kv_len_max, int pos, const int* pos_dev, float theta, cudaStream_t stream);
+// CTAs that share each of `heads` key/value heads (over all sequences) of a supported call behind `longest` positions, and how many
+// such CTAs run at once
+int attention_step_plan(int n_heads, int n_kv_heads, int head_dim, int heads, int longest, int* parts, int* at_once);
 
 }  // namespace tllm

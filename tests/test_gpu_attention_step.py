@@ -1,11 +1,14 @@
 """Attention of one new token on clusters (csrc/attention_step.cu): edges of a warp's, a CTA's and a cluster's share of the
 positions, more positions than one round of copies holds, every group size, against 64 bits; nothing behind the new position is read, and
 other sequences and positions of the cache stay as they are."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 import ternary_llm_b200 as tl
+from ternary_llm_b200 import _lib
 from ternary_llm_b200 import layer_ops as ops
 from ternary_llm_b200 import tllm_format as tf
 
@@ -69,6 +72,39 @@ def test_values_that_are_not_finite():
     ops.attention_decode(q, k, v, kc, vc, out, hk * group, hk, hd, pos, THETA, pos + 1)
     assert (out[1] == 0).all() and out[[0, 2, 3]].isfinite().all()
     assert (out[4:, 7] == float("inf")).all() and out[4:, :7].isfinite().all() and out[4:, 8:].isfinite().all()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+def test_parts_run_at_once(group, hd):
+    """A KV head is shared by more CTAs only while all of them run at the same time, whatever the registers of a group's kernel leave;
+    one sequence behind a long cache is shared by as many as a cluster has."""
+    def plan(batch, pos, hk=8):
+        parts, at_once = ctypes.c_int(), ctypes.c_int()
+        _lib.check(_lib.lib().tllm_b200_attention_step_plan(group * hk, hk, hd, batch, pos, ctypes.byref(parts), ctypes.byref(at_once)))
+        return parts.value, at_once.value
+    assert plan(1, 4000)[0] == 8 and plan(1, 64)[0] == 2 and plan(1, 63)[0] == 1 and plan(1000, 4000)[0] == 1
+    for batch in range(1, 40):
+        parts, at_once = plan(batch, 4000)
+        assert parts == 1 or batch * 8 * parts <= at_once
+
+
+@pytest.mark.parametrize("group,hd", [(8, 64), (8, 128), (4, 128), (1, 128)])
+@pytest.mark.parametrize("batch", [3, 4, 18])
+def test_lock_step_of_every_group(batch, group, hd):
+    """As below, behind more positions than one round of a CTA's copies holds, where groups share a head differently."""
+    cfg = tf.TllmConfig(vocab_size=500, hidden_dim=256, intermediate_dim=256, n_layers=2, n_heads=8 * group, n_kv_heads=8, head_dim=hd,
+                        max_seq_len=640, rope_theta=10000.0, rms_norm_eps=1e-5)
+    dec = tl.Decoder(tf.random_model(cfg, seed=5), int8_decode=False, max_batch=batch)
+    rng = np.random.default_rng(batch)
+    ctx, last = torch.from_numpy(rng.integers(0, 500, (batch, 600)).astype(np.int32)).cuda(), torch.from_numpy(rng.integers(0, 500, batch).astype(np.int32)).cuda()
+    rows = []
+    for order in (list(range(batch)), list(range(batch))[::-1]):
+        for place, i in enumerate(order):
+            dec.forward_seq(place, ctx[i].clone(), 0)
+        rows.append(dec.forward_batch(last[order].contiguous(), 600).clone())
+    assert torch.equal(rows[0], rows[1].flip(0))
+    dec.close()
 
 
 @pytest.mark.parametrize("batch", [3, 24, 50])

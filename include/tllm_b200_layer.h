@@ -61,12 +61,14 @@ int tllm_b200_attention(const void* q, const void* k_cache, const void* v_cache,
                         void* stream);
 
 /* One new token of one sequence: rope_forward on q and k, copy_to_kv_cache of the rotated k
- * and v at position pos, and attention_forward over positions 0..pos, in ONE launch whose
- * CTAs each own 64 cache positions of a KV head.  q [n_heads, head_dim] is rotated in place;
- * k, v [n_kv_heads, head_dim] as the projections wrote them; caches [n_kv_heads, max_seq_len,
- * head_dim].  No counterpart in the reference (it makes three launches,
- * src/transformer.cpp:225-245).  Uses the same per-device scratch as tllm_b200_attention:
- * the first call with given sizes must not happen during stream capture. */
+ * and v at position pos, and attention_forward over positions 0..pos, in ONE launch.
+ * q [n_heads, head_dim] and k, v [n_kv_heads, head_dim] as the projections wrote them, all three only
+ * read; caches [n_kv_heads, max_seq_len, head_dim].  No counterpart in the reference (it makes three
+ * launches, src/transformer.cpp:225-245).  Head sizes 64 and 128 with 1, 2, 4 or 8 query heads to a
+ * KV head need no scratch: any call may happen during stream capture, and calls on several
+ * streams do not disturb one another.  Other sizes use the per-device scratch of
+ * tllm_b200_attention: their first call with given sizes must not happen during stream capture
+ * (TLLM_ERR_LAUNCH), and calls of one device must be issued in stream order. */
 int tllm_b200_attention_decode(void* q, const void* k, const void* v, void* k_cache, void* v_cache, void* output,
                                int n_heads, int n_kv_heads, int head_dim, int pos, float theta, int max_seq_len,
                                void* stream);

@@ -150,9 +150,12 @@ int tllm_b200_attention_decode(void* q, const void* k, const void* v, void* k_ca
     if (st) return st;
     float* ws = nullptr;
     unsigned* counters = nullptr;
-    st = attention_scratch(attention_decode_workspace_bytes(1, n_heads, n_kv_heads, head_dim, max_seq_len), (size_t)n_kv_heads,
-                           S(stream), &ws, &counters);
-    if (st) return st;
+    if (!attention_step_supported((const half*)q, (const half*)k, (const half*)v, (const half*)k_cache, (const half*)v_cache, n_heads, n_kv_heads,
+                                  head_dim)) {
+        st = attention_scratch(attention_decode_workspace_bytes(1, n_heads, n_kv_heads, head_dim, max_seq_len), (size_t)n_kv_heads,
+                               S(stream), &ws, &counters);
+        if (st) return st;
+    }
     return launch_attention_decode((half*)q, (const half*)k, (const half*)v, (half*)k_cache, (half*)v_cache, (half*)output, 1,
                                    n_heads, n_kv_heads, head_dim, max_seq_len, pos, nullptr, theta, ws, counters, S(stream));
 }

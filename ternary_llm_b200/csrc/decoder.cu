@@ -461,7 +461,8 @@ int tllm_b200_decoder_create_batched(const tllm_b200_model_desc* desc, int flags
     {
         const size_t a = attention_workspace_bytes(max_batch, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len);
         const int few = max_batch < kSplitHeads / c.n_kv_heads ? max_batch : kSplitHeads / c.n_kv_heads;
-        const size_t b = attention_decode_workspace_bytes(few < 1 ? 1 : few, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len);
+        const bool clusters = attention_step_supported(D->q, D->k, D->v, D->k_cache, D->v_cache, c.n_heads, c.n_kv_heads, c.head_dim);
+        const size_t b = clusters ? 0 : attention_decode_workspace_bytes(few < 1 ? 1 : few, c.n_heads, c.n_kv_heads, c.head_dim, c.max_seq_len);
         ALLOC(D->dev_alloc(&D->attn_ws, (a > b ? a : b) / sizeof(float), true));
     }
     ALLOC(D->dev_alloc(&D->attn_counters, (size_t)max_batch * c.n_kv_heads, true));

@@ -74,6 +74,24 @@ def test_values_that_are_not_finite():
     assert (out[4:, 7] == float("inf")).all() and out[4:, :7].isfinite().all() and out[4:, 8:].isfinite().all()
 
 
+def test_first_call_under_capture():
+    """No scratch: a size that no call has had before may be captured."""
+    hk, group, hd, pos, mx = 64, 8, 128, 300, 20000                     # records of this cache would be larger than any other test's
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn(h, hd, generator=gen, device="cuda").half() for h in (hk * group, hk, hk))
+    kc, vc = (torch.zeros(hk, mx, hd, dtype=torch.float16, device="cuda") for _ in range(2))
+    kc[:, :pos], vc[:, :pos] = (torch.randn(hk, pos, hd, generator=gen, device="cuda").half() for _ in range(2))
+    out = [torch.zeros(hk * group, hd, dtype=torch.float16, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.attention_decode(q, k, v, kc, vc, out[0], hk * group, hk, hd, pos, THETA, mx)
+    graph.replay()
+    ops.attention_decode(q, k, v, kc, vc, out[1], hk * group, hk, hd, pos, THETA, mx)
+    assert out[1].any() and torch.equal(*out)
+    tl.check_device_errors()
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("group", [1, 2, 4, 8])
 def test_parts_run_at_once(group, hd):

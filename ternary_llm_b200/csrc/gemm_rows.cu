@@ -480,54 +480,77 @@ struct Cut {
     int split = 0, steps = 0;
 };
 
-// Clusters come in GPCs, so fewer CTAs run at once the larger the cluster; a second round of them costs more than a split saves.
-// Among the splits that run at once, the fewest stages of kGroupWarps groups, of which the exchange in a cluster takes as long as one
-// and a half (1024 x 1024: one CTA and two stages 2.3 us, two CTAs and one 2.7; 512 x 2048: two and two 3.1, four and one 2.6; 8192 x 2048:
-// one and four 5.2, two and two 4.1), then the fewest CTAs.
-template <int NB>
-int cut(int rows, int groups, Cut* c)
+// CTAs of a kernel that run at once in clusters of one to kMaxSplit: slots[cluster size], asked once per device.  Clusters come in
+// GPCs, so fewer run at once the larger the cluster.
+template <typename... KArgs>
+int fill_slots(void (*kernel)(KArgs...), size_t smem, int (&slots)[64][kMaxSplit + 1], int* dev)
 {
-    using S = Shape<NB, kRowWarps, kGroupWarps>;
-    const auto kernel = gemm_rows_kernel<NB, kRowWarps, kGroupWarps>;
-    static int slots[64][kMaxSplit + 1] = {};            // CTAs that run at once
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
-    if (!slots[dev][1]) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
-        }
-        prefer_max_shared(reinterpret_cast<const void*>(kernel));
-        for (int split = kMaxSplit; split >= 1; split--) {
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute at = {};
-            at.id = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim.x = split;
-            at.val.clusterDim.y = at.val.clusterDim.z = 1;
-            cfg.gridDim = dim3(split * 1024);
-            cfg.blockDim = dim3(kThreads);
-            cfg.dynamicSmemBytes = S::kSmem;
-            cfg.attrs = &at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
-                cudaGetLastError();
-                return fail(TLLM_ERR_LAUNCH, "gemm_rows: clusters of %d do not run", split);
-            }
-            slots[dev][split] = n * split;
-        }
+    if (cudaGetDevice(dev) != cudaSuccess || *dev < 0 || *dev >= 64) return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
+    if (slots[*dev][1]) return TLLM_OK;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(TLLM_ERR_LAUNCH, "gemm_rows: no current device");
     }
-    const int tiles = (rows + S::kRows - 1) / S::kRows;
+    prefer_max_shared(reinterpret_cast<const void*>(kernel));
+    for (int split = kMaxSplit; split >= 1; split--) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = split;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(split * 1024);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return fail(TLLM_ERR_LAUNCH, "gemm_rows: clusters of %d do not run", split);
+        }
+        slots[*dev][split] = n * split;
+    }
+    return TLLM_OK;
+}
+
+// A second round of clusters costs more than a split saves.  Among the splits that run at once, the fewest stages of kGroupWarps groups,
+// of which the exchange in a cluster takes as long as one and a half (1024 x 1024: one CTA and two stages 2.3 us, two CTAs and one 2.7; 512 x
+// 2048: two and two 3.1, four and one 2.6; 8192 x 2048: one and four 5.2, two and two 4.1), then the fewest CTAs.
+constexpr int kCutRows = kRowWarps * 2 * kTileRows;      // features of a tile
+void choose_cut(const int (&slots)[kMaxSplit + 1], int rows, int groups, Cut* c)
+{
+    const int tiles = (rows + kCutRows - 1) / kCutRows;
     int best = INT_MAX;
     for (int split = 1; split <= kMaxSplit; split++) {
-        if (split > 1 && (tiles * split > slots[dev][split] || groups < split * kGroupWarps)) continue;
+        if (split > 1 && (tiles * split > slots[split] || groups < split * kGroupWarps)) continue;
         const int per = (groups + split - 1) / split, cost = 2 * ((per + kGroupWarps - 1) / kGroupWarps) + (split > 1 ? 3 : 0);
         if (cost >= best) continue;
         best = cost;
         c->split = split;
-        c->steps = per * ((tiles * split + slots[dev][split] - 1) / slots[dev][split]);
+        c->steps = per * ((tiles * split + slots[split] - 1) / slots[split]);
     }
-    return TLLM_OK;
+}
+
+template <int NB>
+int cut(int rows, int groups, Cut* c)
+{
+    using S = Shape<NB, kRowWarps, kGroupWarps>;
+    static_assert(S::kRows == kCutRows, "one cut for all numbers of rows");
+    static int slots[64][kMaxSplit + 1] = {};
+    int dev = 0;
+    const int st = fill_slots(gemm_rows_kernel<NB, kRowWarps, kGroupWarps>, S::kSmem, slots, &dev);
+    if (!st) choose_cut(slots[dev], rows, groups, c);
+    return st;
+}
+// Of the kernel for one vector, whatever part of its shared memory a launch takes.
+template <int INPUT>
+int cut_one(int rows, int groups, Cut* c)
+{
+    static int slots[64][kMaxSplit + 1] = {};
+    int dev = 0;
+    const int st = fill_slots(gemm_row_kernel<INPUT>, kOneSmem, slots, &dev);
+    if (!st) choose_cut(slots[dev], rows, groups, c);
+    return st;
 }
 int cut_for(int m, int rows, int groups, Cut* c)
 {
@@ -560,7 +583,7 @@ int launch_one(OneArgs a, cudaStream_t stream)
 {
     using S = Shape<1, kRowWarps, kGroupWarps>;
     Cut c;
-    const int st = cut<1>(a.rows, a.groups, &c);         // its shared memory is no larger than the other kernel's
+    const int st = cut_one<INPUT>(a.rows, a.groups, &c);
     if (st) return st;
     a.split = c.split;
     a.share = (S::kRows + a.split - 1) / a.split;
@@ -581,7 +604,9 @@ bool row_supported(RowInput input, int rows, int cols)
 {
     Cut c;
     const int groups = cols / kGroup;
-    if (!groups || cut<1>(rows, groups, &c)) return false;
+    if (!groups) return false;
+    if (input == kRowNorm ? cut_one<kRowNorm>(rows, groups, &c) : input == kRowSilu ? cut_one<kRowSilu>(rows, groups, &c) : cut_one<kRowPlain>(rows, groups, &c))
+        return false;
     return (size_t)(input == kRowNorm ? cols : (groups + c.split - 1) / c.split * kGroup) * sizeof(half) <= kOneSmem &&
            (input != kRowNorm || c.steps <= 32);
 }

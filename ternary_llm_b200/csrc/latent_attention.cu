@@ -717,7 +717,9 @@ int launch_latent_expanded(const LatentArgs<bf16>& a, const bf16* kx, const bf16
     int st = check_latent(a);
     if (st) return st;
     if (!latent_expanded_supported(a)) return fail(TLLM_ERR_SHAPE, "latent attention: no expanded form for dim=%d rot=%d vdim=%d", a.dim, a.rot, a.vdim);
-    if (latent_prompt_tcgen05_supported(a) &&
+    // One tile of 64 keys here has the shorter launch (us here / there: 16 heads of 128 + 64, values of 128, 13 tokens 6.2 / 8.2, 45 tokens
+    // 6.2 / 7.8, 4 behind 30 5.4 / 7.5; two tiles, 68 positions, 8.4 / 6.9).
+    if (a.g.start_pos + a.g.seq_len > kExpK && latent_prompt_tcgen05_supported(a) &&
         ((reinterpret_cast<uintptr_t>(kx) | reinterpret_cast<uintptr_t>(vx) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
         return launch_latent_prompt_tcgen05(a, kx, vx, out, stream);
     const dim3 grid((a.g.seq_len + kExpQ - 1) / kExpQ, a.heads), block(kExpThreads);

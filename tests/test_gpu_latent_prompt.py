@@ -59,6 +59,12 @@ def test_against_64_bits(dim, rot, vdim, n, start):
     tl.check_device_errors()
 
 
+@pytest.mark.parametrize("n,start", [(1, 62), (1, 63), (1, 64), (64, 0), (65, 0), (20, 44), (20, 45)])
+def test_both_sides_of_one_tile_of_keys(n, start):
+    """Up to 64 positions go another way (csrc/latent_attention.cu)."""
+    test_against_64_bits(128, 64, 128, n, start)
+
+
 def test_values_that_are_not_finite():
     """An infinity among a position's values reaches the queries that see it and no other."""
     n, H, scale = 300, 2, 0.1

@@ -171,14 +171,18 @@ constexpr int kAbsMaxSplit = 64, kAbsTargetCtas = 2 * 148;
 struct SplitPlan {
     int row_tiles, nsplit, tile;
 };
-// `tile`: positions of a CTA's tile, and what a split is a multiple of.  A step is the chain of one tile, so tiles of 32 where tiles of 64
-// would leave SMs without one (16 heads, rank 512, steps behind 100 / 1900 tokens: 8.0 / 8.6 -> 6.3 / 7.7 us, the merge of twice the
-// records 3.3 / 4.7 -> 3.3 / 5.0); with every SM busy a tile of 64 has half of the barriers.
+// `tile`: positions of a CTA's tile, and what a split is a multiple of.  A step is the chain of one tile, so tiles of 32 while every SM
+// has no more than one of them and the merge requests all records at once (32; of 16 rows alone, as far as there are
+// records).  us with tiles of 64 / 32, attention and merge: 4 heads, rank 512, behind 1071 9.8 / 9.0, two sequences behind 924 9.8 / 8.6; 16
+// heads, 8 tokens behind 465 (120 tiles of 32) 11.9 / 11.2; 64 heads, 3 tokens behind 340 (132) 13.0 / 12.4; two sequences of 32 heads, rank 128,
+// behind 1315 (168 tiles) 7.5 / 8.3; 16 heads, 3 tokens behind 1167 (37 records) 11.2 / 12.0; 16 sequences behind 302 (160 tiles) 13.9 / 14.7; 8
+// heads behind 3159, where 64 records make a CTA walk two tiles of 32, 10.6 / 12.4.
 SplitPlan split_plan(int n_seq, int seq_len, int heads, int keys, bool fits64)
 {
     SplitPlan p;
     p.row_tiles = (seq_len * heads + kAbsRows - 1) / kAbsRows;
-    p.tile = fits64 && (long long)p.row_tiles * n_seq * ((keys + 63) / 64) > 148 ? 64 : 32;
+    const int records = (keys + 31) / 32;
+    p.tile = fits64 && (long long)p.row_tiles * n_seq * records > (records <= kAbsMaxSplit / 2 ? 148 : kAbsMaxSplit) ? 64 : 32;
     int s = kAbsTargetCtas / (p.row_tiles * n_seq);
     const int most = (keys + p.tile - 1) / p.tile;
     if (s > most) s = most;

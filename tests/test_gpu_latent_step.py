@@ -36,3 +36,10 @@ def test_absorbed_steps(n_seq, n, start, heads, rank, rot):
         bound = (2.0 ** -15 + 2 * (dk + ctx) * 2.0 ** -24 * float(reach)) * size + 2.0 ** -8 * want.abs() + 1e-30
         assert ((out[b * n:(b + 1) * n].double() - want).abs() <= bound).all(), b
     tl.check_device_errors()
+
+
+@pytest.mark.parametrize("n_seq,n,start", [(1, 1, 1023), (1, 1, 1024), (1, 1, 2047), (1, 1, 2048), (4, 1, 1023), (4, 1, 1024), (5, 1, 991), (148, 1, 31),
+                                           (149, 1, 31)])
+def test_both_sides_of_the_lines_of_tiles(n_seq, n, start):
+    """Where tiles go from 32 to 64 positions: by their number, and by the number of records of a row."""
+    test_absorbed_steps(n_seq, n, start, 16, 512, 64)

@@ -177,12 +177,13 @@ struct SplitPlan {
 // heads, 8 tokens behind 465 (120 tiles of 32) 11.9 / 11.2; 64 heads, 3 tokens behind 340 (132) 13.0 / 12.4; two sequences of 32 heads, rank 128,
 // behind 1315 (168 tiles) 7.5 / 8.3; 16 heads, 3 tokens behind 1167 (37 records) 11.2 / 12.0; 16 sequences behind 302 (160 tiles) 13.9 / 14.7; 8
 // heads behind 3159, where 64 records make a CTA walk two tiles of 32, 10.6 / 12.4.
-SplitPlan split_plan(int n_seq, int seq_len, int heads, int keys, bool fits64)
+// known: keys is the number of positions, not that of a cache whose position is on the device; behind fewer the tiles of 32 count.
+SplitPlan split_plan(int n_seq, int seq_len, int heads, int keys, bool known, bool fits64)
 {
     SplitPlan p;
     p.row_tiles = (seq_len * heads + kAbsRows - 1) / kAbsRows;
-    const int records = (keys + 31) / 32;
-    p.tile = fits64 && (long long)p.row_tiles * n_seq * records > (records <= kAbsMaxSplit / 2 ? 148 : kAbsMaxSplit) ? 64 : 32;
+    const int records = (keys + 31) / 32, most32 = !known ? 296 : records <= kAbsMaxSplit / 2 ? 148 : kAbsMaxSplit;
+    p.tile = fits64 && (long long)p.row_tiles * n_seq * records > most32 ? 64 : 32;
     int s = kAbsTargetCtas / (p.row_tiles * n_seq);
     const int most = (keys + p.tile - 1) / p.tile;
     if (s > most) s = most;
@@ -671,7 +672,7 @@ int absorbed(const LatentArgs<bf16>& a, const bf16* q_abs, bf16* o_lat, float* w
     const int dk = a.rank + a.rot;
     const bool fits64 = absorbed_smem(64, dk) <= kSmemLimit, fits32 = absorbed_smem(32, dk) <= kSmemLimit;
     if (!fits32 || a.rank > 8 * kAbsWarps * 16) return launch_plain<bf16>(a, q_abs, o_lat, stream);
-    const SplitPlan p = split_plan(a.g.n_seq, a.g.seq_len, a.heads, a.g.pos_dev ? a.max_seq : a.g.start_pos + a.g.seq_len, fits64);
+    const SplitPlan p = split_plan(a.g.n_seq, a.g.seq_len, a.heads, a.g.pos_dev ? a.max_seq : a.g.start_pos + a.g.seq_len, !a.g.pos_dev, fits64);
     int st = p.tile == 64 ? launch_absorbed_tk<64>(a, q_abs, ws, p, stream) : launch_absorbed_tk<32>(a, q_abs, ws, p, stream);
     if (st) return st;
     return launch_pdl("latent_merge", latent_merge_kernel, dim3(a.g.rows() * a.heads, (a.rank + kMergeThreads - 1) / kMergeThreads),

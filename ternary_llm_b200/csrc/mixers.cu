@@ -227,7 +227,9 @@ norm_rows_kernel(const NormArgs<T> a)
 // ---------------------------------------------------------------------------
 // Causal convolution per channel
 // ---------------------------------------------------------------------------
-constexpr int kConvThreads = 128, kConvChunk = 16;
+// kConvFew: portions up to this many tokens go one by one: what a tile of eight does for those that are not there takes longer (four
+// taps, FP32, one token 2.6 us in a tile, 1.7 alone; BF16, two tokens 2.3 and 1.9).
+constexpr int kConvThreads = 128, kConvChunk = 16, kConvFew = 4;
 constexpr int kMaxGridY = 65535;
 
 template <typename T> struct Pair;
@@ -275,40 +277,55 @@ causal_conv_kernel(const ConvArgs<T> a, int chunk)
         }
 #pragma unroll
         for (int j = 1; j < TAPS; j++) win[j] = input(t0 - TAPS + j);
-        // Eight tokens at a time, the next eight as they lie in memory on their way: the compiler does not move a load over a store, nor
-        // a conversion away from its load, and bound by latency each of these costs a round trip.  Four taps, Petulix prompt of 2000
-        // tokens, us a launch: a token at a time 21, eight without the next ones and chunks of 32 16.8, now 11.6 (its bytes take 5).
-        constexpr int kTokens = 8;
-        using Raw = typename Two<T>::type;
-        Raw next[kTokens];
-        auto request = [&](int t) {
-#pragma unroll
-            for (int u = 0; u < kTokens; u++) next[u] = t + u < t1 ? *reinterpret_cast<const Raw*>(x + (size_t)(t + u) * a.ldx) : Raw();
-        };
-        request(t0);
-        for (int t = t0; t < t1; t += kTokens) {
-            Raw in[kTokens];
-            float v[2 * kTokens];
-#pragma unroll
-            for (int u = 0; u < kTokens; u++) in[u] = next[u];
-            request(t + kTokens);
-#pragma unroll
-            for (int u = 0; u < kTokens; u++) {
+        if (n <= kConvFew) {
+            for (int t = t0; t < t1; t++) {
 #pragma unroll
                 for (int j = 0; j + 1 < TAPS; j++) win[j] = win[j + 1];
-                win[TAPS - 1] = two(in[u]);
-                v[2 * u] = b0;
-                v[2 * u + 1] = b1;
+                win[TAPS ? TAPS - 1 : 0] = ld2(x + (size_t)t * a.ldx);
+                float v0 = b0, v1 = b1;
 #pragma unroll
                 for (int j = 0; j < TAPS; j++) {
-                    v[2 * u] = fmaf(w0[j], win[j].x, v[2 * u]);
-                    v[2 * u + 1] = fmaf(w1[j], win[j].y, v[2 * u + 1]);
+                    v0 = fmaf(w0[j], win[j].x, v0);
+                    v1 = fmaf(w1[j], win[j].y, v1);
                 }
+                st2(y + (size_t)t * a.channels, make_float2(apply_act(a.act, v0), apply_act(a.act, v1)));
             }
-            apply_act_n<2 * kTokens>(a.act, v);
+        } else {
+            // Eight tokens at a time, the next eight as they lie in memory on their way: the compiler does not move a load over a store, nor
+            // a conversion away from its load, and bound by latency each of these costs a round trip.  Four taps, Petulix prompt of 2000
+            // tokens, us a launch: a token at a time 21, eight without the next ones and chunks of 32 16.8, now 11.6 (its bytes take 5).
+            constexpr int kTokens = 8;
+            using Raw = typename Two<T>::type;
+            Raw next[kTokens];
+            auto request = [&](int t) {
 #pragma unroll
-            for (int u = 0; u < kTokens; u++)
-                if (t + u < t1) st2(y + (size_t)(t + u) * a.channels, make_float2(v[2 * u], v[2 * u + 1]));
+                for (int u = 0; u < kTokens; u++) next[u] = t + u < t1 ? *reinterpret_cast<const Raw*>(x + (size_t)(t + u) * a.ldx) : Raw();
+            };
+            request(t0);
+            for (int t = t0; t < t1; t += kTokens) {
+                Raw in[kTokens];
+                float v[2 * kTokens];
+#pragma unroll
+                for (int u = 0; u < kTokens; u++) in[u] = next[u];
+                request(t + kTokens);
+#pragma unroll
+                for (int u = 0; u < kTokens; u++) {
+#pragma unroll
+                    for (int j = 0; j + 1 < TAPS; j++) win[j] = win[j + 1];
+                    win[TAPS - 1] = two(in[u]);
+                    v[2 * u] = b0;
+                    v[2 * u + 1] = b1;
+#pragma unroll
+                    for (int j = 0; j < TAPS; j++) {
+                        v[2 * u] = fmaf(w0[j], win[j].x, v[2 * u]);
+                        v[2 * u + 1] = fmaf(w1[j], win[j].y, v[2 * u + 1]);
+                    }
+                }
+                apply_act_n<2 * kTokens>(a.act, v);
+#pragma unroll
+                for (int u = 0; u < kTokens; u++)
+                    if (t + u < t1) st2(y + (size_t)(t + u) * a.channels, make_float2(v[2 * u], v[2 * u + 1]));
+            }
         }
     } else {
         for (int t = t0; t < t1; t++) {

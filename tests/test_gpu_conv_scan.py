@@ -1,4 +1,4 @@
-"""Causal convolution of very many tokens (csrc/mixers.cu), against 64 bits."""
+"""Causal convolution of few and of very many tokens (csrc/mixers.cu), against 64 bits."""
 import pytest
 import torch
 
@@ -6,7 +6,32 @@ import ternary_llm_b200 as tl
 from ternary_llm_b200 import mixed_ops as ops
 
 pytestmark = pytest.mark.gpu
-BF16 = torch.bfloat16
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+@pytest.mark.parametrize("dt", [BF16, F32])
+@pytest.mark.parametrize("taps", [2, 3, 4, 5])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+def test_conv_of_few_tokens(n, taps, dt):
+    gen = torch.Generator(device="cuda").manual_seed(10 * n + taps)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    C, seqs = 264, 2
+    x, w, b = rand(seqs, n, C).to(dt), rand(C, taps), rand(C)
+    for start in (0, 7):
+        state = rand(seqs, taps - 1, C).to(dt)
+        before = state.double() if start else torch.zeros_like(state).double()
+        if not start: state.fill_(float("nan"))                     # a new sequence must not read it
+        y = torch.full((seqs + 1, n, C), 7.0, device="cuda", dtype=dt)
+        ops.causal_conv(x, w, b, state, y[:seqs], C, taps, seqs, n, start, "silu")
+        full = torch.cat([before, x.double()], dim=1)
+        z = sum(full[:, j:j + n] * w[:, j].double() for j in range(taps)) + b.double()
+        size = sum(full[:, j:j + n].abs() * w[:, j].double().abs() for j in range(taps)) + b.double().abs()
+        want = z * torch.sigmoid(z)
+        # taps products and sums in FP32, through SiLU's slope of at most 1.1 and its own FP32 steps, then the type of the result
+        bound = 1.1 * (taps + 1) * 2.0 ** -23 * size + 2.0 ** -20 * want.abs() + (2.0 ** -8 if dt == BF16 else 0.0) * want.abs() + 1e-30
+        assert ((y[:seqs].double() - want).abs() <= bound).all() and (y[seqs] == 7.0).all()
+        assert torch.equal(state.double(), full[:, n:])
+    tl.check_device_errors()
 
 
 @pytest.mark.parametrize("taps", [4, 9])

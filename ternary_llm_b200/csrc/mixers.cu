@@ -705,17 +705,21 @@ int scan16_passes(const ScanArgs<float>&, int, cudaStream_t) { return TLLM_ERR_S
 // ---------------------------------------------------------------------------
 // Real-gated linear recurrence: one thread per channel and time chunk
 // ---------------------------------------------------------------------------
-// Bound by the latency of its loads, so a thread has those of TT tokens under way at once: 16 in the first pass, 8 in the second, which
-// carries the outputs' gate too (16 there cost 38 us: fewer threads fit).  A Petulix prompt of 2000 tokens, us: first pass 35.5 with 8
-// tokens and each load converted where it stands, 25.0 with the conversions behind, 17.4 with 16 tokens; second 36.2 -> 29.7.  Requesting
-// a tile ahead of the sums was slower in every form (32 and 41 with tiles of 4, 33 and 62 with 8).
+// Bound by the latency of its loads, so a thread has those of TT tokens under way at once, 8 of them as they lie in memory, converted
+// when all are requested (each converted where it stands: first pass of 2000 tokens 35.5 us, so 25.0).  Tiles of 16 in the first pass
+// are as quick there and lose where a chunk is little more than 32 tokens (2048 channels, BF16, both passes, 16 / 8: 712 tokens 28.8 /
+// 24.2).  Requesting a tile ahead of the sums was slower in every form (32 and 41 us with tiles of 4, 33 and 62 with 8).
 constexpr int kGateThreads = 64;
+// The second pass carries the outputs' gate too; in tiles of 4 more threads fit, which hides more where there are CTAs for them, and
+// costs where there are not.  Both passes, us, tiles of 8 / 4: BF16 1984 channels, 2788 tokens (992 CTAs) 62 / 72; 2560, two sequences of
+// 1513 (2560) 82 / 75; 2120, five of 652 (3400) 79 / 72; FP32 896, 3701 (448) 49 / 51; 1272, five of 263 (800) 24.4 / 21.8; 1280, five of 785
+// (2400) 62 / 58.
+template <typename T> constexpr int kGateManyCtas = sizeof(T) == 4 ? 5 * 148 : 11 * 148;
 
-template <typename T, bool OUT>
+template <typename T, bool OUT, int TT>
 __global__ void __launch_bounds__(kGateThreads, 1)
 gated_scan_kernel(const GatedScanArgs<T> a, int nchunk)
 {
-    constexpr int TT = OUT ? 8 : 16;
     pdl_launch_dependents();
     const int c = blockIdx.x * kGateThreads + threadIdx.x, chunk = blockIdx.y, b = blockIdx.z;
     const int n = a.g.seq_len, len = (n + nchunk - 1) / nchunk, t0 = min(n, chunk * len), t1 = min(n, t0 + len);
@@ -880,10 +884,12 @@ int launch_gated_scan(const GatedScanArgs<T>& a, cudaStream_t stream)
     if (nchunk > 1 && !a.rec) return fail(TLLM_ERR_NULL, "gated_scan: no record buffer");
     const unsigned gx = (a.channels + kGateThreads - 1) / kGateThreads;
     if (nchunk > 1) {
-        const int st = launch_pdl("gated_scan", gated_scan_kernel<T, false>, dim3(gx, nchunk - 1, a.g.n_seq), dim3(kGateThreads), 0, stream, a, nchunk);
+        const int st = launch_pdl("gated_scan", gated_scan_kernel<T, false, 8>, dim3(gx, nchunk - 1, a.g.n_seq), dim3(kGateThreads), 0, stream, a, nchunk);
         if (st) return st;
     }
-    return launch_pdl("gated_scan", gated_scan_kernel<T, true>, dim3(gx, nchunk, a.g.n_seq), dim3(kGateThreads), 0, stream, a, nchunk);
+    const bool many = (long long)gx * nchunk * a.g.n_seq > kGateManyCtas<T>;
+    return launch_pdl("gated_scan", many ? gated_scan_kernel<T, true, 4> : gated_scan_kernel<T, true, 8>, dim3(gx, nchunk, a.g.n_seq),
+                      dim3(kGateThreads), 0, stream, a, nchunk);
 }
 
 #define TLLM_INSTANTIATE(T)                                                \

@@ -1,8 +1,10 @@
-"""Causal convolution of few and of very many tokens (csrc/mixers.cu), against 64 bits."""
+"""Causal convolution of few and of very many tokens, gated scan of few and of many CTAs (csrc/mixers.cu), against 64 bits."""
+import numpy as np
 import pytest
 import torch
 
 import ternary_llm_b200 as tl
+from oracle import mixed_oracle as O
 from ternary_llm_b200 import mixed_ops as ops
 
 pytestmark = pytest.mark.gpu
@@ -46,4 +48,24 @@ def test_conv_of_more_chunks_than_a_grid_is_high(taps):
     want, size = (sum(f(full[j:j + n]) * f(w[:, j].double()) for j in range(taps)) for f in (lambda t: t, torch.abs))
     assert ((y.double() - want).abs() <= taps * 2.0 ** -23 * size + 2.0 ** -8 * want.abs() + 1e-30).all()
     assert torch.equal(state, x[n - taps + 1:])
+    tl.check_device_errors()
+
+
+@pytest.mark.parametrize("dt,channels,seqs", [(F32, 1280, 18), (F32, 1280, 19), (BF16, 1280, 40), (BF16, 1288, 41)])
+def test_gated_scan_of_many_ctas(dt, channels, seqs):
+    """Either side of the line between the second pass's tiles of 8 and 4 tokens, chunks that end inside both."""
+    n, C = 67, channels
+    rng = np.random.default_rng(seqs)
+    u, y = (torch.from_numpy(rng.standard_normal((seqs, n, C))).to(dt) for _ in range(2))
+    r, i = (rng.uniform(0.01, 1, (seqs, n, C)).astype(np.float32) for _ in range(2))
+    lam = rng.uniform(-12, 1, C).astype(np.float32)
+    gates, soft = torch.from_numpy(np.stack([r, i], axis=2)).cuda(), torch.from_numpy(O.softplus(lam.astype(np.float64)).astype(np.float32)).cuda()
+    state, out = torch.full((seqs, C), float("nan"), device="cuda"), torch.full((seqs + 1, n, C), 7.0, device="cuda", dtype=dt)
+    ops.gated_scan(u.cuda(), gates, soft, y.cuda(), state, out[:seqs], C, 1, seqs, n, 0)
+    assert (out[seqs] == 7.0).all()
+    for s in (0, 1, seqs - 1):
+        want = O.gated_linear_recurrence(u[s].double().numpy(), r[s].astype(np.float64), i[s].astype(np.float64), lam.astype(np.float64)) * O.gelu_tanh(y[s].double().numpy())
+        got = out[s].double().cpu().numpy()
+        # as the operator's other tests: of the largest value, FP32 sums over the tokens, or the rounding to BF16
+        assert np.abs(got - want).max() <= (6e-3 if dt == BF16 else 2e-5) * np.abs(want).max()
     tl.check_device_errors()

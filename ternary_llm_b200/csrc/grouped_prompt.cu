@@ -632,13 +632,28 @@ int launch_latent_prompt_tcgen05(const LatentArgs<bf16>& a, const bf16* kx, cons
     return launch<bf16, true>(p, x, dq, mq, mk, mv, a.heads, 1, stream);
 }
 
-// Two or three queries of single heads of 64 behind a few positions: a CTA per query and key/value head on the CUDA cores
-// (attention.cu) has the shorter launch while all CTAs run at once.  us there / here: 32 heads, 2 queries of 16 positions 5.9 / 6.5, of 32
-// 6.0 / 6.6, of 48 6.2 / 6.7, of 64 equal; one head, 2 of 16 5.6 / 5.9.  Elsewhere a tile is as quick or quicker: 8 queries of one head behind
-// 256 8.1 / 7.4, behind 1000 25.4 / 19.8; 32 heads over 8, 2 queries behind 400 13.6 / 12.0.
+// Few queries over few channels: a CTA per query and key/value head on the CUDA cores (attention.cu) has the shorter launch, and one
+// chunk of 256 positions there is two tiles here.  us there / here, heads of 64 without groups unless said:
+//   * up to 32 positions, while all CTAs run at once: one head of two sequences, 6 queries of 11 5.5 / 6.0, 4 heads of two, 2 of 2 5.3 / 6.1,
+//     32 heads of two, 5 of 10 6.9 / 6.9, 8 heads, 16 of 21 6.4 / 6.1; groups of two, 4 heads, 4 of 4 5.8 / 6.2, of 8 sequences, 8 of 13 7.1 / 6.9;
+//     heads of 128, 8 heads, 6 of 11 7.2 / 7.5; groups of four only where the tiles here share SMs: 8 heads of 8 sequences, 3 of 13
+//     7.8 / 8.5, 4 heads of one, 2 of 22 7.4 / 6.3;
+//   * up to 48 positions for two or three queries: 32 heads, 3 of 33 6.2 / 6.5; of 63 6.2 / 5.9 (8 heads);
+//   * up to 128 positions, one tile here, never;
+//   * one chunk there behind them, while few CTAs share an SM: 4 heads, 3 of 153 7.2 / 8.1; 8 heads, 5 of 205 7.8 / 8.0; 4 heads, 8 of 248
+//     8.2 / 7.7; 2 heads of 8 sequences, 8 of 208 9.3 / 8.3; heads of 128, 2 heads, 8 of 158 9.3 / 9.7, 8 sequences of one, 3 of 203 9.9 / 9.5;
+//   * behind more never: 8 queries of one head behind 1000 25.4 / 19.8; 32 heads over 8, 2 queries behind 400 13.6 / 12.0.
 static bool few_queries(int batch, int group, int n_kv_heads, int head_dim, int seq_len, int kv_len)
 {
-    return head_dim == 64 && group == 1 && seq_len <= 3 && kv_len <= 48 && (long long)batch * n_kv_heads * seq_len <= 444;
+    const long long ctas = (long long)batch * n_kv_heads * seq_len;
+    const int channels = group * head_dim;
+    if (seq_len > 12 && seq_len * group > 16) return false;
+    if (kv_len <= 32) {
+        if (channels <= 128) return ctas <= (channels == 64 ? 444 : head_dim == 64 ? 192 : 148);
+        return head_dim == 64 && channels <= 256 && seq_len <= 8 && ctas >= 64 && ctas <= 192;
+    }
+    if (kv_len <= 128) return channels == 64 && seq_len <= 3 && kv_len <= 48 && ctas <= 444;
+    return channels <= 128 && ctas <= 64 && kv_len <= (channels == 64 ? 208 : 160);
 }
 
 bool attention_prompt_supported(const half* q, const half* k_cache, const half* v_cache, const half* out, int batch, int n_heads, int n_kv_heads,

@@ -63,6 +63,15 @@ def test_both_sides_of_the_lines_for_few_queries(b, hq, hk, hd, seq, kv_len):
     assert (np.abs(out.cpu().numpy().astype(np.float64) - want) <= 2.0 ** -11 * np.abs(want) + 2e-5 * np.abs(vc.astype(np.float64)).max()).all()
 
 
+@pytest.mark.parametrize("b,hq,hk,hd,seq,kv_len", [
+    (1, 1, 1, 64, 6, 32), (1, 1, 1, 64, 6, 33), (1, 4, 4, 64, 3, 48), (1, 4, 4, 64, 3, 49), (1, 8, 8, 64, 4, 128), (1, 8, 8, 64, 4, 129),
+    (1, 8, 8, 64, 8, 208), (1, 8, 8, 64, 8, 209), (1, 9, 9, 64, 8, 200), (1, 4, 4, 128, 4, 160), (1, 4, 4, 128, 4, 161), (1, 8, 4, 64, 4, 160), (1, 8, 4, 64, 4, 161),
+    (8, 32, 8, 64, 3, 20), (9, 32, 8, 64, 3, 20), (8, 7, 1, 64, 8, 20), (1, 16, 4, 64, 8, 20), (2, 32, 8, 64, 8, 32), (48, 8, 4, 64, 1, 9), (24, 8, 4, 64, 2, 9),
+    (25, 8, 4, 64, 2, 9), (37, 4, 4, 64, 3, 9), (38, 4, 4, 64, 3, 9)])
+def test_more_lines_for_few_queries(b, hq, hk, hd, seq, kv_len):
+    test_both_sides_of_the_lines_for_few_queries(b, hq, hk, hd, seq, kv_len)
+
+
 def test_scores_far_apart():
     """One position's score far above the others', first, last or in between: the running maximum
     moves, and the weights of the others are nothing."""

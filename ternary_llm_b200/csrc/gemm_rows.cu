@@ -475,9 +475,9 @@ gemm_row_kernel(const OneArgs a)
 }
 
 
-// How a product is cut: CTAs that share the scale groups of a tile, and the groups that one of them walks in all rounds of CTAs.
+// How a product is cut: tiles, CTAs that share the scale groups of one, rounds of CTAs, and the groups that one of them walks in all rounds.
 struct Cut {
-    int split = 0, steps = 0;
+    int tiles = 0, split = 0, rounds = 0, steps = 0;
 };
 
 // CTAs of a kernel that run at once in clusters of one to kMaxSplit: slots[cluster size], asked once per device.  Clusters come in
@@ -526,8 +526,10 @@ void choose_cut(const int (&slots)[kMaxSplit + 1], int rows, int groups, Cut* c)
         const int per = (groups + split - 1) / split, cost = 2 * ((per + kGroupWarps - 1) / kGroupWarps) + (split > 1 ? 3 : 0);
         if (cost >= best) continue;
         best = cost;
+        c->tiles = tiles;
         c->split = split;
-        c->steps = per * ((tiles * split + slots[split] - 1) / slots[split]);
+        c->rounds = (tiles * split + slots[split] - 1) / slots[split];
+        c->steps = per * c->rounds;
     }
 }
 
@@ -661,11 +663,16 @@ int launch_gemm_rows(const uint8_t* packed, const half* x, const RowsOut* out, i
 //     vectors: 8192 x 24576 64 / 37 before these figures
 //   m = 5..8, two GEMV passes: quicker everywhere, 512 x 2048 9.6 / 2.6, 28672 x 4096 22.1 / 19.8, 14336 x 14336 41 / 33
 //   m = 9..16, tcgen05: 2048 x 14336 11.7 / 8.2, 8192 x 14336 (two CTAs, 56 steps) 25.1 / 22.8, 14336 x 4096 (one, 32) 13.7 / 13.1 - 13.4, 28672
-//     x 4096 (one, 64) 24.0 / 24.1 - 25.3, 14336 x 1280 (one, 10) 6.4 / 5.6 - 6.1, 12800 x 1664 (one, 13) 7.2 / 7.1 - 7.7
+//     x 4096 (one, 64) 24.0 / 24.1 - 25.3.  Of one CTA a tile one round of them: m = 10, 29209 x 256 (457 tiles) 4.4 / 5.5, m = 9, 26384 x 640 (413)
+//     5.7 / 6.7, m = 11, 14672 x 512 (230) 4.3 / 3.5.  Above 12 up to 10 steps and up to 74 tiles, or more than one an SM: m = 16, 5648 x 640
+//     (89) 3.8 / 4.4, m = 14, 8496 x 768 (133) 4.1 / 4.6, m = 16, 13744 x 512 (215) 4.2 / 3.8
 //   m = 17..24: 2048 x 14336 12.0 / 10.3, 4096 x 14336 (four CTAs, 28 steps) 16.0 / 15.1 - 16.0, 8192 x 2048 (two, 8) 7.2 / 6.8, 6144 x 4096
-//     (two, 16) 10.4 / 10.1 - 10.7, 4600 x 8192 (three, 22) 12.9 / 13.3 - 14.2, 1024 x 1024 (one, 8) 4.4 / 3.6 - 4.0, 10240 x 1024 5.5 / 5.4 - 6.0
-//   m = 25..32: 2048 x 8192 (eight, 8) 9.3 / 8.6, 4096 x 4096 (four, 8) 8.9 / 7.4 - 7.8, 2048 x 14336 (eight, 14) 12.0 / 12.6, 1024 x
-//     1024 4.4 / 4.7
+//     (two, 16) 10.4 / 10.1 - 10.7, 4600 x 8192 (three, 22) 12.9 / 13.3 - 14.2.  One CTA a tile where tiles are few and no stage has a single
+//     group: m = 20, 2769 x 1024 (44 tiles, 8 steps) 4.7 / 3.9, m = 19, 528 x 768 (6 steps) 4.0 / 3.8, m = 24, 603 x 640 (5) 3.7 / 4.0, m = 22, 464 x 256
+//     (2) 2.8 / 3.2, m = 24, 5440 x 256 (85 tiles) 3.1 / 4.1
+//   m = 25..32, up to 8 steps: 2048 x 8192 (eight CTAs) 9.3 / 8.6, 4096 x 4096 (four) 8.9 / 7.4 - 7.8, of three CTAs up to 34 tiles: m = 32, 1392 x 2432 (22)
+//     6.1 / 6.0, m = 30, 2768 x 2176 (44) 6.6 / 7.5, m = 29, 5904 x 2560 (93) 8.5 / 11.3.  Up to 12 steps where tiles are few: m = 27, 362 x 10240 (6)
+//     7.3 / 6.4, m = 28, 3511 x 6272 (55) 10.1 / 13.0
 bool linear_takes_rows(int m, int rows, int cols)
 {
     if (m < 4 || m > kRowsMax) return false;
@@ -675,9 +682,12 @@ bool linear_takes_rows(int m, int rows, int cols)
     const int split = c.split, steps = c.steps;
     if (m == 4) return split >= 4 || steps <= 20 || cols > 20480;
     if (m <= 8) return true;
-    if (m <= 16) return split > 1 || steps <= (m <= 12 ? 32 : 10);
-    if (m <= 24) return split >= 7 || (split >= 4 && steps <= 28) || (steps <= 8 && (split > 1 || rows <= 4736));
-    return split >= 3 && steps <= 12;
+    if (m <= 12) return split > 1 || (c.rounds == 1 && steps <= 32);
+    if (m <= 16) return split > 1 || (c.rounds == 1 && steps <= 10 && (c.tiles <= 74 || c.tiles > 148));
+    if (m <= 24)
+        return split >= 7 || (split >= 4 && steps <= 28) || (split > 1 && steps <= 8) ||
+               (split == 1 && steps >= 3 && steps <= 8 && steps % kGroupWarps != 1 && c.tiles <= 60);
+    return (steps <= 8 && (split >= 4 || (split == 3 && c.tiles <= 34))) || (steps <= 12 && split >= 3 && c.tiles <= 13);
 }
 
 // Matrices packed back to back on this kernel or the tcgen05 GEMM (m > 8, or where this one is taken).

@@ -68,6 +68,26 @@ def test_both_sides_of_the_lines(n):
     tl.check_device_errors()
 
 
+@pytest.mark.parametrize("n,k,ms", [
+    (832, 10240, (25, 32)), (833, 10240, (25, 32)), (2176, 2816, (25, 32)), (2177, 2816, (25, 32)), (3840, 1024, (17, 24)), (3841, 1024, (17, 24)),
+    (600, 640, (17, 24)), (600, 768, (17, 24)), (4736, 640, (13, 16)), (4737, 640, (13, 16)), (9472, 640, (9, 13, 16)), (9473, 640, (9, 13, 16)),
+    (18944, 640, (9, 12, 13)), (18945, 640, (9, 12, 13))])
+def test_both_sides_of_the_lines_of_tiles(n, k, ms):
+    """Where the number of tiles or of a stage's groups decides on the kernel."""
+    nz, sg, sc, x = oracle.make_case(n, k, seed=n, batch=max(ms))
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (nz, sg, sc, x)]
+    w = tl.PreparedWeight(*dev[:3], n, k, register=False)
+    wd = torch.from_numpy(oracle.unpack_bitmasks(nz, sg).astype(np.float32) * np.repeat(sc.astype(np.float32), 128, axis=1)).cuda().double()
+    want, size = dev[3].double() @ wd.T, dev[3].double().abs() @ wd.T.abs()
+    for m in ms:
+        y = torch.full((m + 1, n), 7.0, dtype=torch.float16, device="cuda")
+        tl.ternary_gemm_packed(dev[3][:m].contiguous(), w, y, m)
+        assert (y[m] == 7.0).all()
+        bound = k * 2.0 ** -23 * size[:m] + 2.0 ** -11 * want[:m].abs() + 2.0 ** -25      # as above
+        assert ((y[:m].double() - want[:m]).abs() <= bound).all(), m
+    tl.check_device_errors()
+
+
 @pytest.mark.parametrize("n", [4, 5, 8, 9, 16, 17, 32, 33, 65])
 def test_matrices_packed_back_to_back(n):
     """q|k|v and gate|up of a prompt in one launch each, k and v of 48 rows, whose borders fall inside the tiles of 64

@@ -348,9 +348,9 @@ int launch_rope(half* q, half* k, const half* v, half* k_cache, half* v_cache, i
 // SwiGLU   out = half(g / (1 + exp(-g)) * u)       reference: kernels/activations.cu:18-74
 // ---------------------------------------------------------------------------
 // Eight elements a thread (whole 16-byte pieces): bound by the exponential and the division, so that what an element costs
-// beside them counts.  us a launch, two elements a thread / eight: 2000 x 14336 63 / 32, 300 x 8192 5.7 / 3.7, 24 x 8192 1.8 / 3.1: two
-// while all threads run at once.
-constexpr long long kSiluPairs = 2 * 148 * 2048;
+// beside them counts; two elements a thread start more threads at once.  us a launch, two / eight: 2000 x 14336 63 / 32, 300 x 8192 5.4 / 3.4, 1.2
+// million 2.8 / 2.5, one million 2.3 / 2.9, 700000 1.9 / 2.8.
+constexpr long long kSiluPairs = 1 << 20;
 
 __global__ void __launch_bounds__(256)
 silu_mul8_kernel(const uint4* gate, const uint4* up, uint4* out, long long pieces)

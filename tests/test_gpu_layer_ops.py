@@ -203,6 +203,17 @@ def test_attention_several_tokens_is_causal_softmax(seq, kv_len):
     assert np.abs(host(out).astype(np.float32) - want.astype(np.float32)).max() <= 4e-3
 
 
+@pytest.mark.parametrize("size", [(1 << 20) - 8, 1 << 20, (1 << 20) + 8, (1 << 20) + 12, 3 * 2 ** 20 + 8])
+def test_silu_mul_on_both_sides_of_eight_elements_a_thread(size):
+    gen = torch.Generator(device="cuda").manual_seed(size)
+    g, u = (4 * torch.randn(size, generator=gen, device="cuda")).half(), torch.randn(size, generator=gen, device="cuda").half()
+    out = torch.full((size + 8,), 7.0, device="cuda", dtype=torch.float16)
+    ops.silu_mul_forward(g, u, out[:size], size)
+    want = g.double() * torch.sigmoid(g.double()) * u.double()
+    # FP32 steps of the exponential, quotient and products, then one rounding to FP16
+    assert ((out[:size].double() - want).abs() <= (2.0 ** -11 + 2.0 ** -20) * want.abs() + 2.0 ** -25).all() and (out[size:] == 7.0).all()
+
+
 @pytest.mark.parametrize("size", [1, 2, 33, 8192, 14336 * 3 + 1])
 def test_silu_mul_and_add(size):
     rng = np.random.default_rng(size)

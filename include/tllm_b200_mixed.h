@@ -149,6 +149,23 @@ int tllm_b200_decoder_forward_logits(void* decoder, int seq, const int* token_id
  * then n up rows and y = act(gate) * up; y in the activation type then. */
 int tllm_b200_dense_linear(int bf16, const void* x, const void* w, const float* bias, void* y, int rows, int n, int cols, int act,
                            int glu, void* stream);
+/* A BF16 product of more than 8 rows with everything that a layer asks of it: y[m, z, n] = sum_k w[z, n, k] x[m, z, k] for z of
+ * `batch` entries.  x: row stride ldx, entry z from column z * x_batch on; w: [batch * w_rows, ldw]; y: BF16, or float with
+ * y_f32, row stride ldy, entry z from column z * y_batch on; bias float [batch * n] or NULL; gate BF16 or NULL: y *=
+ * sigmoid(gate[m * gate_ld + z]); features [act_lo, act_hi) take the activation, those from f32_from on go to y2 as float
+ * (row stride ldy2), all three multiples of 64, act_hi and f32_from INT_MAX for none, with one entry and no glu; glu as above. */
+typedef struct tllm_b200_dense_args {
+    const void *x, *w, *gate;
+    const float* bias;
+    void* y;
+    float* y2;
+    int rows, n, cols, batch;
+    int ldx, x_batch, ldw, w_rows, ldy, y_batch, ldy2, gate_ld;
+    int act, act_lo, act_hi, f32_from, glu, y_f32;
+} tllm_b200_dense_args;
+int tllm_b200_dense_product(const tllm_b200_dense_args* args, void* stream);
+/* The way that product takes on the current device: features of a tile, whether pairs of CTAs share one, CTAs that share its K. */
+int tllm_b200_dense_way(const tllm_b200_dense_args* args, int* features, int* pair, int* split);
 /* state: activation type [n_seq][taps - 1][channels]; w float [channels, taps]; act: TLLM_ACT_... */
 int tllm_b200_causal_conv(int bf16, const void* x, const float* w, const float* bias, void* state, void* y, int channels, int taps,
                           int act, int n_seq, int seq_len, int start_pos, void* stream);

@@ -67,6 +67,8 @@ SIGNATURES = {
     "tllm_b200_mixed_decoder_runs": (_int, [_vp]),
     "tllm_b200_decoder_forward_logits": (_int, [_vp, _int, _vp, _int, _int, _vp, _int, _vp, _vp, _vp]),
     "tllm_b200_dense_linear": (_int, [_int] + [_vp] * 4 + [_int] * 5 + [_vp]),
+    "tllm_b200_dense_product": (_int, [_vp, _vp]),
+    "tllm_b200_dense_way": (_int, [_vp] * 4),
     "tllm_b200_causal_conv": (_int, [_int] + [_vp] * 5 + [_int] * 6 + [_vp]),
     "tllm_b200_selective_scan": (_int, [_int] + [_vp] * 8 + [_int] * 5 + [_vp]),
     "tllm_b200_gated_scan": (_int, [_int] + [_vp] * 6 + [_int, _int, ctypes.c_float] + [_int] * 4 + [_vp]),
@@ -113,6 +115,13 @@ class MixedLayerDesc(ctypes.Structure):
                [(n, _int) for n in ("gate_act", "ff", "ff_act", "experts", "top", "kv_heads", "chunk", "in_act")] + \
                [("out_scale", ctypes.c_float), ("head_decay", ctypes.POINTER(ctypes.c_float)), ("beside", _vp),
                 ("t", _vp * TENSORS_PER_LAYER)]
+
+
+class DenseArgs(ctypes.Structure):
+    """tllm_b200_dense_args."""
+    _fields_ = [(n, _vp) for n in ("x", "w", "gate", "bias", "y", "y2")] + \
+               [(n, _int) for n in ("rows", "n", "cols", "batch", "ldx", "x_batch", "ldw", "w_rows", "ldy", "y_batch", "ldy2", "gate_ld",
+                                    "act", "act_lo", "act_hi", "f32_from", "glu", "y_f32")]
 
 
 class MixedDesc(ctypes.Structure):

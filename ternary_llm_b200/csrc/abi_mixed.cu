@@ -271,6 +271,67 @@ int tllm_b200_dense_linear(int bf16_, const void* x, const void* w, const float*
                  : dense_linear<float>(x, w, bias, y, rows, n, cols, act, glu, S(stream));
 }
 
+static LinearArgs<bf16> dense_product(const tllm_b200_dense_args& a)
+{
+    LinearArgs<bf16> l;
+    l.w = static_cast<const bf16*>(a.w);
+    l.ldw = a.ldw;
+    l.w_rows = a.w_rows;
+    l.x = static_cast<const bf16*>(a.x);
+    l.ldx = a.ldx;
+    l.x_batch = a.x_batch;
+    l.y = a.y;
+    l.ldy = a.ldy;
+    l.y_batch = a.y_batch;
+    l.y_f32 = a.y_f32 != 0;
+    l.M = a.rows;
+    l.N = a.n;
+    l.K = a.cols;
+    l.batch = a.batch;
+    l.bias = a.bias;
+    l.act = a.act;
+    l.act_lo = a.act_lo;
+    l.act_hi = a.act_hi;
+    l.f32_from = a.f32_from;
+    l.y2 = a.y2;
+    l.ldy2 = a.ldy2;
+    l.glu = a.glu != 0;
+    l.gate = static_cast<const bf16*>(a.gate);
+    l.gate_ld = a.gate_ld;
+    return l;
+}
+
+static int check_product(const tllm_b200_dense_args* a)
+{
+    if (!a) return fail(TLLM_ERR_NULL, "dense_product: null pointer");
+    if (a->rows < 9 || a->n < 1 || a->cols < 8 || a->cols % 8 || a->batch < 1)
+        return fail(TLLM_ERR_SHAPE, "dense_product: rows=%d (more than 8) n=%d cols=%d (a multiple of 8) batch=%d", a->rows, a->n, a->cols, a->batch);
+    return check_device();
+}
+
+int tllm_b200_dense_product(const tllm_b200_dense_args* args, void* stream)
+{
+    const int st = check_product(args);
+    if (st) return st;
+    if (!args->x || !args->w || !args->y || (args->f32_from < args->n && !args->y2)) return fail(TLLM_ERR_NULL, "dense_product: null pointer");
+    return launch_dense_gemm_tcgen05(dense_product(*args), S(stream));
+}
+
+int tllm_b200_dense_way(const tllm_b200_dense_args* args, int* features, int* pair, int* split)
+{
+    const int st = check_product(args);
+    if (st) return st;
+    if (!features || !pair || !split) return fail(TLLM_ERR_NULL, "dense_way: null pointer");
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return fail(TLLM_ERR_LAUNCH, "dense_way: no current device");
+    const DenseWay w = dense_way(dense_product(*args), sms);
+    *features = w.features;
+    *pair = w.pair;
+    *split = w.split;
+    return TLLM_OK;
+}
+
 int tllm_b200_causal_conv(int bf16_, const void* x, const float* w, const float* bias, void* state, void* y, int channels, int taps,
                           int act, int n_seq, int seq_len, int start_pos, void* stream)
 {

@@ -113,6 +113,13 @@ bool gemv_tail_fits(int k, int taps);
 template <typename T>
 bool gemv_norm_fits(int k);
 int launch_dense_gemm_tcgen05(const LinearArgs<bf16>& a, cudaStream_t stream);
+// the way it takes on a device of so many SMs
+struct DenseWay {
+    int features;       // of a tile
+    bool pair;          // two CTAs a tile of 256 tokens
+    int split;          // CTAs that share a tile's K
+};
+DenseWay dense_way(const LinearArgs<bf16>& a, int sms);
 int launch_dense_gemm_f32(const LinearArgs<float>& a, cudaStream_t stream);
 // dispatch by the number of rows
 int linear(const LinearArgs<bf16>& a, cudaStream_t stream);

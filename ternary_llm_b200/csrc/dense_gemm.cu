@@ -524,6 +524,55 @@ int launch_tn(EncodeTiledFn enc, const LinearArgs<bf16>& l, DenseEpi e, int sms,
 
 }  // namespace
 
+// The way of a product: the tile's features, whether pairs of CTAs share a tile, and the CTAs that share its K.
+DenseWay dense_way(const LinearArgs<bf16>& l, int sms)
+{
+    const long long mt = (l.M + kTok - 1) / kTok;
+    auto tiles = [&](int tn, long long m) {
+        const int outs = l.glu ? tn / 2 : tn;
+        return m * ((l.N + outs - 1) / outs) * l.batch;
+    };
+    DenseWay r = {64, false, 1};
+    if (l.group) {                           // their number is known on the device alone: the widest tile that still gives most SMs one
+        r.features = tiles(256, mt) * 10 >= 7LL * sms ? 256 : tiles(128, mt) * 10 >= 7LL * sms ? 128 : 64;
+        return r;
+    }
+    // The quickest by rounds of tiles: 64 columns of K take 0.21, 0.27, 0.39 us in a tile of 64, 128, 256 features (its operands' 24,
+    // 32, 48 KB through 64 bytes a clock), 0.235 and 0.36 in a pair's tile of 128 and 256 (24 and 32 KB a CTA); the outputs of a tile
+    // 0.8 and 0.02 a feature, of gated pairs 1.6 and 0.016, beside the next tile's product; a launch 2.5, of pairs 4.  us measured with 64, 128, 256, pair 128, pair
+    // 256, the one taken in brackets: 2000 tokens 2048 x 2048 31 22 (20) 20 21, 8192 x 2048 gated 183 116 96 107 (89), 4096 x 128
+    // 16.2 16.2 (15.2) 18.8 17.0; 1000 tokens 2048 x 8192 55 35 53 (31) 48; 300 tokens 4096 x 4096 30 21 32 (19) 30, 14336 x 4096 gated
+    // 128 85 (83) 95 89; 100 tokens 8192 x 2048 (12.3) 14.4 20.7 14.3 19.8.  Gated and short: 400 tokens 4864 x 512 13.2 (10.1) 11.6 12.1 12.4; 64
+    // tokens 12032 x 200 11.4 (8.9).
+    const struct { int tn; bool pair; double step; } way[] = {{64, false, 0.21}, {128, false, 0.27}, {256, false, 0.39}, {128, true, 0.235}, {256, true, 0.36}};
+    auto outputs = [&](int tn) { return l.glu ? 1.6 + 0.016 * tn : 0.8 + 0.02 * tn; };
+    double best = 0.;
+    for (const auto& w : way) {
+        if (w.pair && mt == 1) continue;
+        const long long at_once = w.pair ? sms / 2 : sms, n = tiles(w.tn, w.pair ? (mt + 1) / 2 : mt);
+        const double product = (l.K + kBlkK - 1) / kBlkK * w.step, output = outputs(w.tn);
+        const double t = (double)((n + at_once - 1) / at_once) * (product > output ? product : output) + (product > output ? output : product) + (w.pair ? 4. : 2.5);
+        if (best == 0. || t < best) {
+            best = t;
+            r.features = w.tn;
+            r.pair = w.pair;
+        }
+    }
+    // Few tiles: K over a cluster's CTAs while all of them run at once; exchanging the sums takes 3.7 us.  One CTA a tile / so, 100
+    // tokens: 2048 x 8192 29 / 15, 4096 x 14336 48 / 32, 2048 x 2048 10.6 / 9.7, 2048 x 1024 7.5 / 8.6.
+    const long long n = tiles(64, mt), most[3] = {sms, sms * 8 / 9, sms * 4 / 5};
+    for (int i = 0, split = 2; i < 3 && n * split <= most[i]; i++, split *= 2) {
+        const int steps = (l.K + kBlkK - 1) / kBlkK;
+        if (steps < split) break;
+        const double t = (steps + split - 1) / split * 0.21 + outputs(64) + 2.5 + 3.7;
+        if (t < best) {
+            best = t;
+            r = {64, false, split};
+        }
+    }
+    return r;
+}
+
 int launch_dense_gemm_tcgen05(const LinearArgs<bf16>& l, cudaStream_t stream)
 {
     if (l.M == 0 || l.N == 0 || l.batch == 0) return TLLM_OK;
@@ -573,53 +622,11 @@ int launch_dense_gemm_tcgen05(const LinearArgs<bf16>& l, cudaStream_t stream)
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return fail(TLLM_ERR_LAUNCH, "dense_gemm: no current device");
     if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    const long long mt = (l.M + kTok - 1) / kTok;
-    auto tiles = [&](int tn, long long m) {
-        const int outs = l.glu ? tn / 2 : tn;
-        return m * ((l.N + outs - 1) / outs) * l.batch;
-    };
-    int tn = 64;
-    bool pair = false;
-    if (l.group) {                           // their number is known on the device alone: the widest tile that still gives most SMs one
-        tn = tiles(256, mt) * 10 >= 7LL * sms[dev] ? 256 : tiles(128, mt) * 10 >= 7LL * sms[dev] ? 128 : 64;
-    } else {
-        // The quickest by rounds of tiles: 64 columns of K take 0.21, 0.27, 0.39 us in a tile of 64, 128, 256 features (its operands' 24,
-        // 32, 48 KB through 64 bytes a clock), 0.235 and 0.36 in a pair's tile of 128 and 256 (24 and 32 KB a CTA); the outputs of a tile
-        // 0.8 and 0.02 a feature, beside the next tile's product; a launch 2.5, of pairs 4.  us measured with 64, 128, 256, pair 128, pair
-        // 256, the one taken in brackets: 2000 tokens 2048 x 2048 31 22 (20) 20 21, 8192 x 2048 gated 183 116 96 107 (89), 4096 x 128
-        // 16.2 16.2 (15.2) 18.8 17.0; 1000 tokens 2048 x 8192 55 35 53 (31) 48; 300 tokens 4096 x 4096 30 21 32 (19) 30, 14336 x 4096 gated
-        // 128 85 (83) 95 89; 100 tokens 8192 x 2048 (12.3) 14.4 20.7 14.3 19.8.
-        const struct { int tn; bool pair; double step; } way[] = {{64, false, 0.21}, {128, false, 0.27}, {256, false, 0.39}, {128, true, 0.235}, {256, true, 0.36}};
-        double best = 0.;
-        for (const auto& w : way) {
-            if (w.pair && mt == 1) continue;
-            const long long at_once = w.pair ? sms[dev] / 2 : sms[dev], n = tiles(w.tn, w.pair ? (mt + 1) / 2 : mt);
-            const double product = (l.K + kBlkK - 1) / kBlkK * w.step, output = 0.8 + 0.02 * w.tn;
-            const double t = (double)((n + at_once - 1) / at_once) * (product > output ? product : output) + (product > output ? output : product) + (w.pair ? 4. : 2.5);
-            if (best == 0. || t < best) {
-                best = t;
-                tn = w.tn;
-                pair = w.pair;
-            }
-        }
-        // Few tiles: K over a cluster's CTAs while all of them run at once; exchanging the sums takes 3.7 us.  One CTA a tile / so, 100
-        // tokens: 2048 x 8192 29 / 15, 4096 x 14336 48 / 32, 2048 x 2048 10.6 / 9.7, 2048 x 1024 7.5 / 8.6.
-        const long long n = tiles(64, mt), most[3] = {sms[dev], sms[dev] * 8 / 9, sms[dev] * 4 / 5};
-        for (int i = 0, split = 2; i < 3 && n * split <= most[i]; i++, split *= 2) {
-            const int steps = (l.K + kBlkK - 1) / kBlkK;
-            if (steps < split) break;
-            const double t = (steps + split - 1) / split * 0.21 + 0.8 + 0.02 * 64 + 2.5 + 3.7;
-            if (t < best) {
-                best = t;
-                tn = 64;
-                pair = false;
-                e.split = split;
-            }
-        }
-    }
-    if (tn == 256) return pair ? launch_tn<256, kPair>(enc, l, e, sms[dev], stream) : launch_tn<256, kSingle>(enc, l, e, sms[dev], stream);
-    if (tn == 128) return pair ? launch_tn<128, kPair>(enc, l, e, sms[dev], stream) : launch_tn<128, kSingle>(enc, l, e, sms[dev], stream);
-    if (e.split > 1) return launch_tn<64, kSplit>(enc, l, e, sms[dev], stream);
+    const DenseWay r = dense_way(l, sms[dev]);
+    e.split = r.split;
+    if (r.features == 256) return r.pair ? launch_tn<256, kPair>(enc, l, e, sms[dev], stream) : launch_tn<256, kSingle>(enc, l, e, sms[dev], stream);
+    if (r.features == 128) return r.pair ? launch_tn<128, kPair>(enc, l, e, sms[dev], stream) : launch_tn<128, kSingle>(enc, l, e, sms[dev], stream);
+    if (r.split > 1) return launch_tn<64, kSplit>(enc, l, e, sms[dev], stream);
     return launch_tn<64, kSingle>(enc, l, e, sms[dev], stream);
 }
 

@@ -705,10 +705,11 @@ int scan16_passes(const ScanArgs<float>&, int, cudaStream_t) { return TLLM_ERR_S
 // ---------------------------------------------------------------------------
 // Real-gated linear recurrence: one thread per channel and time chunk
 // ---------------------------------------------------------------------------
-// Bound by the latency of its loads, so a thread has those of TT tokens under way at once, 8 of them as they lie in memory, converted
-// when all are requested (each converted where it stands: first pass of 2000 tokens 35.5 us, so 25.0).  Tiles of 16 in the first pass
-// are as quick there and lose where a chunk is little more than 32 tokens (2048 channels, BF16, both passes, 16 / 8: 712 tokens 28.8 /
-// 24.2).  Requesting a tile ahead of the sums was slower in every form (32 and 41 us with tiles of 4, 33 and 62 with 8).
+// Bound by the latency of its loads, so a thread has those of TT tokens under way at once, as they lie in memory, converted when all are
+// requested (each converted where it stands: first pass of 2000 tokens 35.5 us, 8 at once 25.0).  The first pass takes 16 at once where
+// a chunk's last tile is more than half full, else 8 (2048 channels, BF16, both passes, us, 16 / 8: 2000 tokens, chunks of 63, 46.9 / 47.3;
+// 1024 channels 34.7 / 35.9; 1000 tokens, chunks of 33, 32.7 / 30.9; 100 tokens, of 34, 16.2 / 15.1).  Requesting a tile ahead of the sums
+// was slower in every form (32 and 41 us with tiles of 4, 33 and 62 with 8).
 constexpr int kGateThreads = 64;
 // The second pass carries the outputs' gate too; in tiles of 4 more threads fit, which hides more where there are CTAs for them, and
 // costs where there are not.  Both passes, us, tiles of 8 / 4: BF16 1984 channels, 2788 tokens (992 CTAs) 62 / 72; 2560, two sequences of
@@ -884,7 +885,9 @@ int launch_gated_scan(const GatedScanArgs<T>& a, cudaStream_t stream)
     if (nchunk > 1 && !a.rec) return fail(TLLM_ERR_NULL, "gated_scan: no record buffer");
     const unsigned gx = (a.channels + kGateThreads - 1) / kGateThreads;
     if (nchunk > 1) {
-        const int st = launch_pdl("gated_scan", gated_scan_kernel<T, false, 8>, dim3(gx, nchunk - 1, a.g.n_seq), dim3(kGateThreads), 0, stream, a, nchunk);
+        const int rest = ((a.g.seq_len + nchunk - 1) / nchunk) % 16;       // tokens of a chunk's last tile of 16
+        const int st = launch_pdl("gated_scan", rest == 0 || rest > 8 ? gated_scan_kernel<T, false, 16> : gated_scan_kernel<T, false, 8>,
+                                  dim3(gx, nchunk - 1, a.g.n_seq), dim3(kGateThreads), 0, stream, a, nchunk);
         if (st) return st;
     }
     const bool many = (long long)gx * nchunk * a.g.n_seq > kGateManyCtas<T>;

@@ -69,3 +69,18 @@ def test_gated_scan_of_many_ctas(dt, channels, seqs):
         # as the operator's other tests: of the largest value, FP32 sums over the tokens, or the rounding to BF16
         assert np.abs(got - want).max() <= (6e-3 if dt == BF16 else 2e-5) * np.abs(want).max()
     tl.check_device_errors()
+
+
+@pytest.mark.parametrize("n", [64, 66, 80, 81, 82, 94, 95, 96, 97, 1040, 1056])
+def test_gated_scan_of_chunks_of_all_lengths(n):
+    """Chunks of 32 to 48 tokens, whose last tile of 16 is whole, nearly whole or nearly empty."""
+    C, rng = 72, np.random.default_rng(n)
+    u, y = (torch.from_numpy(rng.standard_normal((n, C))).float() for _ in range(2))
+    r, i = (rng.uniform(0.01, 1, (n, C)).astype(np.float32) for _ in range(2))
+    lam = rng.uniform(-12, 1, C).astype(np.float32)
+    soft = torch.from_numpy(O.softplus(lam.astype(np.float64)).astype(np.float32)).cuda()
+    state, out = torch.full((1, C), float("nan"), device="cuda"), torch.full((n + 1, C), 7.0, device="cuda")
+    ops.gated_scan(u.cuda(), torch.from_numpy(np.stack([r, i], axis=1)).cuda(), soft, y.cuda(), state, out[:n], C, 1, 1, n, 0)
+    want = O.gated_linear_recurrence(u.double().numpy(), r.astype(np.float64), i.astype(np.float64), lam.astype(np.float64)) * O.gelu_tanh(y.double().numpy())
+    assert np.abs(out[:n].double().cpu().numpy() - want).max() <= 2e-5 * np.abs(want).max() and (out[n] == 7.0).all()
+    tl.check_device_errors()

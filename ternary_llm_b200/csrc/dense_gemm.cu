@@ -6,15 +6,16 @@
 // cta_group::2): each loads its 128 tokens and half of the features' weights and keeps the sums of
 // its tokens, the first one issues the MMAs of both.  What bounds a tile is the copies of its operands into
 // shared memory (64 bytes a clock and SM): 48 KB for 64 columns of K and 256 features, 32 KB a CTA of a
-// pair.  Gate and up of 8192 x 2048, 2000 tokens: 92 -> 81 us = 1.66 PFLOP/s in a prompt; in tiles of 64
+// pair.  Gate and up of 8192 x 2048, 2000 tokens: 92 -> 81 us in a prompt (1.66 PFLOP/s, where cuBLAS reaches 1.63 at
+// 8192^3 by itself), 101 -> 90 in a row of its own; in tiles of 64
 // and 128 features what bounded was the loop of one thread that issued the MMAs (2048 x 8192, 100 tokens
 // 40.5 -> 29.2 us with the loop run by a warp and one elected lane).
 // Where tiles are few, the CTAs of a cluster share one, each a part of K (SPLIT); they send one another
 // their sums of the tokens that the other finishes, and add them in rank order.
 // One persistent CTA per SM walks tiles with three roles
 // that run ahead of one another: a TMA producer (K-major tiles of 64 columns, 128-byte swizzle;
-// out-of-range rows and columns read as zero, so no size needs to divide a tile), one thread
-// that issues tcgen05.mma kind::f16 (M = 128, N = TN, K = 16) into one of two accumulators in
+// out-of-range rows and columns read as zero, so no size needs to divide a tile), a warp
+// whose elected lane issues tcgen05.mma kind::f16 (M = 128, of a pair 256, N = TN, K = 16) into one of two accumulators in
 // tensor memory, and eight epilogue warps that empty the other one: a TMEM lane is a token, the
 // rows pass through a small shared-memory tile per warp so that global stores are whole lines.
 // A gated feed-forward loads TN/2 gate rows and the TN/2 up rows with the same numbers into one

@@ -4,8 +4,8 @@
 // features walks its weights through tensor memory one scale group at a time, a chain of about a
 // microsecond per group that a decode batch cannot fill; here every warp expands its own weights
 // into mma.sync.m16n8k16 operand registers, so that all SMs stream at once and no step waits for
-// another warp.  scale * t is exact in FP16, so this is the same FP16 contraction with FP32 sums as
-// the tcgen05 kernel's (gemm_tcgen05.cu).
+// another warp.  A code is exact in FP16 and its scale joins the group's sum in FP32: FP16 products with FP32
+// sums, as in the tcgen05 kernel (gemm_tcgen05.cu), whose weights carry their scale.
 //
 //   * A CTA owns RG * R row blocks of 16 features and a range of scale groups; warp (rg, kw) takes R
 //     row blocks and every KW-th group.  A lane's 16 bytes of codes per (row block, group) are four

@@ -3,8 +3,8 @@
 // for the LLaMA design (its other sizes run on attention.cu).
 //
 // A CTA takes 128 queries of one head and walks over tiles of 128 positions that some of its queries
-// sees; two CTAs share an SM, so that one's softmax runs beside the other's products.  Roles: a TMA
-// producer, one thread that issues tcgen05.mma, four warps with a query row per thread.
+// sees; two CTAs share an SM, so that one's softmax runs beside the other's products.  Roles: a warp
+// for the TMA copies and one for tcgen05.mma, an elected lane of each issuing, four warps with a query row per thread.
 //   S = Q K^T      both operands in shared memory, 128 FP32 columns of tensor memory
 //   softmax        a thread reads its row; the weights go back over S as two BF16 numbers each
 //   O += P V       weights from tensor memory, values as they lie in the cache (feature-major
@@ -28,7 +28,7 @@
 //
 // Latent attention over expanded keys and values (BF16, key parts and values in pieces of 64) is the same walk with a key of two
 // parts; its operands leave room for one CTA an SM.  16 heads of 128 + 64, 2000 tokens: 192 -> 75 us a launch against
-// mma.sync on 64 queries (latent_attention.cu, which keeps the other sizes).  Tried: the scores read from tensor memory twice, 64 at a time,
+// mma.sync on 64 queries (latent_attention.cu, which keeps the other sizes and up to 64 positions).  Tried: the scores read from tensor memory twice, 64 at a time,
 // which leaves no spills: 75 -> 85, 90 -> 100 (FP16, 128).
 // All mbarrier waits are bounded (see dense_gemm.cu).
 #include <cfloat>

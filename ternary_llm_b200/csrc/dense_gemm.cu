@@ -540,13 +540,15 @@ DenseWay dense_way(const LinearArgs<bf16>& l, int sms)
     }
     // The quickest by rounds of tiles: 64 columns of K take 0.21, 0.27, 0.39 us in a tile of 64, 128, 256 features (its operands' 24,
     // 32, 48 KB through 64 bytes a clock), 0.235 and 0.36 in a pair's tile of 128 and 256 (24 and 32 KB a CTA); the outputs of a tile
-    // 0.8 and 0.02 a feature, of gated pairs 1.6 and 0.016, beside the next tile's product; a launch 2.5, of pairs 4.  us measured with 64, 128, 256, pair 128, pair
+    // 0.8 and 0.02 a feature (twice that where rows of Y are no whole 16-byte pieces), of gated pairs 1.6 and 0.016, beside the next tile's product; a launch 2.5, of pairs 4.  us measured with 64, 128, 256, pair 128, pair
     // 256, the one taken in brackets: 2000 tokens 2048 x 2048 31 22 (20) 20 21, 8192 x 2048 gated 183 116 96 107 (89), 4096 x 128
     // 16.2 16.2 (15.2) 18.8 17.0; 1000 tokens 2048 x 8192 55 35 53 (31) 48; 300 tokens 4096 x 4096 30 21 32 (19) 30, 14336 x 4096 gated
     // 128 85 (83) 95 89; 100 tokens 8192 x 2048 (12.3) 14.4 20.7 14.3 19.8.  Gated and short: 400 tokens 4864 x 512 13.2 (10.1) 11.6 12.1 12.4; 64
     // tokens 12032 x 200 11.4 (8.9).
     const struct { int tn; bool pair; double step; } way[] = {{64, false, 0.21}, {128, false, 0.27}, {256, false, 0.39}, {128, true, 0.235}, {256, true, 0.36}};
-    auto outputs = [&](int tn) { return l.glu ? 1.6 + 0.016 * tn : 0.8 + 0.02 * tn; };
+    const size_t es = l.y_f32 ? 4 : 2;
+    const double ragged = l.ldy * es % 16 || l.y_batch * es % 16 ? 2. : 1.;              // rows of Y are stored element by element
+    auto outputs = [&](int tn) { return l.glu ? 1.6 + 0.016 * tn : ragged * (0.8 + 0.02 * tn); };
     double best = 0.;
     for (const auto& w : way) {
         if (w.pair && mt == 1) continue;
